@@ -245,35 +245,108 @@ __global__ void __launch_bounds__(NT) tq_attn_split_kernel(const TqAttnParams p)
     }
 }
 
-// Merge n_splits partials of one (lane, q-head); optionally inverse-rotate and
-// store f16 (fused form).  grid = lanes * n_q, block = HD.
+// Merge n_splits partials of one (lane, q-head); optionally inverse-rotate and store f16 (fused form).
+// grid = lanes * n_q.  The partials are added in groups of MERGE_RUN consecutive splits, then the groups in order (with at
+// most MERGE_RUN splits that is plain split order, as the tensor-core kernel's own merge does it).  chunk != 0: the
+// queue form's lanes differ in their number of partials.  Thread
+// (column pair c, run r) adds run r, r + rows, ... of dims 2c, 2c + 1: the launch is a chain of L2 round trips, so all loads
+// of a run are in flight together and the runs are spread over the block.
+constexpr int MERGE_RUN = 8, MERGE_MAX_THREADS = 1024;
 template <bool FUSED>
-__global__ void tq_attn_merge_kernel(const float *__restrict__ partial, const float *__restrict__ signs,
-                                     float *__restrict__ out_f32, __half *__restrict__ out_f16, unsigned hd,
-                                     unsigned n_splits) {
+__global__ void __launch_bounds__(MERGE_MAX_THREADS)
+tq_attn_merge_kernel(const float *__restrict__ partial, const float *__restrict__ signs, float *__restrict__ out_f32,
+                     __half *__restrict__ out_f16, unsigned hd, unsigned n_splits, const uint32_t *__restrict__ positions,
+                     unsigned n_q, unsigned lane_capacity, unsigned chunk) {
     lc_pdl_trigger();  // successors may be scheduled; they wait for this grid before reading its output
     lc_pdl_wait();     // everything below may read what the predecessor wrote
-    __shared__ float sh[512];
-    const unsigned t = threadIdx.x;
-    const size_t qh = blockIdx.x;
-    const float *pp = partial + qh * n_splits * (size_t)(hd + 2);
-    float gmax = -INFINITY;
-    for (unsigned s = 0; s < n_splits; s++) gmax = fmaxf(gmax, pp[s * (size_t)(hd + 2)]);
-    float gsum = 0.f, o = 0.f;
-    for (unsigned s = 0; s < n_splits; s++) {
-        const float *ps = pp + s * (size_t)(hd + 2);
-        const float f = (ps[0] == -INFINITY) ? 0.f : expf(ps[0] - gmax);
-        gsum += f * ps[1];
-        o += f * ps[2 + t];
+    __shared__ float sh[MERGE_MAX_THREADS];
+    __shared__ float red[2 * MERGE_MAX_THREADS];        // [run row][hd]
+    __shared__ float sum_s[MERGE_MAX_THREADS / 32];     // one per run row (hd >= 64: at most 32 rows)
+    __shared__ float max_s[MERGE_MAX_THREADS / 32];
+    const unsigned t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const size_t qh = blockIdx.x, row = hd + 2;
+    const float *pp = partial + qh * n_splits * row;
+    if (chunk) {   // queue form: only as many partials as the lane has items
+        const unsigned keys = min(positions[qh / n_q] + 1u, lane_capacity);
+        n_splits = lc_attn_items(keys, chunk);
     }
-    const float v = gsum > 0.f ? o / gsum : 0.f;
+    const unsigned cols = hd / 2, c = t % cols, r0 = t / cols, rows = blockDim.x / cols;
+    const unsigned runs = (n_splits + MERGE_RUN - 1) / MERGE_RUN;
+    // first run's values are requested before anything else needs them
+    float2 a[MERGE_RUN], ml[MERGE_RUN];
+    auto load = [&](unsigned run) {
+#pragma unroll
+        for (int u = 0; u < MERGE_RUN; u++) {
+            const unsigned s = run * MERGE_RUN + u;
+            const bool ok = r0 < rows && s < n_splits;
+            ml[u] = ok ? *reinterpret_cast<const float2 *>(pp + s * row) : make_float2(-INFINITY, 0.f);
+            a[u] = ok ? *reinterpret_cast<const float2 *>(pp + s * row + 2 + 2 * c) : make_float2(0.f, 0.f);
+        }
+    };
+    load(r0);
+    float gmax = -INFINITY;
+    for (unsigned s = t; s < n_splits; s += blockDim.x) gmax = fmaxf(gmax, pp[s * row]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
+    if (lane == 0) max_s[warp] = gmax;
+    __syncthreads();
+    for (unsigned w = 0; w < (blockDim.x + 31) / 32; w++) gmax = fmaxf(gmax, max_s[w]);
+    float gsum = 0.f;
+    float2 o = make_float2(0.f, 0.f);
+    // Runs are added in order: each round of the block covers `rows` consecutive runs, whose sums meet in shared memory.
+    for (unsigned run0 = 0; run0 < runs; run0 += rows) {
+        if (run0) load(run0 + r0);
+        float ps = 0.f;
+        float2 po = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < MERGE_RUN; u++) {
+            const float f = (ml[u].x == -INFINITY) ? 0.f : expf(ml[u].x - gmax);
+            ps += f * ml[u].y;
+            po.x += f * a[u].x;
+            po.y += f * a[u].y;
+        }
+        if (runs == 1) {
+            gsum = ps;
+            o = po;
+            break;
+        }
+        if (r0 < rows) {
+            if (c == 0) sum_s[r0] = ps;
+            *reinterpret_cast<float2 *>(red + r0 * hd + 2 * c) = po;
+        }
+        __syncthreads();
+        if (r0 == 0) {
+            const unsigned n = runs - run0 < rows ? runs - run0 : rows;
+            for (unsigned r = 0; r < n; r++) {
+                const float2 v = *reinterpret_cast<const float2 *>(red + r * hd + 2 * c);
+                gsum += sum_s[r];
+                o.x += v.x;
+                o.y += v.y;
+            }
+        }
+        __syncthreads();
+    }
+    if (r0 == 0) {
+        sh[2 * c] = gsum > 0.f ? o.x / gsum : 0.f;
+        sh[2 * c + 1] = gsum > 0.f ? o.y / gsum : 0.f;
+    }
+    __syncthreads();
+    const float v = t < hd ? sh[t] : 0.f;
     if (!FUSED) {
-        out_f32[qh * hd + t] = v;
+        if (t < hd) out_f32[qh * hd + t] = v;
         return;
     }
-    // inverse rotation
-    const float w = lc_fwht_value(v, sh, hd, t);
-    out_f16[qh * hd + t] = __float2half_rn(w * (1.0f / sqrtf((float)hd)) * signs[t]);
+    // inverse rotation (threads past hd only take part in the barrier)
+    const float w = lc_fwht_value(v, red, hd, t);
+    if (t < hd) out_f16[qh * hd + t] = __float2half_rn(w * (1.0f / sqrtf((float)hd)) * signs[t]);
+}
+
+// block of the merge launch: one run of splits per hd / 2 threads, at least hd threads
+unsigned merge_threads(unsigned hd, unsigned n_splits) {
+    const unsigned runs = (n_splits + MERGE_RUN - 1) / MERGE_RUN;
+    unsigned t = hd / 2 * runs;
+    if (t < hd) t = hd;
+    return t > MERGE_MAX_THREADS ? MERGE_MAX_THREADS : t;
 }
 
 template <int HD, int BITS, int G>
@@ -361,31 +434,29 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
 
     const uint32_t group = n_q / n_kv;
     int g = group >= 8 ? 8 : (group > 4 ? 8 : (group > 2 ? 4 : (group > 1 ? 2 : 1)));
-    // tq2 at head_dim 256 runs on the tensor-core kernel (8 heads per CTA); LOCAL_CUDA_ATTN_MMA=0 keeps the
-    // CUDA-core kernel, which also serves every other head size and bit width.
+    // Head sizes 128 / 256 / 512 run on the tensor-core kernel (8 heads per CTA; a group of fewer heads leaves MMA columns
+    // empty, and a single head per kv-head is left to the CUDA cores).  It loads queries and signs as 16-byte vectors and
+    // 32-key tiles that wrap at most once: other buffers and rings take the CUDA-core kernel, as does LOCAL_CUDA_ATTN_MMA=0.
     static const bool mma_allowed = []() { const char *e = getenv("LOCAL_CUDA_ATTN_MMA"); return !(e && e[0] == '0'); }();
-    // (the tensor-core kernel copies norms as aligned 4-byte words)
-    const size_t norm_words = ((rows * n_kv + 1) & ~(size_t)1) * 2;
-    // (... and loads the query and the signs as 16-byte vectors: buffers wrapped at other offsets take the CUDA-core kernel)
-    const bool use_mma = mma_allowed && hd == 256 && bits == 2 && lc_aligned(kn->dptr, 4) && lc_aligned(vn->dptr, 4) &&
-                         kn->bytes >= norm_words && vn->bytes >= norm_words && (ring == 0 || ring >= 16) &&
+    const bool use_mma = mma_allowed && lc_tq_attn_mma_supported(hd, bits) && group >= 2 && (ring == 0 || ring >= 32) &&
                          lc_aligned(rq_or_q->dptr, 16) && (!fused || lc_aligned(signs->dptr, 16));
     if (use_mma) g = 8;
     const uint32_t gchunks = (group + g - 1) / g;
     const uint32_t base = n_lanes * n_kv * gchunks;
-    uint32_t want = (2u * (uint32_t)k->ctx->sm_count + base - 1) / base;
+    const uint32_t sms = (uint32_t)k->ctx->sm_count;
+    uint32_t want = (2u * sms + base - 1) / base;
     uint32_t by_len = (len_max + NW * TILE - 1) / (NW * TILE);
     if (by_len < 1) by_len = 1;
     uint32_t n_splits = want < by_len ? want : by_len;
     if (n_splits < 1) n_splits = 1;
     if (n_splits > 64) n_splits = 64;
+    uint32_t chunk = 0;
     if (use_mma) {
-        // One CTA per SM (registers), so the launch runs in whole waves; every CTA pays a fixed prologue worth
-        // about 320 keys.  Pick the split count that minimises waves x (prologue + keys per split).
-        const uint32_t sms = (uint32_t)k->ctx->sm_count;
-        uint32_t max_s = len_max / 256u;   // at least two 16-key tiles for each of the 8 warps
+        // One CTA per SM (shared memory), so the launch runs in whole waves; every CTA pays a fixed prologue and epilogue
+        // worth about 320 keys.  Pick the split count that minimises waves x (overhead + keys per split).
+        uint32_t max_s = len_max / (len_max < 4096 ? 256u : 128u);   // a 32-key tile for all (half) of the eight warps
         if (max_s < 1) max_s = 1;
-        if (max_s > 64) max_s = 64;
+        if (max_s > sms) max_s = sms;
         uint64_t best_cost = ~0ull;
         for (uint32_t s = 1; s <= max_s; s++) {
             const uint64_t waves = ((uint64_t)base * s + sms - 1) / sms;
@@ -393,7 +464,27 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
             if (cost < best_cost) { best_cost = cost; n_splits = s; }
         }
     }
-    const bool direct = (n_splits == 1 && !fused);
+    const bool out_vec = lc_aligned(out->dptr, 16) && (!fused || lc_aligned(signs->dptr, 16));
+    // Queue form for pools of lanes that attend all of their keys.  Lanes differ in length, which the host cannot see, and
+    // equal splits per lane leave most SMs waiting for the longest lane; so one persistent CTA per SM draws items of at
+    // most `chunk` keys.  An item costs about 450 keys' worth of fixed work.  The chunk minimises the sum of two
+    // estimates: every lane full, and lane lengths spread evenly up to the longest.  Below about ten lanes, or 2048 keys, the
+    // splits of the launch above are as good and merge in one launch.
+    if (use_mma && positions && window == 0 && ring == 0 && n_lanes <= LC_ATTN_QUEUE_LANES && base * 16u >= sms && len_max > 2048) {
+        const uint32_t fixed = 450, lo_s = len_max > 32u * 2048u ? 32u : (len_max + 4095) / 4096;
+        uint64_t best_cost = ~0ull;
+        for (uint32_t s = lo_s; s <= 32; s++) {
+            uint32_t per = ((len_max - 64u) / s + 255u) & ~255u;   // whole rounds of eight warps x 32 keys
+            if (per < 256u) per = 256u;
+            const uint64_t full = (((uint64_t)base * s + sms - 1) / sms) * (fixed + per);
+            const uint64_t mean = ((uint64_t)base * (len_max + fixed * (s + 1)) / 2) / sms;
+            const uint64_t cost = full + (mean > fixed + per ? mean : fixed + per);
+            if (cost < best_cost) { best_cost = cost; chunk = per + 64u; }   // (a few keys over do not make another item)
+        }
+        n_splits = (len_max + chunk - 1) / chunk;
+    }
+    const bool queue = chunk != 0;
+    const bool direct = !queue && n_splits == 1 && !fused;
     // The tensor-core kernel merges up to 8 splits itself (one thread-block cluster per lane and kv head, exchange
     // through distributed shared memory, inverse rotation in the kernel): one launch instead of split + merge, the same
     // arithmetic in the same order, bit-identical output.  Alone 57 vs 59 us at 8193 keys x 64 lanes, 12.4 vs 14.6 us
@@ -401,11 +492,11 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     // weight prefetch ahead of their dependency wait it was the slower form in situ, 3.48 vs 3.36 ms.)
     // LOCAL_CUDA_ATTN_CLUSTER=0 selects the two-launch form.
     static const bool cluster_allowed = []() { const char *e = getenv("LOCAL_CUDA_ATTN_CLUSTER"); return !(e && e[0] == '0'); }();
-    const bool cluster_merge = use_mma && cluster_allowed && n_splits <= 8 &&
-                               lc_aligned(out->dptr, 16) && (!fused || lc_aligned(signs->dptr, 16));
+    const bool cluster_merge = use_mma && !queue && cluster_allowed && n_splits <= 8 && out_vec;
 
     if (!direct && !cluster_merge) {
-        int st = lc_reserve_scratch(k, b, qn / hd * n_splits * (size_t)(hd + 2) * sizeof(float), 0);
+        const size_t rows_y = (size_t)n_kv * gchunks;
+        int st = lc_reserve_scratch(k, b, qn / hd * n_splits * (size_t)(hd + 2) * sizeof(float), queue ? rows_y : 0);
         if (st != LC_OK) return st;
     }
     TqAttnParams p;
@@ -419,6 +510,9 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     p.levels = (const float *)levels->dptr;
     p.out = (direct || (cluster_merge && !fused)) ? (float *)out->dptr : nullptr;
     p.out_f16 = (cluster_merge && fused) ? (__half *)out->dptr : nullptr;
+    p.queue_chunk = chunk;
+    p.n_lanes = n_lanes;
+    p.counters = k->counters;
     p.cluster_merge = cluster_merge ? 1 : 0;
     p.partial = (float *)k->scratch;
     p.positions = positions ? (const uint32_t *)positions->dptr : nullptr;
@@ -443,9 +537,13 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
         p.qfrag = (const uint4 *)qfrag->dptr;
     }
     dim3 grid(n_splits, n_kv * gchunks, n_lanes);
+    if (queue) {
+        const uint32_t per_y = sms / grid.y ? sms / grid.y : 1u;
+        grid = dim3(per_y < n_lanes * n_splits ? per_y : n_lanes * n_splits, grid.y, 1);
+    }
     int st;
     if (use_mma) {
-        st = lc_tq2_attn_mma_launch(b, p, grid);
+        st = lc_tq_attn_mma_launch(b, p, grid, hd, bits);
     } else {
         switch (hd) {
             case 64: st = launch_split_b<64>(b, p, grid, g, bits); break;
@@ -456,9 +554,9 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     }
     if (st != LC_OK || direct || cluster_merge) return st;
     if (fused)
-        LC_LAUNCH_CHECKED(lc_launch(tq_attn_merge_kernel<true>, dim3(n_lanes * n_q), dim3(hd), 0, b, (const float *)k->scratch, (const float *)signs->dptr, nullptr, (__half *)out->dptr, hd, n_splits));
+        LC_LAUNCH_CHECKED(lc_launch(tq_attn_merge_kernel<true>, dim3(n_lanes * n_q), dim3(merge_threads(hd, n_splits)), 0, b, (const float *)k->scratch, (const float *)signs->dptr, nullptr, (__half *)out->dptr, hd, n_splits, p.positions, n_q, lane_capacity, chunk));
     else
-        LC_LAUNCH_CHECKED(lc_launch(tq_attn_merge_kernel<false>, dim3(n_lanes * n_q), dim3(hd), 0, b, (const float *)k->scratch, nullptr, (float *)out->dptr, nullptr, hd, n_splits));
+        LC_LAUNCH_CHECKED(lc_launch(tq_attn_merge_kernel<false>, dim3(n_lanes * n_q), dim3(merge_threads(hd, n_splits)), 0, b, (const float *)k->scratch, nullptr, (float *)out->dptr, nullptr, hd, n_splits, p.positions, n_q, lane_capacity, chunk));
     LC_CHECK_LAUNCH("flash_attention_tq merge");
     b->dispatch_count++;
     return LC_OK;
@@ -557,7 +655,7 @@ int lc_tq_attention_batched_into(lc_kernels *k, lc_batch *b, const lc_buf *q, co
 }  // extern "C"
 
 bool lc_qfrag_supported(uint32_t head_dim, uint32_t bits, uint32_t n_q_heads, uint32_t n_kv_heads) {
-    return head_dim == 256 && bits == 2 && n_kv_heads >= 1 && n_q_heads % n_kv_heads == 0 &&
+    return head_dim == 256 && bits >= 2 && bits <= 4 && n_kv_heads >= 1 && n_q_heads % n_kv_heads == 0 &&
            (n_q_heads / n_kv_heads) % 8 == 0;
 }
 
@@ -687,6 +785,9 @@ extern "C" int lc_tq_attention_noalloc_into(lc_batch *b, const lc_buf *q, const 
     p.qfrag = nullptr;
     p.early_kv = 0;
     p.cluster_merge = 0;
+    p.queue_chunk = 0;
+    p.n_lanes = 1;
+    p.counters = nullptr;
     p.rq = nullptr;
     p.q = (const __half *)q->dptr;
     p.signs = (const float *)signs->dptr;
@@ -720,8 +821,8 @@ extern "C" int lc_tq_attention_noalloc_into(lc_batch *b, const lc_buf *q, const 
         default: st = launch_split_b<512>(b, p, grid, g, bits); break;
     }
     if (st != LC_OK) return st;
-    LC_LAUNCH_CHECKED(lc_launch(tq_attn_merge_kernel<true>, dim3(num_q_heads), dim3(head_dim), 0, b, scratch, (const float *)signs->dptr, nullptr,
-                                                                       (__half *)attn_out->dptr, head_dim, n_splits));
+    LC_LAUNCH_CHECKED(lc_launch(tq_attn_merge_kernel<true>, dim3(num_q_heads), dim3(merge_threads(head_dim, n_splits)), 0, b, scratch, (const float *)signs->dptr, nullptr,
+                                                                       (__half *)attn_out->dptr, head_dim, n_splits, nullptr, num_q_heads, 0u, 0u));
     LC_CHECK_LAUNCH("tq_attention_noalloc merge");
     b->dispatch_count++;
     return LC_OK;

@@ -35,14 +35,36 @@ struct TqAttnParams {
     // 1: `positions` and every key below the lanes' positions were complete before the predecessor kernels started, so
     // the kernel may read them ahead of its dependency wait (tensor-core kernel, per-lane positions only).
     uint32_t early_kv;
+    // Queue form (tensor-core kernel, per-lane positions; 0: off): lanes are cut into items of at most about queue_chunk
+    // keys (lc_attn_items) and a grid of one CTA per SM draws them from a ticket counter; a merge launch follows.
+    // counters: gridDim.y tickets, zero between launches.  n_splits is then the row length of the partial buffer: the
+    // most items a lane can have.
+    uint32_t queue_chunk, n_lanes;
+    unsigned int *counters;
 };
+constexpr uint32_t LC_ATTN_QUEUE_LANES = 512;   // most lanes of the queue form (its schedule lives in shared memory)
 
-// Tensor-core variant for tq2 / head_dim 256 (attention_tq_mma.cu). Same grid and partial layout as the
-// CUDA-core split kernel: grid = (n_splits, n_kv * gchunks, n_lanes) with 8 q-heads per chunk.
-int lc_tq2_attn_mma_launch(lc_batch *b, const TqAttnParams &p, dim3 grid);
+#ifdef __CUDACC__
+// Queue form: a lane of n keys is cut into ceil(n / chunk) items of equal size, in whole 32-key tiles.  The cut depends on
+// the lane alone, so a lane's result does not depend on its neighbours.
+__host__ __device__ __forceinline__ uint32_t lc_attn_item_keys(uint32_t n, uint32_t chunk) {
+    const uint32_t pieces = (n + chunk - 1u) / chunk;
+    const uint32_t per = pieces ? (n + pieces - 1u) / pieces : 1u;
+    return (per + 31u) & ~31u;
+}
+__host__ __device__ __forceinline__ uint32_t lc_attn_items(uint32_t n, uint32_t chunk) {
+    const uint32_t per = lc_attn_item_keys(n, chunk);
+    return n ? (n + per - 1u) / per : 1u;
+}
+#endif
+
+// Tensor-core variant (attention_tq_mma.cu). Same grid and partial layout as the CUDA-core split kernel:
+// grid = (n_splits, n_kv * gchunks, n_lanes) with 8 q-heads per chunk; queue form: (CTAs, n_kv * gchunks, 1).
+bool lc_tq_attn_mma_supported(uint32_t head_dim, uint32_t bits);
+int lc_tq_attn_mma_launch(lc_batch *b, const TqAttnParams &p, dim3 grid, uint32_t head_dim, uint32_t bits);
 
 // Library-internal forms used by the decode step: lc_qkv_post_batched_into that also leaves the query fragments
-// described at TqAttnParams::qfrag in `qfrag` (n_lanes * n_q_heads * head_dim * 4 bytes; requires head_dim 256, 2-bit codes and n_q_heads / n_kv_heads a multiple of 8), and lc_tq_attention_batched_into that reads them.
+// described at TqAttnParams::qfrag in `qfrag` (n_lanes * n_q_heads * head_dim * 4 bytes; requires head_dim 256 and n_q_heads / n_kv_heads a multiple of 8), and lc_tq_attention_batched_into that reads them.
 // The fragments hold exactly the values the attention kernel would derive from q, so results do not change.
 bool lc_qfrag_supported(uint32_t head_dim, uint32_t bits, uint32_t n_q_heads, uint32_t n_kv_heads);
 int lc_qkv_post_frag(lc_kernels *k, lc_batch *b, lc_buf *q, const lc_buf *q_norm_weight, uint32_t n_q_heads,

@@ -1,58 +1,83 @@
-// Tensor-core decode attention over TurboQuant tq2 codes, head_dim 256, up to 8 q-heads per kv-head:
-// the shape of the synthetic E2B-like decoder and of the attention benchmark configuration.  Same
-// contract, grid and split-K partial layout as tq_attn_split_kernel (attention_tq.cu), which remains
-// the general path (other head sizes, tq3 / tq4).
+// Tensor-core decode attention over TurboQuant codes: tq2 / tq3 / tq4, head_dim 128 / 256 / 512, 8 q-heads of a kv-head
+// per CTA.  Same contract, grid and split-K partial layout as tq_attn_split_kernel (attention_tq.cu), which serves what is
+// left: head_dim 64, operands at odd offsets, very short rings.
 //
-// Why a second kernel: with 8 q-heads sharing every K/V row the CUDA-core kernel needs 4096 FMAs per
-// 132 bytes of KV, which binds long before HBM does.  Here both contractions run on tensor cores, with
-// operands built directly in registers:
-//   * a shared-memory table maps one code byte (four 2-bit codes) to four f16 levels with a single
-//     8-byte load; the table is replicated 16 times so the lookups of a half-warp never collide on a bank;
-//   * S^T[16 keys x 8 heads] = K[16 x 256] . RQ^T: the contraction index (dims) is free to permute, so
-//     thread (g, t) of a warp feeds the MMA with the 64 dims held in its own 16 code bytes of keys g, g+8;
-//   * O^T[256 dims x 8 heads] += V^T[256 x 16 keys] . P: the A operand wants (dim; two adjacent keys) per
-//     register, so thread (g, t) decodes bytes 8g..8g+7 of keys 2t, 2t+1, 2t+8, 2t+9 itself and pairs the
-//     table entries of adjacent keys with byte permutes (no cross-lane traffic); P reaches the B operand
-//     through one movmatrix transpose per 8 keys;
-//   * codes and norms stream through a per-warp cp.async ring in shared memory (five tiles in flight).
-// f16 levels: the table stores levels / gamma, with gamma searched (1024 mantissas) so that all levels
-// are f16-representable to ~1e-6 relative; gamma is folded into the row norms in f32.  Logits, softmax
-// and accumulation stay f32.
+// With 8 q-heads sharing every K/V row the CUDA-core kernel needs 16 x head_dim FMAs per key, which binds long before HBM
+// does.  Here both contractions run on tensor cores, with operands built in registers from the packed codes:
+//   * a shared-memory table maps one field of code bits (8 bits: four tq2 or two tq4 codes; 6 bits: two tq3 codes) to
+//     f16 levels with a single 8-byte load; it is replicated 16 times so that the lookups of a half-warp never collide;
+//   * S^T[16 keys x 8 heads] = K[16 x HD] . RQ^T: the contraction index (dims) is free to permute, so thread (g, t) of a
+//     warp feeds the MMA with the HD / 4 dims held in its own quarter of the code bytes of keys g, g + 8;
+//   * O^T[HD dims x 8 heads] += V^T[HD x 16 keys] . P: the A operand wants (dim; two adjacent keys) per register, so
+//     thread (g, t) decodes its eighth of the code bytes of keys 2t, 2t + 1, 2t + 8, 2t + 9 and pairs the table entries of
+//     adjacent keys with byte permutes; P reaches the B operand through one movmatrix transpose per 8 keys.
+// A warp step is KT = 32 keys (16 at head_dim 512): two independent sets of accumulation chains, and the softmax, the
+// running-maximum shuffles and the refill arithmetic are paid once per 32 keys.  Codes stream through a per-warp
+// cp.async ring; consecutive lanes copy consecutive 16-byte pieces, so a tile of one kv-head is one contiguous read.
+//
+// What bounds it: instruction issue and fetch, not a pipe (ncu, tq2: 37 warp instructions per key against 55 with 16-key
+// steps and per-thread copies; ALU 38 %, tensor 27 %, shared memory 41 % busy; 12 or 16 warps with the query in shared memory
+// are no faster).  About 14 cycles per key and SM at tq2, 25 at tq4.  64 lanes x 8193 keys: 57 -> 47 us (tq2), 480 -> 79 us
+// (tq4, from the CUDA-core kernel); 64 ragged lanes up to 8192 keys at tq4: 259 -> 49 us.
+//
+// Precision.  The query is split into an f16 and the f16 of the remainder (two MMAs), because logits reach |q||k| ~ head_dim
+// at softmax scale 1.  tq2: the table holds levels / gamma, with gamma searched (1024 mantissas) so that all four levels are
+// f16-representable to ~1e-6; gamma is folded into the row norms in f32.  tq3 / tq4 have too many levels for that: the
+// table holds each level as an f16 and the f16 of its remainder, and so is P (three MMAs per contraction step).
 #include <math.h>
+#include <utility>
 
 #include "attention_tq.h"
 
 namespace {
 
-constexpr int HD = 256;
-constexpr int CB = 64;           // code bytes per row (tq2)
-constexpr int NT = 256;
-constexpr int NW = NT / 32;
 constexpr int G = 8;             // q-heads per CTA (MMA N)
-constexpr int KT = 16;           // keys per warp step (MMA M for QK, MMA K for PV)
 constexpr int LUT_COPIES = 16;   // an 8-byte shared load is served per half-warp, so 16 copies are conflict-free
-constexpr int LUT_BYTES = 256 * LUT_COPIES * 8;
-constexpr int ACC_BYTES = NW * 16 * 4 * 32 * 4;   // merge staging, reuses the front of shared memory
-constexpr int DEPTH = 6;         // ring slots per warp (DEPTH - 1 tiles in flight)
-constexpr int RING_OFF = LUT_BYTES + G * HD * 4 + 256 * 8;
-constexpr int SMEM_BYTES = RING_OFF + NW * DEPTH * (4 * 32 * 16 + 32 * 4);
-static_assert(SMEM_BYTES >= ACC_BYTES + 1024 + G * HD * 4, "merge staging must fit");
-static_assert(NW == G && NT == 256, "the prologue maps warps to heads and threads to code bytes");
 
-__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+template <int HD_, int BITS_>
+struct AttnCfg {
+    static constexpr int HD = HD_, BITS = BITS_;
+    static constexpr int CB = HD * BITS / 8;            // code bytes per row
+    static constexpr int FB = BITS == 3 ? 6 : 8;        // table index bits
+    static constexpr int NENT = 1 << FB;
+    static constexpr bool HILO = BITS > 2;
+    static constexpr int MT = HD == 512 ? 1 : 2;        // 16-key MMA tiles per warp step
+    static constexpr int KT = 16 * MT;
+    static constexpr int NW = 8, NT = NW * 32;
+    static constexpr int NS = HD / 16;                  // k16 steps of QK, 16-dim tiles of PV
+    static constexpr int DPL = HD / 32;                 // dims per lane where a warp owns a head
+    static constexpr bool QSMEM = HD == 512;            // query fragments stay in shared memory (registers hold the accumulators)
+    // Row strides in the ring: chosen so that the fragment reads spread over the banks.
+    static constexpr int KRS = (BITS == 2 && HD == 256) ? CB : CB + 16;
+    static constexpr int VRS = CB + 16;
+    static constexpr int STAGE = KT * (KRS + VRS);
+    static constexpr int LUT_BYTES = NENT * LUT_COPIES * 8;
+    static constexpr int Q_BYTES = NS * 32 * 16;        // query: f32 [NS][32][4], then the packed fragments in place
+    static constexpr int ENT_BYTES = NENT * 8;
+    static constexpr int ACC_BYTES = NW * NS * 4 * 32 * 4;   // merge staging, reuses query and ring memory
+    static constexpr int RING_OFF = LUT_BYTES + Q_BYTES + ENT_BYTES;
+    // the CTA's merged tile: four floats of padding after every HD / 8 dims (its writers' lanes are HD / 8 dims apart)
+    static constexpr int CPS = HD + 32;
+    static constexpr int TAIL_BYTES = (3 * NW * G + 2 * G) * 4 + G * CPS * 4;  // weights of the warp merge, the merged tile
+    static __device__ __forceinline__ int cp_index(int h, int d) { return h * CPS + d + 4 * (d / (HD / 8)); }
+    static constexpr int RING_ROOM = 222 * 1024 - TAIL_BYTES - RING_OFF;
+    static constexpr int DEPTH_FIT = RING_ROOM / (NW * STAGE);
+    static constexpr int DEPTH = DEPTH_FIT > 4 ? 4 : DEPTH_FIT;   // ring slots per warp (DEPTH - 1 tiles in flight)
+    static constexpr int SMEM0 = RING_OFF + NW * DEPTH * STAGE;
+    static constexpr int TAIL_OFF = SMEM0 > LUT_BYTES + ACC_BYTES ? SMEM0 : LUT_BYTES + ACC_BYTES;
+    static constexpr int SMEM = TAIL_OFF + TAIL_BYTES;
+    static_assert(DEPTH >= 2, "the ring needs two slots");
+    static_assert(SMEM <= 224 * 1024, "shared memory, with room for the static part");
+};
+
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -60,6 +85,48 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+// N 32-bit words of shared memory at an address aligned for the widest load that divides N
+template <int N>
+__device__ __forceinline__ void lds_words(uint32_t a, uint32_t (&w)[N]) {
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4)
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(w[i]), "=r"(w[i + 1]), "=r"(w[i + 2]), "=r"(w[i + 3]) : "r"(a + 4 * i));
+    } else if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 2)
+            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];\n" : "=r"(w[i]), "=r"(w[i + 1]) : "r"(a + 4 * i));
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i++) asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(w[i]) : "r"(a + 4 * i));
+    }
+}
+// f(integral_constant<0>) .. f(integral_constant<N - 1>)
+template <typename F, int... I>
+__device__ __forceinline__ void static_for_impl(F &&f, std::integer_sequence<int, I...>) {
+    (f(std::integral_constant<int, I>{}), ...);
+}
+template <int N, typename F>
+__device__ __forceinline__ void static_for(F &&f) {
+    static_for_impl(f, std::make_integer_sequence<int, N>{});
+}
+// Table address of the FB-bit field at bit O of a word run: lane base + index * 128 bytes.  The multiply-add goes to the
+// multiply pipe, which is idle here; the ALU pipe is the busy one.
+template <int FB, int O, int N>
+__device__ __forceinline__ uint32_t field_addr(const uint32_t (&w)[N], uint32_t lane_base) {
+    constexpr int i = O / 32, o = O % 32;
+    uint32_t idx, r;
+    if constexpr (FB == 8) idx = __byte_perm(w[i], 0u, 0x4440 + o / 8);
+    else if constexpr (o + FB > 32) idx = __funnelshift_r(w[i], w[i + 1 < N ? i + 1 : i], o) & ((1u << FB) - 1u);
+    else idx = (w[i] >> o) & ((1u << FB) - 1u);
+    asm("mad.lo.u32 %0, %1, %2, %3;\n" : "=r"(r) : "r"(idx), "n"(LUT_COPIES * 8), "r"(lane_base));
+    return r;
 }
 // a shared-memory word / 16 bytes of CTA `rank` of this cluster (or of this CTA when the launch is not clustered)
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t rank, bool clustered) {
@@ -93,50 +160,76 @@ __device__ __forceinline__ uint32_t pack_h2(float x, float y) {
     __half2 h = __floats2half2_rn(x, y);
     return *reinterpret_cast<uint32_t *>(&h);
 }
-__device__ __forceinline__ uint32_t byte_of(const uint4 &q, int s) {
-    const uint32_t w = s < 4 ? q.x : (s < 8 ? q.y : (s < 12 ? q.z : q.w));
-    return (w >> (8 * (s & 3))) & 0xFFu;
+__device__ __forceinline__ float2 unpack_h2(uint32_t u) { return __half22float2(*reinterpret_cast<__half2 *>(&u)); }
+// f16 of the two values and f16 of what the rounding left
+__device__ __forceinline__ void split_h2(float x, float y, uint32_t &hi, uint32_t &lo) {
+    hi = pack_h2(x, y);
+    const float2 h = unpack_h2(hi);
+    lo = pack_h2(x - h.x, y - h.y);
+}
+template <int BITS>
+__device__ __forceinline__ float soft_exp(float x) {
+    return BITS == 2 ? __expf(x) : expf(x);
 }
 
-// rq_s index of (head h, dim d): the order in which thread (g, t) = lane 4g + t reads its B fragments,
-// so that fragment loads are one conflict-free float4 per (s, lane).  d = 64t + 4s + e.
-__device__ __forceinline__ int rq_index(int h, int d) {
-    return (((d & 63) >> 2) * 32 + h * 4 + (d >> 6)) * 4 + (d & 3);
+// Walsh-Hadamard butterflies over 32 * DPL values held DPL per lane (lane owns consecutive dims), ascending stride.
+template <int DPL>
+__device__ __forceinline__ void warp_fwht(float (&x)[DPL], int lane) {
+#pragma unroll
+    for (int len = 1; len < DPL; len <<= 1) {
+#pragma unroll
+        for (int i = 0; i < DPL; i++) {
+            if (!(i & len)) {
+                const float a = x[i], b2 = x[i + len];
+                x[i] = a + b2;
+                x[i + len] = a - b2;
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) {
+        const bool upper = lane & m;
+#pragma unroll
+        for (int i = 0; i < DPL; i++) {
+            const float o2 = __shfl_xor_sync(0xffffffffu, x[i], m);
+            x[i] = upper ? o2 - x[i] : x[i] + o2;
+        }
+    }
 }
 
-__global__ void __launch_bounds__(NT) tq2_attn_mma_kernel(const TqAttnParams p) {
+template <typename C>
+__global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p) {
+    constexpr int HD = C::HD, CB = C::CB, NW = C::NW, NT = C::NT, KT = C::KT, MT = C::MT, NS = C::NS, DPL = C::DPL, FB = C::FB;
     lc_pdl_trigger();
     extern __shared__ __align__(16) uint8_t smem[];
-    uint2 *lut = reinterpret_cast<uint2 *>(smem);                       // [256 bytes][16 copies] x 4 f16
-    float *rq_s = reinterpret_cast<float *>(smem + LUT_BYTES);          // [16 s][32 lanes][4] rotated, scaled query
-    uint2 *ent_s = reinterpret_cast<uint2 *>(smem + LUT_BYTES + G * HD * sizeof(float));   // [256] one table copy
+    const uint32_t base_a = smem_u32(smem);
+    uint2 *lut = reinterpret_cast<uint2 *>(smem);                       // [NENT][16 copies]
+    float *rq_s = reinterpret_cast<float *>(smem + C::LUT_BYTES);       // [NS][32 lanes][4] rotated, scaled query
+    uint2 *ent_s = reinterpret_cast<uint2 *>(smem + C::LUT_BYTES + C::Q_BYTES);   // one table copy
     __shared__ float gamma_s;
     __shared__ float cand_err[NW];
     __shared__ int cand_idx[NW];
+    __shared__ uint32_t q_first[LC_ATTN_QUEUE_LANES + 1];               // queue form: first item of each lane
+    __shared__ uint32_t q_ticket, q_lane;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const uint32_t split = blockIdx.x;
     const uint32_t gchunks = (p.group + G - 1) / G;
     const uint32_t kv_head = blockIdx.y / gchunks, gchunk = blockIdx.y - kv_head * gchunks;
-    const uint32_t lane_idx = blockIdx.z;
     const int gvalid = min((int)G, (int)(p.group - gchunk * G));
     const uint32_t qh0 = kv_head * p.group + gchunk * G;
 
-    // ---- before the dependency wait: everything that depends on the codec's levels only (a constant operand): the
-    //      gamma search and the byte table.  A CTA that becomes resident while its predecessor drains does this
-    //      part for free. ----
-    const float lv0 = p.levels[0], lv1 = p.levels[1], lv2 = p.levels[2], lv3 = p.levels[3];
-    // ---- prologue 1: gamma such that every level / gamma is (almost) exactly an f16 ----
-    const float ref = fmaxf(fmaxf(fabsf(lv0), fabsf(lv1)), fmaxf(fabsf(lv2), fabsf(lv3)));
-    {
+    // ---- before the dependency wait: everything that depends on the codec's levels only (a constant operand): gamma and
+    //      the table.  A CTA that becomes resident while its predecessor drains does this part for free. ----
+    if constexpr (!C::HILO) {
+        // gamma such that every level / gamma is (almost) exactly an f16
+        const float lv0 = p.levels[0], lv1 = p.levels[1], lv2 = p.levels[2], lv3 = p.levels[3];
+        const float ref = fmaxf(fmaxf(fabsf(lv0), fabsf(lv1)), fmaxf(fabsf(lv2), fabsf(lv3)));
         const float ia0 = lv0 != 0.f ? 1.0f / fabsf(lv0) : 0.f, ia1 = lv1 != 0.f ? 1.0f / fabsf(lv1) : 0.f;
         const float ia2 = lv2 != 0.f ? 1.0f / fabsf(lv2) : 0.f, ia3 = lv3 != 0.f ? 1.0f / fabsf(lv3) : 0.f;
         float best = INFINITY;
         int besti = 0;
-#pragma unroll
-        for (int it = 0; it < 1024 / NT; it++) {
-            const int j = threadIdx.x + it * NT;
+        for (int j = threadIdx.x; j < 1024; j += NT) {
             const float gm = ref > 0.f ? ref / (1.0f + (float)j * (1.0f / 1024.0f)) : 1.0f;  // largest level -> [1, 2)
             const float inv = __frcp_rn(gm);
             float e = fabsf(__half2float(__float2half_rn(lv0 * inv)) * gm - lv0) * ia0;
@@ -152,457 +245,589 @@ __global__ void __launch_bounds__(NT) tq2_attn_mma_kernel(const TqAttnParams p) 
             if (oe < best || (oe == best && oi < besti)) { best = oe; besti = oi; }
         }
         if (lane == 0) { cand_err[warp] = best; cand_idx[warp] = besti; }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float b2 = cand_err[0];
-        int bi = cand_idx[0];
-        for (int i = 1; i < NW; i++)
-            if (cand_err[i] < b2 || (cand_err[i] == b2 && cand_idx[i] < bi)) { b2 = cand_err[i]; bi = cand_idx[i]; }
-        gamma_s = ref > 0.f ? ref / (1.0f + (float)bi * (1.0f / 1024.0f)) : 1.0f;
-    }
-    __syncthreads();
-    const float gamma = gamma_s;
-    // ---- prologue 3: byte -> four f16 levels table; one copy first, then one copy per lane ----
-    {
-        const int byte = threadIdx.x;   // NT == 256
-        const float inv_levels[4] = {lv0 / gamma, lv1 / gamma, lv2 / gamma, lv3 / gamma};
-        float e4[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int c = (byte >> (2 * q)) & 3;
-            e4[q] = c == 0 ? inv_levels[0] : (c == 1 ? inv_levels[1] : (c == 2 ? inv_levels[2] : inv_levels[3]));
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float b2 = cand_err[0];
+            int bi = cand_idx[0];
+            for (int i = 1; i < NW; i++)
+                if (cand_err[i] < b2 || (cand_err[i] == b2 && cand_idx[i] < bi)) { b2 = cand_err[i]; bi = cand_idx[i]; }
+            gamma_s = ref > 0.f ? ref / (1.0f + (float)bi * (1.0f / 1024.0f)) : 1.0f;
         }
+        __syncthreads();
+    } else {
+        // the largest level becomes 1; each level is stored as two f16
+        float ref = 0.f;
+#pragma unroll
+        for (int i = 0; i < (1 << C::BITS); i++) ref = fmaxf(ref, fabsf(p.levels[i]));
+        if (threadIdx.x == 0) gamma_s = ref > 0.f ? ref : 1.0f;
+        __syncthreads();
+    }
+    const float gamma = gamma_s;
+    for (int e = threadIdx.x; e < C::NENT; e += NT) {
         uint2 v;
-        v.x = pack_h2(e4[0], e4[1]);
-        v.y = pack_h2(e4[2], e4[3]);
-        ent_s[byte] = v;
+        if constexpr (!C::HILO) {
+            v.x = pack_h2(p.levels[e & 3] / gamma, p.levels[(e >> 2) & 3] / gamma);
+            v.y = pack_h2(p.levels[(e >> 4) & 3] / gamma, p.levels[(e >> 6) & 3] / gamma);
+        } else {
+            constexpr int M = (1 << C::BITS) - 1;
+            split_h2(p.levels[e & M] / gamma, p.levels[(e >> C::BITS) & M] / gamma, v.x, v.y);   // {two high parts, two low parts}
+        }
+        ent_s[e] = v;
     }
     __syncthreads();
 #pragma unroll 8
-    for (int e = threadIdx.x; e < 256 * LUT_COPIES; e += NT) lut[e] = ent_s[e / LUT_COPIES];
+    for (int e = threadIdx.x; e < C::NENT * LUT_COPIES; e += NT) lut[e] = ent_s[e / LUT_COPIES];
+    const uint32_t lut_lane = base_a + (uint32_t)(lane & (LUT_COPIES - 1)) * 8u;
 
     // Codes and norms of keys below the lanes' positions were written by earlier steps; only the key at the position
     // itself comes from the predecessor.  A caller that also guarantees that `positions` was written before the
     // predecessor kernels started (the decode step: it is an input of the step) sets early_kv, and the first tiles'
     // copies are then in flight while the predecessor finishes.
-    const bool early = p.early_kv != 0u && p.positions != nullptr && p.row_positions == 0u;
-    if (!early) lc_pdl_wait();
-    uint32_t pos, seq_len;
-    if (p.positions) {
-        pos = p.positions[lane_idx];
-        seq_len = pos + 1u;
-        if (p.ring == 0u && seq_len > p.lane_capacity) {   // never read past the lane's rows
-            seq_len = p.lane_capacity;
-            if (p.status && threadIdx.x == 0) atomicExch(p.status, LC_DEV_STATUS_POSITION);
-        }
-    } else {
-        pos = p.current_pos + (p.row_positions ? lane_idx : 0u);
-        seq_len = min(p.kv_len, pos + 1u);
-    }
-    const uint32_t win_start = (p.window > 0u && pos + 1u > p.window) ? (pos + 1u - p.window) : 0u;
-    const uint32_t n_keys = seq_len > win_start ? seq_len - win_start : 0u;
-    uint32_t per = (n_keys + p.n_splits - 1) / p.n_splits;
-    per = (per + KT - 1) & ~(uint32_t)(KT - 1);
-    const uint32_t k_begin = win_start + split * per;
-    const uint32_t k_end = min(seq_len, k_begin + per);
-    const size_t lane_base = (size_t)lane_idx * p.lane_capacity;
+    const bool queue = p.queue_chunk != 0u;
+    const bool early = p.early_kv != 0u && p.positions != nullptr && p.row_positions == 0u && !queue;
+    if (!early && !(queue && p.early_kv)) lc_pdl_wait();
 
-    // Each warp keeps DEPTH - 1 tiles of codes and norms in flight.  Every thread copies, with cp.async, exactly the
-    // bytes it will consume into its own slots of a shared-memory ring, so no cross-thread synchronisation is needed:
-    //   K codes: keys g and g + 8, bytes 16 t .. 16 t + 15 (the thread's 64 dims of the QK contraction);
-    //   V codes: keys 2t, 2t + 1, 2t + 8, 2t + 9, bytes 8 g .. 8 g + 7 (the thread's 32 output dims of PV);
-    //   one 4-byte word holding one norm (lanes 0-15: key norm of key `lane`; 16-31: value norm of key `lane - 16`).
-    uint4 *ring_c = reinterpret_cast<uint4 *>(smem + RING_OFF) + warp * (DEPTH * 4 * 32);
-    uint32_t *ring_n = reinterpret_cast<uint32_t *>(smem + RING_OFF + NW * DEPTH * 4 * 32 * 16) + warp * (DEPTH * 32);
-    uint32_t parity = 0;   // bit `stage`: which half of the copied word is this lane's norm
-    auto issue = [&](uint32_t t0, int stage) {
-        const uint32_t r0 = p.ring ? t0 % p.ring : t0;   // ring slot of the tile's first key (ring >= 16)
-        auto slot_of = [&](uint32_t off) -> size_t {
-            uint32_t r = t0 + off < k_end ? r0 + off : r0;   // t0 is always a valid key
-            if (p.ring && r >= p.ring) r -= p.ring;
-            return (lane_base + r) * p.n_kv + kv_head;
-        };
-        const size_t slot_n = slot_of(lane & 15);
-        uint4 *dst = ring_c + stage * 4 * 32 + lane;
-        cp_async16(dst, p.kc + slot_of(g) * CB + 16 * t);
-        cp_async16(dst + 32, p.kc + slot_of(g + 8) * CB + 16 * t);
-        uint2 *dv = reinterpret_cast<uint2 *>(dst + 64);
-        cp_async8(dv, p.vc + slot_of(2 * t) * CB + 8 * g);
-        cp_async8(dv + 1, p.vc + slot_of(2 * t + 1) * CB + 8 * g);
-        dv = reinterpret_cast<uint2 *>(dst + 96);
-        cp_async8(dv, p.vc + slot_of(2 * t + 8) * CB + 8 * g);
-        cp_async8(dv + 1, p.vc + slot_of(2 * t + 9) * CB + 8 * g);
-        const __half *nsrc = (lane < 16 ? p.kn : p.vn) + (slot_n & ~(size_t)1);
-        cp_async4(ring_n + stage * 32 + lane, nsrc);
-        parity = (parity & ~(1u << stage)) | ((uint32_t)(slot_n & 1) << stage);
+    // keys [win_start, seq_len) of a lane
+    auto lane_range = [&](uint32_t li, uint32_t &pos, uint32_t &seq_len, uint32_t &win_start, bool report) {
+        if (p.positions) {
+            pos = p.positions[li];
+            seq_len = pos + 1u;
+            if (p.ring == 0u && seq_len > p.lane_capacity) {   // never read past the lane's rows
+                seq_len = p.lane_capacity;
+                if (report && p.status && threadIdx.x == 0) atomicExch(p.status, LC_DEV_STATUS_POSITION);
+            }
+        } else {
+            pos = p.current_pos + (p.row_positions ? li : 0u);
+            seq_len = min(p.kv_len, pos + 1u);
+        }
+        win_start = (p.window > 0u && pos + 1u > p.window) ? (pos + 1u - p.window) : 0u;
     };
-    const uint32_t t_first = k_begin + warp * KT;
-    uint32_t t_issue = t_first;
-    // With early_kv the first tiles leave before the dependency wait, up to the tile that holds the key the
-    // predecessor is writing (position pos: the last key of the last split); that tile and the ones after it follow
-    // the wait.  Groups are committed in tile order either way.
-    int issued = 0;
-    if (early) {
+    uint32_t n_items = 0;
+    if (queue) {
+        for (uint32_t li = threadIdx.x; li < p.n_lanes; li += NT) {
+            uint32_t pos, seq_len, ws;
+            lane_range(li, pos, seq_len, ws, false);
+            const uint32_t n = seq_len > ws ? seq_len - ws : 0u;
+            q_first[li + 1] = lc_attn_items(n, p.queue_chunk);   // (an empty lane is one item and stores zeros)
+        }
+        if (threadIdx.x == 0) q_first[0] = 0;
+        __syncthreads();
+        if (warp == 0) {   // prefix sums
+            uint32_t carry = 0;
+            for (uint32_t l0 = 0; l0 < p.n_lanes; l0 += 32) {
+                const uint32_t li = l0 + lane;
+                uint32_t v = li < p.n_lanes ? q_first[li + 1] : 0u;
 #pragma unroll
-        for (int i = 0; i < DEPTH - 1; i++) {
-            if (issued == i && !(t_issue <= pos && pos < t_issue + KT)) {
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
+                    if (lane >= o) v += u;
+                }
+                v += carry;
+                if (li < p.n_lanes) q_first[li + 1] = v;
+                carry = __shfl_sync(0xffffffffu, v, 31);
+            }
+        }
+        __syncthreads();
+        n_items = q_first[p.n_lanes];
+        if (p.early_kv) lc_pdl_wait();
+    }
+    uint32_t ticket = 0;   // thread 0: the item drawn
+    const uint32_t items_all = n_items + gridDim.x;
+    if (queue && threadIdx.x == 0) ticket = atomicAdd(&p.counters[blockIdx.y], 1u);
+
+    // The item at hand: keys [k_begin, k_end) of lane lane_idx, its part number `split`.
+    uint32_t lane_idx = blockIdx.z, split = blockIdx.x, pos = 0, k_begin = 0, k_end = 0;
+    auto next_item = [&]() -> bool {   // (a barrier at the end: every thread has read the schedule's words)
+        if (queue) {
+            if (threadIdx.x == 0) q_ticket = ticket;
+            __syncthreads();
+            const uint32_t item = q_ticket;
+            if (item >= n_items) {
+                // every CTA has drawn its last: zero again for the next launch
+                if (item == items_all - 1u && threadIdx.x == 0) p.counters[blockIdx.y] = 0u;
+                return false;
+            }
+            for (uint32_t li = threadIdx.x; li < p.n_lanes; li += NT)
+                if (q_first[li] <= item && item < q_first[li + 1]) q_lane = li;
+            __syncthreads();
+            lane_idx = q_lane;
+            split = item - q_first[lane_idx];
+        }
+        uint32_t seq_len, win_start;
+        lane_range(lane_idx, pos, seq_len, win_start, true);
+        const uint32_t n_keys = seq_len > win_start ? seq_len - win_start : 0u;
+        uint32_t per;
+        if (queue) {
+            per = lc_attn_item_keys(n_keys, p.queue_chunk);
+        } else {
+            per = (n_keys + p.n_splits - 1) / p.n_splits;
+            per = (per + (KT - 1)) & ~(uint32_t)(KT - 1);
+        }
+        k_begin = win_start + split * per;
+        k_end = min(seq_len, k_begin + per);
+        return true;
+    };
+
+    // Each warp keeps DEPTH - 1 tiles of codes in flight in its own ring: KT rows of K, then KT rows of V.
+    const uint32_t ring_a = base_a + (uint32_t)C::RING_OFF + (uint32_t)(warp * C::DEPTH) * C::STAGE;
+    auto slot_of = [&](uint32_t t0, uint32_t off) -> size_t {
+        uint32_t r = p.ring ? t0 % p.ring : t0;   // (ring >= KT)
+        if (t0 + off < k_end) r += off;           // t0 is always a valid key
+        if (p.ring && r >= p.ring) r -= p.ring;
+        return ((size_t)lane_idx * p.lane_capacity + r) * p.n_kv + kv_head;
+    };
+    auto issue = [&](uint32_t t0, int stage) {
+        constexpr int CPR = CB / 16, PER_LANE = KT * CPR / 32;
+        const uint32_t dst = ring_a + (uint32_t)stage * C::STAGE;
+        const uint32_t r0 = p.ring ? t0 % p.ring : t0;
+        if (t0 + KT <= k_end && (p.ring == 0u || r0 + KT <= p.ring)) {   // the usual tile: KT rows at one stride
+            const size_t s0 = ((size_t)lane_idx * p.lane_capacity + r0) * p.n_kv + kv_head;
+            const uint8_t *kb = p.kc + s0 * CB, *vb = p.vc + s0 * CB;
+            const uint32_t rs = p.n_kv * (uint32_t)CB;
+#pragma unroll
+            for (int i = 0; i < PER_LANE; i++) {
+                const uint32_t c = (uint32_t)(i * 32 + lane), row = c / CPR, off = (c - row * CPR) * 16u;
+                cp_async16(dst + row * C::KRS + off, kb + row * rs + off);
+                cp_async16(dst + KT * C::KRS + row * C::VRS + off, vb + row * rs + off);
+            }
+        } else {
+#pragma unroll 1
+            for (int i = 0; i < PER_LANE; i++) {
+                const uint32_t c = (uint32_t)(i * 32 + lane), row = c / CPR, off = (c - row * CPR) * 16u;
+                const size_t s = slot_of(t0, row);
+                cp_async16(dst + row * C::KRS + off, p.kc + s * CB + off);
+                cp_async16(dst + KT * C::KRS + row * C::VRS + off, p.vc + s * CB + off);
+            }
+        }
+    };
+    // this lane's norms of a tile: key norm of key `lane`, value norm of key `lane` (KT = 16: lanes 16-31 repeat)
+    auto load_norms = [&](uint32_t t0, __half &nk, __half &nv) {
+        if (t0 < k_end) {
+            const size_t s = slot_of(t0, (uint32_t)lane & (KT - 1));
+            nk = p.kn[s];
+            nv = p.vn[s];
+        }
+    };
+    uint32_t t_issue = 0;
+    __half nk_raw = __float2half(0.f), nv_raw = nk_raw;
+    auto start_item = [&](int issued) {   // the item's first tiles but the `issued` ones
+#pragma unroll
+        for (int i = 0; i < C::DEPTH - 1; i++) {
+            if (i >= issued) {
                 if (t_issue < k_end) issue(t_issue, i);
                 cp_async_commit();
                 t_issue += NW * KT;
-                issued = i + 1;
             }
         }
-        lc_pdl_wait();
-    }
+        load_norms(k_begin + warp * KT, nk_raw, nv_raw);
+    };
+    bool more = next_item();
+    if (more) {
+        t_issue = k_begin + warp * KT;
+        // With early_kv the first tiles leave before the dependency wait, up to the tile that holds the key the
+        // predecessor is writing (position pos: the last key of the last split); that tile and the ones after it follow
+        // the wait.  Groups are committed in tile order either way.
+        int issued = 0;
+        if (early) {
 #pragma unroll
-    for (int i = 0; i < DEPTH - 1; i++) {
-        if (i >= issued) {
-            if (t_issue < k_end) issue(t_issue, i);
-            cp_async_commit();
-            t_issue += NW * KT;
+            for (int i = 0; i < C::DEPTH - 1; i++) {
+                if (issued == i && !(t_issue <= pos && pos < t_issue + KT)) {
+                    if (t_issue < k_end) issue(t_issue, i);
+                    cp_async_commit();
+                    t_issue += NW * KT;
+                    issued = i + 1;
+                }
+            }
+            lc_pdl_wait();
         }
+        start_item(issued);
     }
 
-    // ---- after the wait: the query ----
-    const size_t q_row = ((size_t)lane_idx * p.n_q + qh0 + warp) * HD + 8 * lane;   // warp w owns head w
-    uint4 q_raw = make_uint4(0u, 0u, 0u, 0u);
-    float4 q_s0 = make_float4(0.f, 0.f, 0.f, 0.f), q_s1 = q_s0;
-    // B fragments of the query: thread (g, t) holds head g, dims 64t + 4s + {0,1} and + {2,3}, s = 0..15.
-    // The query is the one operand f16 cannot hold well enough when logits are large (softmax scale 1.0):
-    // it is split into a high f16 part and the f16 of the remainder, and each k-step issues two MMAs.
-    uint32_t bq[16][2], bql[16][2];
-    const bool have_frag = p.qfrag != nullptr;   // the launch that wrote q left the fragments ready (group % 8 == 0)
-    if (have_frag) {
-        const uint4 *src = p.qfrag + ((size_t)lane_idx * (p.n_q >> 3) + (qh0 >> 3)) * 512 + lane;
+    while (more) {
+        // ---- after the wait: the query.  B fragments: thread (g, t) holds head g, dims t HD/4 + 4s + {0,1} and + {2,3}.
+        //      It is the one operand f16 cannot hold well enough: a high f16 part and the f16 of the remainder. ----
+        constexpr int NQ = C::QSMEM ? 1 : NS;
+        uint32_t bq[NQ][2], bql[NQ][2];
+        const bool have_frag = p.qfrag != nullptr;   // the launch that wrote q left the fragments ready (group % 8 == 0)
+        if (C::QSMEM && have_frag) {
+            const uint4 *src = p.qfrag + ((size_t)lane_idx * (p.n_q >> 3) + (qh0 >> 3)) * (NS * 32);
+            for (int e = threadIdx.x; e < NS * 32; e += NT) *reinterpret_cast<uint4 *>(rq_s + e * 4) = src[e];
+        } else if (!C::QSMEM && have_frag) {
+            const uint4 *src = p.qfrag + ((size_t)lane_idx * (p.n_q >> 3) + (qh0 >> 3)) * (NS * 32) + lane;
 #pragma unroll
-        for (int s = 0; s < 16; s++) {
-            const uint4 v = src[s * 32];
-            bq[s][0] = v.x;
-            bq[s][1] = v.y;
-            bql[s][0] = v.z;
-            bql[s][1] = v.w;
-        }
-    } else if (warp < gvalid) {
-        if (p.fused_q) {
-            q_raw = *reinterpret_cast<const uint4 *>(p.q + q_row);
-            q_s0 = *reinterpret_cast<const float4 *>(p.signs + 8 * lane);
-            q_s1 = *reinterpret_cast<const float4 *>(p.signs + 8 * lane + 4);
-        } else {
-            q_s0 = *reinterpret_cast<const float4 *>(p.rq + q_row);
-            q_s1 = *reinterpret_cast<const float4 *>(p.rq + q_row + 4);
-        }
-    }
-    // ---- prologue 2 (independent of gamma): rotated, scaled query; warp w owns head w ----
-    if (!have_frag) {
-        const int h = warp;   // NW == G
-        float x[8];
-        if (h < gvalid) {
-            if (p.fused_q) {
-                const __half2 *hp = reinterpret_cast<const __half2 *>(&q_raw);
-                const float sg[8] = {q_s0.x, q_s0.y, q_s0.z, q_s0.w, q_s1.x, q_s1.y, q_s1.z, q_s1.w};
+            for (int s = 0; s < NQ; s++) {
+                const uint4 v = src[s * 32];
+                bq[s][0] = v.x;
+                bq[s][1] = v.y;
+                bql[s][0] = v.z;
+                bql[s][1] = v.w;
+            }
+        } else if (warp < G) {   // warp w rotates and scales head w
+            float x[DPL];
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const float2 f = __half22float2(hp[e]);
-                    x[2 * e] = f.x * sg[2 * e];
-                    x[2 * e + 1] = f.y * sg[2 * e + 1];
-                }
-                // 256-point Walsh-Hadamard butterflies: strides 1, 2, 4 inside the thread, 8..128 across lanes
+            for (int i = 0; i < DPL; i++) x[i] = 0.f;
+            if (warp < gvalid) {
+                const size_t q_row = ((size_t)lane_idx * p.n_q + qh0 + warp) * HD + DPL * lane;
+                if (p.fused_q) {
 #pragma unroll
-                for (int len = 1; len < 8; len <<= 1) {
+                    for (int i = 0; i < DPL; i += 4) {
+                        const uint2 raw = *reinterpret_cast<const uint2 *>(p.q + q_row + i);
+                        const float4 sg = *reinterpret_cast<const float4 *>(p.signs + DPL * lane + i);
+                        const float2 f0 = unpack_h2(raw.x), f1 = unpack_h2(raw.y);
+                        x[i] = f0.x * sg.x;
+                        x[i + 1] = f0.y * sg.y;
+                        x[i + 2] = f1.x * sg.z;
+                        x[i + 3] = f1.y * sg.w;
+                    }
+                    warp_fwht<DPL>(x, lane);
+                    const float f = p.scale / sqrtf((float)HD);
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        if (!(i & len)) {
-                            const float a = x[i], b2 = x[i + len];
-                            x[i] = a + b2;
-                            x[i + len] = a - b2;
-                        }
+                    for (int i = 0; i < DPL; i++) x[i] *= f;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < DPL; i += 4) {
+                        const float4 r = *reinterpret_cast<const float4 *>(p.rq + q_row + i);
+                        x[i] = r.x * p.scale;
+                        x[i + 1] = r.y * p.scale;
+                        x[i + 2] = r.z * p.scale;
+                        x[i + 3] = r.w * p.scale;
                     }
                 }
+            }
 #pragma unroll
-                for (int m = 1; m < 32; m <<= 1) {
-                    const bool upper = lane & m;
+            for (int i = 0; i < DPL; i += 4) {   // dim d = t HD/4 + 4s + e is element e of entry [s][lane 4 head + t]
+                const int d = DPL * lane + i;
+                *reinterpret_cast<float4 *>(rq_s + (((d % (HD / 4)) / 4) * 32 + warp * 4 + d / (HD / 4)) * 4) =
+                    make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+            }
+        }
+        __syncthreads();   // the rotated query is in place; so is every copy of the table
+        if (C::QSMEM) {
+            if (!have_frag)
+            for (int e = threadIdx.x; e < NS * 32; e += NT) {   // in place: entry e is read and written by one thread
+                const float4 r = *reinterpret_cast<const float4 *>(rq_s + e * 4);
+                uint4 v;
+                split_h2(r.x, r.y, v.x, v.z);
+                split_h2(r.z, r.w, v.y, v.w);
+                *reinterpret_cast<uint4 *>(rq_s + e * 4) = v;
+            }
+            __syncthreads();
+        } else if (!have_frag) {
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const float o2 = __shfl_xor_sync(0xffffffffu, x[i], m);
-                        x[i] = upper ? o2 - x[i] : x[i] + o2;
+            for (int s = 0; s < NQ; s++) {
+                const float4 r = *reinterpret_cast<const float4 *>(rq_s + (s * 32 + lane) * 4);
+                split_h2(r.x, r.y, bq[s][0], bql[s][0]);
+                split_h2(r.z, r.w, bq[s][1], bql[s][1]);
+            }
+        }
+        const uint32_t q_a = base_a + (uint32_t)C::LUT_BYTES + (uint32_t)lane * 16u;
+
+        // ---- main loop: each warp takes every 8th tile of this split ----
+        float o[NS][4];
+#pragma unroll
+        for (int s = 0; s < NS; s++) o[s][0] = o[s][1] = o[s][2] = o[s][3] = 0.f;
+        float m_run[2] = {-INFINITY, -INFINITY}, l_part[2] = {0.f, 0.f};   // heads 2t, 2t+1 (l: this thread's keys only)
+
+        int stage = 0;
+        for (uint32_t t0 = k_begin + warp * KT; t0 < k_end; t0 += NW * KT) {
+            cp_async_wait<C::DEPTH - 2>();   // tile t0 is the oldest group in flight
+            __syncwarp();                    // ... for every lane; and every lane is done with the tile before
+            const float nk = __half2float(nk_raw) * gamma, nv = __half2float(nv_raw) * gamma;
+            load_norms(t0 + NW * KT, nk_raw, nv_raw);
+            {
+                const int st_fill = stage == 0 ? C::DEPTH - 1 : stage - 1;
+                if (t_issue < k_end) issue(t_issue, st_fill);
+                cp_async_commit();
+                t_issue += NW * KT;
+            }
+            const uint32_t ka = ring_a + (uint32_t)stage * C::STAGE, va = ka + KT * C::KRS;
+            stage = stage + 1 == C::DEPTH ? 0 : stage + 1;
+
+            // ---- S^T[KT keys x 8 heads] ----
+            constexpr int KW = CB / 16;   // words of one key in this thread's quarter row
+            uint32_t kw[MT][2][KW];
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++) {
+                lds_words<KW>(ka + (uint32_t)(mt * 16 + g) * C::KRS + (uint32_t)t * (KW * 4), kw[mt][0]);
+                lds_words<KW>(ka + (uint32_t)(mt * 16 + g + 8) * C::KRS + (uint32_t)t * (KW * 4), kw[mt][1]);
+            }
+            float c[MT][2][4];   // chains: high and low query parts
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) c[mt][0][i] = c[mt][1][i] = 0.f;
+            auto qk_step = [&](auto S) {
+                constexpr int s = decltype(S)::value;
+                uint32_t b0, b1, l0, l1;
+                if constexpr (C::QSMEM) {
+                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(b0), "=r"(b1), "=r"(l0), "=r"(l1) : "r"(q_a + s * 512));
+                } else {
+                    b0 = bq[s][0]; b1 = bq[s][1]; l0 = bql[s][0]; l1 = bql[s][1];
+                }
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    if constexpr (!C::HILO) {
+                        const uint2 x = lds64(field_addr<FB, s * 8>(kw[mt][0], lut_lane)), y = lds64(field_addr<FB, s * 8>(kw[mt][1], lut_lane));
+                        const uint32_t a[4] = {x.x, y.x, x.y, y.y};
+                        mma16816(c[mt][0], a, b0, b1);
+                        mma16816(c[mt][1], a, l0, l1);
+                    } else {
+                        const uint2 x0 = lds64(field_addr<FB, 2 * s * FB>(kw[mt][0], lut_lane)), x1 = lds64(field_addr<FB, (2 * s + 1) * FB>(kw[mt][0], lut_lane));
+                        const uint2 y0 = lds64(field_addr<FB, 2 * s * FB>(kw[mt][1], lut_lane)), y1 = lds64(field_addr<FB, (2 * s + 1) * FB>(kw[mt][1], lut_lane));
+                        const uint32_t ah[4] = {x0.x, y0.x, x1.x, y1.x}, al[4] = {x0.y, y0.y, x1.y, y1.y};
+                        mma16816(c[mt][0], ah, b0, b1);
+                        mma16816(c[mt][1], ah, l0, l1);
+                        mma16816(c[mt][1], al, b0, b1);
                     }
                 }
-                const float f = p.scale / sqrtf((float)HD);
+            };
+            static_for<NS>(qk_step);
+
+            // ---- online softmax: logits of keys 16 mt + g (row 0), + 8 (row 1) for heads 2t, 2t+1 ----
+            float sc[MT][2][2], tm[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-                for (int i = 0; i < 8; i++) x[i] *= f;
-            } else {
-                const float4 r0 = q_s0, r1 = q_s1;
-                x[0] = r0.x * p.scale; x[1] = r0.y * p.scale; x[2] = r0.z * p.scale; x[3] = r0.w * p.scale;
-                x[4] = r1.x * p.scale; x[5] = r1.y * p.scale; x[6] = r1.z * p.scale; x[7] = r1.w * p.scale;
+            for (int mt = 0; mt < MT; mt++) {
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    const int key = 16 * mt + 8 * r + g;
+                    const float kn = __shfl_sync(0xffffffffu, nk, key);
+                    const bool valid = t0 + key < k_end;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        sc[mt][r][h] = valid ? (c[mt][0][2 * r + h] + c[mt][1][2 * r + h]) * kn : -INFINITY;
+                        tm[h] = fmaxf(tm[h], sc[mt][r][h]);
+                    }
+                }
             }
-        } else {
+            float resc[2];
 #pragma unroll
-            for (int i = 0; i < 8; i++) x[i] = 0.f;
-        }
-        *reinterpret_cast<float4 *>(rq_s + rq_index(h, 8 * lane)) = make_float4(x[0], x[1], x[2], x[3]);
-        *reinterpret_cast<float4 *>(rq_s + rq_index(h, 8 * lane + 4)) = make_float4(x[4], x[5], x[6], x[7]);
-    }
-    __syncthreads();   // the rotated query is in place; so is every copy of the table
-    if (!have_frag) {
-#pragma unroll
-        for (int s = 0; s < 16; s++) {
-            const float4 r4 = *reinterpret_cast<const float4 *>(rq_s + (s * 32 + lane) * 4);
-            const float r[4] = {r4.x, r4.y, r4.z, r4.w};
-            float hi[4], lo[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                hi[e] = __half2float(__float2half_rn(r[e]));
-                lo[e] = r[e] - hi[e];
+            for (int h = 0; h < 2; h++) {
+                tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 4));
+                tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 8));
+                tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 16));
+                const float m_new = fmaxf(m_run[h], tm[h]);    // finite: key t0 is valid
+                resc[h] = soft_exp<C::BITS>(m_run[h] - m_new);
+                m_run[h] = m_new;
+                l_part[h] *= resc[h];
             }
-            bq[s][0] = pack_h2(hi[0], hi[1]);
-            bq[s][1] = pack_h2(hi[2], hi[3]);
-            bql[s][0] = pack_h2(lo[0], lo[1]);
-            bql[s][1] = pack_h2(lo[2], lo[3]);
-        }
-    }
-    const uint2 *lut_lane = lut + (lane & (LUT_COPIES - 1));
+            // P (times the value norms) into the B operand: (key g | g+8; heads 2t, 2t+1) -> (keys 2t, 2t+1 | +8; head g)
+            uint32_t bp[MT][2], bpl[MT][2];
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++) {
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    const float vn = __shfl_sync(0xffffffffu, nv, (KT == 32 ? 16 * mt : 0) + 8 * r + g);
+                    const float p0 = soft_exp<C::BITS>(sc[mt][r][0] - m_run[0]), p1 = soft_exp<C::BITS>(sc[mt][r][1] - m_run[1]);
+                    l_part[0] += p0;
+                    l_part[1] += p1;
+                    if constexpr (!C::HILO) {
+                        bp[mt][r] = movmatrix_trans(pack_h2(p0 * vn, p1 * vn));
+                    } else {
+                        uint32_t hi, lo;
+                        split_h2(p0 * vn, p1 * vn, hi, lo);
+                        bp[mt][r] = movmatrix_trans(hi);
+                        bpl[mt][r] = movmatrix_trans(lo);
+                    }
+                }
+            }
+            if (__any_sync(0xffffffffu, resc[0] != 1.0f || resc[1] != 1.0f)) {   // the running max moved for some head
+#pragma unroll
+                for (int s = 0; s < NS; s++) {
+                    o[s][0] *= resc[0]; o[s][1] *= resc[1]; o[s][2] *= resc[0]; o[s][3] *= resc[1];
+                }
+            }
 
-    // ---- main loop: each warp takes every 8th 16-key tile of this split ----
-    float o[16][4];
+            // ---- O^T[HD dims x 8 heads] += V^T . P.  MMA tile j has rows (g, g + 8) = dims (g HD/8 + 2j, + 1). ----
 #pragma unroll
-    for (int s = 0; s < 16; s++) o[s][0] = o[s][1] = o[s][2] = o[s][3] = 0.f;
-    float m_run[2] = {-INFINITY, -INFINITY}, l_part[2] = {0.f, 0.f};   // heads 2t, 2t+1 (l: this thread's keys only)
-
-    int stage = 0;
-    for (uint32_t t0 = t_first; t0 < k_end; t0 += NW * KT) {
-        // tile t0 is the oldest group in flight; DEPTH - 2 newer ones may still be pending
-        cp_async_wait<DEPTH - 2>();
-        const uint4 *src = ring_c + stage * 4 * 32 + lane;
-        const uint4 kqa = src[0], kqb = src[32], vqa = src[64], vqb = src[96];
-        const uint32_t nw = ring_n[stage * 32 + lane];
-        const float n_own = __half2float(__ushort_as_half((unsigned short)((parity >> stage) & 1u ? nw >> 16 : nw & 0xFFFFu))) * gamma;
-        const float kna = __shfl_sync(0xffffffffu, n_own, g), knb = __shfl_sync(0xffffffffu, n_own, g + 8);
-        const float vna = __shfl_sync(0xffffffffu, n_own, 16 + g), vnb = __shfl_sync(0xffffffffu, n_own, 24 + g);
-        // refill: the slot of the tile consumed in the previous iteration is free (its values were used by then)
-        {
-            const int st_fill = stage == 0 ? DEPTH - 1 : stage - 1;
-            if (t_issue < k_end) issue(t_issue, st_fill);
-            cp_async_commit();
-            t_issue += NW * KT;
+            for (int mt = 0; mt < MT; mt++) {
+                constexpr int VW = CB % 32 == 0 ? CB / 32 : 2;   // words of one key in this thread's eighth row
+                uint32_t vw[4][VW];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const uint32_t row = va + (uint32_t)(16 * mt + 2 * t + (q & 1) + 8 * (q >> 1)) * C::VRS;
+                    if constexpr (CB % 32 == 0) {
+                        lds_words<VW>(row + (uint32_t)g * (VW * 4), vw[q]);
+                    } else {   // 6-byte pieces (tq3 at head_dim 128): two aligned words, shifted into place
+                        const uint32_t a = row + (uint32_t)g * 6u, sh = (a & 2u) * 8u;
+                        uint32_t w[2];
+                        asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(w[0]) : "r"(a & ~3u));
+                        asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(w[1]) : "r"((a & ~3u) + 4u));
+                        vw[q][0] = __funnelshift_r(w[0], w[1], sh);
+                        vw[q][1] = w[1] >> sh;
+                    }
+                }
+                auto pv_step = [&](auto U) {
+                    constexpr int u = decltype(U)::value;
+                    const uint2 e0 = lds64(field_addr<FB, u * FB>(vw[0], lut_lane)), e1 = lds64(field_addr<FB, u * FB>(vw[1], lut_lane));   // keys 2t, 2t+1
+                    const uint2 e2 = lds64(field_addr<FB, u * FB>(vw[2], lut_lane)), e3 = lds64(field_addr<FB, u * FB>(vw[3], lut_lane));   // keys 2t+8, 2t+9
+                    // .x: first two dims (tq2) / high parts; .y: next two dims / low parts
+                    const uint32_t ax[4] = {__byte_perm(e0.x, e1.x, 0x5410), __byte_perm(e0.x, e1.x, 0x7632), __byte_perm(e2.x, e3.x, 0x5410),
+                                            __byte_perm(e2.x, e3.x, 0x7632)};
+                    const uint32_t ay[4] = {__byte_perm(e0.y, e1.y, 0x5410), __byte_perm(e0.y, e1.y, 0x7632), __byte_perm(e2.y, e3.y, 0x5410),
+                                            __byte_perm(e2.y, e3.y, 0x7632)};
+                    if constexpr (!C::HILO) {
+                        mma16816(o[2 * u], ax, bp[mt][0], bp[mt][1]);
+                        mma16816(o[2 * u + 1], ay, bp[mt][0], bp[mt][1]);
+                    } else {
+                        mma16816(o[u], ax, bp[mt][0], bp[mt][1]);
+                        mma16816(o[u], ax, bpl[mt][0], bpl[mt][1]);
+                        mma16816(o[u], ay, bp[mt][0], bp[mt][1]);
+                    }
+                };
+                static_for<(C::HILO ? NS : NS / 2)>(pv_step);
+            }
         }
-        stage = stage + 1 == DEPTH ? 0 : stage + 1;
-        const bool va = t0 + g < k_end, vb = t0 + g + 8 < k_end;
 
-        // S^T[16 keys x 8 heads]
-        // eight independent accumulation chains (k-step mod 4, high / low query parts)
-        float c8[8][4];
-#pragma unroll
-        for (int i = 0; i < 8; i++) c8[i][0] = c8[i][1] = c8[i][2] = c8[i][3] = 0.f;
-#pragma unroll
-        for (int s = 0; s < 16; s++) {
-            const uint2 la = lut_lane[byte_of(kqa, s) * LUT_COPIES], lb = lut_lane[byte_of(kqb, s) * LUT_COPIES];
-            const uint32_t a[4] = {la.x, lb.x, la.y, lb.y};
-            mma16816(c8[2 * (s & 3)], a, bq[s]);
-            mma16816(c8[2 * (s & 3) + 1], a, bql[s]);
-        }
-        float c[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-            c[e] = ((c8[0][e] + c8[2][e]) + (c8[4][e] + c8[6][e])) + ((c8[1][e] + c8[3][e]) + (c8[5][e] + c8[7][e]));
-        // logits of keys g (c0, c1) and g+8 (c2, c3) for heads 2t, 2t+1
-        float sA[2] = {va ? c[0] * kna : -INFINITY, va ? c[1] * kna : -INFINITY};
-        float sB[2] = {vb ? c[2] * knb : -INFINITY, vb ? c[3] * knb : -INFINITY};
-        float pa[2], pb[2], resc[2];
+        // the next ticket, drawn as late as hides the round trip: items are then handed out in the order of need
+        if (queue && threadIdx.x == 0) ticket = atomicAdd(&p.counters[blockIdx.y], 1u);
+
+        // ---- merge the 8 warps; query and ring memory is reused for the per-warp accumulators ----
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            float tm = fmaxf(sA[h], sB[h]);
-            tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 4));
-            tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 8));
-            tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 16));
-            const float m_new = fmaxf(m_run[h], tm);    // finite: key t0 is valid
-            resc[h] = __expf(m_run[h] - m_new);
-            pa[h] = __expf(sA[h] - m_new);
-            pb[h] = __expf(sB[h] - m_new);
-            l_part[h] = l_part[h] * resc[h] + pa[h] + pb[h];
-            m_run[h] = m_new;
+            l_part[h] += __shfl_xor_sync(0xffffffffu, l_part[h], 4);
+            l_part[h] += __shfl_xor_sync(0xffffffffu, l_part[h], 8);
+            l_part[h] += __shfl_xor_sync(0xffffffffu, l_part[h], 16);
         }
-        if (__any_sync(0xffffffffu, resc[0] != 1.0f || resc[1] != 1.0f)) {   // the running max moved for some head
+        __syncthreads();   // every warp is done with its ring
+        float *acc_s = reinterpret_cast<float *>(smem + C::LUT_BYTES);                   // [NW][NS][4][32 lanes]
+        float *m_s = reinterpret_cast<float *>(smem + C::TAIL_OFF);                      // [NW][G]
+        float *l_s = m_s + NW * G;
+        if (g == 0) {
+            m_s[warp * G + 2 * t] = m_run[0];
+            m_s[warp * G + 2 * t + 1] = m_run[1];
+            l_s[warp * G + 2 * t] = l_part[0];
+            l_s[warp * G + 2 * t + 1] = l_part[1];
+        }
+        // Accumulators go to shared memory in fragment order [warp][s][j][lane] (conflict-free both ways).
 #pragma unroll
-            for (int s = 0; s < 16; s++) {
-                o[s][0] *= resc[0]; o[s][1] *= resc[1]; o[s][2] *= resc[0]; o[s][3] *= resc[1];
+        for (int s = 0; s < NS; s++) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc_s[((warp * NS + s) * 4 + j) * 32 + lane] = o[s][j];
+        }
+        __syncthreads();
+        // Per (warp, head) weights exp(m_w - max) and the merged (max, sum); thread h < G does head h.
+        float *f_s = l_s + NW * G;       // [NW][G]
+        float *ml_s = f_s + NW * G;      // [G][2]
+        float *cpart = ml_s + 2 * G;     // this CTA's merged, unnormalised tile (cp_index)
+        if (threadIdx.x < G) {
+            const int h = threadIdx.x;
+            float gmax = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < NW; w++) gmax = fmaxf(gmax, m_s[w * G + h]);
+            float gsum = 0.f;
+#pragma unroll
+            for (int w = 0; w < NW; w++) {
+                const float mw = m_s[w * G + h];
+                const float f = (mw == -INFINITY) ? 0.f : soft_exp<C::BITS>(mw - gmax);
+                f_s[w * G + h] = f;
+                gsum += f * l_s[w * G + h];
+            }
+            ml_s[2 * h] = gmax;
+            ml_s[2 * h + 1] = gsum;
+        }
+        __syncthreads();
+        const size_t part_row = HD + 2;
+        const uint32_t it_lane = lane_idx, it_split = split;
+        // where head h's partial of this split goes
+        auto part_of = [&](int h, uint32_t sp) -> float * {
+            const size_t qh = (size_t)it_lane * p.n_q + qh0 + h;
+            return p.partial + (qh * p.n_splits + sp) * part_row;
+        };
+        // Thread (warp, lane) merges fragment position `lane` of its tiles s: element j of tile s is
+        // head 2t + (j & 1), dim (HD / 8) g + 2 s + (j >> 1).
+        for (int s = warp; s < NS; s += NW) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int h = 2 * t + (j & 1);
+                const int d = (HD / 8) * g + 2 * s + (j >> 1);
+                float acc = 0.f;
+#pragma unroll
+                for (int w = 0; w < NW; w++) acc += f_s[w * G + h] * acc_s[((w * NS + s) * 4 + j) * 32 + lane];
+                cpart[C::cp_index(h, d)] = acc;
             }
         }
-        // P (times the value norms) into the B operand: (key g | g+8; heads 2t, 2t+1) -> (keys 2t, 2t+1 | +8; head g)
-        uint32_t bp[2];
-        bp[0] = movmatrix_trans(pack_h2(pa[0] * vna, pa[1] * vna));
-        bp[1] = movmatrix_trans(pack_h2(pb[0] * vnb, pb[1] * vnb));
-        // O^T[256 dims x 8 heads] += V^T . P.  Code byte u of this thread's 8 (dims 32 g + 4 u .. + 3) of its four keys
-        // feeds two MMAs: tile 2u has rows (g, g + 8) = dims (32 g + 4 u, + 1), tile 2u + 1 the next two dims.  The
-        // A fragment wants (dim; two adjacent keys) per register: a byte permute of two table entries.
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const uint2 e0 = lut_lane[byte_of(vqa, u) * LUT_COPIES], e1 = lut_lane[byte_of(vqa, 8 + u) * LUT_COPIES];   // keys 2t, 2t+1
-            const uint2 e2 = lut_lane[byte_of(vqb, u) * LUT_COPIES], e3 = lut_lane[byte_of(vqb, 8 + u) * LUT_COPIES];   // keys 2t+8, 2t+9
-            uint32_t a[4];
-            a[0] = __byte_perm(e0.x, e1.x, 0x5410);
-            a[1] = __byte_perm(e0.x, e1.x, 0x7632);
-            a[2] = __byte_perm(e2.x, e3.x, 0x5410);
-            a[3] = __byte_perm(e2.x, e3.x, 0x7632);
-            mma16816(o[2 * u], a, bp);
-            a[0] = __byte_perm(e0.y, e1.y, 0x5410);
-            a[1] = __byte_perm(e0.y, e1.y, 0x7632);
-            a[2] = __byte_perm(e2.y, e3.y, 0x5410);
-            a[3] = __byte_perm(e2.y, e3.y, 0x7632);
-            mma16816(o[2 * u + 1], a, bp);
+        __syncthreads();   // the tile is complete; the ring is free
+        if (queue) {
+            more = next_item();
+            if (more) {
+                t_issue = k_begin + warp * KT;
+                start_item(0);
+            }
+        } else {
+            more = false;
         }
-    }
-
-    // ---- merge the 8 warps; lut memory is reused for the per-warp accumulators ----
-    l_part[0] += __shfl_xor_sync(0xffffffffu, l_part[0], 4);
-    l_part[0] += __shfl_xor_sync(0xffffffffu, l_part[0], 8);
-    l_part[0] += __shfl_xor_sync(0xffffffffu, l_part[0], 16);
-    l_part[1] += __shfl_xor_sync(0xffffffffu, l_part[1], 4);
-    l_part[1] += __shfl_xor_sync(0xffffffffu, l_part[1], 8);
-    l_part[1] += __shfl_xor_sync(0xffffffffu, l_part[1], 16);
-    __syncthreads();   // every warp is done with the table
-    float *acc_s = reinterpret_cast<float *>(smem);   // [NW][G][HD]
-    float *m_s = reinterpret_cast<float *>(smem + ACC_BYTES);   // [NW][G]  (query, table and ring are all dead)
-    float *l_s = m_s + NW * G;
-    if (g == 0) {
-        m_s[warp * G + 2 * t] = m_run[0];
-        m_s[warp * G + 2 * t + 1] = m_run[1];
-        l_s[warp * G + 2 * t] = l_part[0];
-        l_s[warp * G + 2 * t + 1] = l_part[1];
-    }
-    // Accumulators go to shared memory in fragment order [warp][s][j][lane] (conflict-free both ways).
-#pragma unroll
-    for (int s = 0; s < 16; s++) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc_s[((warp * 16 + s) * 4 + j) * 32 + lane] = o[s][j];
-    }
-    __syncthreads();
-    // Per (warp, head) weights exp(m_w - max) and the merged (max, sum); thread h < G does head h.
-    float *f_s = l_s + NW * G;       // [NW][G]
-    float *ml_s = f_s + NW * G;      // [G][2]
-    float *cpart = ml_s + 2 * G + 16;  // [G][HD] this CTA's merged, unnormalised tile (cluster merge only)
-    if (threadIdx.x < G) {
-        const int h = threadIdx.x;
-        float gmax = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < NW; w++) gmax = fmaxf(gmax, m_s[w * G + h]);
-        float gsum = 0.f;
-#pragma unroll
-        for (int w = 0; w < NW; w++) {
-            const float mw = m_s[w * G + h];
-            const float f = (mw == -INFINITY) ? 0.f : __expf(mw - gmax);
-            f_s[w * G + h] = f;
-            gsum += f * l_s[w * G + h];
-        }
-        ml_s[2 * h] = gmax;
-        ml_s[2 * h + 1] = gsum;
-    }
-    __syncthreads();
-    // Thread (warp, lane) merges fragment position `lane` of tiles s = 2 warp, 2 warp + 1: element j of tile s is
-    // head 2t + (j & 1), dim 32 g + 2 s + (j >> 1).
-#pragma unroll
-    for (int ss = 0; ss < 2; ss++) {
-        const int s = 2 * warp + ss;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int h = 2 * t + (j & 1);
-            const int d = 32 * g + 2 * s + (j >> 1);
-            float acc = 0.f;
-#pragma unroll
-            for (int w = 0; w < NW; w++) acc += f_s[w * G + h] * acc_s[((w * 16 + s) * 4 + j) * 32 + lane];
-            if (p.cluster_merge) {
-                cpart[h * HD + d] = acc;
-            } else if (h < gvalid) {
-                const size_t qh = (size_t)lane_idx * p.n_q + qh0 + h;
+        if (!p.cluster_merge) {   // a merge launch follows (unless there is nothing to merge)
+            for (int e = threadIdx.x; e < gvalid * (HD / 2); e += NT) {
+                const int h = e / (HD / 2), d = 2 * (e % (HD / 2));
+                const float2 v = *reinterpret_cast<const float2 *>(cpart + C::cp_index(h, d));
                 if (p.direct_out) {
                     const float gsum = ml_s[2 * h + 1];
-                    p.out[qh * HD + d] = gsum > 0.f ? acc / gsum : 0.f;
+                    float *dst = p.out + ((size_t)it_lane * p.n_q + qh0 + h) * HD + d;
+                    dst[0] = gsum > 0.f ? v.x / gsum : 0.f;
+                    dst[1] = gsum > 0.f ? v.y / gsum : 0.f;
                 } else {
-                    p.partial[(qh * p.n_splits + split) * (size_t)(HD + 2) + 2 + d] = acc;
+                    *reinterpret_cast<float2 *>(part_of(h, it_split) + 2 + d) = v;
                 }
             }
-        }
-    }
-    if (!p.cluster_merge) {
-        if (!p.direct_out && threadIdx.x < 2 * gvalid) {
-            const int h = threadIdx.x >> 1;
-            const size_t qh = (size_t)lane_idx * p.n_q + qh0 + h;
-            p.partial[(qh * p.n_splits + split) * (size_t)(HD + 2) + (threadIdx.x & 1)] = ml_s[threadIdx.x];
-        }
-        return;
-    }
-    // ---- splits of this (lane, kv head): one cluster.  Head h is finished by CTA h mod n_splits, one warp per head:
-    // the same arithmetic, in the same order, as tq_attn_merge_kernel (attention_tq.cu) ----
-    if (p.n_splits > 1) cluster_sync(); else __syncthreads();
-    const uint32_t ml_a = smem_u32(ml_s), cp_a = smem_u32(cpart);
-    for (int h = (int)split + (int)p.n_splits * warp; h < gvalid; h += (int)p.n_splits * NW) {
-        float gmax = -INFINITY;
-        for (uint32_t sp = 0; sp < p.n_splits; sp++) gmax = fmaxf(gmax, ld_cluster_f32(ml_a + (2 * h) * 4, sp, p.n_splits > 1));
-        float gsum = 0.f, ov[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) ov[i] = 0.f;
-        for (uint32_t sp = 0; sp < p.n_splits; sp++) {
-            const float ms = ld_cluster_f32(ml_a + (2 * h) * 4, sp, p.n_splits > 1);
-            const float ls = ld_cluster_f32(ml_a + (2 * h + 1) * 4, sp, p.n_splits > 1);
-            const float f = (ms == -INFINITY) ? 0.f : expf(ms - gmax);
-            gsum += f * ls;
-            const float4 a0 = ld_cluster_f4(cp_a + (h * HD + 8 * lane) * 4, sp, p.n_splits > 1);
-            const float4 a1 = ld_cluster_f4(cp_a + (h * HD + 8 * lane + 4) * 4, sp, p.n_splits > 1);
-            ov[0] += f * a0.x; ov[1] += f * a0.y; ov[2] += f * a0.z; ov[3] += f * a0.w;
-            ov[4] += f * a1.x; ov[5] += f * a1.y; ov[6] += f * a1.z; ov[7] += f * a1.w;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++) ov[i] = gsum > 0.f ? ov[i] / gsum : 0.f;
-        const size_t qh = (size_t)lane_idx * p.n_q + qh0 + h;
-        if (!p.fused_q) {
-            *reinterpret_cast<float4 *>(p.out + qh * HD + 8 * lane) = make_float4(ov[0], ov[1], ov[2], ov[3]);
-            *reinterpret_cast<float4 *>(p.out + qh * HD + 8 * lane + 4) = make_float4(ov[4], ov[5], ov[6], ov[7]);
+            if (!p.direct_out && threadIdx.x < gvalid)
+                *reinterpret_cast<float2 *>(part_of(threadIdx.x, it_split)) = make_float2(ml_s[2 * threadIdx.x], ml_s[2 * threadIdx.x + 1]);
             continue;
         }
-        // inverse rotation: Walsh-Hadamard butterflies (strides 1, 2, 4 in the thread, 8..128 across lanes), 1/sqrt(d), signs
+        // The splits of this (lane, kv head) are one cluster: head h is finished by CTA h mod n_splits.
+        if (p.n_splits > 1) cluster_sync();
+        // One warp per head: the same arithmetic, in the same order, as tq_attn_merge_kernel (attention_tq.cu).
+        const bool clustered = p.n_splits > 1;
+        const uint32_t ml_a = smem_u32(ml_s), cp_a = smem_u32(cpart);
+        for (int h = (int)it_split + (int)p.n_splits * warp; h < gvalid; h += (int)p.n_splits * NW) {
+            float gmax = -INFINITY;
+            for (uint32_t sp = 0; sp < p.n_splits; sp++) gmax = fmaxf(gmax, ld_cluster_f32(ml_a + (2 * h) * 4, sp, clustered));
+            float gsum = 0.f, ov[DPL];
 #pragma unroll
-        for (int len = 1; len < 8; len <<= 1) {
+            for (int i = 0; i < DPL; i++) ov[i] = 0.f;
+            for (uint32_t sp = 0; sp < p.n_splits; sp++) {
+                const float ms = ld_cluster_f32(ml_a + (2 * h) * 4, sp, clustered);
+                const float ls = ld_cluster_f32(ml_a + (2 * h + 1) * 4, sp, clustered);
+                const float f = (ms == -INFINITY) ? 0.f : expf(ms - gmax);
+                gsum += f * ls;
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                if (!(i & len)) {
-                    const float a = ov[i], b2 = ov[i + len];
-                    ov[i] = a + b2;
-                    ov[i + len] = a - b2;
+                for (int i = 0; i < DPL; i += 4) {
+                    const float4 a = ld_cluster_f4(cp_a + C::cp_index(h, DPL * lane + i) * 4, sp, clustered);
+                    ov[i] += f * a.x; ov[i + 1] += f * a.y; ov[i + 2] += f * a.z; ov[i + 3] += f * a.w;
                 }
             }
-        }
 #pragma unroll
-        for (int m = 1; m < 32; m <<= 1) {
-            const bool upper = lane & m;
+            for (int i = 0; i < DPL; i++) ov[i] = gsum > 0.f ? ov[i] / gsum : 0.f;
+            const size_t qh = (size_t)it_lane * p.n_q + qh0 + h;
+            if (!p.fused_q) {
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const float o2 = __shfl_xor_sync(0xffffffffu, ov[i], m);
-                ov[i] = upper ? o2 - ov[i] : ov[i] + o2;
+                for (int i = 0; i < DPL; i += 4)
+                    *reinterpret_cast<float4 *>(p.out + qh * HD + DPL * lane + i) = make_float4(ov[i], ov[i + 1], ov[i + 2], ov[i + 3]);
+                continue;
+            }
+            // inverse rotation, 1/sqrt(d), signs
+            warp_fwht<DPL>(ov, lane);
+            const float inv = 1.0f / sqrtf((float)HD);
+#pragma unroll
+            for (int i = 0; i < DPL; i += 4) {
+                const float4 sg = *reinterpret_cast<const float4 *>(p.signs + DPL * lane + i);
+                uint2 packed;
+                packed.x = pack_h2(ov[i] * inv * sg.x, ov[i + 1] * inv * sg.y);
+                packed.y = pack_h2(ov[i + 2] * inv * sg.z, ov[i + 3] * inv * sg.w);
+                *reinterpret_cast<uint2 *>(p.out_f16 + qh * HD + DPL * lane + i) = packed;
             }
         }
-        const float4 s0 = *reinterpret_cast<const float4 *>(p.signs + 8 * lane);
-        const float4 s1 = *reinterpret_cast<const float4 *>(p.signs + 8 * lane + 4);
-        const float sg[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-        const float inv = 1.0f / sqrtf((float)HD);
-        uint4 packed;
-        __half2 *hp = reinterpret_cast<__half2 *>(&packed);
-#pragma unroll
-        for (int i = 0; i < 4; i++) hp[i] = __floats2half2_rn(ov[2 * i] * inv * sg[2 * i], ov[2 * i + 1] * inv * sg[2 * i + 1]);
-        *reinterpret_cast<uint4 *>(p.out_f16 + qh * HD + 8 * lane) = packed;
+        if (p.n_splits > 1) cluster_sync();   // no CTA leaves while a peer may still read its shared memory
     }
-    if (p.n_splits > 1) cluster_sync();   // no CTA leaves while a peer may still read its shared memory
 }
 
-}  // namespace
-
-int lc_tq2_attn_mma_launch(lc_batch *b, const TqAttnParams &p, dim3 grid) {
-    const size_t smem = SMEM_BYTES;
+template <typename C>
+int launch(lc_batch *b, const TqAttnParams &p, dim3 grid) {
     static lc_smem_optin optin;
-    LC_CUDA_TRY(lc_ensure_smem(tq2_attn_mma_kernel, optin, b->ctx, smem));
+    LC_CUDA_TRY(lc_ensure_smem(tq_attn_mma_kernel<C>, optin, b->ctx, C::SMEM));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = smem;
+    cfg.blockDim = dim3(C::NT);
+    cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = b->stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
@@ -620,7 +845,28 @@ int lc_tq2_attn_mma_launch(lc_batch *b, const TqAttnParams &p, dim3 grid) {
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    LC_LAUNCH_CHECKED(cudaLaunchKernelEx(&cfg, tq2_attn_mma_kernel, p));
+    LC_LAUNCH_CHECKED(cudaLaunchKernelEx(&cfg, tq_attn_mma_kernel<C>, p));
     b->dispatch_count++;
     return LC_OK;
+}
+
+template <int HD>
+int launch_bits(lc_batch *b, const TqAttnParams &p, dim3 grid, uint32_t bits) {
+    switch (bits) {
+        case 2: return launch<AttnCfg<HD, 2>>(b, p, grid);
+        case 3: return launch<AttnCfg<HD, 3>>(b, p, grid);
+        default: return launch<AttnCfg<HD, 4>>(b, p, grid);
+    }
+}
+
+}  // namespace
+
+bool lc_tq_attn_mma_supported(uint32_t hd, uint32_t bits) { return (hd == 128 || hd == 256 || hd == 512) && bits >= 2 && bits <= 4; }
+
+int lc_tq_attn_mma_launch(lc_batch *b, const TqAttnParams &p, dim3 grid, uint32_t hd, uint32_t bits) {
+    switch (hd) {
+        case 128: return launch_bits<128>(b, p, grid, bits);
+        case 256: return launch_bits<256>(b, p, grid, bits);
+        default: return launch_bits<512>(b, p, grid, bits);
+    }
 }
