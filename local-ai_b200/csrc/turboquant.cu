@@ -298,6 +298,29 @@ int rotate_into(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *inpu
     return LC_OK;
 }
 
+// One Lloyd-Max sweep: every grid cell adds to the first nearest level.  Cells and levels both ascend, so the nearest
+// level only moves up from cell to cell.
+#define LLOYD_SWEEP_BODY                                                                                            \
+    uint32_t best = 0;                                                                                              \
+    float s = 0.f, w = 0.f;                                                                                         \
+    for (int i = 0; i < n; i++) {                                                                                   \
+        while (best + 1 < k && fabsf(xs[i] - levels[best + 1]) < fabsf(xs[i] - levels[best])) {                     \
+            sum[best] = s;                                                                                          \
+            wsum[best] = w;                                                                                         \
+            s = w = 0.f;                                                                                            \
+            best++;                                                                                                 \
+        }                                                                                                           \
+        s = __builtin_fmaf(pdf[i], xs[i], s);                                                                       \
+        w += pdf[i];                                                                                                \
+    }                                                                                                               \
+    sum[best] = s;                                                                                                  \
+    wsum[best] = w;
+void lloyd_sweep(const float *xs, const float *pdf, int n, const float *levels, uint32_t k, float *sum, float *wsum) { LLOYD_SWEEP_BODY }
+#if defined(__x86_64__)
+__attribute__((target("fma"))) void lloyd_sweep_fma(const float *xs, const float *pdf, int n, const float *levels, uint32_t k,
+                                                    float *sum, float *wsum) { LLOYD_SWEEP_BODY }
+#endif
+
 }  // namespace
 
 extern "C" {
@@ -336,18 +359,14 @@ int lc_tq_levels(uint32_t dim, uint32_t bits, float *levels) {
     }
     for (uint32_t i = 0; i < k; i++) levels[i] = 6.0f * ((((float)i + 0.5f) / (float)k) - 0.5f);
     float sum[16], wsum[16];
+    // (hardware multiply-adds where the host has them: the library call rounds the same and takes four times as long)
+    void (*sweep)(const float *, const float *, int, const float *, uint32_t, float *, float *) = lloyd_sweep;
+#if defined(__x86_64__)
+    if (__builtin_cpu_supports("fma")) sweep = lloyd_sweep_fma;
+#endif
     for (int it = 0; it < 100; it++) {
         for (uint32_t j = 0; j < k; j++) sum[j] = wsum[j] = 0.f;
-        for (int i = 0; i < N; i++) {
-            uint32_t best = 0;
-            float bd = INFINITY;
-            for (uint32_t j = 0; j < k; j++) {
-                const float d = fabsf(xs[i] - levels[j]);
-                if (d < bd) { bd = d; best = j; }
-            }
-            sum[best] = fmaf(pdf[i], xs[i], sum[best]);
-            wsum[best] += pdf[i];
-        }
+        sweep(xs, pdf, N, levels, k, sum, wsum);
         for (uint32_t j = 0; j < k; j++)
             if (wsum[j] > 1e-12f) levels[j] = sum[j] / wsum[j];
     }
