@@ -9,6 +9,7 @@ computes on the CPU.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import re
 from pathlib import Path
 
@@ -62,6 +63,17 @@ def parse_header(path: Path = HEADER) -> dict[str, tuple]:
 
 _lib = None
 _decls = None
+_fast = None
+
+
+def fastcall():
+    """The generated CPython extension (fastcall.py): handles and calls without ctypes.  `load` binds its functions."""
+    global _fast
+    if _fast is None:
+        spec = importlib.util.spec_from_file_location("_fastcall", build.build_fastcall())
+        _fast = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_fast)
+    return _fast
 
 
 def declarations() -> dict[str, tuple]:

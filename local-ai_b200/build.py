@@ -3,15 +3,18 @@
 The library is rebuilt when the hash of its sources (csrc/*.cu, csrc/*.h,
 include/local_cuda.h) differs from the hash recorded beside the built file,
 so a stale binary is never loaded.  Each .cu is compiled to an object file in
-parallel, then linked.
+parallel, then linked.  The CPython extension of fastcall.py (the argument
+conversion of the Python mirror) is generated from the header and built beside it.
 """
 from __future__ import annotations
 
 import hashlib
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -21,6 +24,8 @@ CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "liblocal_cuda.so"
 HASH = PKG / "liblocal_cuda.build_hash"
+FAST = PKG / ("_fastcall" + sysconfig.get_config_var("EXT_SUFFIX"))
+FAST_HASH = PKG / "_fastcall.build_hash"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -54,8 +59,39 @@ def find_nvcc() -> str | None:
     return None
 
 
+def fastcall_hash() -> str:
+    h = hashlib.sha256(FAST.name.encode())
+    for f in (PKG / "fastcall.py", ROOT / "include" / "local_cuda.h"):
+        h.update(f.read_bytes())
+    return h.hexdigest()
+
+
+def build_fastcall(force: bool = False) -> Path:
+    """Generate and compile the CPython extension for the running interpreter."""
+    if not force and FAST.exists() and FAST_HASH.exists() and FAST_HASH.read_text().strip() == fastcall_hash():
+        return FAST
+    spec = importlib.util.spec_from_file_location("local_ai_b200_fastcall_gen", PKG / "fastcall.py")
+    gen = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(gen)
+    OBJ.mkdir(exist_ok=True)
+    src = OBJ / "_fastcall.c"
+    src.write_text(gen.generate(ROOT / "include" / "local_cuda.h"))
+    cc = shutil.which("gcc") or shutil.which("cc")
+    if cc is None:
+        raise RuntimeError("no C compiler: cannot build the _fastcall extension")
+    cmd = [cc, "-O2", "-std=gnu11", "-shared", "-fPIC", "-fvisibility=hidden", f"-I{sysconfig.get_paths()['include']}",
+           f"-I{ROOT / 'include'}", str(src), "-o", str(FAST)]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(f"$ {' '.join(cmd)}\n{r.stdout}{r.stderr}")
+        raise RuntimeError("gcc failed on the _fastcall extension")
+    FAST_HASH.write_text(fastcall_hash() + "\n")
+    return FAST
+
+
 def build_library(force: bool = False, verbose: bool = False, extra_flags: list[str] | None = None) -> Path:
-    """Compile every CUDA source for sm_100a and link the shared library."""
+    """Compile every CUDA source for sm_100a, link the shared library, build the CPython extension."""
+    build_fastcall(force)
     if not force and is_current():
         return LIB
     nvcc = find_nvcc()

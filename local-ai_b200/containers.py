@@ -8,16 +8,15 @@ import ctypes as C
 
 import numpy as np
 
-from . import _lib
-from .kernels import CommandBatch, CudaBuffer, CudaContext, Kernels, _check
+from .kernels import CommandBatch, CudaBuffer, CudaContext, Handle, Kernels, _check, _fast, _load
 
 STOP_REASONS = {0: None, 1: "Eos", 2: "MaxTokens", 3: "Capacity"}
 
 
-class QuantizedKvCache:
+class QuantizedKvCache(Handle):
     def __init__(self, ctx: CudaContext, n_kv_heads: int, head_dim: int, max_positions: int,
                  physical_positions: int | None = None, sliding_window: int = 0, bits: int = 2):
-        self._lib, self.ctx = _lib.load(), ctx
+        self._lib, self.ctx = _load(), ctx
         h = C.c_void_p()
         phys = max_positions if physical_positions is None else physical_positions
         _check(self._lib.lc_kv_cache_create(ctx._h, n_kv_heads, head_dim, max_positions, phys, sliding_window, bits, C.byref(h)))
@@ -51,16 +50,16 @@ class QuantizedKvCache:
 
     def write_kv_gpu_into(self, batch: CommandBatch, kernels: Kernels, k_src: CudaBuffer, v_src: CudaBuffer, position: int,
                           n_rows: int) -> None:
-        _check(self._lib.lc_kv_cache_write_kv_gpu_into(self._h, batch._h, kernels._h, k_src._h, v_src._h, position, n_rows))
+        _fast.lc_kv_cache_write_kv_gpu_into(self, batch, kernels, k_src, v_src, position, n_rows)
 
     def fused_attention_into(self, batch, kernels, q, attn_out, seq_len, current_pos, n_q_heads, window, softmax_scale=1.0):
-        _check(self._lib.lc_kv_cache_fused_attention_into(self._h, batch._h, kernels._h, q._h, attn_out._h, seq_len, current_pos,
-                                                          n_q_heads, window, softmax_scale))
+        _fast.lc_kv_cache_fused_attention_into(self, batch, kernels, q, attn_out, seq_len, current_pos, n_q_heads, window,
+                                               softmax_scale)
 
     def fused_attention_batch_into(self, batch, kernels, q, attn_out, kv_len, start_pos, n_rows, n_q_heads, window,
                                    softmax_scale=1.0):
-        _check(self._lib.lc_kv_cache_fused_attention_batch_into(self._h, batch._h, kernels._h, q._h, attn_out._h, kv_len,
-                                                                start_pos, n_rows, n_q_heads, window, softmax_scale))
+        _fast.lc_kv_cache_fused_attention_batch_into(self, batch, kernels, q, attn_out, kv_len, start_pos, n_rows, n_q_heads,
+                                                     window, softmax_scale)
 
     def max_snapshot_positions(self) -> int:
         return self._lib.lc_kv_cache_max_snapshot_positions(self._h)
@@ -85,11 +84,11 @@ class QuantizedKvCache:
             self._h = None
 
 
-class LaneScheduler:
+class LaneScheduler(Handle):
     """Continuous batching over the lanes of a DecodeModel (or host logic only, with model=None)."""
 
     def __init__(self, model, n_lanes: int, lane_capacity: int, eos_token: int):
-        self._lib = _lib.load()
+        self._lib = _load()
         h = C.c_void_p()
         _check(self._lib.lc_lane_sched_create(model._h if model is not None else None, n_lanes, lane_capacity, eos_token, C.byref(h)))
         self._h, self.n_lanes = h, n_lanes

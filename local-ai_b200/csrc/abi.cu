@@ -5,6 +5,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <mutex>
 
 #include "lc_internal.h"
 
@@ -20,6 +21,56 @@ int lc_fail(int code, const char *fmt, ...) {
     return code;
 }
 void lc_clear_error() { g_last_error.clear(); }
+
+// Completion events of lc_batch_commit_async, kept for the next batch: creating and destroying one costs as much as
+// recording it.  One pool per device, at most POOLED_EVENTS events, emptied when the device's last context goes.
+namespace {
+constexpr size_t POOLED_EVENTS = 64;
+struct EventPool {
+    std::mutex mutex;
+    std::vector<cudaEvent_t> events;
+    int contexts = 0;
+};
+EventPool g_events[LC_MAX_DEVICES];
+EventPool *event_pool(int device) { return device >= 0 && device < LC_MAX_DEVICES ? &g_events[device] : nullptr; }
+cudaError_t take_event(int device, cudaEvent_t *ev) {
+    if (EventPool *p = event_pool(device)) {
+        std::lock_guard<std::mutex> lock(p->mutex);
+        if (!p->events.empty()) {
+            *ev = p->events.back();
+            p->events.pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+}
+void return_event(int device, cudaEvent_t ev) {
+    if (EventPool *p = event_pool(device)) {
+        std::lock_guard<std::mutex> lock(p->mutex);
+        if (p->contexts > 0 && p->events.size() < POOLED_EVENTS) {
+            p->events.push_back(ev);
+            return;
+        }
+    }
+    cudaEventDestroy(ev);
+}
+void count_context(int device, int by) {
+    if (EventPool *p = event_pool(device)) {
+        std::lock_guard<std::mutex> lock(p->mutex);
+        p->contexts += by;
+        if (p->contexts == 0) {
+            for (cudaEvent_t e : p->events) cudaEventDestroy(e);
+            p->events.clear();
+        }
+    }
+}
+// make `device` current; reading the current device is cheaper than setting it
+cudaError_t use_device(int device) {
+    int now = -1;
+    if (cudaGetDevice(&now) == cudaSuccess && now == device) return cudaSuccess;
+    return cudaSetDevice(device);
+}
+}  // namespace
 
 extern "C" {
 
@@ -75,6 +126,7 @@ int lc_ctx_create(int device, lc_ctx **out) {
     cudaMemGetInfo(&fr, &tot);
     c->total_mem = tot;
     { const char *e = getenv("LOCAL_CUDA_PDL"); c->pdl = !(e && strcmp(e, "0") == 0); }
+    count_context(device, 1);
     *out = c;
     return LC_OK;
 }
@@ -86,6 +138,7 @@ void lc_ctx_destroy(lc_ctx *ctx) {
         cudaStreamSynchronize(ctx->stream);
         cudaStreamDestroy(ctx->stream);
     }
+    count_context(ctx->device, -1);
     delete ctx;
 }
 
@@ -220,7 +273,7 @@ int lc_buf_fill(lc_buf *buf, size_t offset, size_t bytes, int value) {
 // ------------------------------------------------------------------ batch --
 int lc_batch_begin(lc_ctx *ctx, lc_batch **out) {
     if (!ctx || !out) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_batch_begin: NULL argument");
-    LC_CUDA_TRY(cudaSetDevice(ctx->device));
+    LC_CUDA_TRY(use_device(ctx->device));
     lc_batch *b = new lc_batch();
     b->ctx = ctx;
     b->stream = ctx->stream;
@@ -282,8 +335,8 @@ int lc_batch_commit_async(lc_batch *batch, lc_pending **out) {
     if (batch->capturing)
         return lc_fail(LC_ERR_INVALID_ARGUMENT, "batch is capturing: use lc_batch_end_capture");
     lc_pending *p = new lc_pending();
-    p->ctx = batch->ctx;
-    cudaError_t e = cudaEventCreateWithFlags(&p->ev, cudaEventDisableTiming);
+    p->device = batch->ctx->device;
+    cudaError_t e = take_event(p->device, &p->ev);
     if (e == cudaSuccess) e = cudaEventRecord(p->ev, batch->stream);
     delete batch;
     if (e != cudaSuccess) {
@@ -298,7 +351,7 @@ int lc_batch_commit_async(lc_batch *batch, lc_pending **out) {
 int lc_pending_wait(lc_pending *pending) {
     if (!pending) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_pending_wait: pending is NULL");
     cudaError_t e = cudaEventSynchronize(pending->ev);
-    cudaEventDestroy(pending->ev);
+    return_event(pending->device, pending->ev);
     delete pending;
     if (e != cudaSuccess) return lc_fail(LC_ERR_COMMAND_BUFFER, "%s", cudaGetErrorString(e));
     return LC_OK;

@@ -18,6 +18,11 @@
 
 constexpr uint32_t LC_MAX_PREFILL_CHUNK = 256;   // quant_cache.rs:42-46: rows one multi-row write may add
 
+// turboquant.cu
+int lc_encode_kv_pair(lc_kernels *k, lc_batch *b, const lc_buf *k_in, const lc_buf *v_in, const lc_buf *levels, const lc_buf *signs,
+                      lc_buf *k_packed, lc_buf *k_norms, lc_buf *v_packed, lc_buf *v_norms, uint32_t head_dim, uint32_t n_kv_heads,
+                      uint32_t num_tokens, uint32_t bits, uint32_t position, uint32_t ring_capacity);
+
 struct lc_kv_cache {
     lc_ctx *ctx = nullptr;
     lc_buf *keys_q = nullptr, *values_q = nullptr, *key_norms = nullptr, *value_norms = nullptr;
@@ -123,11 +128,8 @@ int lc_kv_cache_write_kv_gpu_into(lc_kv_cache *c, lc_batch *b, lc_kernels *k, co
         return lc_fail(LC_ERR_INVALID_ARGUMENT, "KV write [%u..%llu) exceeds capacity %u", position,
                        (unsigned long long)position + n_rows, c->max_positions);
     const uint32_t ring = ring_of(c);
-    int st = lc_encode_kv_turboquant_into(k, b, k_src, c->levels, c->signs, c->keys_q, c->key_norms, c->head_dim, c->n_kv_heads,
-                                          n_rows, c->bits, position, ring);
-    if (st != LC_OK) return st;
-    return lc_encode_kv_turboquant_into(k, b, v_src, c->levels, c->signs, c->values_q, c->value_norms, c->head_dim,
-                                        c->n_kv_heads, n_rows, c->bits, position, ring);
+    return lc_encode_kv_pair(k, b, k_src, v_src, c->levels, c->signs, c->keys_q, c->key_norms, c->values_q, c->value_norms, c->head_dim,
+                             c->n_kv_heads, n_rows, c->bits, position, ring);
 }
 
 // QuantizedKvCache::fused_attention_into (quant_cache.rs:548-598): rotate, attend over codes, rotate back, as one

@@ -34,7 +34,7 @@ struct lc_batch {
 };
 
 struct lc_pending {
-    lc_ctx *ctx = nullptr;
+    int device = 0;   // not the context: a pending batch may outlive it
     cudaEvent_t ev = nullptr;
 };
 

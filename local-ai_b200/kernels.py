@@ -10,7 +10,9 @@ reference's enum case (`InvalidArgument`, `BufferAllocation`, ...).
 
 Every `Kernels` method is generated from the C header: `lc_<name>(kernels,
 ...)` becomes `Kernels.<name>(...)`.  Buffers, batches and contexts are passed
-as the wrapper objects; scalars as Python numbers.
+as the wrapper objects; scalars as Python numbers.  The calls a program makes
+per token (begin, enqueue, commit, wait, graph launch) go through the generated
+extension of fastcall.py; set-up calls use ctypes.
 """
 from __future__ import annotations
 
@@ -31,25 +33,36 @@ class Error(RuntimeError):
         super().__init__(f"{self.kind}: {message}")
 
 
+def _error(status: int) -> Error:
+    return Error(status, _lib.load().lc_last_error().decode())
+
+
 def _check(status: int) -> None:
     if status != 0:
-        raise Error(status, _lib.load().lc_last_error().decode())
+        raise _error(status)
 
 
-def _handle(x):
-    if x is None:
-        return None
-    h = getattr(x, "_h", None)
-    if h is None:
-        raise TypeError(f"expected a local-cuda object, got {type(x).__name__}")
-    return h
+_fast = _lib.fastcall()
+Handle = _fast.Handle
 
 
-class CudaContext:
+def _load():
+    """The library, with the extension's calls bound to it."""
+    lib = _lib.load()
+    if not _load.bound:
+        _fast.bind({n: C.cast(getattr(lib, n), C.c_void_p).value for n in _lib.declarations()}, _error)
+        _load.bound = True
+    return lib
+
+
+_load.bound = False
+
+
+class CudaContext(Handle):
     """MetalContext: one device, one in-order stream."""
 
     def __init__(self, device: int = 0):
-        self._lib = _lib.load()
+        self._lib = _load()
         h = C.c_void_p()
         _check(self._lib.lc_ctx_create(device, C.byref(h)))
         self._h = h
@@ -68,8 +81,7 @@ class CudaContext:
     def stream(self) -> int:
         return self._lib.lc_ctx_stream(self._h) or 0
 
-    def synchronize(self) -> None:
-        _check(self._lib.lc_ctx_synchronize(self._h))
+    synchronize = _fast.method(_fast.lc_ctx_synchronize)
 
     def close(self) -> None:
         if self._h:
@@ -77,7 +89,7 @@ class CudaContext:
             self._h = None
 
 
-class CudaBuffer:
+class CudaBuffer(Handle):
     """MetalBuffer.  Device memory; the CPU sees it through explicit copies."""
 
     def __init__(self, ctx: CudaContext, handle, nbytes: int):
@@ -137,23 +149,20 @@ class CudaBuffer:
             self._h = None
 
 
-class PendingCommandBuffer:
-    def __init__(self, lib, handle):
-        self._lib, self._h = lib, handle
+class PendingCommandBuffer(Handle):
+    __slots__ = ()
 
-    def wait(self) -> None:
-        h, self._h = self._h, None
-        _check(self._lib.lc_pending_wait(h))
+    def wait(self, _wait=_fast.lc_pending_wait, _take=_fast.take) -> None:   # (bound early: callable at interpreter exit)
+        _wait(_take(self))
 
 
-class CudaGraph:
+class CudaGraph(Handle):
     """A captured batch that can be replayed (no twin in the reference)."""
 
     def __init__(self, lib, handle):
         self._lib, self._h = lib, handle
 
-    def launch(self) -> None:
-        _check(self._lib.lc_graph_launch(self._h))
+    launch = _fast.method(_fast.lc_graph_launch)
 
     def destroy(self) -> None:
         if self._h:
@@ -161,15 +170,19 @@ class CudaGraph:
             self._h = None
 
 
-class CommandBatch:
+class CommandBatch(Handle):
     """CommandBatch: dispatches run in encode order on the context's stream."""
+
+    __slots__ = ("_lib", "_ctx")
 
     def __init__(self, ctx: CudaContext, capture: bool = False):
         self._lib = ctx._lib
         self._ctx = ctx
+        if not capture:
+            _fast.begin(self, ctx)
+            return
         h = C.c_void_p()
-        fn = self._lib.lc_batch_begin_capture if capture else self._lib.lc_batch_begin
-        _check(fn(ctx._h, C.byref(h)))
+        _check(self._lib.lc_batch_begin_capture(ctx._h, C.byref(h)))
         self._h = h
 
     @classmethod
@@ -184,23 +197,21 @@ class CommandBatch:
         return self._lib.lc_batch_dispatch_count(self._h)
 
     def blit_buffer_copy(self, src: CudaBuffer, src_off: int, dst: CudaBuffer, dst_off: int, nbytes: int) -> None:
-        _check(self._lib.lc_batch_copy(self._h, src._h, src_off, dst._h, dst_off, nbytes))
+        _fast.lc_batch_copy(self, src, src_off, dst, dst_off, nbytes)
 
     def upload(self, dst: CudaBuffer, dst_off: int, host_ptr: int, nbytes: int) -> None:
-        _check(self._lib.lc_batch_upload(self._h, dst._h, dst_off, host_ptr, nbytes))
+        _fast.lc_batch_upload(self, dst, dst_off, host_ptr, nbytes)
 
     def download(self, src: CudaBuffer, src_off: int, host_ptr: int, nbytes: int) -> None:
-        _check(self._lib.lc_batch_download(self._h, src._h, src_off, host_ptr, nbytes))
+        _fast.lc_batch_download(self, src, src_off, host_ptr, nbytes)
 
     def commit_and_wait(self) -> None:
-        h, self._h = self._h, None
-        _check(self._lib.lc_batch_commit_and_wait(h))
+        _fast.lc_batch_commit_and_wait(_fast.take(self))
 
     def commit_async(self) -> PendingCommandBuffer:
-        h, self._h = self._h, None
-        p = C.c_void_p()
-        _check(self._lib.lc_batch_commit_async(h, C.byref(p)))
-        return PendingCommandBuffer(self._lib, p)
+        p = PendingCommandBuffer()
+        _fast.commit(self, p)
+        return p
 
     def end_capture(self) -> CudaGraph:
         h, self._h = self._h, None
@@ -213,7 +224,7 @@ class PinnedHost:
     """Page-locked host array for asynchronous copies."""
 
     def __init__(self, nbytes: int, dtype=np.uint8):
-        self._lib = _lib.load()
+        self._lib = _load()
         p = C.c_void_p()
         _check(self._lib.lc_host_alloc(nbytes, C.byref(p)))
         self.ptr = p.value
@@ -228,7 +239,7 @@ class PinnedHost:
             self.ptr = None
 
 
-class Kernels:
+class Kernels(Handle):
     """Kernels (local-metal/src/kernels.rs): one method per dispatcher."""
 
     def __init__(self, ctx: CudaContext):
@@ -248,7 +259,7 @@ class Kernels:
             self._h = None
 
 
-class Communicator:
+class Communicator(Handle):
     """NCCL behind the C ABI (lc_comm_*): one communicator per process / GPU.  `unique_id()` runs on one rank; the
     host carries the bytes to the others (a file, a socket, an existing process group); every rank then constructs
     its Communicator (collective)."""
@@ -257,7 +268,7 @@ class Communicator:
 
     @staticmethod
     def available() -> bool:
-        return _lib.load().lc_comm_available() == 0
+        return _load().lc_comm_available() == 0
 
     @staticmethod
     def unique_id() -> bytes:
@@ -284,33 +295,12 @@ class Communicator:
             self._h = None
 
 
-def _make_method(cname: str, restype, argnames):
-    def method(self, *args):
-        if len(args) != len(argnames) - 1:
-            raise TypeError(f"{cname[3:]}() takes {len(argnames) - 1} arguments ({', '.join(argnames[1:])}), got {len(args)}")
-        conv = []
-        for a in args:
-            if isinstance(a, (list, tuple)):   # an array of handles (const lc_buf *const *)
-                conv.append((C.c_void_p * len(a))(*[x._h for x in a]))
-            else:
-                conv.append(a._h if hasattr(a, "_h") else a)
-        r = getattr(self._lib, cname)(self._h, *conv)
-        if restype is C.c_int:
-            _check(r)
-            return None
-        return r
-
-    method.__name__ = cname[3:]
-    method.__doc__ = f"{cname}({', '.join(argnames)}) from include/local_cuda.h"
-    return method
-
-
 def _install_kernel_methods() -> None:
     skip = {"lc_kernels_create", "lc_kernels_destroy"}
-    for cname, (restype, argtypes, argnames) in _lib.declarations().items():
+    for cname, (_, _, argnames) in _lib.declarations().items():
         if cname in skip or not argnames or argnames[0] != "k":
             continue
-        setattr(Kernels, cname[3:], _make_method(cname, restype, argnames))
+        setattr(Kernels, cname[3:], _fast.method(getattr(_fast, cname)))
 
 
 _install_kernel_methods()
@@ -345,6 +335,6 @@ def tq_attention_noalloc_into(batch: CommandBatch, q, k_codes, k_norms, v_codes,
                               softmax_scale) -> None:
     """lc_tq_attention_noalloc_into: fused code-space attention whose split-K scratch is a fixed
     array inside the library, for callers that cannot allocate device memory (no `Kernels` needed)."""
-    _check(_lib.load().lc_tq_attention_noalloc_into(
-        batch._h, q._h, k_codes._h, k_norms._h, v_codes._h, v_norms._h, levels._h, signs._h, attn_out._h,
-        head_dim, kv_len, current_pos, num_q_heads, num_kv_heads, window, bits, ring_capacity, softmax_scale))
+    _fast.lc_tq_attention_noalloc_into(
+        batch, q, k_codes, k_norms, v_codes, v_norms, levels, signs, attn_out,
+        head_dim, kv_len, current_pos, num_q_heads, num_kv_heads, window, bits, ring_capacity, softmax_scale)

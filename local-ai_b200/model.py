@@ -9,8 +9,8 @@ from dataclasses import dataclass
 
 import numpy as np
 
-from . import _lib, synth
-from .kernels import CommandBatch, CudaBuffer, CudaContext, Kernels, _check
+from . import synth
+from .kernels import CommandBatch, CudaBuffer, CudaContext, Handle, Kernels, _check, _fast, _load
 
 
 class ModelConfig(C.Structure):
@@ -60,9 +60,9 @@ def synth_embedding(cfg: ModelConfig, seed: int = 0):
     return emb, fnorm
 
 
-class DecodeModel:
+class DecodeModel(Handle):
     def __init__(self, ctx: CudaContext, kernels: Kernels, cfg: ModelConfig):
-        self._lib = _lib.load()
+        self._lib = _load()
         self.ctx, self.kernels, self.cfg = ctx, kernels, cfg
         h = C.c_void_p()
         _check(self._lib.lc_model_create(ctx._h, kernels._h, C.addressof(cfg), C.byref(h)))
@@ -108,9 +108,7 @@ class DecodeModel:
 
     def decode_batch_step_into(self, batch: CommandBatch, tokens: CudaBuffer, positions: CudaBuffer, n_lanes: int,
                                want_logits: bool = True, next_tokens: CudaBuffer | None = None) -> None:
-        _check(self._lib.lc_model_decode_batch_step_into(self._h, batch._h, tokens._h, positions._h, n_lanes,
-                                                         1 if want_logits else 0,
-                                                         next_tokens._h if next_tokens is not None else None))
+        _fast.lc_model_decode_batch_step_into(self, batch, tokens, positions, n_lanes, 1 if want_logits else 0, next_tokens)
 
     def close(self) -> None:
         if self._h:
