@@ -35,6 +35,16 @@ int lc_qgemm_mma_grouped(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const
 int lc_qgemm_tcd_launch(lc_kernels *k, lc_batch *b, const lc_buf *input, int ng, const lc_buf *const *weights,
                         lc_buf *const *outputs, const uint32_t *ns, uint32_t m, uint32_t kk, bool geglu);
 
+// qmatmul_sm.cu: small-batch tensor-core kernel (both formats, f16 and f32 out, m <= 16); same return contract.
+int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng, const lc_buf *const *weights,
+                       lc_buf *const *outputs, const uint32_t *ns, uint32_t m, uint32_t kk, bool geglu);
+int lc_qgemv_mma_stream(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, const lc_buf *weight,
+                        lc_buf *output, uint32_t m, uint32_t kk, uint32_t n);
+constexpr uint32_t SM_MAX_M = 16;
+static bool small_batch_ok(const lc_kernels *k, int fmt, uint32_t m) {
+    return k->mma && k->decode_mma && m <= SM_MAX_M && (fmt == 0 || (k->decode_tc && m > k->small_m));
+}
+
 // qmatmul_tcv.cu: persistent tcgen05 kernel for very tall Q4_0 matrices (the vocabulary projection), f32 out, m <= 64;
 // same return contract.
 int lc_qgemm_tcv_launch(lc_kernels *k, lc_batch *b, const lc_buf *input, const lc_buf *weight, lc_buf *output, uint32_t m,
@@ -48,6 +58,14 @@ static int route(int fmt, bool f32out, const char *name, lc_kernels *k, lc_batch
     const lc_buf *ws[1] = {weight};
     lc_buf *os[1] = {output};
     const uint32_t ns[1] = {n};
+    if (small_batch_ok(k, fmt, m)) {
+        st = m <= 8 ? lc_qgemv_mma_stream(fmt, f32out, k, b, input, weight, output, m, kk, n) : -1;
+        if (st >= 0) return st;
+        if (!(k->vocab_tc && fmt == 0 && f32out && m > 8 && n >= 128u * (uint32_t)k->ctx->sm_count)) {   // (the vocabulary kernel's shapes)
+            st = lc_qgemm_sm_launch(fmt, f32out, k, b, input, 1, ws, os, ns, m, kk, false);
+            if (st >= 0) return st;
+        }
+    }
     if (k->mma && k->decode_tc && fmt == 1 && !f32out && m > k->small_m && m <= 64) {
         st = lc_qgemm_tcd_launch(k, b, input, 1, ws, os, ns, m, kk, false);
         if (st >= 0) return st;
@@ -100,6 +118,10 @@ int lc_matmul_nt_tq2_0_grouped(lc_kernels *k, lc_batch *b, const lc_buf *input, 
         int st = lc_check_qargs(1, "matmul_nt_tq2_0", k, b, weights[g], input, outputs[g], m, kk, ns[g], 2);
         if (st != LC_OK) return st;
     }
+    if (small_batch_ok(k, 1, m)) {
+        const int st = lc_qgemm_sm_launch(1, false, k, b, input, ng, weights, outputs, ns, m, kk, false);
+        if (st >= 0) return st;
+    }
     if (k->mma && k->decode_tc && m > k->small_m && m <= 64) {
         const int st = lc_qgemm_tcd_launch(k, b, input, ng, weights, outputs, ns, m, kk, false);
         if (st >= 0) return st;
@@ -140,6 +162,10 @@ int lc_matmul_nt_tq2_0_geglu_into(lc_kernels *k, lc_batch *b, const lc_buf *inpu
             const lc_buf *ws[2] = {w_gate, w_up};
             lc_buf *os[2] = {output, output};
             const uint32_t ns[2] = {n, n};
+            if (small_batch_ok(k, 1, m)) {
+                st = lc_qgemm_sm_launch(1, false, k, b, input, 2, ws, os, ns, m, kk, true);
+                if (st >= 0) return st;
+            }
             st = lc_qgemm_tcd_launch(k, b, input, 2, ws, os, ns, m, kk, true);
             if (st >= 0) return st;
         }

@@ -1,0 +1,377 @@
+// Small-batch quantized matmul C[m, n] = A[m, K] (f16) x W[n, K]^T, W in GGUF Q4_0 / TQ2_0 blocks, m <= 16: the projections
+// of one token or of a small decode batch (shaders/matvec_quant.metal:64-387 and the m <= 8 kernels at :389-577), alone, up
+// to three matrices on the same activations, or gate and up of a GeGLU pair (local-engine/src/layer.rs:825-838).
+//
+// Such a projection is a few megabytes that sit behind the kernel before it, so what counts is the chain after that kernel
+// has finished: read the activations, multiply, add up, store.  The chain here has no shared-memory staging of the
+// activations, no tensor memory and no exchange between CTAs:
+//   * a CTA owns 16 / 32 / 64 weight rows and all of K; its raw blocks come in by one bulk copy per row before the
+//     dependency wait, and the CTA is small enough that the next launch's CTAs become resident and fetch theirs meanwhile;
+//   * the twelve warps split K into 128-k steps: a warp reads its part of the activations straight into MMA fragments,
+//     16 bytes per lane, all of them in flight together; K is permuted so that a lane's weights come from the code bytes it
+//     holds and its activations are contiguous;
+//   * the warps' partial sums meet once in shared memory and are added in a fixed order.
+// Issue slots bound what is left, so the conversion of the weights is two instructions per two of them: codes masked in place
+// are f16 subnormals, q 4^l 2^-24 (TQ2_0, bit pair l of a byte) or q 16^l 2^-24 (Q4_0, nibble l), and one multiply-add makes
+// them (q - z) 2^-9, exactly and at one scale.  The operands are integers times a power of two; every block's sum is scaled by
+// d 2^9 in f32, the reference's d * sum((q - z) x).  (With a byte table and permutes, as the tcgen05 kernels decode, the
+// kernel issued twice the instructions and 8192 x 1536 at m = 1 took 6.1 us.  Leaving z to a sum of the activations saves
+// the multiply-add but cancels: twice the rounding error.)
+#include <stdlib.h>
+
+#include "lc_internal.h"
+#include "tcgen05_util.cuh"
+
+namespace {
+
+constexpr int FMT_Q4_0 = 0, FMT_TQ2_0 = 1;
+constexpr int SM_NW = 12, SM_NT = SM_NW * 32, SM_UNIT = 128;   // warps (each a part of K), threads, k per step of a warp
+constexpr int SM_GROUPS = 3;
+constexpr uint32_t SM_WAIT_LIMIT = 1u << 22;
+
+struct SmParams {
+    const uint8_t *w[SM_GROUPS];
+    void *out[SM_GROUPS];
+    int n[SM_GROUPS], tile_end[SM_GROUPS];
+    int ngroups;
+    const __half *x;
+    int m, K, nb;          // nb = blocks per weight row
+    int raw_rs;            // bytes reserved per row of raw blocks
+    int *status;
+    uint32_t wait_limit;
+    uint32_t extra_arrivals;   // 0; 1 in the expiry self-test
+};
+
+// gelu_tanh(gate) * up with gate and up rounded to f16 first, as the separate projections would store them, and the
+// element-wise kernel's arithmetic (shaders/gelu.metal:23-37)
+__device__ __forceinline__ float geglu_f(float gate, float up) {
+    const float x = __half2float(__float2half_rn(gate)), u = __half2float(__float2half_rn(up));
+    float inner = 0.7978845608f * (x + 0.044715f * (x * x * x));
+    inner = fminf(fmaxf(inner, -10.0f), 10.0f);
+    return 0.5f * x * (1.0f + tanhf(inner)) * u;
+}
+__device__ __forceinline__ void sm_store(__half *p, float v) { *p = __float2half_rn(v); }
+__device__ __forceinline__ void sm_store(float *p, float v) { *p = v; }
+__device__ __forceinline__ void sm_store2(__half *p, float2 v) { *reinterpret_cast<__half2 *>(p) = __floats2half2_rn(v.x, v.y); }
+__device__ __forceinline__ void sm_store2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
+__device__ __forceinline__ void sm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// N consecutive 32-bit words at a 2-byte aligned shared-memory address, the bytes of each in the order 0, 2, 1, 3: a mask
+// then pairs neighbouring codes in the halves of a register.
+template <int N>
+__device__ __forceinline__ void lds_codes(uint32_t a, uint32_t (&w)[N]) {
+    const uint32_t sel = (a & 2u) ? 0x5342u : 0x3120u, base = a & ~3u;
+    uint32_t r[N + 1];
+#pragma unroll
+    for (int i = 0; i <= N; i++) r[i] = lds32(base + 4 * i);
+#pragma unroll
+    for (int i = 0; i < N; i++) w[i] = __byte_perm(r[i], r[i + 1], sel);
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t a) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(v) : "r"(a));
+    return v;
+}
+
+// two codes, BITS wide at bit BITS * l of each half of w, as f16 (q - Z) 2^-9
+template <int BITS, int Z>
+__device__ __forceinline__ uint32_t codes_f16(uint32_t w, int l) {
+    constexpr uint32_t one = (1u << BITS) - 1u;
+    const uint32_t v = w & ((one | one << 16) << (BITS * l));      // q 2^(BITS l - 24)
+    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&v), __float2half2_rn((float)(1 << (15 - BITS * l))),
+                              __float2half2_rn(-(float)Z / 512.0f));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+
+// NT8: batch columns / 8.  MTW: 16-row tiles of the CTA (every warp works on all of them).  SINGLE: a warp has at most one
+// step, so a tile's sums go to shared memory at once and four tiles fit the registers of two CTAs per SM.
+template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT>
+__global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_kernel(const __grid_constant__ SmParams p) {
+    constexpr int BB = FMT == FMT_Q4_0 ? 18 : 66;
+    constexpr int ROWS = MTW * 16, OROWS = GEGLU ? ROWS / 2 : ROWS;
+    constexpr int RS = ROWS + 4;                // padded column of partial sums
+    lc_pdl_trigger();
+    extern __shared__ __align__(16) uint8_t smem[];
+    uint8_t *raw = smem;                                                       // [ROWS][raw_rs]
+    float *red = reinterpret_cast<float *>(smem + ROWS * p.raw_rs);            // [SM_NW][NT8 * 8][RS]
+    __shared__ __align__(8) uint64_t raw_full;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    int grp = 0;
+    if (!GEGLU)
+        while (grp + 1 < p.ngroups && (int)blockIdx.x >= p.tile_end[grp]) grp++;
+    const int n0 = ((int)blockIdx.x - (grp ? p.tile_end[grp - 1] : 0)) * OROWS;   // first output row
+    const int n_rows = p.n[grp];
+    const size_t rb = (size_t)p.nb * BB, w_bytes = rb * (size_t)n_rows;
+
+    // ---- before the dependency wait: the raw blocks (constant operands) ----
+    const uint32_t bar = smem_u32(&raw_full);
+    if (tid == 0) {
+        mbar_init(bar, ROWS + p.extra_arrivals);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    if (tid < ROWS) {
+        const int row = n0 + (GEGLU ? tid % OROWS : tid);
+        const uint8_t *wm = p.w[GEGLU ? tid / OROWS : grp];
+        bool counted = false;
+        if (row < n_rows) {
+            const size_t g0 = (size_t)row * rb, a0 = g0 & ~(size_t)15;
+            const uint32_t bytes = (uint32_t)(((g0 + rb - a0) + 15) & ~(size_t)15);
+            uint8_t *dst = raw + tid * p.raw_rs;
+            if (a0 + bytes <= w_bytes) {
+                mbar_arrive_expect_tx(bar, bytes);
+                bulk_g2s(smem_u32(dst), wm + a0, bytes, bar);
+                counted = true;
+            } else {   // the last bytes of the matrix: nothing is read past its end
+                for (uint32_t i = 0; i < bytes; i++) dst[i] = (a0 + i < w_bytes) ? wm[a0 + i] : 0;
+            }
+        }
+        if (!counted) mbar_arrive(bar);
+    }
+    // this lane's operand rows: 16 mt + g and + 8
+    auto row_at = [&](int mt, int h, bool &ok_) -> uint32_t {
+        const int r = mt * 16 + h * 8 + g, row = n0 + (GEGLU ? r % OROWS : r);
+        ok_ = row < n_rows;
+        return smem_u32(raw) + (uint32_t)(r * p.raw_rs) + (uint32_t)(((size_t)row * rb) & 15);
+    };
+    const int units = (p.K + SM_UNIT - 1) / SM_UNIT;
+    lc_pdl_wait();
+
+    // ---- activations of one step as B fragments.  TQ2_0: k = 32 l + 8t .. + 7 (l = 0..3), one 16-byte load each.
+    //      Q4_0: block l of the step, k = 32 l + 4t .. + 3 and 32 l + 16 + 4t .. + 3, two 8-byte loads. ----
+    uint4 xr[NT8][4];
+    auto load_x = [&](int u, uint4 (&x)[NT8][4]) {
+#pragma unroll
+        for (int nt = 0; nt < NT8; nt++) {
+            const int col = nt * 8 + g;
+            const __half *src = p.x + (size_t)col * p.K + (size_t)u * SM_UNIT;
+#pragma unroll
+            for (int l = 0; l < 4; l++) {
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (col < p.m && u < units && (FMT == FMT_TQ2_0 || u * 4 + l < p.nb)) {
+                    if (FMT == FMT_TQ2_0) {
+                        v = *reinterpret_cast<const uint4 *>(src + 32 * l + 8 * t);
+                    } else {
+                        const uint2 lo = *reinterpret_cast<const uint2 *>(src + 32 * l + 4 * t), hi = *reinterpret_cast<const uint2 *>(src + 32 * l + 16 + 4 * t);
+                        v = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                    }
+                }
+                x[nt][l] = v;
+            }
+        }
+    };
+    load_x(warp, xr);
+    bool ok;
+    {
+        uint32_t w = 1;
+        if (lane == 0) w = mbar_wait(bar, 0u, p.wait_limit) ? 1u : 0u;
+        ok = __shfl_sync(0xffffffffu, w, 0);
+    }
+    // acc += this step's part of rows 16 mt + g, + 8
+    auto step = [&](int u, int mt, const uint4 (&x)[NT8][4], float (&acc)[NT8][4]) {
+        bool rok[2];
+        const uint32_t ra[2] = {row_at(mt, 0, rok[0]), row_at(mt, 1, rok[1])};
+        if constexpr (FMT == FMT_TQ2_0) {
+            uint32_t cw[2][2], sh[2][2];
+            float d[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t a = ra[h] + (uint32_t)((u >> 1) * BB);
+                lds_codes<2>(a + (uint32_t)(32 * (u & 1) + 8 * t), cw[h]);
+                sh[h][0] = cw[h][0] >> 8;
+                sh[h][1] = cw[h][1] >> 8;
+                d[h] = rok[h] ? __half2float(__ushort_as_half((unsigned short)lds16(a + 64u))) * 512.0f : 0.f;
+            }
+            float c[2][NT8][4] = {};
+#pragma unroll
+            for (int l = 0; l < 4; l++) {
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const uint32_t a0 = codes_f16<2, 1>(cw[0][q], l), a1 = codes_f16<2, 1>(cw[1][q], l), a2 = codes_f16<2, 1>(sh[0][q], l),
+                                   a3 = codes_f16<2, 1>(sh[1][q], l);
+#pragma unroll
+                    for (int nt = 0; nt < NT8; nt++) sm_mma(c[q][nt], a0, a1, a2, a3, q ? x[nt][l].z : x[nt][l].x, q ? x[nt][l].w : x[nt][l].y);
+                }
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT8; nt++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) acc[nt][i] = fmaf(c[0][nt][i] + c[1][nt][i], d[i >> 1], acc[nt][i]);
+        } else {
+#pragma unroll
+            for (int l = 0; l < 4; l++) {
+                const int blk = u * 4 + l;
+                if (blk >= p.nb) break;
+                uint32_t cw[2], sh[2];
+                float d[2];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint32_t a = ra[h] + (uint32_t)(blk * BB);
+                    uint32_t w[1];
+                    lds_codes<1>(a + 2u + (uint32_t)(4 * t), w);
+                    cw[h] = w[0];
+                    sh[h] = w[0] >> 8;
+                    d[h] = rok[h] ? __half2float(__ushort_as_half((unsigned short)lds16(a))) * 512.0f : 0.f;
+                }
+#pragma unroll
+                for (int nt = 0; nt < NT8; nt++) {
+                    float c[4] = {0.f, 0.f, 0.f, 0.f};
+                    sm_mma(c, codes_f16<4, 8>(cw[0], 0), codes_f16<4, 8>(cw[1], 0), codes_f16<4, 8>(sh[0], 0), codes_f16<4, 8>(sh[1], 0), x[nt][l].x, x[nt][l].y);
+                    sm_mma(c, codes_f16<4, 8>(cw[0], 1), codes_f16<4, 8>(cw[1], 1), codes_f16<4, 8>(sh[0], 1), codes_f16<4, 8>(sh[1], 1), x[nt][l].z, x[nt][l].w);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) acc[nt][i] = fmaf(c[i], d[i >> 1], acc[nt][i]);
+                }
+            }
+        }
+    };
+    // this warp's sums of a tile into shared memory
+    auto put = [&](int mt, const float (&acc)[NT8][4]) {
+#pragma unroll
+        for (int nt = 0; nt < NT8; nt++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) red[(warp * (NT8 * 8) + nt * 8 + 2 * t + (i & 1)) * RS + mt * 16 + g + 8 * (i >> 1)] = acc[nt][i];
+    };
+    if constexpr (SINGLE) {
+#pragma unroll 1
+        for (int mt = 0; mt < MTW; mt++) {
+            float acc[NT8][4];
+#pragma unroll
+            for (int nt = 0; nt < NT8; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+            if (ok && warp < units) step(warp, mt, xr, acc);
+            put(mt, acc);
+        }
+    } else {
+        float acc[MTW][NT8][4];
+#pragma unroll
+        for (int mt = 0; mt < MTW; mt++)
+#pragma unroll
+            for (int nt = 0; nt < NT8; nt++) acc[mt][nt][0] = acc[mt][nt][1] = acc[mt][nt][2] = acc[mt][nt][3] = 0.f;
+        if (ok) {
+            for (int u = warp; u < units; u += SM_NW) {
+                uint4 x[NT8][4];
+#pragma unroll
+                for (int nt = 0; nt < NT8; nt++)
+#pragma unroll
+                    for (int l = 0; l < 4; l++) x[nt][l] = xr[nt][l];
+                load_x(u + SM_NW, xr);
+#pragma unroll
+                for (int mt = 0; mt < MTW; mt++) step(u, mt, x, acc[mt]);
+            }
+        }
+#pragma unroll
+        for (int mt = 0; mt < MTW; mt++) put(mt, acc[mt]);
+    }
+    const bool failed = __syncthreads_or(!ok);
+    if (failed) {
+        tc_wait_expired(p.status, LC_DEV_STATUS_WAIT_EXPIRED_TCD, tid);
+        return;
+    }
+    const int parts = min(units, SM_NW);
+    auto total = [&](int col, int r) -> float2 {   // rows r, r + 1
+        float2 s = make_float2(0.f, 0.f);
+        const float *src = red + col * RS + r;
+#pragma unroll 4
+        for (int i = 0; i < parts; i++) {
+            const float2 v = *reinterpret_cast<const float2 *>(src + i * (NT8 * 8) * RS);
+            s.x += v.x;
+            s.y += v.y;
+        }
+        return s;
+    };
+    OutT *out = reinterpret_cast<OutT *>(p.out[grp]);
+    const bool pairs = (n_rows & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & (2 * sizeof(OutT) - 1)) == 0;   // (n0 is even)
+    for (int i = tid; i < OROWS / 2 * p.m; i += SM_NT) {
+        const int r = 2 * (i % (OROWS / 2)), col = i / (OROWS / 2);
+        if (n0 + r >= n_rows) continue;
+        float2 v = total(col, r);
+        if (GEGLU) {
+            const float2 up = total(col, r + OROWS);
+            v = make_float2(geglu_f(v.x, up.x), geglu_f(v.y, up.y));
+        }
+        OutT *dst = out + (size_t)col * n_rows + n0 + r;
+        if (pairs) {
+            sm_store2(dst, v);
+        } else {
+            sm_store(dst, v.x);
+            if (n0 + r + 1 < n_rows) sm_store(dst + 1, v.y);
+        }
+    }
+}
+
+template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT>
+int launch_sm(lc_batch *b, const SmParams &p, int tiles) {
+    auto kern = qgemm_sm_kernel<FMT, NT8, MTW, SINGLE, GEGLU, OutT>;
+    const size_t smem = (size_t)MTW * 16 * p.raw_rs + sizeof(float) * SM_NW * NT8 * 8 * (MTW * 16 + 4);
+    static lc_smem_optin optin;
+    LC_CUDA_TRY(lc_ensure_smem(kern, optin, b->ctx, smem));
+    LC_LAUNCH_CHECKED(lc_launch(kern, dim3(tiles), dim3(SM_NT), smem, b, p));
+    b->dispatch_count++;
+    return LC_OK;
+}
+template <int FMT, int NT8, bool GEGLU, typename OutT>
+int launch_rows(lc_batch *b, const SmParams &p, int tiles, int rows) {
+    if (p.K <= SM_NW * SM_UNIT) {
+        if (rows == 64) return launch_sm<FMT, NT8, 4, true, GEGLU, OutT>(b, p, tiles);
+        if (rows == 32) return launch_sm<FMT, NT8, 2, true, GEGLU, OutT>(b, p, tiles);
+        return launch_sm<FMT, NT8, 1, true, GEGLU, OutT>(b, p, tiles);
+    }
+    if (rows == 32) return launch_sm<FMT, NT8, 2, false, GEGLU, OutT>(b, p, tiles);
+    return launch_sm<FMT, NT8, 1, false, GEGLU, OutT>(b, p, tiles);
+}
+template <int FMT, bool GEGLU, typename OutT>
+int launch_nt(lc_batch *b, const SmParams &p, int tiles, int rows) {
+    return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT>(b, p, tiles, rows) : launch_rows<FMT, 2, GEGLU, OutT>(b, p, tiles, rows);
+}
+
+}  // namespace
+
+// Grouped launch: `ng` matrices [ns[g], kk] on the same activations `input` [m, kk]; with `geglu` (TQ2_0), two matrices of one
+// shape and one output gelu_tanh(x Wg^T) * (x Wu^T).  Returns LC_OK after a launch, a positive status on error, or -1 when
+// the shape is outside what this kernel covers.
+int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng, const lc_buf *const *weights,
+                       lc_buf *const *outputs, const uint32_t *ns, uint32_t m, uint32_t kk, bool geglu) {
+    if (m < 1 || m > 16 || ng < 1 || ng > SM_GROUPS || !lc_aligned(input->dptr, 16)) return -1;
+    if (geglu && (ng != 2 || ns[0] != ns[1] || fmt != FMT_TQ2_0 || f32out)) return -1;
+    if (fmt == FMT_Q4_0 && kk % 4 != 0) return -1;
+    SmParams p;
+    p.x = (const __half *)input->dptr;
+    p.m = (int)m;
+    p.K = (int)kk;
+    p.nb = (int)(fmt == FMT_Q4_0 ? kk / 32 : kk / 256);
+    p.ngroups = geglu ? 1 : ng;
+    const size_t rb = (size_t)p.nb * (fmt == FMT_Q4_0 ? 18 : 66);
+    // a row's enclosing 16-byte range; an odd number of 32-byte pieces spreads the lanes' rows over the banks
+    size_t rs = (rb + 15 + 15) / 16 * 16;
+    rs += (32 + 64 - rs % 64) % 64;
+    p.raw_rs = (int)rs;
+    uint64_t rows_all = 0;
+    for (int g = 0; g < ng; g++) rows_all += ns[g];
+    // Rows per CTA: the fewest CTAs that still give every SM one (a CTA reads all activations), but never so many rows that
+    // the raw blocks of two CTAs do not fit an SM together (the next launch's CTA fetches its blocks while this one runs).
+    const size_t room = 100 * 1024, sms = (size_t)k->ctx->sm_count;
+    int rows = kk <= SM_NW * SM_UNIT ? 64 : 32;
+    while (rows > 16 && ((rows_all + rows - 1) / rows < sms * 3 / 4 || rows * rs > room)) rows >>= 1;
+    if (rows * rs > room) return -1;
+    int tiles = 0;
+    const int orows = geglu ? rows / 2 : rows;
+    for (int g = 0; g < SM_GROUPS; g++) {
+        const int gi = g < ng ? g : ng - 1;
+        if (!lc_aligned(weights[gi]->dptr, 16)) return -1;
+        p.w[g] = (const uint8_t *)weights[gi]->dptr;
+        p.out[g] = outputs[gi]->dptr;
+        p.n[g] = (int)ns[gi];
+        if (g < ng && !(geglu && g > 0)) tiles += ((int)ns[g] + orows - 1) / orows;
+        p.tile_end[g] = tiles;
+    }
+    if (tiles < 1) return -1;
+    p.status = k->dev_status;
+    p.wait_limit = k->test_wait_expiry ? 4096u : SM_WAIT_LIMIT;
+    p.extra_arrivals = k->test_wait_expiry ? 1u : 0u;
+    if (geglu) return launch_nt<FMT_TQ2_0, true, __half>(b, p, tiles, rows);
+    if (fmt == FMT_Q4_0) return f32out ? launch_nt<FMT_Q4_0, false, float>(b, p, tiles, rows) : launch_nt<FMT_Q4_0, false, __half>(b, p, tiles, rows);
+    return f32out ? launch_nt<FMT_TQ2_0, false, float>(b, p, tiles, rows) : launch_nt<FMT_TQ2_0, false, __half>(b, p, tiles, rows);
+}

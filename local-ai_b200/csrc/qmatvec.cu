@@ -281,6 +281,10 @@ int lc_qgemv_mma_stream(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const 
 int lc_qgemv_mma_stream_group(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int count,
                               const lc_buf *const *weights, lc_buf *const *outputs, uint32_t m, uint32_t kk, uint32_t n);
 
+// qmatmul_sm.cu: small-batch tensor-core kernel, m <= 16; returns -1 for what it does not cover.
+int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng, const lc_buf *const *weights,
+                       lc_buf *const *outputs, const uint32_t *ns, uint32_t m, uint32_t kk, bool geglu);
+
 int lc_qgemm_cuda_core(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input,
                        const lc_buf *weight, lc_buf *output, uint32_t m, uint32_t kk, uint32_t n) {
     if (n == 0) return LC_OK;
@@ -300,6 +304,18 @@ int lc_qgemm_cuda_core(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     return dispatch_qgemv<FMT_TQ2_0, __half>(k, b, w, wb, x, (__half *)output->dptr, n, kk, m);
 }
 
+// One matrix at m <= 16: the streaming kernel for matrices that are bandwidth, the small-batch kernel for the rest.
+static int small_batch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, const lc_buf *weight, lc_buf *output,
+                       uint32_t m, uint32_t kk, uint32_t n) {
+    if (n == 0) return LC_OK;
+    if (k->mma && k->decode_mma) {
+        int st = m <= 8 ? lc_qgemv_mma_stream(fmt, f32out, k, b, input, weight, output, m, kk, n) : -1;
+        if (st < 0) st = lc_qgemm_sm_launch(fmt, f32out, k, b, input, 1, &weight, &output, &n, m, kk, false);
+        if (st >= 0) return st;
+    }
+    return lc_qgemm_cuda_core(fmt, f32out, k, b, input, weight, output, m, kk, n);
+}
+
 extern "C" {
 
 #define LC_MATVEC_PAIR(NAME, FMT, F32OUT)                                                                  \
@@ -307,7 +323,7 @@ extern "C" {
                     uint32_t rows, uint32_t cols) {                                                        \
         int st = check_qargs<FMT>(#NAME, k, b, matrix, vector, output, 1, cols, rows, F32OUT ? 4 : 2);     \
         if (st != LC_OK) return st;                                                                        \
-        return lc_qgemm_cuda_core(FMT, F32OUT, k, b, vector, matrix, output, 1, cols, rows);               \
+        return small_batch(FMT, F32OUT, k, b, vector, matrix, output, 1, cols, rows);                      \
     }                                                                                                      \
     int NAME(lc_kernels *k, lc_ctx *ctx, const lc_buf *matrix, const lc_buf *vector, lc_buf *output,       \
              uint32_t rows, uint32_t cols) {                                                               \
@@ -334,7 +350,7 @@ extern "C" {
             if (st >= 0) return st;                                                                                  \
         }                                                                                                            \
         for (uint32_t i = 0; i < count; i++) {                                                                       \
-            int st = lc_qgemm_cuda_core(FMT, false, k, b, vector, matrices[i], outputs[i], 1, cols, rows);          \
+            int st = small_batch(FMT, false, k, b, vector, matrices[i], outputs[i], 1, cols, rows);                 \
             if (st != LC_OK) return st;                                                                              \
         }                                                                                                            \
         return LC_OK;                                                                                                \
@@ -372,7 +388,7 @@ int lc_multivec_nt_q4_0_into(lc_kernels *k, lc_batch *b, const lc_buf *input, co
     if (st != LC_OK) return st;
     // kernels.rs:6393-6398
     if (m < 1 || m > 16) return lc_fail(LC_ERR_INVALID_ARGUMENT, "multivec_nt_q4_0: m %u not in 1..=16", m);
-    return lc_qgemm_cuda_core(FMT_Q4_0, false, k, b, input, weight, output, m, kk, n);
+    return small_batch(FMT_Q4_0, false, k, b, input, weight, output, m, kk, n);
 }
 
 int lc_multivec_nt_tq2_0_into(lc_kernels *k, lc_batch *b, const lc_buf *input, const lc_buf *weight,
@@ -380,7 +396,7 @@ int lc_multivec_nt_tq2_0_into(lc_kernels *k, lc_batch *b, const lc_buf *input, c
     int st = check_qargs<FMT_TQ2_0>("multivec_nt_tq2_0", k, b, weight, input, output, m, kk, n, 2);
     if (st != LC_OK) return st;
     if (m < 1 || m > 16) return lc_fail(LC_ERR_INVALID_ARGUMENT, "multivec_nt_tq2_0: m %u not in 1..=16", m);
-    return lc_qgemm_cuda_core(FMT_TQ2_0, false, k, b, input, weight, output, m, kk, n);
+    return small_batch(FMT_TQ2_0, false, k, b, input, weight, output, m, kk, n);
 }
 
 int lc_tq2_dequant(lc_kernels *k, lc_ctx *ctx, const lc_buf *packed, const lc_buf *scales, lc_buf *output,
