@@ -454,7 +454,10 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     if (use_mma) {
         // One CTA per SM (shared memory), so the launch runs in whole waves; every CTA pays a fixed prologue and epilogue
         // worth about 320 keys.  Pick the split count that minimises waves x (overhead + keys per split).
-        uint32_t max_s = len_max / (len_max < 4096 ? 256u : 128u);   // a 32-key tile for all (half) of the eight warps
+        // Short contexts split down to two 32-key tiles per CTA (two warps that have the table's banks to themselves finish a
+        // tile sooner than eight), but into no more splits than one launch merges; long ones to half the warps.
+        uint32_t max_s = len_max < 4096 ? len_max / 64u : len_max / 128u;
+        if (len_max < 4096 && max_s > 8) max_s = 8;
         if (max_s < 1) max_s = 1;
         if (max_s > sms) max_s = sms;
         uint64_t best_cost = ~0ull;

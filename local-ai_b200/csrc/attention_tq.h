@@ -65,7 +65,8 @@ int lc_tq_attn_mma_launch(lc_batch *b, const TqAttnParams &p, dim3 grid, uint32_
 
 // Library-internal forms used by the decode step: lc_qkv_post_batched_into that also leaves the query fragments
 // described at TqAttnParams::qfrag in `qfrag` (n_lanes * n_q_heads * head_dim * 4 bytes; requires head_dim 256 and n_q_heads / n_kv_heads a multiple of 8), and lc_tq_attention_batched_into that reads them.
-// The fragments hold exactly the values the attention kernel would derive from q, so results do not change.
+// The fragments hold exactly the values the attention kernel would derive from q, so results do not change.  Both forms may
+// read `positions` ahead of their dependency wait: it has to be complete before the predecessor kernels start.
 bool lc_qfrag_supported(uint32_t head_dim, uint32_t bits, uint32_t n_q_heads, uint32_t n_kv_heads);
 int lc_qkv_post_frag(lc_kernels *k, lc_batch *b, lc_buf *q, const lc_buf *q_norm_weight, uint32_t n_q_heads,
                      const lc_buf *k_in, const lc_buf *v_in, const lc_buf *k_norm_weight, const lc_buf *positions,

@@ -779,20 +779,44 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
         const bool clustered = p.n_splits > 1;
         const uint32_t ml_a = smem_u32(ml_s), cp_a = smem_u32(cpart);
         for (int h = (int)it_split + (int)p.n_splits * warp; h < gvalid; h += (int)p.n_splits * NW) {
-            float gmax = -INFINITY;
-            for (uint32_t sp = 0; sp < p.n_splits; sp++) gmax = fmaxf(gmax, ld_cluster_f32(ml_a + (2 * h) * 4, sp, clustered));
+            // (loads of several splits in flight together: a read of a peer's shared memory takes most of a microsecond)
+            float ms[8], ls[8], gmax = -INFINITY;
+#pragma unroll
+            for (int sp = 0; sp < 8; sp++) {
+                ms[sp] = -INFINITY;
+                ls[sp] = 0.f;
+                if (sp < (int)p.n_splits) {
+                    ms[sp] = ld_cluster_f32(ml_a + (2 * h) * 4, sp, clustered);
+                    ls[sp] = ld_cluster_f32(ml_a + (2 * h + 1) * 4, sp, clustered);
+                }
+            }
+#pragma unroll
+            for (int sp = 0; sp < 8; sp++) gmax = fmaxf(gmax, ms[sp]);
             float gsum = 0.f, ov[DPL];
 #pragma unroll
             for (int i = 0; i < DPL; i++) ov[i] = 0.f;
-            for (uint32_t sp = 0; sp < p.n_splits; sp++) {
-                const float ms = ld_cluster_f32(ml_a + (2 * h) * 4, sp, clustered);
-                const float ls = ld_cluster_f32(ml_a + (2 * h + 1) * 4, sp, clustered);
-                const float f = (ms == -INFINITY) ? 0.f : expf(ms - gmax);
-                gsum += f * ls;
 #pragma unroll
-                for (int i = 0; i < DPL; i += 4) {
-                    const float4 a = ld_cluster_f4(cp_a + C::cp_index(h, DPL * lane + i) * 4, sp, clustered);
-                    ov[i] += f * a.x; ov[i + 1] += f * a.y; ov[i + 2] += f * a.z; ov[i + 3] += f * a.w;
+            for (int s0 = 0; s0 < 8; s0 += 4) {
+                if (s0 < (int)p.n_splits) {
+                    float4 a[4][DPL / 4];
+#pragma unroll
+                    for (int sp = 0; sp < 4; sp++)
+#pragma unroll
+                        for (int i = 0; i < DPL; i += 4)
+                            a[sp][i / 4] = s0 + sp < (int)p.n_splits ? ld_cluster_f4(cp_a + C::cp_index(h, DPL * lane + i) * 4, s0 + sp, clustered)
+                                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int sp = 0; sp < 4; sp++) {
+                        if (s0 + sp < (int)p.n_splits) {
+                            const float f = (ms[s0 + sp] == -INFINITY) ? 0.f : expf(ms[s0 + sp] - gmax);
+                            gsum += f * ls[s0 + sp];
+#pragma unroll
+                            for (int i = 0; i < DPL; i += 4) {
+                                const float4 v = a[sp][i / 4];
+                                ov[i] += f * v.x; ov[i + 1] += f * v.y; ov[i + 2] += f * v.z; ov[i + 3] += f * v.w;
+                            }
+                        }
+                    }
                 }
             }
 #pragma unroll

@@ -58,9 +58,26 @@ struct lc_model {
 
 namespace {
 
-int alloc(lc_model *m, size_t bytes, lc_buf **out) {
-    int st = lc_buf_alloc(m->ctx, bytes, out);
-    if (st == LC_OK) m->owned.push_back(*out);
+// The model's buffers are pieces of one zero-filled allocation (four KV pools per layer would otherwise be four allocations
+// and, at the end, four device-wide waits each).  Sizes are collected first, then placed.
+struct Piece {
+    size_t bytes;
+    lc_buf **out;
+};
+int place(lc_model *m, const std::vector<Piece> &pieces) {
+    auto padded = [](size_t n) { return ((n ? n : 1) + 255) & ~(size_t)255; };
+    size_t total = 0;
+    for (const Piece &p : pieces) total += padded(p.bytes);
+    lc_buf *slab = nullptr;
+    int st = lc_buf_alloc(m->ctx, total, &slab);
+    if (st != LC_OK) return st;
+    char *at = (char *)lc_buf_device_ptr(slab);
+    for (const Piece &p : pieces) {
+        if ((st = lc_buf_wrap(m->ctx, at, p.bytes, p.out)) != LC_OK) break;
+        m->owned.push_back(*p.out);
+        at += padded(p.bytes);
+    }
+    m->owned.push_back(slab);   // last: freed after its pieces
     return st;
 }
 
@@ -91,6 +108,7 @@ int lc_model_create(lc_ctx *ctx, lc_kernels *k, const lc_model_config *cfg, lc_m
         lc_model_destroy(m);
         return s;
     };
+    std::vector<Piece> pieces;
     for (uint32_t i = 0; i < c.n_layers; i++) {
         lc_model_layer &L = m->layers[i];
         const bool full = (i % c.full_every) == c.full_every - 1 || c.swa_window == 0;
@@ -99,34 +117,29 @@ int lc_model_create(lc_ctx *ctx, lc_kernels *k, const lc_model_config *cfg, lc_m
         if (L.ring > c.max_context) L.ring = 0, L.window = c.swa_window;  // window never fills: absolute rows
         L.lane_rows = L.ring ? L.ring : c.max_context;
         const size_t rows = (size_t)c.max_lanes * L.lane_rows * c.n_kv_heads;
-        if ((st = alloc(m, rows * cb, &L.k_codes)) || (st = alloc(m, rows * cb, &L.v_codes)) ||
-            (st = alloc(m, rows * 2, &L.k_norms)) || (st = alloc(m, rows * 2, &L.v_norms)))
-            return fail(st);
+        for (const Piece &p : {Piece{rows * cb, &L.k_codes}, Piece{rows * cb, &L.v_codes}, Piece{rows * 2, &L.k_norms}, Piece{rows * 2, &L.v_norms}})
+            pieces.push_back(p);
     }
     // codec constants (TurboQuant::new, turboquant.rs:187-199; seed quant_cache.rs:30)
     std::vector<float> lv(1u << c.kv_bits), sg(c.head_dim);
     lc_tq_levels(c.head_dim, c.kv_bits, lv.data());
     lc_tq_signs(c.head_dim, LC_TQ_SEED, sg.data());
     std::vector<__half> ones(c.head_dim, __float2half(1.0f));
-    if ((st = alloc(m, lv.size() * 4, &m->levels)) || (st = alloc(m, sg.size() * 4, &m->signs)) ||
-        (st = alloc(m, ones.size() * 2, &m->ones)))
-        return fail(st);
+    const size_t n = c.max_lanes, qd = (size_t)c.n_q_heads * c.head_dim, kd = (size_t)c.n_kv_heads * c.head_dim;
+    for (const Piece &p : {Piece{lv.size() * 4, &m->levels}, Piece{sg.size() * 4, &m->signs}, Piece{ones.size() * 2, &m->ones},
+                           Piece{n * c.hidden * 2, &m->x}, Piece{n * c.hidden * 2, &m->x2}, Piece{n * c.hidden * 2, &m->normed},
+                           Piece{n * qd * 2, &m->q}, Piece{n * kd * 2, &m->kbuf}, Piece{n * kd * 2, &m->vbuf}, Piece{n * qd * 2, &m->attn},
+                           Piece{n * c.hidden * 2, &m->resid}, Piece{n * c.inter * 2, &m->gate}, Piece{n * c.inter * 2, &m->up},
+                           Piece{n * c.hidden * 2, &m->ffn}, Piece{n * (size_t)c.vocab * 4, &m->logits}})
+        pieces.push_back(p);
+    // LOCAL_CUDA_QFRAG=0 keeps the attention kernel's own query prologue (same results; for A/B timing and tests)
+    const char *qf_env = getenv("LOCAL_CUDA_QFRAG");
+    if (!(qf_env && qf_env[0] == '0') && lc_qfrag_supported(c.head_dim, c.kv_bits, c.n_q_heads, c.n_kv_heads))
+        pieces.push_back({n * qd * 4, &m->qfrag});
+    if ((st = place(m, pieces)) != LC_OK) return fail(st);
     if ((st = lc_buf_upload(m->levels, 0, lv.data(), lv.size() * 4)) ||
         (st = lc_buf_upload(m->signs, 0, sg.data(), sg.size() * 4)) ||
         (st = lc_buf_upload(m->ones, 0, ones.data(), ones.size() * 2)))
-        return fail(st);
-    const size_t n = c.max_lanes, qd = (size_t)c.n_q_heads * c.head_dim, kd = (size_t)c.n_kv_heads * c.head_dim;
-    if ((st = alloc(m, n * c.hidden * 2, &m->x)) || (st = alloc(m, n * c.hidden * 2, &m->x2)) ||
-        (st = alloc(m, n * c.hidden * 2, &m->normed)) || (st = alloc(m, n * qd * 2, &m->q)) ||
-        (st = alloc(m, n * kd * 2, &m->kbuf)) || (st = alloc(m, n * kd * 2, &m->vbuf)) ||
-        (st = alloc(m, n * qd * 2, &m->attn)) || (st = alloc(m, n * c.hidden * 2, &m->resid)) ||
-        (st = alloc(m, n * c.inter * 2, &m->gate)) || (st = alloc(m, n * c.inter * 2, &m->up)) ||
-        (st = alloc(m, n * c.hidden * 2, &m->ffn)) || (st = alloc(m, n * (size_t)c.vocab * 4, &m->logits)))
-        return fail(st);
-    // LOCAL_CUDA_QFRAG=0 keeps the attention kernel's own query prologue (same results; for A/B timing and tests)
-    const char *qf_env = getenv("LOCAL_CUDA_QFRAG");
-    if (!(qf_env && qf_env[0] == '0') && lc_qfrag_supported(c.head_dim, c.kv_bits, c.n_q_heads, c.n_kv_heads) &&
-        (st = alloc(m, n * qd * 4, &m->qfrag)))
         return fail(st);
     {
         const char *e = getenv("LOCAL_CUDA_DECODE_CHAINS");

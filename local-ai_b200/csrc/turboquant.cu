@@ -139,6 +139,68 @@ __global__ void encode_kv_kernel(const __half *__restrict__ input, const float *
                &norm_sh);
 }
 
+// Rotates x (HD / 32 consecutive dims per lane): Walsh-Hadamard butterflies in ascending stride, lower = a + b, upper = a - b.
+template <int DPL>
+__device__ __forceinline__ void fwht_warp_row(float (&x)[DPL], int lane) {
+#pragma unroll
+    for (int len = 1; len < DPL; len <<= 1)
+#pragma unroll
+        for (int i = 0; i < DPL; i++)
+            if (!(i & len)) {
+                const float a = x[i], b = x[i + len];
+                x[i] = __fadd_rn(a, b);
+                x[i + len] = __fsub_rn(a, b);
+            }
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) {
+        const bool upper = lane & m;
+#pragma unroll
+        for (int i = 0; i < DPL; i++) {
+            const float o = __shfl_xor_sync(0xffffffffu, x[i], m);
+            x[i] = upper ? __fsub_rn(o, x[i]) : __fadd_rn(x[i], o);
+        }
+    }
+}
+// Encodes one row held by a warp, HD / 32 consecutive dims per lane, whose norm is known (TurboQuant::encode_into).
+template <int HD, int BITS>
+__device__ __forceinline__ void encode_warp_row(float (&x)[HD / 32], float norm, const float (&lv)[1 << BITS], const float (&sg)[HD / 32],
+                                                int lane, uint8_t *dst, __half *norm_out) {
+    constexpr int DPL = HD / 32, NLEV = 1 << BITS;
+    const float inv = norm > 0.f ? __fdiv_rn(1.0f, norm) : 0.f;
+#pragma unroll
+    for (int i = 0; i < DPL; i++) x[i] = __fmul_rn(norm > 0.f ? __fmul_rn(x[i], inv) : x[i], sg[i]);
+    fwht_warp_row<DPL>(x, lane);
+    const float inv_sqrt_d = __fdiv_rn(1.0f, __fsqrt_rn((float)HD));
+    unsigned long long word = 0;   // this lane's DPL codes, LSB first
+#pragma unroll
+    for (int i = 0; i < DPL; i++) {
+        const float v = __fmul_rn(x[i], inv_sqrt_d);
+        unsigned best = 0;
+        float bd = INFINITY;
+#pragma unroll
+        for (int j = 0; j < NLEV; j++) {
+            const float dd = fabsf(__fsub_rn(v, lv[j]));
+            if (dd < bd) { bd = dd; best = (unsigned)j; }
+        }
+        word |= (unsigned long long)best << (BITS * i);
+    }
+    constexpr int LB = DPL * BITS;   // bits of one lane: 8 .. 64, or 12 (tq3 at head_dim 128)
+    if constexpr (LB == 12) {        // two lanes share three bytes
+        const unsigned w = (unsigned)word | (__shfl_down_sync(0xffffffffu, (unsigned)word, 1) << 12);
+        if (!(lane & 1)) {
+            dst += (lane >> 1) * 3;
+            dst[0] = (uint8_t)w;
+            dst[1] = (uint8_t)(w >> 8);
+            dst[2] = (uint8_t)(w >> 16);
+        }
+    } else {
+        dst += lane * (LB / 8);
+#pragma unroll
+        for (int i = 0; i < LB / 8; i++) dst[i] = (uint8_t)(word >> (8 * i));
+    }
+    if (lane == 0) *norm_out = __float2half_rn(norm);
+}
+
 // The same rows for head_dim 128 / 256 / 512 and the sequential norm, a warp per row and eight rows per CTA: what one row
 // takes is the dependent chain of the norm's head_dim additions (about a microsecond at 256), so eight of them run side
 // by side in the lanes of one warp, and the rest of a row needs no further barrier.  grid.y = 1 or 2: the K rows and the V
@@ -199,42 +261,6 @@ __global__ void __launch_bounds__(ENC_ROWS * 32) encode_rows_kernel(const Encode
     }
     __syncthreads();
     if (!live) return;
-    const float norm = norm_s[warp];
-    const float inv = norm > 0.f ? __fdiv_rn(1.0f, norm) : 0.f;
-#pragma unroll
-    for (int i = 0; i < DPL; i++) x[i] = __fmul_rn(norm > 0.f ? __fmul_rn(x[i], inv) : x[i], sg[i]);
-#pragma unroll
-    for (int len = 1; len < DPL; len <<= 1)
-#pragma unroll
-        for (int i = 0; i < DPL; i++)
-            if (!(i & len)) {
-                const float a = x[i], b = x[i + len];
-                x[i] = __fadd_rn(a, b);
-                x[i + len] = __fsub_rn(a, b);
-            }
-#pragma unroll
-    for (int m = 1; m < 32; m <<= 1) {
-        const bool upper = lane & m;
-#pragma unroll
-        for (int i = 0; i < DPL; i++) {
-            const float o = __shfl_xor_sync(0xffffffffu, x[i], m);
-            x[i] = upper ? __fsub_rn(o, x[i]) : __fadd_rn(x[i], o);
-        }
-    }
-    const float inv_sqrt_d = __fdiv_rn(1.0f, __fsqrt_rn((float)HD));
-    unsigned long long word = 0;   // this lane's DPL codes, LSB first
-#pragma unroll
-    for (int i = 0; i < DPL; i++) {
-        const float v = __fmul_rn(x[i], inv_sqrt_d);
-        unsigned best = 0;
-        float bd = INFINITY;
-#pragma unroll
-        for (int j = 0; j < NLEV; j++) {
-            const float dd = fabsf(__fsub_rn(v, lv[j]));
-            if (dd < bd) { bd = dd; best = (unsigned)j; }
-        }
-        word |= (unsigned long long)best << (BITS * i);
-    }
     size_t slot;
     const unsigned row = g_in / p.n_kv, head = g_in - row * p.n_kv;
     if (BATCHED) {
@@ -248,22 +274,7 @@ __global__ void __launch_bounds__(ENC_ROWS * 32) encode_rows_kernel(const Encode
         const unsigned logical = p.position + row;
         slot = (size_t)(p.ring ? logical % p.ring : logical) * p.n_kv + head;
     }
-    constexpr int LB = DPL * BITS;   // bits of one lane: 8 .. 64, or 12 (tq3 at head_dim 128)
-    uint8_t *dst = p.packed[y] + slot * (HD * BITS / 8);
-    if constexpr (LB == 12) {        // two lanes share three bytes
-        const unsigned w = (unsigned)word | (__shfl_down_sync(0xffffffffu, (unsigned)word, 1) << 12);
-        if (!(lane & 1)) {
-            dst += (lane >> 1) * 3;
-            dst[0] = (uint8_t)w;
-            dst[1] = (uint8_t)(w >> 8);
-            dst[2] = (uint8_t)(w >> 16);
-        }
-    } else {
-        dst += lane * (LB / 8);
-#pragma unroll
-        for (int i = 0; i < LB / 8; i++) dst[i] = (uint8_t)(word >> (8 * i));
-    }
-    if (lane == 0) p.norms[y][slot] = __float2half_rn(norm);
+    encode_warp_row<HD, BITS>(x, norm_s[warp], lv, sg, lane, p.packed[y] + slot * (HD * BITS / 8), p.norms[y] + slot);
 }
 template <int HD, bool BATCHED>
 cudaError_t launch_encode_rows(lc_batch *b, const EncodeRows &p, unsigned tensors, unsigned bits) {
@@ -375,6 +386,163 @@ __global__ void kv_write_kernel(__half *q, const __half *__restrict__ q_norm_w, 
     const unsigned code_bytes = (hd * bits + 7) >> 3;
     encode_row(xr, t, hd, bits, levels, signs, norm_mode, (role == 1 ? k_packed : v_packed) + slot * code_bytes,
                (role == 1 ? k_norms : v_norms) + slot, sh, red, code_sh, &norm_sh);
+}
+
+// The same launch for head_dim 256 and the sequential norm, a warp per row, eight rows per CTA (see encode_rows_kernel): no
+// barrier but the two around the norms of the K and V rows, which have CTAs of their own and come first.  The order of the
+// additions inside a row is that of the kernel above.  EARLY: `positions` was complete before the predecessor kernels started
+// (an input of the decode step), so the rotation's angles are ready before the dependency wait.
+struct KvWriteRows {
+    __half *q;
+    const __half *q_norm_w, *kin, *vin, *k_norm_w;
+    unsigned n_q, n_lanes, n_kv, kv_ctas, lane_capacity, ring;
+    const uint32_t *positions;
+    const float *levels, *signs;
+    uint8_t *packed[2];
+    __half *norms[2];
+    float eps, theta, rotary_factor, q_scale;
+    int *status;
+    uint4 *qfrag;
+};
+template <int BITS, bool EARLY>
+__global__ void __launch_bounds__(ENC_ROWS * 32) kv_write_rows_kernel(const __grid_constant__ KvWriteRows p) {
+    constexpr int HD = 256, DPL = 8, NLEV = 1 << BITS;
+    lc_pdl_trigger();
+    __shared__ __align__(16) float sq[ENC_ROWS][HD + 4];
+    __shared__ float norm_s[ENC_ROWS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool kv = blockIdx.x < p.kv_ctas;
+    const unsigned per_lane = kv ? 2 * p.n_kv : p.n_q;
+    const unsigned r = (kv ? blockIdx.x : blockIdx.x - p.kv_ctas) * ENC_ROWS + warp, row = r / per_lane, rem = r - row * per_lane;
+    const bool live = row < p.n_lanes;
+    const int role = !kv ? 0 : (rem < p.n_kv ? 1 : 2);   // Q, K, V
+    const unsigned head = role == 2 ? rem - p.n_kv : rem;
+    // constant operands and the rotation frequencies of this lane's dims (dims d and d + 128 turn together)
+    float w[DPL], freq[DPL], sg[DPL], lv[NLEV];
+    const unsigned angles = (unsigned)((float)HD * p.rotary_factor) / 2;
+#pragma unroll
+    for (int i = 0; i < NLEV; i++) lv[i] = p.levels[i];
+#pragma unroll
+    for (int e = 0; e < DPL; e++) {
+        const unsigned d = DPL * lane + e, i = d & (HD / 2 - 1);
+        sg[e] = p.signs[d];
+        w[e] = role == 2 ? 1.0f : __half2float((role == 0 ? p.q_norm_w : p.k_norm_w)[d]);
+        freq[e] = role != 2 && i < angles ? 1.0f / powf(p.theta, (float)(2 * i) / (float)HD) : 0.f;
+    }
+    unsigned pos = 0;
+    float cs[DPL], sn[DPL];
+    auto rotation = [&]() {
+        if (live) pos = p.positions[row];
+#pragma unroll
+        for (int e = 0; e < DPL; e++) {
+            cs[e] = 1.f;
+            sn[e] = 0.f;
+            if (role != 2) {
+                const float ang = (float)pos * freq[e];
+                cs[e] = cosf(ang);
+                sn[e] = sinf(ang);
+            }
+        }
+    };
+    if (EARLY) rotation();
+    lc_pdl_wait();
+    if (!EARLY) rotation();
+    __half *qrow = p.q + ((size_t)row * p.n_q + head) * HD + DPL * lane;
+    const size_t g_in = (size_t)row * p.n_kv + head;
+    float x[DPL];
+    {
+        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+        if (live) raw = *reinterpret_cast<const uint4 *>(role == 0 ? qrow : (role == 1 ? p.kin : p.vin) + g_in * HD + DPL * lane);
+        const __half2 *h = reinterpret_cast<const __half2 *>(&raw);
+#pragma unroll
+        for (int i = 0; i < DPL / 2; i++) {
+            const float2 f = __half22float2(h[i]);
+            x[2 * i] = f.x;
+            x[2 * i + 1] = f.y;
+        }
+    }
+    // mean square: 32-dim groups as shuffle trees (strides 16, 8 across lanes; 4, 2, 1 inside), then the groups in order
+    float tot = 0.f;
+    {
+        float s[DPL];
+#pragma unroll
+        for (int e = 0; e < DPL; e++) {
+            s[e] = x[e] * x[e];
+            s[e] += __shfl_xor_sync(0xffffffffu, s[e], 2);
+            s[e] += __shfl_xor_sync(0xffffffffu, s[e], 1);
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+            for (int e = 0; e < o; e++) s[e] += s[e + o];
+#pragma unroll
+        for (int g = 0; g < 8; g++) tot += __shfl_sync(0xffffffffu, s[0], 4 * g);
+    }
+    const float rms = rsqrtf(tot / (float)HD + p.eps);
+#pragma unroll
+    for (int e = 0; e < DPL; e++) x[e] = __half2float(__float2half_rn(x[e] * rms * w[e]));
+    if (role != 2) {
+#pragma unroll
+        for (int e = 0; e < DPL; e++) {
+            const float other = __shfl_xor_sync(0xffffffffu, x[e], 16);
+            const bool low = lane < 16;
+            const float x0 = low ? x[e] : other, x1 = low ? other : x[e];
+            const float v = low ? x0 * cs[e] - x1 * sn[e] : x0 * sn[e] + x1 * cs[e];
+            if (((unsigned)(DPL * lane + e) & (HD / 2 - 1)) < angles) x[e] = __half2float(__float2half_rn(v));
+        }
+    }
+    if (role == 0) {
+        if (!live) return;
+        uint4 raw;
+        __half2 *h = reinterpret_cast<__half2 *>(&raw);
+#pragma unroll
+        for (int i = 0; i < DPL / 2; i++) h[i] = __floats2half2_rn(x[2 * i], x[2 * i + 1]);
+        *reinterpret_cast<uint4 *>(qrow) = raw;
+        if (p.qfrag) {
+            // the tensor-core attention kernel's first steps (see kv_write_kernel): sign, transform, scale, split
+#pragma unroll
+            for (int e = 0; e < DPL; e++) x[e] = __fmul_rn(x[e], sg[e]);
+            fwht_warp_row<DPL>(x, lane);
+            const float f = __fdiv_rn(p.q_scale, __fsqrt_rn((float)HD));
+            unsigned hi[DPL / 2], lo[DPL / 2];
+#pragma unroll
+            for (int i = 0; i < DPL / 2; i++) {
+                const float v0 = __fmul_rn(x[2 * i], f), v1 = __fmul_rn(x[2 * i + 1], f);
+                const __half2 a = __floats2half2_rn(v0, v1);
+                const __half2 b = __floats2half2_rn(__fsub_rn(v0, __low2float(a)), __fsub_rn(v1, __high2float(a)));
+                hi[i] = *reinterpret_cast<const unsigned *>(&a);
+                lo[i] = *reinterpret_cast<const unsigned *>(&b);
+            }
+            uint4 *dst = p.qfrag + ((size_t)row * (p.n_q >> 3) + (head >> 3)) * 512 + 4 * (head & 7) + (lane >> 3);
+            dst[((lane & 7) * 2) * 32] = make_uint4(hi[0], hi[1], lo[0], lo[1]);
+            dst[((lane & 7) * 2 + 1) * 32] = make_uint4(hi[2], hi[3], lo[2], lo[3]);
+        }
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < DPL; i += 4)
+        *reinterpret_cast<float4 *>(&sq[warp][DPL * lane + i]) =
+            make_float4(__fmul_rn(x[i], x[i]), __fmul_rn(x[i + 1], x[i + 1]), __fmul_rn(x[i + 2], x[i + 2]), __fmul_rn(x[i + 3], x[i + 3]));
+    __syncthreads();
+    if (warp == 0 && lane < ENC_ROWS) {   // the reference's sequential f32 sum, in index order
+        const float4 *r4 = reinterpret_cast<const float4 *>(sq[lane]);
+        float s = 0.f;
+#pragma unroll 8
+        for (int i = 0; i < HD / 4; i++) {
+            const float4 a = r4[i];
+            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a.x), a.y), a.z), a.w);
+        }
+        norm_s[lane] = __fsqrt_rn(s);
+    }
+    __syncthreads();
+    if (!live) return;
+    const unsigned ppos = p.ring ? pos % p.ring : pos;
+    if (ppos >= p.lane_capacity) {   // a device-resident position past the lane's rows: write nothing, report
+        if (lane == 0) atomicExch(p.status, LC_DEV_STATUS_POSITION);
+        return;
+    }
+    const size_t slot = ((size_t)row * p.lane_capacity + ppos) * p.n_kv + head;
+    encode_warp_row<HD, BITS>(x, norm_s[warp], lv, sg, lane, p.packed[role - 1] + slot * (HD * BITS / 8), p.norms[role - 1] + slot);
 }
 
 // dequantize_kv.metal:132-189. grid = n_kv * (num_tokens - token_start).
@@ -720,7 +888,7 @@ static int kv_write_common(const char *name, lc_kernels *k, lc_batch *b, lc_buf 
                            lc_buf *k_norms, lc_buf *v_packed, lc_buf *v_norms, uint32_t head_dim, uint32_t n_kv_heads,
                            uint32_t lane_capacity, uint32_t bits, uint32_t n_lanes, uint32_t ring_capacity, float eps,
                            float rope_theta, float partial_rotary_factor, lc_buf *qfrag = nullptr,
-                           float softmax_scale = 0.f) {
+                           float softmax_scale = 0.f, bool early_positions = false) {
     if (!k || !b || !k_in || !v_in || !k_norm_weight || !positions || !levels || !signs || !k_packed || !k_norms ||
         !v_packed || !v_norms || (n_q_heads && (!q || !q_norm_weight)))
         return lc_fail(LC_ERR_INVALID_ARGUMENT, "%s: NULL argument", name);
@@ -738,7 +906,7 @@ static int kv_write_common(const char *name, lc_kernels *k, lc_batch *b, lc_buf 
     LC_REQUIRE(levels->bytes >= (4u << bits) && signs->bytes >= head_dim * 4u, "%s: codec buffers too small", name);
     if (qfrag) {
         LC_REQUIRE(n_q_heads && lc_qfrag_supported(head_dim, bits, n_q_heads, n_kv_heads),
-                   "%s: query fragments need head_dim 256, 2-bit codes and q heads in groups of 8 per kv head", name);
+                   "%s: query fragments need head_dim 256 and q heads in groups of 8 per kv head", name);
         LC_REQUIRE(qfrag->bytes >= (size_t)n_lanes * n_q_heads * head_dim * 4 && lc_aligned(qfrag->dptr, 16),
                    "%s: query fragment buffer too small or misaligned", name);
     }
@@ -748,6 +916,40 @@ static int kv_write_common(const char *name, lc_kernels *k, lc_batch *b, lc_buf 
                    v_norms->bytes >= rows * 2,
                "%s: pool buffers hold fewer than %zu rows", name, rows);
     if (groups == 0) return LC_OK;
+    if (head_dim == 256 && k->kv_norm_mode == 0 && lc_aligned(k_in->dptr, 16) && lc_aligned(v_in->dptr, 16) && (!n_q_heads || lc_aligned(q->dptr, 16))) {
+        KvWriteRows p;
+        p.q = q ? (__half *)q->dptr : nullptr;
+        p.q_norm_w = q_norm_weight ? (const __half *)q_norm_weight->dptr : nullptr;
+        p.kin = (const __half *)k_in->dptr;
+        p.vin = (const __half *)v_in->dptr;
+        p.k_norm_w = (const __half *)k_norm_weight->dptr;
+        p.n_q = n_q_heads;
+        p.n_lanes = n_lanes;
+        p.n_kv = n_kv_heads;
+        p.kv_ctas = (unsigned)((2 * groups + ENC_ROWS - 1) / ENC_ROWS);
+        p.lane_capacity = lane_capacity;
+        p.ring = ring_capacity;
+        p.positions = (const uint32_t *)positions->dptr;
+        p.levels = (const float *)levels->dptr;
+        p.signs = (const float *)signs->dptr;
+        p.packed[0] = (uint8_t *)k_packed->dptr;
+        p.packed[1] = (uint8_t *)v_packed->dptr;
+        p.norms[0] = (__half *)k_norms->dptr;
+        p.norms[1] = (__half *)v_norms->dptr;
+        p.eps = eps;
+        p.theta = rope_theta;
+        p.rotary_factor = partial_rotary_factor;
+        p.q_scale = softmax_scale;
+        p.status = k->dev_status;
+        p.qfrag = qfrag ? (uint4 *)qfrag->dptr : nullptr;
+        const dim3 grid(p.kv_ctas + (unsigned)(((size_t)n_lanes * n_q_heads + ENC_ROWS - 1) / ENC_ROWS)), block(ENC_ROWS * 32);
+        void (*kern)(KvWriteRows);
+        if (early_positions) kern = bits == 2 ? kv_write_rows_kernel<2, true> : (bits == 3 ? kv_write_rows_kernel<3, true> : kv_write_rows_kernel<4, true>);
+        else kern = bits == 2 ? kv_write_rows_kernel<2, false> : (bits == 3 ? kv_write_rows_kernel<3, false> : kv_write_rows_kernel<4, false>);
+        LC_LAUNCH_CHECKED(lc_launch(kern, grid, block, 0, b, p));
+        b->dispatch_count++;
+        return LC_OK;
+    }
     LC_LAUNCH_CHECKED(lc_launch(kv_write_kernel, dim3(n_lanes, n_q_heads + 2 * n_kv_heads), dim3(head_dim), 0, b,
                                 q ? (__half *)q->dptr : nullptr, q_norm_weight ? (const __half *)q_norm_weight->dptr : nullptr,
                                 n_q_heads, (const __half *)k_in->dptr, (const __half *)v_in->dptr,
@@ -796,5 +998,5 @@ int lc_qkv_post_frag(lc_kernels *k, lc_batch *b, lc_buf *q, const lc_buf *q_norm
         return lc_fail(LC_ERR_INVALID_ARGUMENT, "qkv_post_batched: the query buffer, its norm weight and n_q_heads are required");
     return kv_write_common("qkv_post_batched", k, b, q, q_norm_weight, n_q_heads, k_in, v_in, k_norm_weight, positions, levels,
                            signs, k_packed, k_norms, v_packed, v_norms, head_dim, n_kv_heads, lane_capacity, bits, n_lanes,
-                           ring_capacity, eps, rope_theta, partial_rotary_factor, qfrag, softmax_scale);
+                           ring_capacity, eps, rope_theta, partial_rotary_factor, qfrag, softmax_scale, true);
 }
