@@ -468,6 +468,18 @@ void lc_kernels_destroy(lc_kernels *k) {
     delete k;
 }
 
+int lc_kernels_device_status(lc_kernels *k, int *status) {
+    if (!k || !status) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_kernels_device_status: NULL argument");
+    LC_CUDA_TRY(cudaMemcpyAsync(status, k->dev_status, sizeof(int), cudaMemcpyDeviceToHost, k->ctx->stream));
+    LC_CUDA_TRY(cudaStreamSynchronize(k->ctx->stream));
+    if (*status == LC_DEV_STATUS_POSITION)
+        return lc_fail(LC_ERR_INVALID_ARGUMENT,
+                       "a position in a device buffer pointed past its lane's pool rows (the row was not written / the "
+                       "context was clamped)");
+    if (*status) return lc_fail(LC_ERR_TIMEOUT, "a device-side bounded wait expired (status %d)", *status);
+    return LC_OK;
+}
+
 }  // extern "C"
 
 // A captured graph keeps the scratch and counter addresses it was recorded with, so a block that has

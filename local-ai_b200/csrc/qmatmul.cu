@@ -7,13 +7,13 @@
 // keeps those on the CUDA-core kernel); otherwise the register-resident CUDA-core
 // path that streams the weights once for up to 16 rows (qmatvec.cu, m <= 8), the
 // register-direct mma.sync kernel for decode batches 8 < m <= 64 (qmatmul_mma.cu:
-// Q4_0, f32 out, shapes the tcgen05 kernel declines), and the large-tile tcgen05
-// kernel for larger m (qmatmul_tc.cu).  The matvec entry points (lc_matvec_*) stay
+// Q4_0, f32 out, shapes the tcgen05 kernel declines), and the large-batch tcgen05
+// kernel for larger m (qmatmul_tcl.cu).  The matvec entry points (lc_matvec_*) stay
 // on the CUDA-core kernels.
 // LOCAL_AI_MMA=0 forces the CUDA-core path for every m, as it forces the non-MMA
 // kernels in the reference; LOCAL_CUDA_DECODE_TC=0 / LOCAL_CUDA_DECODE_MMA=0
 // switch the two decode kernels off (with both off, 8 < m <= 64 runs on
-// qmatmul_tc.cu as well).
+// qmatmul_tcl.cu as well).
 #include <stdlib.h>
 #include "lc_internal.h"
 
@@ -21,12 +21,12 @@ int lc_qgemm_cuda_core(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
                        const lc_buf *weight, lc_buf *output, uint32_t m, uint32_t kk, uint32_t n);
 int lc_check_qargs(int fmt, const char *name, lc_kernels *k, lc_batch *b, const lc_buf *w, const lc_buf *x,
                    const lc_buf *out, uint32_t m, uint32_t kk, uint32_t n, size_t out_elem);
-// qmatmul_tc.cu: returns LC_OK when it launched, or a negative value when the
-// shape is outside what the tensor-core kernel covers (caller falls through).
-int lc_qgemm_tcgen05(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input,
-                     const lc_buf *weight, lc_buf *output, uint32_t m, uint32_t kk, uint32_t n);
+// qmatmul_tcl.cu: large-batch tcgen05 kernel, up to three matrices on the same activations; returns LC_OK when it launched, or
+// a negative value when the shape is outside what it covers (caller falls through).
+int lc_qgemm_tcl_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng, const lc_buf *const *weights,
+                        lc_buf *const *outputs, const uint32_t *ns, uint32_t m, uint32_t kk);
 
-// qmatmul_mma.cu: same contract as lc_qgemm_tcgen05_grouped, for 8 < m <= 64.
+// qmatmul_mma.cu: same contract, for 8 < m <= 64.
 int lc_qgemm_mma_grouped(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng,
                          const lc_buf *const *weights, lc_buf *const *outputs, const uint32_t *ns, uint32_t m,
                          uint32_t kk);
@@ -100,15 +100,11 @@ static int route(int fmt, bool f32out, const char *name, lc_kernels *k, lc_batch
                 if (st >= 0) return st;
             }
         }
-        st = lc_qgemm_tcgen05(fmt, f32out, k, b, input, weight, output, m, kk, n);
+        st = lc_qgemm_tcl_launch(fmt, f32out, k, b, input, 1, ws, os, ns, m, kk);
         if (st >= 0) return st;
     }
     return lc_qgemm_cuda_core(fmt, f32out, k, b, input, weight, output, m, kk, n);
 }
-
-int lc_qgemm_tcgen05_grouped(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng,
-                             const lc_buf *const *weights, lc_buf *const *outputs, const uint32_t *ns, uint32_t m,
-                             uint32_t kk);
 
 // Several TQ2_0 projections of the same activations (Q/K/V; gate/up) as one launch when the tensor-core
 // path applies, else one after the other.
@@ -129,7 +125,7 @@ int lc_matmul_nt_tq2_0_grouped(lc_kernels *k, lc_batch *b, const lc_buf *input, 
     if (k->mma && m > 8) {
         int st = -1;
         if (k->decode_mma && m <= 64) st = lc_qgemm_mma_grouped(1, false, k, b, input, ng, weights, outputs, ns, m, kk);
-        if (st < 0) st = lc_qgemm_tcgen05_grouped(1, false, k, b, input, ng, weights, outputs, ns, m, kk);
+        if (st < 0) st = lc_qgemm_tcl_launch(1, false, k, b, input, ng, weights, outputs, ns, m, kk);
         if (st >= 0) return st;
     }
     for (int g = 0; g < ng; g++) {
