@@ -486,8 +486,26 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
         }
         n_splits = (len_max + chunk - 1) / chunk;
     }
+    // Chunks of several rows: the prefill kernel shares each decoded key among 128 MMA rows.  Below about half a tile of rows
+    // the decode kernel's CTA per row is as fast.
+    uint32_t pf_heads = 1, pf_tiles = 0;
+    if (prefill && use_mma && lc_tq_attn_prefill_supported(hd, bits)) {
+        const uint32_t heads = group < 8 ? group : 8;
+        while (pf_heads < heads) pf_heads <<= 1;
+        const uint32_t rows_per_tile = 128 / pf_heads;
+        if (n_rows * 2 >= rows_per_tile) {
+            pf_tiles = (n_rows + rows_per_tile - 1) / rows_per_tile;
+            const uint32_t ctas = n_kv * gchunks * pf_tiles, tile = lc_tq_attn_prefill_tile_keys(hd, bits);
+            const uint32_t seen = len_max + (rows_per_tile < n_rows ? rows_per_tile : n_rows);   // keys of a tile of rows, at most
+            uint32_t most = (seen + tile - 1) / tile;   // at least a tile of keys per split
+            if (most > 64) most = 64;
+            n_splits = ctas < sms ? sms / ctas : 1;
+            if (n_splits > most) n_splits = most;
+        }
+    }
+    const bool pf = pf_tiles != 0;
     const bool queue = chunk != 0;
-    const bool direct = !queue && n_splits == 1 && !fused;
+    const bool direct = !queue && !pf && n_splits == 1 && !fused;
     // The tensor-core kernel merges up to 8 splits itself (one thread-block cluster per lane and kv head, exchange
     // through distributed shared memory, inverse rotation in the kernel): one launch instead of split + merge, the same
     // arithmetic in the same order, bit-identical output.  Alone 57 vs 59 us at 8193 keys x 64 lanes, 12.4 vs 14.6 us
@@ -495,7 +513,7 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     // weight prefetch ahead of their dependency wait it was the slower form in situ, 3.48 vs 3.36 ms.)
     // LOCAL_CUDA_ATTN_CLUSTER=0 selects the two-launch form.
     static const bool cluster_allowed = []() { const char *e = getenv("LOCAL_CUDA_ATTN_CLUSTER"); return !(e && e[0] == '0'); }();
-    const bool cluster_merge = use_mma && !queue && cluster_allowed && n_splits <= 8 && out_vec;
+    const bool cluster_merge = use_mma && !queue && !pf && cluster_allowed && n_splits <= 8 && out_vec;
 
     if (!direct && !cluster_merge) {
         const size_t rows_y = (size_t)n_kv * gchunks;
@@ -516,6 +534,7 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     p.queue_chunk = chunk;
     p.n_lanes = n_lanes;
     p.counters = k->counters;
+    p.pf_heads = pf_heads;
     p.cluster_merge = cluster_merge ? 1 : 0;
     p.partial = (float *)k->scratch;
     p.positions = positions ? (const uint32_t *)positions->dptr : nullptr;
@@ -545,7 +564,9 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
         grid = dim3(per_y < n_lanes * n_splits ? per_y : n_lanes * n_splits, grid.y, 1);
     }
     int st;
-    if (use_mma) {
+    if (pf) {
+        st = lc_tq_attn_prefill_launch(b, p, dim3(n_splits, n_kv * gchunks, pf_tiles), hd, bits);
+    } else if (use_mma) {
         st = lc_tq_attn_mma_launch(b, p, grid, hd, bits);
     } else {
         switch (hd) {
@@ -791,6 +812,7 @@ extern "C" int lc_tq_attention_noalloc_into(lc_batch *b, const lc_buf *q, const 
     p.queue_chunk = 0;
     p.n_lanes = 1;
     p.counters = nullptr;
+    p.pf_heads = 1;
     p.rq = nullptr;
     p.q = (const __half *)q->dptr;
     p.signs = (const float *)signs->dptr;

@@ -39,8 +39,9 @@ struct TqAttnParams {
     // keys (lc_attn_items) and a grid of one CTA per SM draws them from a ticket counter; a merge launch follows.
     // counters: gridDim.y tickets, zero between launches.  n_splits is then the row length of the partial buffer: the
     // most items a lane can have.
-    uint32_t queue_chunk, n_lanes;
+    uint32_t queue_chunk, n_lanes;   // n_lanes: lanes, or query rows of a prefill chunk
     unsigned int *counters;
+    uint32_t pf_heads;   // prefill kernel: MMA rows per query row (heads of a chunk, rounded up to a power of two)
 };
 constexpr uint32_t LC_ATTN_QUEUE_LANES = 512;   // most lanes of the queue form (its schedule lives in shared memory)
 
@@ -62,6 +63,12 @@ __host__ __device__ __forceinline__ uint32_t lc_attn_items(uint32_t n, uint32_t 
 // grid = (n_splits, n_kv * gchunks, n_lanes) with 8 q-heads per chunk; queue form: (CTAs, n_kv * gchunks, 1).
 bool lc_tq_attn_mma_supported(uint32_t head_dim, uint32_t bits);
 int lc_tq_attn_mma_launch(lc_batch *b, const TqAttnParams &p, dim3 grid, uint32_t head_dim, uint32_t bits);
+
+// Prefill variant (attention_tq_pf.cu): 128 / pf_heads query rows per CTA; grid = (n_splits, n_kv * gchunks, row tiles); a merge
+// launch follows.
+bool lc_tq_attn_prefill_supported(uint32_t head_dim, uint32_t bits);
+uint32_t lc_tq_attn_prefill_tile_keys(uint32_t head_dim, uint32_t bits);
+int lc_tq_attn_prefill_launch(lc_batch *b, const TqAttnParams &p, dim3 grid, uint32_t head_dim, uint32_t bits);
 
 // Library-internal forms used by the decode step: lc_qkv_post_batched_into that also leaves the query fragments
 // described at TqAttnParams::qfrag in `qfrag` (n_lanes * n_q_heads * head_dim * 4 bytes; requires head_dim 256 and n_q_heads / n_kv_heads a multiple of 8), and lc_tq_attention_batched_into that reads them.
