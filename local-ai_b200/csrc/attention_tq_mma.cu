@@ -56,10 +56,11 @@ struct AttnCfg {
     static constexpr int ENT_BYTES = NENT * 8;
     static constexpr int ACC_BYTES = NW * NS * 4 * 32 * 4;   // merge staging, reuses query and ring memory
     static constexpr int RING_OFF = LUT_BYTES + Q_BYTES + ENT_BYTES;
-    // the CTA's merged tile: four floats of padding after every HD / 8 dims (its writers' lanes are HD / 8 dims apart)
-    static constexpr int CPS = HD + 32;
-    static constexpr int TAIL_BYTES = (3 * NW * G + 2 * G) * 4 + G * CPS * 4;  // weights of the warp merge, the merged tile
-    static __device__ __forceinline__ int cp_index(int h, int d) { return h * CPS + d + 4 * (d / (HD / 8)); }
+    // Merged rows (a head of one split): four floats of padding after every HD / 8 dims (their writers' lanes are HD / 8 dims
+    // apart).  A CTA of a cluster of n receives n rows for each of its ceil(8 / n) heads, at most 14.
+    static constexpr int CPS = HD + 40, ROWS = 14;
+    static constexpr int TAIL_BYTES = (2 * NW * G + 2 * ROWS) * 4 + ROWS * CPS * 4;  // (max, sum) of warps and rows, the rows
+    static __device__ __forceinline__ int cp_index(int row, int d) { return row * CPS + d + 4 * (d / (HD / 8)); }
     static constexpr int RING_ROOM = 222 * 1024 - TAIL_BYTES - RING_OFF;
     static constexpr int DEPTH_FIT = RING_ROOM / (NW * STAGE);
     static constexpr int DEPTH = DEPTH_FIT > 4 ? 4 : DEPTH_FIT;   // ring slots per warp (DEPTH - 1 tiles in flight)
@@ -83,8 +84,17 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+// the same place in the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(addr), "r"(rank));
+    return ra;
+}
+__device__ __forceinline__ void st_cluster_f2(uint32_t a, float x, float y) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(a), "f"(x), "f"(y) : "memory");
 }
 __device__ __forceinline__ uint2 lds64(uint32_t a) {
     uint2 v;
@@ -127,29 +137,6 @@ __device__ __forceinline__ uint32_t field_addr(const uint32_t (&w)[N], uint32_t 
     else idx = (w[i] >> o) & ((1u << FB) - 1u);
     asm("mad.lo.u32 %0, %1, %2, %3;\n" : "=r"(r) : "r"(idx), "n"(LUT_COPIES * 8), "r"(lane_base));
     return r;
-}
-// a shared-memory word / 16 bytes of CTA `rank` of this cluster (or of this CTA when the launch is not clustered)
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t rank, bool clustered) {
-    float v;
-    if (clustered) {
-        uint32_t ra;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(addr), "r"(rank));
-        asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(ra));
-    } else {
-        asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(v) : "r"(addr));
-    }
-    return v;
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank, bool clustered) {
-    float4 v;
-    if (clustered) {
-        uint32_t ra;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(addr), "r"(rank));
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ra));
-    } else {
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-    }
-    return v;
 }
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
     uint32_t d;
@@ -201,6 +188,7 @@ template <typename C>
 __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p) {
     constexpr int HD = C::HD, CB = C::CB, NW = C::NW, NT = C::NT, KT = C::KT, MT = C::MT, NS = C::NS, DPL = C::DPL, FB = C::FB;
     lc_pdl_trigger();
+    if (p.cluster_merge) cluster_arrive_relaxed();   // awaited before the first store to a peer's shared memory
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t base_a = smem_u32(smem);
     uint2 *lut = reinterpret_cast<uint2 *>(smem);                       // [NENT][16 copies]
@@ -681,51 +669,60 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
         // the next ticket, drawn as late as hides the round trip: items are then handed out in the order of need
         if (queue && threadIdx.x == 0) ticket = atomicAdd(&p.counters[blockIdx.y], 1u);
 
-        // ---- merge the 8 warps; query and ring memory is reused for the per-warp accumulators ----
+        // ---- merge the warps that had keys; query and ring memory is reused for their accumulators.  A step of the decode
+        //      model comes here after one or two tiles per warp, with this code cold in the instruction cache: it is
+        //      kept short (with the finish below 12.4 -> 10.1 us for 64 lanes x 512 keys, 9.5 -> 7.9 us for one lane). ----
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             l_part[h] += __shfl_xor_sync(0xffffffffu, l_part[h], 4);
             l_part[h] += __shfl_xor_sync(0xffffffffu, l_part[h], 8);
             l_part[h] += __shfl_xor_sync(0xffffffffu, l_part[h], 16);
         }
-        __syncthreads();   // every warp is done with its ring
-        float *acc_s = reinterpret_cast<float *>(smem + C::LUT_BYTES);                   // [NW][NS][4][32 lanes]
-        float *m_s = reinterpret_cast<float *>(smem + C::TAIL_OFF);                      // [NW][G]
+        float *acc_s = reinterpret_cast<float *>(smem + C::LUT_BYTES);   // [NW][NS][32 lanes][4]: fragment order
+        float *m_s = reinterpret_cast<float *>(smem + C::TAIL_OFF);      // [NW][G]
         float *l_s = m_s + NW * G;
-        if (g == 0) {
-            m_s[warp * G + 2 * t] = m_run[0];
-            m_s[warp * G + 2 * t + 1] = m_run[1];
-            l_s[warp * G + 2 * t] = l_part[0];
-            l_s[warp * G + 2 * t + 1] = l_part[1];
-        }
-        // Accumulators go to shared memory in fragment order [warp][s][j][lane] (conflict-free both ways).
-#pragma unroll
-        for (int s = 0; s < NS; s++) {
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc_s[((warp * NS + s) * 4 + j) * 32 + lane] = o[s][j];
-        }
-        __syncthreads();
-        // Per (warp, head) weights exp(m_w - max) and the merged (max, sum); thread h < G does head h.
-        float *f_s = l_s + NW * G;       // [NW][G]
-        float *ml_s = f_s + NW * G;      // [G][2]
-        float *cpart = ml_s + 2 * G;     // this CTA's merged, unnormalised tile (cp_index)
-        if (threadIdx.x < G) {
-            const int h = threadIdx.x;
-            float gmax = -INFINITY;
-#pragma unroll
-            for (int w = 0; w < NW; w++) gmax = fmaxf(gmax, m_s[w * G + h]);
-            float gsum = 0.f;
+        float *ml_s = l_s + NW * G;                                      // [ROWS][2]
+        float *cpart = ml_s + 2 * C::ROWS;                               // merged, unnormalised rows (cp_index)
+        if (g == 0) *reinterpret_cast<float2 *>(m_s + warp * G + 2 * t) = make_float2(m_run[0], m_run[1]);
+        __syncthreads();   // every warp is done with its ring, and its maximum is known
+        const uint32_t tiles_all = k_end > k_begin ? (k_end - k_begin + KT - 1) / KT : 0u;
+        const int nwa = tiles_all < (uint32_t)NW ? (int)tiles_all : NW;
+        {
+            float g0 = -INFINITY, g1 = -INFINITY;
 #pragma unroll
             for (int w = 0; w < NW; w++) {
-                const float mw = m_s[w * G + h];
-                const float f = (mw == -INFINITY) ? 0.f : soft_exp<C::BITS>(mw - gmax);
-                f_s[w * G + h] = f;
-                gsum += f * l_s[w * G + h];
+                const float2 v = *reinterpret_cast<const float2 *>(m_s + w * G + 2 * t);
+                g0 = fmaxf(g0, v.x);
+                g1 = fmaxf(g1, v.y);
             }
-            ml_s[2 * h] = gmax;
-            ml_s[2 * h + 1] = gsum;
+            const float f0 = m_run[0] == -INFINITY ? 0.f : soft_exp<C::BITS>(m_run[0] - g0);
+            const float f1 = m_run[1] == -INFINITY ? 0.f : soft_exp<C::BITS>(m_run[1] - g1);
+            if (g == 0) *reinterpret_cast<float2 *>(l_s + warp * G + 2 * t) = make_float2(f0 * l_part[0], f1 * l_part[1]);
+            if (warp < nwa) {
+                float4 *dst = reinterpret_cast<float4 *>(acc_s) + warp * NS * 32 + lane;
+#pragma unroll
+                for (int s = 0; s < NS; s++) dst[s * 32] = make_float4(o[s][0] * f0, o[s][1] * f1, o[s][2] * f0, o[s][3] * f1);
+            }
         }
+        // Head h's row: of this CTA alone row h; in a cluster row (h / n) * n + split of CTA h mod n, which finishes head h.
+        auto row_of = [&](int h) -> int { return p.cluster_merge ? (h / (int)p.n_splits) * (int)p.n_splits + (int)split : h; };
+        auto peer_addr = [&](const float *a, int h) -> uint32_t { return cluster_addr(smem_u32(a), (uint32_t)h % p.n_splits); };
+        if (p.cluster_merge) cluster_wait();   // (of the arrival at the start) every CTA of the cluster runs
         __syncthreads();
+        if (threadIdx.x < G) {   // merged (max, sum) of head h
+            const int h = threadIdx.x;
+            float gmax = -INFINITY, gsum = 0.f;
+#pragma unroll
+            for (int w = 0; w < NW; w++) {
+                gmax = fmaxf(gmax, m_s[w * G + h]);
+                gsum += l_s[w * G + h];
+            }
+            float *dst = ml_s + 2 * row_of(h);
+            if (p.cluster_merge)
+                st_cluster_f2(peer_addr(dst, h), gmax, gsum);
+            else
+                *reinterpret_cast<float2 *>(dst) = make_float2(gmax, gsum);
+        }
         const size_t part_row = HD + 2;
         const uint32_t it_lane = lane_idx, it_split = split;
         // where head h's partial of this split goes
@@ -733,18 +730,91 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
             const size_t qh = (size_t)it_lane * p.n_q + qh0 + h;
             return p.partial + (qh * p.n_splits + sp) * part_row;
         };
-        // Thread (warp, lane) merges fragment position `lane` of its tiles s: element j of tile s is
-        // head 2t + (j & 1), dim (HD / 8) g + 2 s + (j >> 1).
-        for (int s = warp; s < NS; s += NW) {
+        // Thread (warp, lane) adds fragment position `lane` of its tiles s: heads 2t and 2t + 1 at dims (HD / 8) g + 2 s + 0, 1.
+        {
+            constexpr int TW = NS / NW;
+            float4 acc[TW];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int h = 2 * t + (j & 1);
-                const int d = (HD / 8) * g + 2 * s + (j >> 1);
-                float acc = 0.f;
+            for (int i = 0; i < TW; i++) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 *src = reinterpret_cast<const float4 *>(acc_s) + warp * 32 + lane;
 #pragma unroll
-                for (int w = 0; w < NW; w++) acc += f_s[w * G + h] * acc_s[((w * NS + s) * 4 + j) * 32 + lane];
-                cpart[C::cp_index(h, d)] = acc;
+            for (int w = 0; w < NW; w++) {
+#pragma unroll
+                for (int i = 0; i < TW; i++) {
+                    const float4 v = w < nwa ? src[(w * NS + i * NW) * 32] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    acc[i].x += v.x; acc[i].y += v.y; acc[i].z += v.z; acc[i].w += v.w;
+                }
             }
+            float *r0 = cpart + C::cp_index(row_of(2 * t), (HD / 8) * g), *r1 = cpart + C::cp_index(row_of(2 * t + 1), (HD / 8) * g);
+            if (p.cluster_merge) {
+                const uint32_t a0 = peer_addr(r0, 2 * t), a1 = peer_addr(r1, 2 * t + 1);
+#pragma unroll
+                for (int i = 0; i < TW; i++) {
+                    st_cluster_f2(a0 + (uint32_t)(warp + i * NW) * 8u, acc[i].x, acc[i].z);
+                    st_cluster_f2(a1 + (uint32_t)(warp + i * NW) * 8u, acc[i].y, acc[i].w);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < TW; i++) {
+                    *reinterpret_cast<float2 *>(r0 + 2 * (warp + i * NW)) = make_float2(acc[i].x, acc[i].z);
+                    *reinterpret_cast<float2 *>(r1 + 2 * (warp + i * NW)) = make_float2(acc[i].y, acc[i].w);
+                }
+            }
+        }
+        if (p.cluster_merge) {
+            // The splits of this (lane, kv head) are one cluster, and every row this CTA finishes is in its own shared memory
+            // after the barrier: nobody reads a peer's, so there is no second barrier.  One warp per head: the same arithmetic,
+            // in the same order, as tq_attn_merge_kernel (attention_tq.cu).
+            const int n = (int)p.n_splits;
+            float4 sg[DPL / 4];   // (the load's round trip passes at the barrier)
+            if (p.fused_q) {
+#pragma unroll
+                for (int i = 0; i < DPL / 4; i++) sg[i] = *reinterpret_cast<const float4 *>(p.signs + DPL * lane + 4 * i);
+            }
+            cluster_arrive_release();
+            cluster_wait();
+            for (int h = (int)split + n * warp; h < gvalid; h += n * NW) {
+                const int row0 = (h / n) * n;
+                const float2 ml = lane < n ? *reinterpret_cast<const float2 *>(ml_s + 2 * (row0 + lane)) : make_float2(-INFINITY, 0.f);
+                float gmax = ml.x;
+                gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 1));
+                gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 2));
+                gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 4));
+                const float fl = ml.x == -INFINITY ? 0.f : expf(ml.x - gmax);   // (lanes past the eighth hold nothing)
+                float gsum = 0.f, ov[DPL];
+#pragma unroll
+                for (int i = 0; i < DPL; i++) ov[i] = 0.f;
+#pragma unroll 2
+                for (int sp = 0; sp < n; sp++) {
+                    const float f = __shfl_sync(0xffffffffu, fl, sp);
+                    gsum += f * __shfl_sync(0xffffffffu, ml.y, sp);
+#pragma unroll
+                    for (int i = 0; i < DPL; i += 4) {
+                        const float4 v = *reinterpret_cast<const float4 *>(cpart + C::cp_index(row0 + sp, DPL * lane + i));
+                        ov[i] += f * v.x; ov[i + 1] += f * v.y; ov[i + 2] += f * v.z; ov[i + 3] += f * v.w;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < DPL; i++) ov[i] = gsum > 0.f ? ov[i] / gsum : 0.f;
+                const size_t qh = (size_t)it_lane * p.n_q + qh0 + h;
+                if (!p.fused_q) {
+#pragma unroll
+                    for (int i = 0; i < DPL; i += 4)
+                        *reinterpret_cast<float4 *>(p.out + qh * HD + DPL * lane + i) = make_float4(ov[i], ov[i + 1], ov[i + 2], ov[i + 3]);
+                    continue;
+                }
+                // inverse rotation, 1/sqrt(d), signs
+                warp_fwht<DPL>(ov, lane);
+                const float inv = 1.0f / sqrtf((float)HD);
+#pragma unroll
+                for (int i = 0; i < DPL; i += 4) {
+                    uint2 packed;
+                    packed.x = pack_h2(ov[i] * inv * sg[i / 4].x, ov[i + 1] * inv * sg[i / 4].y);
+                    packed.y = pack_h2(ov[i + 2] * inv * sg[i / 4].z, ov[i + 3] * inv * sg[i / 4].w);
+                    *reinterpret_cast<uint2 *>(p.out_f16 + qh * HD + DPL * lane + i) = packed;
+                }
+            }
+            return;
         }
         __syncthreads();   // the tile is complete; the ring is free
         if (queue) {
@@ -756,91 +826,21 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
         } else {
             more = false;
         }
-        if (!p.cluster_merge) {   // a merge launch follows (unless there is nothing to merge)
-            for (int e = threadIdx.x; e < gvalid * (HD / 2); e += NT) {
-                const int h = e / (HD / 2), d = 2 * (e % (HD / 2));
-                const float2 v = *reinterpret_cast<const float2 *>(cpart + C::cp_index(h, d));
-                if (p.direct_out) {
-                    const float gsum = ml_s[2 * h + 1];
-                    float *dst = p.out + ((size_t)it_lane * p.n_q + qh0 + h) * HD + d;
-                    dst[0] = gsum > 0.f ? v.x / gsum : 0.f;
-                    dst[1] = gsum > 0.f ? v.y / gsum : 0.f;
-                } else {
-                    *reinterpret_cast<float2 *>(part_of(h, it_split) + 2 + d) = v;
-                }
-            }
-            if (!p.direct_out && threadIdx.x < gvalid)
-                *reinterpret_cast<float2 *>(part_of(threadIdx.x, it_split)) = make_float2(ml_s[2 * threadIdx.x], ml_s[2 * threadIdx.x + 1]);
-            continue;
-        }
-        // The splits of this (lane, kv head) are one cluster: head h is finished by CTA h mod n_splits.
-        if (p.n_splits > 1) cluster_sync();
-        // One warp per head: the same arithmetic, in the same order, as tq_attn_merge_kernel (attention_tq.cu).
-        const bool clustered = p.n_splits > 1;
-        const uint32_t ml_a = smem_u32(ml_s), cp_a = smem_u32(cpart);
-        for (int h = (int)it_split + (int)p.n_splits * warp; h < gvalid; h += (int)p.n_splits * NW) {
-            // (loads of several splits in flight together: a read of a peer's shared memory takes most of a microsecond)
-            float ms[8], ls[8], gmax = -INFINITY;
-#pragma unroll
-            for (int sp = 0; sp < 8; sp++) {
-                ms[sp] = -INFINITY;
-                ls[sp] = 0.f;
-                if (sp < (int)p.n_splits) {
-                    ms[sp] = ld_cluster_f32(ml_a + (2 * h) * 4, sp, clustered);
-                    ls[sp] = ld_cluster_f32(ml_a + (2 * h + 1) * 4, sp, clustered);
-                }
-            }
-#pragma unroll
-            for (int sp = 0; sp < 8; sp++) gmax = fmaxf(gmax, ms[sp]);
-            float gsum = 0.f, ov[DPL];
-#pragma unroll
-            for (int i = 0; i < DPL; i++) ov[i] = 0.f;
-#pragma unroll
-            for (int s0 = 0; s0 < 8; s0 += 4) {
-                if (s0 < (int)p.n_splits) {
-                    float4 a[4][DPL / 4];
-#pragma unroll
-                    for (int sp = 0; sp < 4; sp++)
-#pragma unroll
-                        for (int i = 0; i < DPL; i += 4)
-                            a[sp][i / 4] = s0 + sp < (int)p.n_splits ? ld_cluster_f4(cp_a + C::cp_index(h, DPL * lane + i) * 4, s0 + sp, clustered)
-                                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                    for (int sp = 0; sp < 4; sp++) {
-                        if (s0 + sp < (int)p.n_splits) {
-                            const float f = (ms[s0 + sp] == -INFINITY) ? 0.f : expf(ms[s0 + sp] - gmax);
-                            gsum += f * ls[s0 + sp];
-#pragma unroll
-                            for (int i = 0; i < DPL; i += 4) {
-                                const float4 v = a[sp][i / 4];
-                                ov[i] += f * v.x; ov[i + 1] += f * v.y; ov[i + 2] += f * v.z; ov[i + 3] += f * v.w;
-                            }
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < DPL; i++) ov[i] = gsum > 0.f ? ov[i] / gsum : 0.f;
-            const size_t qh = (size_t)it_lane * p.n_q + qh0 + h;
-            if (!p.fused_q) {
-#pragma unroll
-                for (int i = 0; i < DPL; i += 4)
-                    *reinterpret_cast<float4 *>(p.out + qh * HD + DPL * lane + i) = make_float4(ov[i], ov[i + 1], ov[i + 2], ov[i + 3]);
-                continue;
-            }
-            // inverse rotation, 1/sqrt(d), signs
-            warp_fwht<DPL>(ov, lane);
-            const float inv = 1.0f / sqrtf((float)HD);
-#pragma unroll
-            for (int i = 0; i < DPL; i += 4) {
-                const float4 sg = *reinterpret_cast<const float4 *>(p.signs + DPL * lane + i);
-                uint2 packed;
-                packed.x = pack_h2(ov[i] * inv * sg.x, ov[i + 1] * inv * sg.y);
-                packed.y = pack_h2(ov[i + 2] * inv * sg.z, ov[i + 3] * inv * sg.w);
-                *reinterpret_cast<uint2 *>(p.out_f16 + qh * HD + DPL * lane + i) = packed;
+        // a merge launch follows (unless there is nothing to merge)
+        for (int e = threadIdx.x; e < gvalid * (HD / 2); e += NT) {
+            const int h = e / (HD / 2), d = 2 * (e % (HD / 2));
+            const float2 v = *reinterpret_cast<const float2 *>(cpart + C::cp_index(h, d));
+            if (p.direct_out) {
+                const float gsum = ml_s[2 * h + 1];
+                float *dst = p.out + ((size_t)it_lane * p.n_q + qh0 + h) * HD + d;
+                dst[0] = gsum > 0.f ? v.x / gsum : 0.f;
+                dst[1] = gsum > 0.f ? v.y / gsum : 0.f;
+            } else {
+                *reinterpret_cast<float2 *>(part_of(h, it_split) + 2 + d) = v;
             }
         }
-        if (p.n_splits > 1) cluster_sync();   // no CTA leaves while a peer may still read its shared memory
+        if (!p.direct_out && threadIdx.x < gvalid)
+            *reinterpret_cast<float2 *>(part_of(threadIdx.x, it_split)) = make_float2(ml_s[2 * threadIdx.x], ml_s[2 * threadIdx.x + 1]);
     }
 }
 
@@ -860,7 +860,7 @@ int launch(lc_batch *b, const TqAttnParams &p, dim3 grid) {
         attr[na].val.programmaticStreamSerializationAllowed = 1;
         na++;
     }
-    if (p.cluster_merge && p.n_splits > 1) {
+    if (p.cluster_merge) {
         attr[na].id = cudaLaunchAttributeClusterDimension;
         attr[na].val.clusterDim.x = p.n_splits;
         attr[na].val.clusterDim.y = 1;
