@@ -1,0 +1,122 @@
+"""The tensor-core kernels at the sizes where their tiling can go wrong: tile edges, remainders, the smallest and the
+largest of each dispatch range, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from gpu_util import Guarded, rel_close
+from test_attention_gpu import Cache, f16_case
+from test_matvec_gpu import device_status_ok, run_matmul
+from test_turboquant_gpu import gpu_encode
+
+pytestmark = pytest.mark.gpu
+
+
+# m <= 16: one 8- or 16-row tile; K in 32- (Q4_0) or 256-wide (TQ2_0) blocks, uneven over the warps; ragged last rows of W.
+# m > 64, and Q4_0 from 17: 128-row weight tiles, batch tiles of 64 / 128 columns, K splits with a remainder.
+@pytest.mark.parametrize("fmt,m,k,n", [
+    ("q4_0", 1, 32, 1), ("q4_0", 8, 96, 65), ("q4_0", 9, 1536, 129), ("q4_0", 16, 2080, 63), ("q4_0", 16, 6144, 1537),
+    ("tq2_0", 9, 256, 127), ("tq2_0", 16, 768, 8193), ("tq2_0", 13, 2048, 33), ("tq2_0", 16, 6144, 1537),
+    ("q4_0", 17, 96, 127), ("q4_0", 64, 1568, 129), ("q4_0", 65, 32, 1), ("q4_0", 129, 2080, 130), ("q4_0", 257, 1536, 300),
+    ("tq2_0", 65, 256, 127), ("tq2_0", 128, 1536, 129), ("tq2_0", 129, 6144, 260), ("tq2_0", 300, 768, 1)])
+def test_quantised_matmul_at_tile_edges(la, orc, ctx, kernels, fmt, m, k, n):
+    raw = (la.synth.q4_0_weights if fmt == "q4_0" else la.synth.tq2_0_weights)(n, k, 31)
+    a = la.synth.normal_f16((m, k), 32)
+    want = orc.matmul_nt(orc.Q4_0 if fmt == "q4_0" else orc.TQ2_0, a, raw, m, k, n)
+    rel_close(run_matmul(la, ctx, kernels, f"matmul_nt_{fmt}_into", a, raw, m, k, n), want, 1e-3, f"{fmt} m={m} k={k} n={n}")
+    if fmt == "q4_0":
+        rel_close(run_matmul(la, ctx, kernels, "matmul_nt_q4_0_f32out_into", a, raw, m, k, n, f32out=True), want, 5e-4, "f32 out")
+    device_status_ok(kernels)
+
+
+@pytest.mark.parametrize("hd,n_q,n_kv,bits,total,window,ring", [
+    (128, 8, 1, 2, 33, 0, 0), (128, 8, 1, 3, 1025, 0, 0), (128, 12, 2, 4, 2600, 0, 0), (512, 8, 1, 2, 17, 0, 0),
+    (512, 6, 2, 3, 700, 300, 0), (512, 4, 2, 4, 513, 0, 0), (256, 5, 1, 3, 1600, 512, 512), (256, 10, 1, 4, 4097, 0, 0)])
+def test_code_attention_head_sizes_and_code_widths(la, orc, ctx, kernels, hd, n_q, n_kv, bits, total, window, ring):
+    c = Cache(la, orc, ctx, hd, n_kv, bits, ring or total, seed=41 + total)
+    c.fill_single(total, ring)
+    kc, kn, vc, vn, lv, _ = c.device()
+    rq = orc.hadamard_rotate(la.synth.normal(43, n_q * hd).astype(np.float32), c.signs, hd, n_q, True, False)
+    out = Guarded(la, ctx, n_q * hd * 4)
+    b = la.CommandBatch.new(ctx)
+    kernels.flash_attention_tq_into(b, la.CudaBuffer.from_slice(ctx, rq), kc, kn, vc, vn, lv, out.view, hd, total, total - 1,
+                                    n_q, n_kv, window, bits, ring, 0.0625)
+    b.commit_and_wait()
+    want = orc.flash_attention_tq(rq, c.kc, c.kn, c.vc, c.vn, c.levels, hd, total, total - 1, n_q, n_kv, window, bits, ring, 0.0625)
+    rel_close(out.read(np.float32), want, 1e-3, "attention over codes")
+
+
+@pytest.mark.parametrize("hd,n_q,n_kv,bits", [(256, 8, 1, 4), (128, 8, 2, 2)])
+def test_ragged_pool_attention_in_work_items(la, orc, ctx, kernels, hd, n_q, n_kv, bits):
+    """Pools of ten lanes or more and over 2048 keys: lanes are cut into items that the CTAs draw.  Twice with the same
+    object: the draw's counters are back at zero."""
+    cap = 2600
+    positions = np.array([0, 31, 255, 256, 700, 1023, 2047, 2048, 2598, 2599, 5, 1800], np.uint32)
+    n = positions.size
+    c = Cache(la, orc, ctx, hd, n_kv, bits, n * cap, seed=90)
+    c.fill_pool(positions, cap, 0)
+    kc, kn, vc, vn, lv, sg = c.device()
+    q = la.synth.normal_f16((n, n_q, hd), 91)
+    want = orc.tq_attention_fused(q, c.kc, c.kn, c.vc, c.vn, c.levels, c.signs, positions, hd, cap, n_q, n_kv, 0, bits, n, 0, 0.0625)
+    outs = []
+    for _ in range(2):
+        out = Guarded(la, ctx, n * n_q * hd * 2)
+        b = la.CommandBatch.new(ctx)
+        kernels.tq_attention_batched_into(b, la.CudaBuffer.from_slice(ctx, q), kc, kn, vc, vn, lv, sg, out.view,
+                                          la.CudaBuffer.from_slice(ctx, positions), hd, cap, n_q, n_kv, 0, bits, n, 0, 0.0625)
+        b.commit_and_wait()
+        outs.append(out.read(np.float16))
+        rel_close(outs[-1], want.astype(np.float32), 2e-3, "ragged pool")
+    assert np.array_equal(outs[0].view(np.uint16), outs[1].view(np.uint16))
+
+
+# 128 rows (query rows x heads, heads rounded up to a power of two) to a tile, 32 or 64 keys to a step
+@pytest.mark.parametrize("hd,n_q,n_kv,bits,rows,start,window", [
+    (256, 8, 1, 2, 8, 0, 0), (256, 8, 1, 2, 17, 63, 0), (256, 8, 1, 4, 33, 500, 128), (256, 3, 1, 3, 16, 31, 0),
+    (256, 16, 2, 2, 65, 1000, 512), (128, 8, 2, 3, 32, 95, 0), (128, 12, 1, 4, 40, 300, 64), (128, 2, 1, 2, 130, 1, 0)])
+def test_prefill_attention_at_tile_edges(la, orc, ctx, kernels, hd, n_q, n_kv, bits, rows, start, window):
+    total = start + rows
+    c = Cache(la, orc, ctx, hd, n_kv, bits, total, seed=60 + total)
+    c.fill_single(total, 0)
+    kc, kn, vc, vn, lv, sg = c.device()
+    q = la.synth.normal_f16((rows, n_q, hd), 61)
+    rq = orc.hadamard_rotate(q.astype(np.float32), c.signs, hd, rows * n_q, True, False)
+    want = orc.flash_attention_tq_prefill(rq, c.kc, c.kn, c.vc, c.vn, c.levels, hd, total, start, rows, n_q, n_kv, window, bits, 0, 0.0625)
+    out, fused = Guarded(la, ctx, rows * n_q * hd * 4), Guarded(la, ctx, rows * n_q * hd * 2)
+    b = la.CommandBatch.new(ctx)
+    kernels.flash_attention_tq_prefill_into(b, la.CudaBuffer.from_slice(ctx, rq), kc, kn, vc, vn, lv, out.view, hd, total, start, rows,
+                                            n_q, n_kv, window, bits, 0, 0.0625)
+    kernels.tq_attention_prefill_into(b, la.CudaBuffer.from_slice(ctx, q), kc, kn, vc, vn, lv, sg, fused.view, hd, total, start, rows,
+                                      n_q, n_kv, window, bits, 0, 0.0625)
+    b.commit_and_wait()
+    rel_close(out.read(np.float32), want, 1e-3, "prefill")
+    back = orc.hadamard_rotate(want, c.signs, hd, rows * n_q, False, True)
+    rel_close(fused.read(np.float16), back.astype(np.float16).astype(np.float32), 2e-3, "fused prefill")
+    device_status_ok(kernels)
+
+
+@pytest.mark.parametrize("hd,n_q,n_kv,total,window", [(64, 8, 1, 1, 0), (64, 6, 2, 1001, 0), (128, 16, 1, 63, 0), (256, 8, 1, 8191, 0),
+                                                      (512, 8, 2, 129, 0), (256, 7, 1, 700, 333)])
+def test_f16_attention_at_odd_lengths(la, orc, ctx, kernels, hd, n_q, n_kv, total, window):
+    q, k, v = f16_case(la, hd, n_q, n_kv, total, 71)
+    out = Guarded(la, ctx, n_q * hd * 2)
+    f = lambda x: la.CudaBuffer.from_slice(ctx, x)
+    if window:
+        kernels.attention_sliding(ctx, f(q), f(k), f(v), out.view, hd, total, total - 1, window, n_q, n_kv)
+    else:
+        b = la.CommandBatch.new(ctx)
+        kernels.flash_decoding_into(ctx, b, f(q), f(k), f(v), out.view, hd, total, total - 1, n_q, n_kv)
+        b.commit_and_wait()
+    rel_close(out.read(np.float16), orc.attention_f16(q, k, v, hd, total, total - 1, n_q, n_kv, window).astype(np.float32), 2e-3, "f16")
+
+
+@pytest.mark.parametrize("hd", [128, 256, 512])
+@pytest.mark.parametrize("rows", [1, 7, 9, 65])
+def test_encoder_rows_at_block_edges(la, orc, ctx, kernels, hd, rows):
+    bits, n_kv = 2 + rows % 3, 1
+    levels, signs = la.tq_levels(hd, bits), la.tq_signs(hd, la.TQ_SEED)
+    x = la.synth.normal_f16((rows, n_kv, hd), 81)
+    cb = la.tq_code_bytes(hd, bits)
+    want_c, want_n = np.zeros(rows * cb, np.uint8), np.zeros(rows, np.float16)
+    orc.encode_kv(x, levels, signs, want_c, want_n, hd, n_kv, rows, bits, 0, 0)
+    codes, norms = gpu_encode(la, ctx, kernels, x, levels, signs, hd, n_kv, rows, bits, 0, 0, rows)
+    assert np.array_equal(codes, want_c) and np.array_equal(norms, want_n.view(np.uint16))
