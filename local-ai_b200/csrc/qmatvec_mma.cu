@@ -6,22 +6,28 @@
 // A batch-1 matvec is HBM-bound in principle, but on CUDA cores the dequantisation costs 5-6 instructions per
 // weight and binds long before HBM does.  Here the multiply-adds run on mma.sync (the 1..8 batch rows take the
 // MMA's N = 8), which leaves about two integer instructions per four weights:
-//   * a persistent CTA streams groups of 64 consecutive weight rows -- one contiguous byte range, so every
-//     cp.async is a fully coalesced 16-byte piece and DRAM sees sequential reads -- through a three-slot ring;
-//   * the activations (8 rows x K) stay in shared memory for the whole launch;
+//   * a persistent CTA streams groups of 64 consecutive weight rows -- one contiguous byte range, so a group is one bulk
+//     copy and DRAM sees sequential reads -- through a ring of three slots; a warp of its own fetches, and the others
+//     meet it at mbarriers only, so a warp that is done with a group goes on to the next;
+//   * the activations (8 rows x K) stay in shared memory, or in registers, for the whole launch;
 //   * warp (rg, kq) of 16 owns rows 16 rg .. + 15 of the group and quarter kq of K; its threads turn 2-byte pieces
 //     of code bytes into A fragments in registers (thread t of a quad owns bytes 2t, 2t+1 of every 8-byte group);
-//   * the four K quarters are added through shared memory once per group and stored.
-// Numerics keep the exact-weight semantic of the CUDA-core kernels: TQ2_0 weights (q - 1) d are exact in f16;
-// for Q4_0 the A operand holds the integers q - 8, every 32-k block is accumulated on its own and scaled by d in
-// f32.  Accumulation is f32.
+//   * the four K quarters meet at a barrier of their four warps, and each adds and stores a quarter of the sums.
+// Numerics keep the exact-weight semantic of the CUDA-core kernels: the A operand holds the integers q - z (times 2^-9), every
+// block (Q4_0) or half block (TQ2_0) is accumulated on its own and scaled by d in f32.  Accumulation is f32.
+// Issue slots bound it: 2-byte shared loads, masks, one multiply-add per two weights.  262144 x 1536 Q4_0 at m = 1 takes 57.4 us
+// (3.95 TB/s); 67 us with cp.async by every thread, two barriers of the whole CTA per group and permutes for the conversion.
+// TQ2_0 gains more, as its conversion had a permute and a multiply per two weights: 90 matrices of 8192 x 1536 in one
+// launch 2.4 -> 1.6 us each.
 #include "lc_internal.h"
+#include "tcgen05_util.cuh"
 
 namespace {
 
 constexpr int FMT_Q4_0 = 0;
 constexpr int FMT_TQ2_0 = 1;
-constexpr int NW = 16, NT = NW * 32;
+constexpr int NW = 16, NT = (NW + 1) * 32;   // sixteen working warps and one that fetches
+constexpr uint32_t STREAM_WAIT_LIMIT = 1u << 22;
 constexpr int GROUP_ROWS = 64;       // rows per ring slot: 4 row groups of 16
 constexpr int SLOTS = 3;
 constexpr int UNIT_K = 128;          // K is split over the four warp quarters in units of 128 k
@@ -37,9 +43,9 @@ struct StreamParams {
     int groups;             // n_mat * gpm
     int xs;                 // bytes per activation row in shared memory
     int slot_bytes;         // bytes reserved per ring slot
+    int *status;
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t src_bytes = 16u) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
@@ -56,8 +62,15 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
 __device__ __forceinline__ void ldmatrix_x2(uint32_t &b0, uint32_t &b1, uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];\n" : "=r"(b0), "=r"(b1) : "r"(addr));
 }
-__device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t *>(&h); }
-__device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<__half2 *>(&u); }
+// two codes, BITS wide at bit BITS * l of each half of w, as f16 (q - Z) 2^-9: in place they are the f16 subnormals
+// q 2^(BITS l - 24), which one multiply-add moves to the common scale, exactly
+template <int BITS, int Z>
+__device__ __forceinline__ uint32_t codes_f16(uint32_t w, int l) {
+    constexpr uint32_t one = (1u << BITS) - 1u;
+    const uint32_t v = w & ((one | one << 16) << (BITS * l));
+    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&v), __float2half2_rn((float)(1 << (15 - BITS * l))), __float2half2_rn(-(float)Z / 512.0f));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
 __device__ __forceinline__ void store_c(__half *p, float v) { *p = __float2half_rn(v); }
 __device__ __forceinline__ void store_c(float *p, float v) { *p = v; }
 __device__ __forceinline__ uint32_t lds_u16(const uint8_t *p) { return *reinterpret_cast<const uint16_t *>(p); }
@@ -82,28 +95,37 @@ __global__ void __launch_bounds__(NT, 1) qgemv_mma_stream_kernel(const __grid_co
     uint8_t *ring = smem + 8 * p.xs + 2 * NW * 32 * 16;               // [SLOTS][slot_bytes]
     const int my_groups = (p.groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
-    // group `it` of this CTA: group (blockIdx.x + it gridDim.x) of the launch = rows 64 gi .. of matrix mi; one
-    // contiguous byte range
+    __shared__ __align__(8) uint64_t full_s[SLOTS], empty_s[SLOTS];
+    __shared__ int abort_s;
+    volatile int *abort_flag = &abort_s;
+    const uint32_t full = smem_u32(full_s), empty = smem_u32(empty_s);
+    // Group `it` of this CTA: group (blockIdx.x + it gridDim.x) of the launch = rows 64 gi .. of matrix mi; one contiguous byte
+    // range, one bulk copy (one thread).
     auto load_group = [&](int it) {
         const int gl = (int)blockIdx.x + it * (int)gridDim.x, mi = MULTI ? gl / p.gpm : 0, grp = gl - mi * p.gpm;
         const uint8_t *wm = p.w[mi];
         const size_t start = (size_t)grp * GROUP_ROWS * rb;
         const size_t len = (size_t)min(GROUP_ROWS, p.n - grp * GROUP_ROWS) * rb;
         const size_t a0 = start & ~(size_t)15;
-        const int n16 = (int)((start - a0 + len + 15) >> 4);
+        uint32_t bytes = (uint32_t)((start - a0 + len + 15) & ~(size_t)15);
         uint8_t *slot = ring + (size_t)(it % SLOTS) * p.slot_bytes;
-        for (int i = tid; i < n16; i += NT) {
-            const size_t ga = a0 + ((size_t)i << 4);
-            if (ga + 16 <= w_bytes) {
-                cp_async16(smem_u32(slot + ((size_t)i << 4)), wm + ga);
-            } else {
-                for (int b = 0; b < 16; b++) slot[((size_t)i << 4) + b] = (ga + b < w_bytes) ? wm[ga + b] : 0;
-            }
+        if (a0 + bytes > w_bytes) {   // nothing is read past the matrix's end
+            bytes -= 16;
+            for (uint32_t b = 0; b < 16; b++) slot[bytes + b] = (a0 + bytes + b < w_bytes) ? wm[a0 + bytes + b] : 0;
         }
+        mbar_arrive_expect_tx(full + 8 * (it % SLOTS), bytes);
+        if (bytes) bulk_g2s(smem_u32(slot), wm + a0, bytes, full + 8 * (it % SLOTS));
     };
-    // the weights of the first two groups do not depend on the previous kernel
-    if (my_groups > 0) load_group(0);
-    if (my_groups > 1) load_group(1);
+    // the weights of the first groups do not depend on the previous kernel
+    if (tid == NW * 32) {
+        for (int s = 0; s < SLOTS; s++) {
+            mbar_init(full + 8 * s, 1);
+            mbar_init(empty + 8 * s, NW);
+        }
+        abort_s = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        for (int it = 0; it < SLOTS && it < my_groups; it++) load_group(it);
+    }
     lc_pdl_wait();
     for (int i = tid; i < 8 * (p.K / 8); i += NT) {
         const int r = i / (p.K / 8), pc = i - r * (p.K / 8);
@@ -111,109 +133,111 @@ __global__ void __launch_bounds__(NT, 1) qgemv_mma_stream_kernel(const __grid_co
         cp_async16(smem_u32(x_s + r * p.xs + pc * 16), ok ? (const void *)(p.x + (size_t)r * p.K + pc * 8) : (const void *)p.x,
                    ok ? 16u : 0u);
     }
-    cp_async_commit();      // group 0: weights of groups 0 and 1 + the activations
-    cp_async_commit();      // group 1: empty (keeps the wait arithmetic uniform)
-
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();          // the activations have landed, the barriers are ready
+    bool alive = true;   // no wait of this warp has run out
+    auto warp_wait = [&](uint32_t bar, uint32_t parity) -> bool {
+        if (alive && !__all_sync(0xffffffffu, mbar_wait(bar, parity, STREAM_WAIT_LIMIT))) {
+            alive = false;
+            *abort_flag = 1;
+        }
+        return alive;
+    };
+    if (warp == NW) {
+        for (int it = SLOTS; it < my_groups; it++) {
+            if (!warp_wait(empty + 8 * (it % SLOTS), (uint32_t)((it / SLOTS - 1) & 1))) break;
+            if (lane == 0) load_group(it);
+            __syncwarp();
+        }
+    } else {
     // this warp's quarter of K, in units of 128 k
     const int nu = p.K / UNIT_K, upq = (nu + 3) / 4;
     const int u0 = kq * upq, u1 = min(nu, u0 + upq);
     // ldmatrix.x2 lane address: lanes 0-7 rows of the first k half, lanes 8-15 the second
     const uint32_t xl = smem_u32(x_s) + (uint32_t)((lane & 7) * p.xs + ((lane >> 3) & 1) * 16);
     uint32_t breg[UPQ > 0 ? UPQ * 8 : 1][2];
+    // Code bytes 2t, 2t + 8 pair up in a register, and so do 2t + 1, 2t + 9: the activations' k follow.
+    auto load_b = [&](uint32_t &b0, uint32_t &b1, uint32_t addr) {
+        uint32_t r0, r1;
+        ldmatrix_x2(r0, r1, addr);
+        b0 = __byte_perm(r0, r1, 0x5410);
+        b1 = __byte_perm(r0, r1, 0x7632);
+    };
     if (UPQ > 0) {
-        cp_async_wait<1>();
-        __syncthreads();          // the activations have landed
 #pragma unroll
         for (int uu = 0; uu < (UPQ > 0 ? UPQ : 1); uu++)
 #pragma unroll
             for (int s8 = 0; s8 < 8; s8++) {
                 breg[uu * 8 + s8][0] = breg[uu * 8 + s8][1] = 0u;
-                if (u0 + uu < u1) ldmatrix_x2(breg[uu * 8 + s8][0], breg[uu * 8 + s8][1], xl + (uint32_t)(((u0 + uu) * UNIT_K + 16 * s8) * 2));
+                if (u0 + uu < u1) load_b(breg[uu * 8 + s8][0], breg[uu * 8 + s8][1], xl + (uint32_t)(((u0 + uu) * UNIT_K + 16 * s8) * 2));
             }
     }
 
-    auto reduce_store = [&](int it) {      // warps kq == 0: add the four quarters of group `it` and store
+    // The four quarters of a group of sixteen rows meet at a named barrier; warp kq adds fragment element kq and stores.
+    auto reduce_store = [&](int it) {
         const int gl = (int)blockIdx.x + it * (int)gridDim.x, mi = MULTI ? gl / p.gpm : 0, grp = gl - mi * p.gpm;
-        OutT *out = reinterpret_cast<OutT *>(p.out[mi]);
-        const float4 *rp = red + (size_t)(it & 1) * NW * 32;
-        float4 v = rp[(0 * 4 + rg) * 32 + lane];
-#pragma unroll
-        for (int q = 1; q < 4; q++) {
-            const float4 o = rp[(q * 4 + rg) * 32 + lane];
-            v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-        }
-        const float e4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int row = grp * GROUP_ROWS + rg * 16 + g + 8 * (e >> 1), col = 2 * t + (e & 1);
-            if (row < p.n && col < p.m) store_c(out + (size_t)col * p.n + row, e4[e]);
-        }
+        const float *rp = reinterpret_cast<const float *>(red + (size_t)(it & 1) * NW * 32 + rg * 32 + lane) + kq;
+        const float v = ((rp[0] + rp[4 * 32 * 4]) + rp[2 * 4 * 32 * 4]) + rp[3 * 4 * 32 * 4];
+        const int row = grp * GROUP_ROWS + rg * 16 + g + 8 * (kq >> 1), col = 2 * t + (kq & 1);
+        if (row < p.n && col < p.m) store_c(reinterpret_cast<OutT *>(p.out[mi]) + (size_t)col * p.n + row, v);
     };
 
     for (int it = 0; it < my_groups; it++) {
-        cp_async_wait<1>();
-        __syncthreads();          // group `it` has landed everywhere; everyone is done with group it - 1
-        if (it + 2 < my_groups) load_group(it + 2);
-        cp_async_commit();
-        if (it > 0 && kq == 0) reduce_store(it - 1);
-
+        // (an expired wait does not leave the loop: the other quarters count on this warp at their barrier)
+        const bool landed = warp_wait(full + 8 * (it % SLOTS), (uint32_t)((it / SLOTS) & 1));
         const int gl = (int)blockIdx.x + it * (int)gridDim.x, grp = MULTI ? gl % p.gpm : gl;
         const size_t start = (size_t)grp * GROUP_ROWS * rb;
         const uint8_t *slot = ring + (size_t)(it % SLOTS) * p.slot_bytes + (start & 15);
         const uint8_t *rbase[2];
-        bool rvalid[2];
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             const int r = rg * 16 + g + 8 * i;
-            rbase[i] = slot + (size_t)r * rb;
-            rvalid[i] = grp * GROUP_ROWS + r < p.n;
+            rbase[i] = slot + (size_t)r * rb;   // (rows past the matrix's last hold leftovers; nothing of them is stored)
         }
         float c[4] = {0.f, 0.f, 0.f, 0.f};
-        if (FMT == FMT_TQ2_0) {
+        if (!landed) {
+        } else if (FMT == FMT_TQ2_0) {
             // unit u = half h of block b: element 128 h + 32 l + j of the block is bit pair l of code byte 32 h + j
 #pragma unroll
             for (int uu = 0; uu < (UPQ > 0 ? UPQ : 64); uu++) {
                 const int u = u0 + uu;
                 if (u >= u1) break;
                 const int b = u >> 1, h = u & 1;
-                uint32_t lut_lo[2], lut_hi[2], wq[2][2];
+                uint32_t wq[2][2], sh[2][2];
+                float df[2];
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
                     const uint8_t *bp = rbase[i] + b * BB;
-                    const __half d = rvalid[i] ? *reinterpret_cast<const __half *>(bp + 64) : __float2half(0.0f);
-                    const uint32_t p01 = (uint32_t)__half_as_ushort(__hneg(d));                       // {-d, 0}
-                    const uint32_t p23 = (uint32_t)__half_as_ushort(d) | ((uint32_t)__half_as_ushort(__hadd(d, d)) << 16);
-                    lut_lo[i] = __byte_perm(p01, p23, 0x6420);
-                    lut_hi[i] = __byte_perm(p01, p23, 0x7531);
+                    df[i] = __half2float(*reinterpret_cast<const __half *>(bp + 64)) * 512.0f;
                     const uint8_t *hp = bp + h * 32 + 2 * t;
                     wq[i][0] = lds_u16(hp) | (lds_u16(hp + 8) << 16);
                     wq[i][1] = lds_u16(hp + 16) | (lds_u16(hp + 24) << 16);
+                    sh[i][0] = wq[i][0] >> 8;
+                    sh[i][1] = wq[i][1] >> 8;
                 }
+                float cu[2][4] = {};
 #pragma unroll
                 for (int l = 0; l < 4; l++) {
 #pragma unroll
                     for (int qp = 0; qp < 2; qp++) {
-                        uint32_t a[4];
-#pragma unroll
-                        for (int i = 0; i < 2; i++) {
-                            const uint32_t sel = ((wq[i][qp] >> (2 * l)) & 0x03030303u) * 0x11u + 0x40404040u;
-                            a[i] = __byte_perm(lut_lo[i], lut_hi[i], sel);
-                            a[i + 2] = __byte_perm(lut_lo[i], lut_hi[i], sel >> 16);
-                        }
+                        const uint32_t a[4] = {codes_f16<2, 1>(wq[0][qp], l), codes_f16<2, 1>(wq[1][qp], l), codes_f16<2, 1>(sh[0][qp], l),
+                                               codes_f16<2, 1>(sh[1][qp], l)};
                         uint32_t b0, b1;
                         if (UPQ > 0) {
                             b0 = breg[uu * 8 + 2 * l + qp][0];
                             b1 = breg[uu * 8 + 2 * l + qp][1];
                         } else {
-                            ldmatrix_x2(b0, b1, xl + (uint32_t)((u * UNIT_K + 32 * l + 16 * qp) * 2));
+                            load_b(b0, b1, xl + (uint32_t)((u * UNIT_K + 32 * l + 16 * qp) * 2));
                         }
-                        mma16816(c, a, b0, b1);
+                        mma16816(cu[qp], a, b0, b1);
                     }
                 }
+#pragma unroll
+                for (int e = 0; e < 4; e++) c[e] = fmaf(df[e >> 1], cu[0][e] + cu[1][e], c[e]);
             }
         } else {
             // unit u = blocks 4u .. 4u+3; block: f16 scale, then byte i holds k = i (low nibble) and i + 16 (high)
-            const __half2 c1032 = __float2half2_rn(1032.0f);
 #pragma unroll
             for (int uu = 0; uu < (UPQ > 0 ? UPQ : 64); uu++) {
                 const int u = u0 + uu;
@@ -226,25 +250,20 @@ __global__ void __launch_bounds__(NT, 1) qgemv_mma_stream_kernel(const __grid_co
 #pragma unroll
                     for (int i = 0; i < 2; i++) {
                         const uint8_t *bp = rbase[i] + b * BB;
-                        df[i] = rvalid[i] ? __half2float(*reinterpret_cast<const __half *>(bp)) : 0.f;
+                        df[i] = __half2float(*reinterpret_cast<const __half *>(bp)) * 512.0f;
                         wq[i] = lds_u16(bp + 2 + 2 * t) | (lds_u16(bp + 10 + 2 * t) << 16);
                     }
                     float cb[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                     for (int part = 0; part < 2; part++) {
-                        uint32_t a[4];
-#pragma unroll
-                        for (int i = 0; i < 2; i++) {
-                            const uint32_t codes = (wq[i] >> (4 * part)) & 0x0F0F0F0Fu;
-                            a[i] = h2_bits(__hsub2(bits_h2(__byte_perm(codes, 0x64u, 0x4140)), c1032));
-                            a[i + 2] = h2_bits(__hsub2(bits_h2(__byte_perm(codes, 0x64u, 0x4342)), c1032));
-                        }
+                        const uint32_t a[4] = {codes_f16<4, 8>(wq[0], part), codes_f16<4, 8>(wq[1], part), codes_f16<4, 8>(wq[0] >> 8, part),
+                                               codes_f16<4, 8>(wq[1] >> 8, part)};
                         uint32_t b0, b1;
                         if (UPQ > 0) {
                             b0 = breg[uu * 8 + 2 * bi + part][0];
                             b1 = breg[uu * 8 + 2 * bi + part][1];
                         } else {
-                            ldmatrix_x2(b0, b1, xl + (uint32_t)((b * 32 + 16 * part) * 2));
+                            load_b(b0, b1, xl + (uint32_t)((b * 32 + 16 * part) * 2));
                         }
                         mma16816(cb, a, b0, b1);
                     }
@@ -255,11 +274,15 @@ __global__ void __launch_bounds__(NT, 1) qgemv_mma_stream_kernel(const __grid_co
                 }
             }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty + 8 * (it % SLOTS));
         red[((size_t)(it & 1) * NW + kq * 4 + rg) * 32 + lane] = make_float4(c[0], c[1], c[2], c[3]);
+        asm volatile("bar.sync %0, 128;\n" ::"r"(1 + rg) : "memory");
+        if (landed) reduce_store(it);
     }
-    cp_async_wait<0>();
+    }
     __syncthreads();
-    if (my_groups > 0 && kq == 0) reduce_store(my_groups - 1);
+    if (*abort_flag) tc_wait_expired(p.status, LC_DEV_STATUS_WAIT_EXPIRED, tid);
 }
 
 template <int FMT, typename OutT, int UPQ, bool MULTI>
@@ -311,12 +334,13 @@ int lc_qgemv_mma_stream_group(int fmt, bool f32out, lc_kernels *k, lc_batch *b, 
     p.K = (int)kk;
     p.nb = (int)(kk / be);
     p.gpm = (int)((n + GROUP_ROWS - 1) / GROUP_ROWS);
+    p.status = k->dev_status;
     p.groups = p.gpm * count;
     p.xs = (int)kk * 2 + 16;
     const size_t rb = (size_t)p.nb * bb;
     p.slot_bytes = (int)(((size_t)GROUP_ROWS * rb + 15 + 15) / 16 * 16 + 16);
     const size_t smem = (size_t)8 * p.xs + 2 * NW * 32 * 16 + (size_t)SLOTS * p.slot_bytes;
-    if (smem > k->ctx->smem_optin) return -1;
+    if (smem + 256 > k->ctx->smem_optin) return -1;   // (the barriers are static)
     // worth it only when every SM gets a few groups to stream
     if (p.groups < 2 * k->ctx->sm_count) return -1;
     if (fmt == FMT_Q4_0)
