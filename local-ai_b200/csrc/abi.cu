@@ -447,6 +447,7 @@ int lc_kernels_create(lc_ctx *ctx, lc_kernels **out) {
     { const char *e = getenv("LOCAL_CUDA_TEST_WAIT_EXPIRY"); k->test_wait_expiry = e && strcmp(e, "1") == 0; }
     const char *nm = getenv("LOCAL_CUDA_TQ_NORM");
     k->kv_norm_mode = (nm && strcmp(nm, "tree") == 0) ? 1 : 0;
+    lc_cluster_capacity(ctx, k->cluster_cap);
     cudaError_t e = cudaMalloc((void **)&k->dev_status, 128);  // status word + tuning stamps
     if (e == cudaSuccess) e = cudaMemsetAsync(k->dev_status, 0, 128, ctx->stream);
     if (e != cudaSuccess) {

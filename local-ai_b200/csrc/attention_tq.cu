@@ -451,6 +451,11 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     if (n_splits < 1) n_splits = 1;
     if (n_splits > 64) n_splits = 64;
     uint32_t chunk = 0;
+    // The tensor-core kernel merges up to 8 splits itself (one thread-block cluster per lane and kv head, exchange
+    // through distributed shared memory, inverse rotation in the kernel): one launch instead of split + merge, the same
+    // arithmetic in the same order, bit-identical output.  LOCAL_CUDA_ATTN_CLUSTER=0 selects the two-launch form.
+    static const bool cluster_allowed = []() { const char *e = getenv("LOCAL_CUDA_ATTN_CLUSTER"); return !(e && e[0] == '0'); }();
+    const bool clusters = use_mma && cluster_allowed && lc_aligned(out->dptr, 16) && (!fused || lc_aligned(signs->dptr, 16));
     if (use_mma) {
         // One CTA per SM (shared memory), so the launch runs in whole waves; every CTA pays a fixed prologue and epilogue
         // worth about 320 keys.  Pick the split count that minimises waves x (overhead + keys per split).
@@ -460,14 +465,14 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
         if (len_max < 4096 && max_s > 8) max_s = 8;
         if (max_s < 1) max_s = 1;
         if (max_s > sms) max_s = sms;
+        // Up to 8 splits are a cluster, and of those fewer fit at once (17 lanes x 512 keys: 8 splits 17.2 us, 6 splits 9.3).
         uint64_t best_cost = ~0ull;
         for (uint32_t s = 1; s <= max_s; s++) {
-            const uint64_t waves = ((uint64_t)base * s + sms - 1) / sms;
+            const uint64_t waves = s <= 8 && clusters ? (base + k->cluster_cap[s] - 1) / k->cluster_cap[s] : ((uint64_t)base * s + sms - 1) / sms;
             const uint64_t cost = waves * (320u + (len_max + s - 1) / s);
             if (cost < best_cost) { best_cost = cost; n_splits = s; }
         }
     }
-    const bool out_vec = lc_aligned(out->dptr, 16) && (!fused || lc_aligned(signs->dptr, 16));
     // Queue form for pools of lanes that attend all of their keys.  Lanes differ in length, which the host cannot see, and
     // equal splits per lane leave most SMs waiting for the longest lane; so one persistent CTA per SM draws items of at
     // most `chunk` keys.  An item costs about 450 keys' worth of fixed work.  The chunk minimises the sum of two
@@ -506,14 +511,7 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     const bool pf = pf_tiles != 0;
     const bool queue = chunk != 0;
     const bool direct = !queue && !pf && n_splits == 1 && !fused;
-    // The tensor-core kernel merges up to 8 splits itself (one thread-block cluster per lane and kv head, exchange
-    // through distributed shared memory, inverse rotation in the kernel): one launch instead of split + merge, the same
-    // arithmetic in the same order, bit-identical output.  Alone 57 vs 59 us at 8193 keys x 64 lanes, 12.4 vs 14.6 us
-    // for a 512-key window; inside the decode step 2.314 vs 2.331 ms.  (Before the step's other kernels did their
-    // weight prefetch ahead of their dependency wait it was the slower form in situ, 3.48 vs 3.36 ms.)
-    // LOCAL_CUDA_ATTN_CLUSTER=0 selects the two-launch form.
-    static const bool cluster_allowed = []() { const char *e = getenv("LOCAL_CUDA_ATTN_CLUSTER"); return !(e && e[0] == '0'); }();
-    const bool cluster_merge = use_mma && !queue && !pf && cluster_allowed && n_splits <= 8 && out_vec;
+    const bool cluster_merge = clusters && !queue && !pf && n_splits <= 8;
 
     if (!direct && !cluster_merge) {
         const size_t rows_y = (size_t)n_kv * gchunks;

@@ -894,3 +894,31 @@ int lc_tq_attn_mma_launch(lc_batch *b, const TqAttnParams &p, dim3 grid, uint32_
         default: return launch_bits<512>(b, p, grid, bits);
     }
 }
+
+// (asked of one of the kernels that fill an SM's shared memory; the others that do differ in nothing that counts here)
+void lc_cluster_capacity(const lc_ctx *ctx, uint32_t (&cap)[9]) {
+    using C = AttnCfg<256, 2>;
+    auto kern = tq_attn_mma_kernel<C>;
+    cap[0] = 0;
+    cap[1] = (uint32_t)ctx->sm_count;
+    const bool ready = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) == cudaSuccess;
+    for (uint32_t s = 2; s <= 8; s++) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(s);
+        cfg.blockDim = dim3(C::NT);
+        cfg.dynamicSmemBytes = C::SMEM;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = s;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (!ready || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = ctx->sm_count * 3 / 4 / (int)s;
+        }
+        cap[s] = n < 1 ? 1u : (uint32_t)n;
+    }
+}

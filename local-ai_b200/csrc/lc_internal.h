@@ -62,13 +62,17 @@ struct lc_kernels {
     size_t counters_len = 0;
     std::vector<void *> retired;  // outgrown scratch / counter blocks: graphs recorded earlier still point at them
     int *dev_status = nullptr;  // device-side error word (bounded waits report here)
+    // Clusters of s CTAs, an SM each, that the device runs at once (lc_cluster_capacity).  A cluster needs all its SMs in one
+    // GPC, so this is well below SMs / s: 74 pairs, but 45 triples, 33 fours and 15 eights on 148 SMs.  A launch of one more
+    // runs a second wave and takes twice as long.
+    uint32_t cluster_cap[9] = {0};
     // LOCAL_CUDA_TEST_WAIT_EXPIRY=1 (read at creation): the tcgen05 matmul's barrier waits use a short limit and wait for
     // an arrival that never comes, so the expiry path (status word, early exit, TMEM release) can be exercised on purpose.
     bool test_wait_expiry = false;
 };
 
 // Values of the device-side status word (lc_kernels::dev_status).
-constexpr int LC_DEV_STATUS_WAIT_EXPIRED = 1;      // a bounded barrier wait ran out (large-tile tcgen05 matmul)
+constexpr int LC_DEV_STATUS_WAIT_EXPIRED = 1;      // a bounded barrier wait ran out (large-batch matmul, prefill attention, streaming matvec)
 constexpr int LC_DEV_STATUS_WAIT_EXPIRED_TCD = 2;  // the same in the decode tcgen05 matmul
 constexpr int LC_DEV_STATUS_POSITION = 3;          // a device-resident position pointed past its lane's pool rows
 
@@ -187,6 +191,8 @@ static inline cudaError_t lc_ensure_smem(Kern kern, lc_smem_optin &state, const 
 }
 
 static inline bool lc_aligned(const void *p, size_t a) { return ((uintptr_t)p & (a - 1)) == 0; }
+
+void lc_cluster_capacity(const lc_ctx *ctx, uint32_t (&cap)[9]);   // attention_tq_mma.cu
 
 // Grow the kernels object's split-K scratch (no-op when large enough). Fails
 // during graph capture if growth would be needed.

@@ -463,7 +463,7 @@ int lc_qgemm_tcl_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const 
     p.steps = ((int)kk + step_k - 1) / step_k;
     // Batch rows per CTA and K splits: a step costs its tensor-memory stores (about 900 cycles) or its MMAs (8 per column),
     // whichever is more; a launch costs about 2500 cycles around its steps, the exchange of a split 3000 more.  Clusters
-    // cannot use every SM (7/8 are counted on), other launches can.
+    // cannot use every SM, other launches can.
     const int sms = k->ctx->sm_count;
     uint64_t best = ~0ull;
     p.m_tiles = 1;
@@ -471,8 +471,7 @@ int lc_qgemm_tcl_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const 
     for (int mt = ((int)m + MAX_NB - 1) / MAX_NB; mt <= ((int)m + 47) / 48; mt++) {
         const int nb = (((int)m + mt - 1) / mt + 15) / 16 * 16, real_mt = ((int)m + nb - 1) / nb;
         for (int ks = 1; ks <= MAX_KS && (ks == 1 || 2 * ks <= p.steps); ks++) {
-            const int slots = ks > 1 ? sms * 7 / 8 : sms;
-            const uint64_t ctas = (uint64_t)tiles * real_mt * ks, waves = (ctas + slots - 1) / slots;
+            const uint64_t at_once = ks > 1 ? k->cluster_cap[ks] : (uint64_t)sms, waves = ((uint64_t)tiles * real_mt + at_once - 1) / at_once;
             const uint64_t cost = waves * (2500u + (uint64_t)((p.steps + ks - 1) / ks) * (uint64_t)(8 * nb > 900 ? 8 * nb : 900) + (ks > 1 ? 3000u + 10u * nb : 0u));
             if (cost < best) {
                 best = cost;
