@@ -184,13 +184,15 @@ class QuantMatvec:
     def kernel_name(self) -> str:
         if self.grouped:
             return "qgemv_mma_stream_kernel (grouped)"
-        if self.m == 1:
-            return "qgemv_mma_stream_kernel" if self.rows >= 18944 else "qgemv_kernel"
+        if self.m <= 8 and self.rows >= 18944:
+            return "qgemv_mma_stream_kernel"
+        if self.m <= 16 and not (self.f32out and self.m > 8 and self.rows >= 18944):
+            return "qgemm_sm_kernel"
         if self.f32out and 8 < self.m <= 64 and self.cols % 256 == 0 and self.rows >= 128 * 148:
             return "qgemm_tcv_kernel (tcgen05)"
         if self.fmt == "tq2_0" and 8 < self.m <= 64:
             return "qgemm_tcd_kernel (tcgen05)"
-        return "qgemm_mma_kernel" if self.m <= 64 else "qgemm_tc_kernel (tcgen05)"
+        return "qgemm_tcl_kernel (tcgen05)"
 
     def value(self, ms_per_step: float) -> float:
         return self.alg_bytes_per_launch * self.units_per_step / (ms_per_step * 1e-3) / 1e9
@@ -305,7 +307,7 @@ class TqAttention:
         achieved = self.alg_bytes_per_launch / (us * 1e-6) / 1e9
         return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": None, "peak_kind": peak_kind,
-                "kernel": "tq2_attn_mma_kernel (splits merged in the kernel through a thread-block cluster)", "us_per_launch": us,
+                "kernel": "tq_attn_mma_kernel (splits merged in the kernel through a thread-block cluster)", "us_per_launch": us,
                 "algorithmic_bytes_per_launch": self.alg_bytes_per_launch, "frac_of_nominal_8tbs": achieved / 8000.0}
 
     def cpu_sample(self, orc, threads: int):
@@ -505,7 +507,7 @@ class DecodeStep:
         return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": self.FFN_TRAFFIC["bytes"] if m == 64 else None,
                 "traffic_source": self.FFN_TRAFFIC if m == 64 else None, "peak_kind": peak_kind,
-                "kernel": (f"{'qgemv_kernel' if m <= 8 else 'qgemm_tcd_kernel (tcgen05)' if m <= 64 else 'qgemm_tc_kernel (tcgen05) + gelu_mul'}"
+                "kernel": (f"{'qgemm_sm_kernel' if m <= 16 else 'qgemm_tcd_kernel (tcgen05)' if m <= 64 else 'qgemm_tcl_kernel (tcgen05) + gelu_mul'}"
                            f"<TQ2_0, m={m}>: GeGLU + down projections of {cfg.n_layers} layers, {n_launch} launches"),
                 "us_per_launch": us, "algorithmic_bytes_per_launch": per_launch,
                 "launches_timed_alone_share_of_step": ms / ms_per_step,
