@@ -456,9 +456,12 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     // arithmetic in the same order, bit-identical output.  LOCAL_CUDA_ATTN_CLUSTER=0 selects the two-launch form.
     static const bool cluster_allowed = []() { const char *e = getenv("LOCAL_CUDA_ATTN_CLUSTER"); return !(e && e[0] == '0'); }();
     const bool clusters = use_mma && cluster_allowed && lc_aligned(out->dptr, 16) && (!fused || lc_aligned(signs->dptr, 16));
+    uint64_t grid_cost = ~0ull;
+    auto in_keys = [&](uint32_t tq2_keys) -> uint32_t { return tq2_keys * (bits == 2 ? 8u : 5u) * 32u / hd; };
     if (use_mma) {
-        // One CTA per SM (shared memory), so the launch runs in whole waves; every CTA pays a fixed prologue and epilogue
-        // worth about 320 keys.  Pick the split count that minimises waves x (overhead + keys per split).
+        // One CTA per SM (shared memory), so the launch runs in whole waves.  Pick the split count that minimises their
+        // time, in keys of tq2 at head_dim 256 (8.5 ns each; more bits take 8/5 of that): 700 for the launch, 1050 for
+        // every further wave, 640 for a merge launch.
         // Short contexts split down to two 32-key tiles per CTA (two warps that have the table's banks to themselves finish a
         // tile sooner than eight), but into no more splits than one launch merges; long ones to half the warps.
         uint32_t max_s = len_max < 4096 ? len_max / 64u : len_max / 128u;
@@ -466,30 +469,36 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
         if (max_s < 1) max_s = 1;
         if (max_s > sms) max_s = sms;
         // Up to 8 splits are a cluster, and of those fewer fit at once (17 lanes x 512 keys: 8 splits 17.2 us, 6 splits 9.3).
-        uint64_t best_cost = ~0ull;
         for (uint32_t s = 1; s <= max_s; s++) {
-            const uint64_t waves = s <= 8 && clusters ? (base + k->cluster_cap[s] - 1) / k->cluster_cap[s] : ((uint64_t)base * s + sms - 1) / sms;
-            const uint64_t cost = waves * (320u + (len_max + s - 1) / s);
-            if (cost < best_cost) { best_cost = cost; n_splits = s; }
+            const bool one_launch = s <= 8 && clusters;
+            const uint64_t waves = one_launch ? (base + k->cluster_cap[s] - 1) / k->cluster_cap[s] : ((uint64_t)base * s + sms - 1) / sms;
+            const uint64_t cost = in_keys(700u) + waves * ((len_max + s - 1) / s) + (waves - 1) * in_keys(1050u) + (one_launch || s == 1 ? 0u : in_keys(640u));
+            if (cost < grid_cost) { grid_cost = cost; n_splits = s; }
         }
     }
     // Queue form for pools of lanes that attend all of their keys.  Lanes differ in length, which the host cannot see, and
     // equal splits per lane leave most SMs waiting for the longest lane; so one persistent CTA per SM draws items of at
-    // most `chunk` keys.  An item costs about 450 keys' worth of fixed work.  The chunk minimises the sum of two
-    // estimates: every lane full, and lane lengths spread evenly up to the longest.  Below about ten lanes, or 2048 keys, the
-    // splits of the launch above are as good and merge in one launch.
+    // most `chunk` keys.  An item after a CTA's first costs about 620 keys' worth more, and a merge launch follows.  The chunk minimises
+    // the sum of two estimates: every lane full, and lane lengths spread evenly up to the longest.  The splits above take
+    // their longest lane's time in both, in one launch, and stay unless the queue promises less: measured full / ragged,
+    // 32 lanes x 8192 tq2 keys 28.5 / 23.5 us against 36.8 / 22.1 for the queue, 64 lanes 46.6 / 44.3 against 57.4 / 33.3,
+    // 64 lanes of tq4 keys 74.5 / 72.3 against 85.7 / 48.3.
     if (use_mma && positions && window == 0 && ring == 0 && n_lanes <= LC_ATTN_QUEUE_LANES && base * 16u >= sms && len_max > 2048) {
-        const uint32_t fixed = 450, lo_s = len_max > 32u * 2048u ? 32u : (len_max + 4095) / 4096;
+        const uint32_t item = in_keys(620u), launch = in_keys(700u + 640u), lo_s = len_max > 32u * 2048u ? 32u : (len_max + 4095) / 4096;
         uint64_t best_cost = ~0ull;
+        uint32_t best_chunk = 0;
         for (uint32_t s = lo_s; s <= 32; s++) {
             uint32_t per = ((len_max - 64u) / s + 255u) & ~255u;   // whole rounds of eight warps x 32 keys
             if (per < 256u) per = 256u;
-            const uint64_t full = (((uint64_t)base * s + sms - 1) / sms) * (fixed + per);
-            const uint64_t mean = ((uint64_t)base * (len_max + fixed * (s + 1)) / 2) / sms;
-            const uint64_t cost = full + (mean > fixed + per ? mean : fixed + per);
-            if (cost < best_cost) { best_cost = cost; chunk = per + 64u; }   // (a few keys over do not make another item)
+            const uint64_t rounds = ((uint64_t)base * s + sms - 1) / sms, full = rounds * per + (rounds - 1) * item;
+            const uint64_t mean = ((uint64_t)base * (len_max + item * (s + 1)) / 2) / sms;
+            const uint64_t cost = full + (mean > per ? mean : per) + 2u * launch;
+            if (cost < best_cost) { best_cost = cost; best_chunk = per + 64u; }   // (a few keys over do not make another item)
         }
-        n_splits = (len_max + chunk - 1) / chunk;
+        if (best_cost < 2u * grid_cost) {
+            chunk = best_chunk;
+            n_splits = (len_max + chunk - 1) / chunk;
+        }
     }
     // Chunks of several rows: the prefill kernel shares each decoded key among 128 MMA rows.  Below about half a tile of rows
     // the decode kernel's CTA per row is as fast.
