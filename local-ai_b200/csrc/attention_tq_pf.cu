@@ -1,6 +1,6 @@
 // Prefill / multi-row attention over TurboQuant codes on tcgen05: head_dim 128 / 256, tq2 / tq3 / tq4.  Stands in for
 // shaders/attention_flash_tq.metal:290-556 (flash_attention_tq_prefill and its query-tiled form) for chunks of several rows;
-// leaves the split-K partials that tq_attn_merge_kernel (attention_tq.cu) adds up.
+// leaves the split-K partials that a merge launch (attention_tq.cu) adds up.
 //
 // The decode kernel serves one query row per CTA, so a chunk of 256 rows decoded the same cache 256 times.  Here a CTA owns 128
 // query rows of the MMA's M (16 tokens x 8 heads of a kv-head) and a range of keys:
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
     float *norms = reinterpret_cast<float *>(smem + C::NORM_OFF);
     constexpr int BAR_OFF = C::TAIL > C::STAGE ? C::TAIL : C::STAGE;
     const uint32_t bars = base + BAR_OFF;
-    const uint32_t k_full = bars, v_full = bars + 8, p_full = bars + 16, pv_done = bars + 24, qk_done = bars + 32;   // qk_done: two
+    const uint32_t k_full = bars, v_full = bars + 8, p_full = bars + 16, pv_done = bars + 24, qk_done = bars + 32, rot_done = bars + 56;   // qk_done: two
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + BAR_OFF + 48);
     volatile uint32_t *abort_flag = tmem_slot + 1;
     __shared__ float m_s[M], l_s[2][M], mx_s[2][2][M], gamma_s, cand_err[PF_NT / 32];
@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
         mbar_init(pv_done, 1);
         mbar_init(qk_done, 1);
         mbar_init(qk_done + 8, 1);
+        mbar_init(rot_done, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -210,26 +211,127 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
     lc_pdl_wait();
 
     // ---- query rows: sign, transform, scale, split into two f16 operand tiles (K-major, 128-byte swizzle) ----
-    // (four rows of a warp at a time, their loads first: a row is a microsecond of memory latency and little else)
-    if (warp < MMA_WARP) {
-        constexpr int QB = 4;
+    auto warp_wait = [&](uint32_t bar, uint32_t parity) -> bool {
+        uint32_t ok = 1;
+        if (lane == 0) ok = *abort_flag == 0u && mbar_wait(bar, parity, PF_WAIT_LIMIT) ? 1u : 0u;
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (!ok || *abort_flag) {
+            *abort_flag = 1;
+            return false;
+        }
+        return true;
+    };
+    // The transform of 128 rows by shuffles took 13 of this kernel's 61 thousand cycles (16 rows over 2000 keys 21.0 -> 19.1 us
+    // without it, 256 over 4096 39.4 -> 37.8).  With signs of +-1 the signed row is an f16 still, exactly, and 64 dims of it at a
+    // time go through the tensor cores: D = A . H64 (Sylvester's matrix, its rows in the order of the operand tiles), then butterflies over the 64-dim blocks when a row is read back.
+    bool unit = p.fused_q != 0u;
+    uint32_t flip[DPL / 2];
+    if (p.fused_q) {
+#pragma unroll
+        for (int i = 0; i < DPL; i += 2) {
+            const float2 sg = *reinterpret_cast<const float2 *>(p.signs + DPL * lane + i);
+            unit = unit && fabsf(sg.x) == 1.0f && fabsf(sg.y) == 1.0f;
+            flip[i / 2] = (sg.x < 0.f ? 0x8000u : 0u) | (sg.y < 0.f ? 0x80000000u : 0u);
+        }
+    }
+    unit = __all_sync(0xffffffffu, unit);   // (every warp sees all signs)
+    if (unit) {
+        if (warp < MMA_WARP) {
+            constexpr int QB = 4;   // rows of a warp whose loads are in flight together
 #pragma unroll 1
-        for (int rb = warp; rb < M; rb += MMA_WARP * QB) {
-            uint2 raw[QB][DPL / 4];
+            for (int rb = warp; rb < M; rb += MMA_WARP * QB) {
+                uint2 raw[QB][DPL / 4];
 #pragma unroll
-            for (int j = 0; j < QB; j++) {
-                const int r = rb + j * MMA_WARP, tk = r / gc, h = r - tk * gc;
+                for (int j = 0; j < QB; j++) {
+                    const int r = rb + j * MMA_WARP, tk = r / gc, h = r - tk * gc;
 #pragma unroll
-                for (int i = 0; i < DPL / 4; i++) {
-                    raw[j][i] = make_uint2(0u, 0u);
-                    if (p.fused_q && r < M && tk < nt && h < gvalid)
-                        raw[j][i] = *reinterpret_cast<const uint2 *>(p.q + ((size_t)(tok0 + tk) * p.n_q + qh0 + h) * HD + DPL * lane + 4 * i);
+                    for (int i = 0; i < DPL / 4; i++) {
+                        raw[j][i] = make_uint2(0u, 0u);
+                        if (r < M && tk < nt && h < gvalid)
+                            raw[j][i] = *reinterpret_cast<const uint2 *>(p.q + ((size_t)(tok0 + tk) * p.n_q + qh0 + h) * HD + DPL * lane + 4 * i);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < QB; j++) {
+                    const int r = rb + j * MMA_WARP;
+                    if (r >= M) break;
+#pragma unroll
+                    for (int i = 0; i < DPL / 4; i++) {
+                        const int d = DPL * lane + 4 * i;
+                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(base + (uint32_t)(C::Q_OFF + (d >> 6) * M * 128 + r * 128 + ((((d & 63) >> 3) ^ (r & 7)) << 4) + (d & 4) * 2)),
+                                     "r"(raw[j][i].x ^ flip[2 * i]), "r"(raw[j][i].y ^ flip[2 * i + 1])
+                                     : "memory");
+                    }
                 }
             }
+        }
+        for (int e = tid; e < 64 * 8; e += PF_NT) {   // H64 in the place of the first keys: row n is output dim tile_pos(n) (its own inverse)
+            const int n = e >> 3, c = e & 7, d = tile_pos<BITS>(n);
+            uint32_t v[4];
 #pragma unroll
-            for (int j = 0; j < QB; j++) {
-            const int r = rb + j * MMA_WARP, tk = r / gc, h = r - tk * gc;
-            if (r >= M) break;
+            for (int i = 0; i < 4; i++) {
+                const int k = 8 * c + 2 * i;
+                v[i] = ((__popc(d & k) & 1) ? 0xBC00u : 0x3C00u) | ((__popc(d & (k + 1)) & 1) ? 0xBC000000u : 0x3C000000u);
+            }
+            sts16(base + (uint32_t)(C::K_OFF + n * 128 + ((c ^ (n & 7)) << 4)), v);
+        }
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        const uint32_t d_tmem = *tmem_slot + (uint32_t)C::O_COL;
+        if (warp == MMA_WARP) {
+            const bool leader = elect_one();
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+            if (leader) {
+#pragma unroll
+                for (int nb = 0; nb < NB; nb++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        umma_ss(d_tmem + 64u * nb, make_desc(base + C::Q_OFF + nb * M * 128) + 2 * j, make_desc(base + C::K_OFF) + 2 * j, idesc, j > 0 ? 1u : 0u);
+                umma_commit(rot_done);
+            }
+            __syncwarp();
+        }
+        if (warp < SMW) {   // two threads per row, half of each block's columns each
+            const int half = warp >> 2, r = (warp & 3) * 32 + lane;
+            const uint32_t tq = d_tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+            const float f = p.scale / sqrtf((float)HD);
+            warp_wait(rot_done, 0u);
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 4 * half; c < 4 * half + 4; c++) {
+                uint32_t v[NB][8];
+#pragma unroll
+                for (int nb = 0; nb < NB; nb++) tmem_ld8(tq + (uint32_t)(64 * nb + 8 * c), v[nb]);
+                tmem_ld_wait();
+#pragma unroll
+                for (int len = 1; len < NB; len <<= 1)
+#pragma unroll
+                    for (int nb = 0; nb < NB; nb++)
+                        if (!(nb & len)) {
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                const float a = __uint_as_float(v[nb][i]), b = __uint_as_float(v[nb + len][i]);
+                                v[nb][i] = __float_as_uint(a + b);
+                                v[nb + len][i] = __float_as_uint(a - b);
+                            }
+                        }
+#pragma unroll
+                for (int nb = 0; nb < NB; nb++) {
+                    uint32_t hi[4], lo[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) split2(__uint_as_float(v[nb][2 * i]) * f, __uint_as_float(v[nb][2 * i + 1]) * f, hi[i], lo[i]);
+                    const uint32_t off = base + (uint32_t)(C::Q_OFF + nb * M * 128 + r * 128 + ((c ^ (r & 7)) << 4));
+                    sts16(off, hi);
+                    sts16(off + C::Q_PART, lo);
+                }
+            }
+        }
+    } else if (warp < MMA_WARP) {   // queries rotated already, or other signs
+#pragma unroll 1
+        for (int r = warp; r < M; r += MMA_WARP) {
+            const int tk = r / gc, h = r - tk * gc;
             float x[DPL];
 #pragma unroll
             for (int i = 0; i < DPL; i++) x[i] = 0.f;
@@ -237,7 +339,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
                 if (p.fused_q) {
 #pragma unroll
                     for (int i = 0; i < DPL; i += 4) {
-                        const uint2 q4 = raw[j][i / 4];
+                        const uint2 q4 = *reinterpret_cast<const uint2 *>(p.q + ((size_t)(tok0 + tk) * p.n_q + qh0 + h) * HD + DPL * lane + i);
                         const float4 sg = *reinterpret_cast<const float4 *>(p.signs + DPL * lane + i);
                         const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&q4.x)), f1 = __half22float2(*reinterpret_cast<const __half2 *>(&q4.y));
                         x[i] = f0.x * sg.x;
@@ -294,7 +396,6 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
                     *reinterpret_cast<__half *>(smem + C::Q_OFF + C::Q_PART + off) = lo;
                 }
             }
-            }
         }
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -302,16 +403,6 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    auto warp_wait = [&](uint32_t bar, uint32_t parity) -> bool {
-        uint32_t ok = 1;
-        if (lane == 0) ok = *abort_flag == 0u && mbar_wait(bar, parity, PF_WAIT_LIMIT) ? 1u : 0u;
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok || *abort_flag) {
-            *abort_flag = 1;
-            return false;
-        }
-        return true;
-    };
 
     float m_ref = -INFINITY, l_sum = 0.f;   // softmax threads: reference maximum and sum of this thread's row
     // =========================== decoding warps: codes -> f16 operand tiles ===========================
