@@ -182,7 +182,7 @@ struct lc_smem_optin {
 };
 template <typename Kern>
 static inline cudaError_t lc_ensure_smem(Kern kern, lc_smem_optin &state, const lc_ctx *ctx, size_t smem) {
-    if (smem <= 48 * 1024) return cudaSuccess;
+    if (smem <= 40 * 1024) return cudaSuccess;   // (48 KB less what a kernel may have of static shared memory)
     const int dev = ctx->device;
     if (dev >= 0 && dev < LC_MAX_DEVICES && state.granted[dev].load(std::memory_order_relaxed) >= smem) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 # m > 64, and Q4_0 from 17: 128-row weight tiles, batch tiles of 64 / 128 columns, K splits with a remainder.
 @pytest.mark.parametrize("fmt,m,k,n", [
     ("q4_0", 1, 32, 1), ("q4_0", 8, 96, 65), ("q4_0", 9, 1536, 129), ("q4_0", 16, 2080, 63), ("q4_0", 16, 6144, 1537),
-    ("tq2_0", 9, 256, 127), ("tq2_0", 16, 768, 8193), ("tq2_0", 13, 2048, 33), ("tq2_0", 16, 6144, 1537),
+    ("tq2_0", 9, 256, 127), ("tq2_0", 16, 768, 8193), ("tq2_0", 13, 2048, 33), ("tq2_0", 16, 2304, 6000),
+    ("tq2_0", 16, 6144, 1537),
     ("q4_0", 17, 96, 127), ("q4_0", 64, 1568, 129), ("q4_0", 65, 32, 1), ("q4_0", 129, 2080, 130), ("q4_0", 257, 1536, 300),
     ("tq2_0", 65, 256, 127), ("tq2_0", 128, 1536, 129), ("tq2_0", 129, 6144, 260), ("tq2_0", 300, 768, 1)])
 def test_quantised_matmul_at_tile_edges(la, orc, ctx, kernels, fmt, m, k, n):
