@@ -117,20 +117,19 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
     if (tid < ROWS) {
         const int row = n0 + (GEGLU ? tid % OROWS : tid);
         const uint8_t *wm = p.w[GEGLU ? tid / OROWS : grp];
-        bool counted = false;
         if (row < n_rows) {
             const size_t g0 = (size_t)row * rb, a0 = g0 & ~(size_t)15;
-            const uint32_t bytes = (uint32_t)(((g0 + rb - a0) + 15) & ~(size_t)15);
+            uint32_t bytes = (uint32_t)(((g0 + rb - a0) + 15) & ~(size_t)15);
             uint8_t *dst = raw + tid * p.raw_rs;
-            if (a0 + bytes <= w_bytes) {
-                mbar_arrive_expect_tx(bar, bytes);
-                bulk_g2s(smem_u32(dst), wm + a0, bytes, bar);
-                counted = true;
-            } else {   // the last bytes of the matrix: nothing is read past its end
-                for (uint32_t i = 0; i < bytes; i++) dst[i] = (a0 + i < w_bytes) ? wm[a0 + i] : 0;
+            if (a0 + bytes > w_bytes) {   // the last bytes of the matrix: nothing is read past its end
+                bytes -= 16;
+                for (uint32_t i = 0; i < 16; i++) dst[bytes + i] = (a0 + bytes + i < w_bytes) ? wm[a0 + bytes + i] : 0;
             }
+            mbar_arrive_expect_tx(bar, bytes);
+            if (bytes) bulk_g2s(smem_u32(dst), wm + a0, bytes, bar);
+        } else {
+            mbar_arrive(bar);
         }
-        if (!counted) mbar_arrive(bar);
     }
     // this lane's operand rows: 16 mt + g and + 8
     auto row_at = [&](int mt, int h, bool &ok_) -> uint32_t {
@@ -355,6 +354,8 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     const size_t room = 100 * 1024, sms = (size_t)k->ctx->sm_count;
     int rows = kk <= SM_NW * SM_UNIT ? 64 : 32;
     while (rows > 16 && ((rows_all + rows - 1) / rows < sms * 3 / 4 || rows * rs > room)) rows >>= 1;
+    // ... and, where registers leave an SM one CTA (more than 8 batch rows, several steps per warp), not a little over one wave.
+    if (rows == 16 && m > 8 && kk > SM_NW * SM_UNIT && (rows_all + 15) / 16 > sms && 32 * rs <= room) rows = 32;
     if (rows * rs > room) return -1;
     int tiles = 0;
     const int orows = geglu ? rows / 2 : rows;
