@@ -630,8 +630,10 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
             n_splits = (len_max + chunk - 1) / chunk;
         }
     }
-    // Chunks of several rows: the prefill kernel shares each decoded key among 128 MMA rows.  Below about half a tile of rows
-    // the decode kernel's CTA per row is as fast.
+    // Chunks of several rows: the prefill kernel shares each decoded key among 128 MMA rows, but takes 1900 keys' time (16 us)
+    // before and after its key tiles, of 240 (tq2; else 360) each.  Fewer than half a tile of rows, and chunks whose rows the decode
+    // kernel's CTAs finish sooner by the estimate above, stay there: 64 rows over 400 keys 9.7 us against 16.6, 256 over 330
+    // 20.0 against 19.5, 256 over 4096 87 against 38.
     uint32_t pf_heads = 1, pf_tiles = 0;
     if (prefill && use_mma && lc_tq_attn_prefill_supported(hd, bits)) {
         const uint32_t heads = group < 8 ? group : 8;
@@ -641,10 +643,16 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
             pf_tiles = (n_rows + rows_per_tile - 1) / rows_per_tile;
             const uint32_t ctas = n_kv * gchunks * pf_tiles, tile = lc_tq_attn_prefill_tile_keys(hd, bits);
             const uint32_t seen = len_max + (rows_per_tile < n_rows ? rows_per_tile : n_rows);   // keys of a tile of rows, at most
-            uint32_t most = (seen + tile - 1) / tile;   // at least a tile of keys per split
-            if (most > 64) most = 64;
-            n_splits = ctas < sms ? sms / ctas : 1;
-            if (n_splits > most) n_splits = most;
+            const uint32_t key_tiles = (seen + tile - 1) / tile;
+            uint32_t splits = ctas < sms ? sms / ctas : 1;
+            if (splits > key_tiles) splits = key_tiles;
+            if (splits > MERGE_ROWS_MAX_SPLITS) splits = MERGE_ROWS_MAX_SPLITS;
+            const uint64_t waves = ((uint64_t)ctas * splits + sms - 1) / sms, steps = (key_tiles + splits - 1) / splits;
+            const uint64_t merge = (uint64_t)n_rows * n_q * splits * hd / 6400u;   // partials: 25 KB of them in a key's time
+            if (waves * (in_keys(1900u) + steps * in_keys(bits == 2 ? 240u : 360u)) + in_keys((uint32_t)merge) < grid_cost)
+                n_splits = splits;
+            else
+                pf_tiles = 0;
         }
     }
     const bool pf = pf_tiles != 0;

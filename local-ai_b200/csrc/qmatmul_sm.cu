@@ -355,8 +355,8 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     int rows = kk <= SM_NW * SM_UNIT ? 64 : 32;
     while (rows > 16 && ((rows_all + rows - 1) / rows < sms * 3 / 4 || rows * rs > room)) rows >>= 1;
     // ... and, where registers leave an SM one CTA (more than 8 batch rows, several steps per warp), not a little over one wave.
-    if (rows == 16 && m > 8 && kk > SM_NW * SM_UNIT && (rows_all + 15) / 16 > sms && 32 * rs <= room) rows = 32;
-    if (rows * rs > room) return -1;
+    if (rows == 16 && m > 8 && kk > SM_NW * SM_UNIT && (rows_all + 15) / 16 > sms && 32 * rs <= 190 * 1024) rows = 32;
+    if (rows * rs > (rows == 32 ? 190 * 1024 : room)) return -1;
     int tiles = 0;
     const int orows = geglu ? rows / 2 : rows;
     for (int g = 0; g < SM_GROUPS; g++) {

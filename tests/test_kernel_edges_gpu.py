@@ -93,10 +93,11 @@ def test_merge_of_many_rows(la, orc, ctx, kernels, hd, bits, cap):
     rel_close(buf.as_slice(np.uint8)[8:].view(np.float16), want.astype(np.float32), 2e-3, "merge of many rows")
 
 
-# 128 rows (query rows x heads, heads rounded up to a power of two) to a tile, 32 or 64 keys to a step
+# 128 rows (query rows x heads, heads rounded up to a power of two) to a tile, 32 or 64 keys to a step; chunks of enough rows
+# that the prefill kernel is the one that runs, and one that is too small for it
 @pytest.mark.parametrize("hd,n_q,n_kv,bits,rows,start,window", [
-    (256, 8, 1, 2, 8, 0, 0), (256, 8, 1, 2, 17, 63, 0), (256, 8, 1, 4, 33, 500, 128), (256, 3, 1, 3, 16, 31, 0),
-    (256, 16, 2, 2, 65, 1000, 512), (128, 8, 2, 3, 32, 95, 0), (128, 12, 1, 4, 40, 300, 64), (128, 2, 1, 2, 130, 1, 0)])
+    (256, 8, 1, 2, 150, 463, 0), (256, 8, 1, 4, 300, 500, 128), (256, 3, 1, 3, 300, 31, 0), (256, 16, 2, 2, 155, 1000, 512),
+    (128, 8, 2, 3, 160, 95, 0), (128, 12, 1, 4, 161, 300, 64), (128, 2, 1, 2, 310, 1, 0), (256, 8, 1, 4, 33, 500, 128)])
 def test_prefill_attention_at_tile_edges(la, orc, ctx, kernels, hd, n_q, n_kv, bits, rows, start, window):
     total = start + rows
     c = Cache(la, orc, ctx, hd, n_kv, bits, total, seed=60 + total)
