@@ -96,7 +96,7 @@ static int route(int fmt, bool f32out, const char *name, lc_kernels *k, lc_batch
     }
     if (k->mma && m > 8) {
         if (m <= 64) {
-            if (k->decode_mma && !(k->decode_tc && fmt == 0)) {
+            if (k->decode_mma && !(k->decode_tc && fmt == 0 && m > SM_MAX_M)) {   // (Q4_0 from 17 rows: the large-batch kernel)
                 st = lc_qgemm_mma_grouped(fmt, f32out, k, b, input, 1, ws, os, ns, m, kk);
                 if (st >= 0) return st;
             }

@@ -357,6 +357,9 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     // ... and, where registers leave an SM one CTA (more than 8 batch rows, several steps per warp), not a little over one wave.
     if (rows == 16 && m > 8 && kk > SM_NW * SM_UNIT && (rows_all + 15) / 16 > sms && 32 * rs <= 190 * 1024) rows = 32;
     if (rows * rs > (rows == 32 ? 190 * 1024 : room)) return -1;
+    // Q4_0 with few steps per warp, 9 to 16 rows of activations and more than two waves of tiles: the register-direct kernel's
+    // 64-row tiles read the activations half as often (11 x 1792 x 15996: 18.0 us here, 13.7 there, 16 x 2048 x 12000 15.0 and 12.9; at K = 3072 24 against 28).
+    if (fmt == FMT_Q4_0 && !f32out && m > 8 && kk > SM_NW * SM_UNIT && kk <= 2560 && (rows_all + 31) / 32 > 2 * sms) return -1;
     int tiles = 0;
     const int orows = geglu ? rows / 2 : rows;
     for (int g = 0; g < SM_GROUPS; g++) {

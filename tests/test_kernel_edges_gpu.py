@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 # m <= 16: one 8- or 16-row tile; K in 32- (Q4_0) or 256-wide (TQ2_0) blocks, uneven over the warps; ragged last rows of W.
 # m > 64, and Q4_0 from 17: 128-row weight tiles, batch tiles of 64 / 128 columns, K splits with a remainder.
 @pytest.mark.parametrize("fmt,m,k,n", [
-    ("q4_0", 1, 32, 1), ("q4_0", 8, 96, 65), ("q4_0", 9, 1536, 129), ("q4_0", 16, 2080, 63), ("q4_0", 16, 6144, 1537),
+    ("q4_0", 1, 32, 1), ("q4_0", 8, 96, 65), ("q4_0", 9, 1536, 129), ("q4_0", 16, 2080, 63), ("q4_0", 16, 6144, 1537), ("q4_0", 11, 1792, 14213),
     ("tq2_0", 9, 256, 127), ("tq2_0", 16, 768, 8193), ("tq2_0", 13, 2048, 33), ("tq2_0", 16, 2304, 6000),
     ("tq2_0", 16, 6144, 1537),
     ("q4_0", 17, 96, 127), ("q4_0", 64, 1568, 129), ("q4_0", 65, 32, 1), ("q4_0", 129, 2080, 130), ("q4_0", 257, 1536, 300),
