@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
             uint8_t *dst = raw + tid * p.raw_rs;
             if (a0 + bytes > w_bytes) {   // the last bytes of the matrix: nothing is read past its end
                 bytes -= 16;
+#pragma unroll 1
                 for (uint32_t i = 0; i < 16; i++) dst[bytes + i] = (a0 + bytes + i < w_bytes) ? wm[a0 + bytes + i] : 0;
             }
             mbar_arrive_expect_tx(bar, bytes);
