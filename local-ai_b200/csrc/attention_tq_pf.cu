@@ -9,8 +9,8 @@
 //   * S[128 x KN] = Q . K^T with the query as an f16 and the f16 of its remainder (two MMAs per slice), f32 in tensor memory,
 //     two buffers, so the next tile's product runs beside this one's softmax;
 //   * eight warps own half a query row per thread: row norms, causal and window mask, online softmax with the running maximum moved
-//     only when it has grown by more than 8 (a rescale is a pass over the accumulator); P times the value norms goes back to
-//     tensor memory;
+//     only when it has grown by more than LAZY (a rescale is a pass over the accumulator), or at all where a tile's value norms
+//     are so large that P could leave f16's range; P times the value norms goes back to tensor memory;
 //   * O[128 x HD] += P . V with P read from tensor memory.
 // Precision as in attention_tq_mma.cu: tq2 levels are f16-exact up to a factor gamma that is folded into the norms, P is an f16;
 // tq3 / tq4 levels and P are an f16 and the f16 of the remainder, which doubles the operand tiles.
@@ -26,6 +26,10 @@ namespace {
 constexpr int M = 128;
 constexpr int SMW = 8, DKW = 8, DVW = 4, MMA_WARP = SMW + DKW + DVW, PF_NT = (MMA_WARP + 1) * 32;   // softmax, K, V, issue
 constexpr uint32_t PF_WAIT_LIMIT = 1u << 22;
+// A weight is at most e^LAZY while the running maximum lags, and P, the weight times v_norm * gamma, is stored as f16: tiles with
+// a larger factor than LAZY_VMAX (e^8 * 21 = 62600 < 65504) move the maximum whenever it grows, which leaves P <= v_norm * gamma.
+// Unit normal V rows have 1 - 3, so the usual tile keeps the lag.
+constexpr float LAZY = 8.0f, LAZY_VMAX = 21.0f;
 
 template <int HD_, int BITS_>
 struct PfCfg {
@@ -43,6 +47,7 @@ struct PfCfg {
     static constexpr int STAGE = M * (HD + 4) * 4;               // results, reuses the operand tiles
     static constexpr int TAIL = NORM_OFF + NORM_BYTES;
     static constexpr int SMEM = (TAIL > STAGE ? TAIL : STAGE) + 256 + 1024;
+    static constexpr int NVW = KN / 32;                          // warps that fetch a tile's V norms, one lane per key
     static_assert(NUK >= 1 && NUV >= 1 && SMEM <= 226 * 1024, "shared memory");
     static constexpr int S_COL = 0, P_COL = 128, PL_COL = 160, O_COL = 256;   // tensor memory: S x 2, P, remainder of P, O
 };
@@ -124,7 +129,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
     const uint32_t k_full = bars, v_full = bars + 8, p_full = bars + 16, pv_done = bars + 24, qk_done = bars + 32, rot_done = bars + 56;   // qk_done: two
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + BAR_OFF + 48);
     volatile uint32_t *abort_flag = tmem_slot + 1;
-    __shared__ float m_s[M], l_s[2][M], mx_s[2][2][M], gamma_s, cand_err[PF_NT / 32];
+    __shared__ float m_s[M], l_s[2][M], mx_s[2][2][M], vmax_s[4][C::NVW], gamma_s, cand_err[PF_NT / 32];
     __shared__ int cand_idx[PF_NT / 32];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -498,7 +503,13 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
             for (int j = 0; j < NU; j++)
 #pragma unroll
                 for (int i = 0; i < W; i++) now[j][i] = raw[j][i];
-            if (with_norms && dt < 2 * KN) norms[(t & 3) * 2 * KN + dt] = norm_next;   // (read before QK of tile t + 2 was issued)
+            if (with_norms && dt < 2 * KN) {   // (read before QK of tile t + 2 was issued)
+                norms[(t & 3) * 2 * KN + dt] = norm_next;
+                if (dt >= KN) {   // whole warps: the largest magnitude (as integers, so that a NaN is the largest)
+                    const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(norm_next)));
+                    if (lane == 0) vmax_s[t & 3][(dt - KN) / 32] = __uint_as_float(most);
+                }
+            }
             if (t + 1 < tiles) fetch(t + 1);
             if (t > 0 && !free_wait(t - 1)) break;
             decode(now);
@@ -588,6 +599,8 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
             }
             const float *kn = norms + (t & 3) * 2 * KN + half * KH, *vn = kn + KN;
             const uint32_t t0 = k_begin + (uint32_t)(t * KN + half * KH), end = min(row_end, k_end);
+            const bool in_range = vmax_s[t & 3][0] <= LAZY_VMAX && vmax_s[t & 3][C::NVW - 1] <= LAZY_VMAX;
+            const float lag = in_range ? LAZY : 0.f;
             float mx = -INFINITY;
 #pragma unroll
             for (int i = 0; i < KH; i += 4) {
@@ -607,7 +620,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
             mx = fmaxf(mx, mx_s[t & 1][half ^ 1][r]);
             if (t == 0) {
                 m_ref = mx;
-            } else if (__any_sync(0xffffffffu, mx > m_ref + 8.0f)) {
+            } else if (__any_sync(0xffffffffu, mx > m_ref + lag)) {
                 // the accumulator moves to the new maximum: PV of the tile before has to be complete
                 warp_wait(pv_done, (uint32_t)((t - 1) & 1));
                 tc_fence_after();

@@ -145,3 +145,45 @@ def test_encoder_rows_at_block_edges(la, orc, ctx, kernels, hd, rows):
     orc.encode_kv(x, levels, signs, want_c, want_n, hd, n_kv, rows, bits, 0, 0)
     codes, norms = gpu_encode(la, ctx, kernels, x, levels, signs, hd, n_kv, rows, bits, 0, 0, rows)
     assert np.array_equal(codes, want_c) and np.array_equal(norms, want_n.view(np.uint16))
+
+
+# V rows far above unit norm and logits that grow along the context: P, the softmax weight times v_norm * gamma, is stored as
+# f16, so the weights that a lagging maximum allows (up to e^8) must not carry it past 65504
+@pytest.mark.parametrize("bits,vnorm,window,ring", [(2, 1000.0, 0, 0), (2, 60000.0, 512, 1024), (4, 1000.0, 0, 0), (4, 200.0, 512, 1024),
+                                                    (3, 60000.0, 0, 0)])
+def test_prefill_attention_keeps_large_value_norms_in_range(la, orc, ctx, kernels, bits, vnorm, window, ring):
+    hd, n_q, n_kv, rows, total = 256, 8, 1, 400, 1200
+    slots = ring or total
+    levels, signs = la.tq_levels(hd, bits), la.tq_signs(hd, la.TQ_SEED)
+    cb = la.tq_code_bytes(hd, bits)
+    rng = np.random.default_rng(bits)
+    one = rng.integers(0, 256, cb, dtype=np.uint8)                      # every K row has one direction; its norms set the logits
+    k0 = levels[(np.unpackbits(one, bitorder="little").reshape(hd, bits) * (1 << np.arange(bits))).sum(1)].astype(np.float64)
+    slot = np.arange(total) % slots                                     # (later positions overwrite the ring's earlier ones)
+    kc, vc = np.tile(one, slots), rng.integers(0, 256, slots * cb, dtype=np.uint8)
+    kn, vn = np.zeros(slots, np.float16), np.zeros(slots, np.float16)
+    kn[slot] = (0.5 + np.arange(total) / total + 6.0 * (np.arange(total) % 240 >= 130)).astype(np.float16)   # steps of 4.5 .. 6.9
+    vn[slot] = np.where(np.arange(total) // 100 % 2, vnorm, 1.0).astype(np.float16)
+    rq = (np.linspace(0.75, 1.15, rows * n_q)[:, None] * (k0 / (k0 @ k0))).astype(np.float32).reshape(-1)   # logits 0.4 .. 8.6
+    q16 = orc.hadamard_rotate(rq, signs, hd, rows * n_q, False, True).astype(np.float16)
+    f = lambda a: la.CudaBuffer.from_slice(ctx, a)
+    bufs = (f(kc), f(kn), f(vc), f(vn), f(levels))
+    out, fused = Guarded(la, ctx, rows * n_q * hd * 4), Guarded(la, ctx, rows * n_q * hd * 2)
+    start = total - rows
+    b = la.CommandBatch.new(ctx)
+    kernels.flash_attention_tq_prefill_into(b, f(rq), *bufs, out.view, hd, total, start, rows, n_q, n_kv, window, bits, ring, 1.0)
+    kernels.tq_attention_prefill_into(b, f(q16), *bufs, f(signs), fused.view, hd, total, start, rows, n_q, n_kv, window, bits, ring, 1.0)
+    b.commit_and_wait()
+    attend = lambda x: orc.flash_attention_tq_prefill(x, kc, kn, vc, vn, levels, hd, total, start, rows, n_q, n_kv, window, bits, ring, 1.0)
+    # The weights sum to 1.  tq2 rounds each P to f16: 2^-11 of it.  tq3 / tq4 keep P, levels and query in two f16 parts, 2^-22 each;
+    # of logits up to 8.6 that is 2^-19, and 2^-16 leaves as much again for f32 sums and exponentials.  The inverse rotation keeps
+    # a row's 2-norm, and its f16 result adds 2^-11.
+    most = np.abs(levels).max() * vnorm
+    tol = most * (2.0 ** -11 if bits == 2 else 2.0 ** -16)
+    got, want = out.read(np.float32), attend(rq)
+    assert np.isfinite(got).all() and np.abs(got - want).max() <= tol, np.abs(got - want).max() / tol
+    back = orc.hadamard_rotate(attend(orc.hadamard_rotate(q16.astype(np.float32), signs, hd, rows * n_q, True, False)), signs, hd, rows * n_q, False, True)
+    back, got = back.reshape(-1, hd), fused.read(np.float16).astype(np.float64).reshape(-1, hd)
+    off = np.linalg.norm(got - back, axis=1)
+    assert np.all(off <= tol * np.sqrt(hd) + 2.0 ** -11 * np.linalg.norm(back, axis=1)), off.max()
+    device_status_ok(kernels)
