@@ -25,8 +25,10 @@ int lc_check_qargs(int fmt, const char *name, lc_kernels *k, lc_batch *b, const 
 // a negative value when the shape is outside what it covers (caller falls through).
 int lc_qgemm_tcl_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng, const lc_buf *const *weights,
                         lc_buf *const *outputs, const uint32_t *ns, uint32_t m, uint32_t kk);
+uint64_t lc_qgemm_tcl_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uint32_t n);   // ns, one Q4_0 matrix, 16 < m <= 64
 
 // qmatmul_mma.cu: same contract, for 8 < m <= 64.
+uint64_t lc_qgemm_mma_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uint32_t n);   // as above
 int lc_qgemm_mma_grouped(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng,
                          const lc_buf *const *weights, lc_buf *const *outputs, const uint32_t *ns, uint32_t m,
                          uint32_t kk);
@@ -96,7 +98,10 @@ static int route(int fmt, bool f32out, const char *name, lc_kernels *k, lc_batch
     }
     if (k->mma && m > 8) {
         if (m <= 64) {
-            if (k->decode_mma && !(k->decode_tc && fmt == 0 && m > SM_MAX_M)) {   // (Q4_0 from 17 rows: the large-batch kernel)
+            // Q4_0 from 17 rows: whichever kernel's estimate is less.  40 x 6144 x 1536 9.4 us on the large-batch kernel, 15.3 on the
+            // other; 24 x 6144 x 4096 20.0 and 17.2; 25 x 70991 x 512 30.8 and 20.2; 64 x 262144 x 256 93 and 61.
+            const bool choose = k->decode_tc && fmt == 0 && m > SM_MAX_M;
+            if (k->decode_mma && (!choose || lc_qgemm_mma_estimate(k, m, kk, n) < lc_qgemm_tcl_estimate(k, m, kk, n))) {
                 st = lc_qgemm_mma_grouped(fmt, f32out, k, b, input, 1, ws, os, ns, m, kk);
                 if (st >= 0) return st;
             }

@@ -562,13 +562,69 @@ int launch_wide(lc_kernels *k, lc_batch *b, const WideParams &p) {
 
 }  // namespace
 
+// How a launch of `tiles` 128-row tiles splits K (at most 8 ways: one cluster per tile): while the grid stays within 1.5 CTAs
+// per SM (measured optimum: more splits cost more in the exchange than they gain in parallelism); whole 256-k chunks per split.
+struct MmaPlan {
+    int ks, cps, bps, nbt, raw_rs;   // splits of cps chunks (bps blocks); 8-row batch tiles
+    size_t smem;                     // (more than an SM has: the K range is too long for one CTA's raw rows)
+};
+static MmaPlan mma_plan(int fmt, const lc_kernels *k, uint32_t m, uint32_t kk, int tiles) {
+    const int be = fmt == FMT_Q4_0 ? 32 : 256, bb = fmt == FMT_Q4_0 ? 18 : 66;
+    MmaPlan pl;
+    pl.nbt = m <= 16 ? 2 : (m <= 32 ? 4 : 8);
+    const int chb = CHUNK_K / be, nchunk = ((int)(kk / be) + chb - 1) / chb;   // blocks per 256 k
+    pl.ks = (3 * k->ctx->sm_count / 2) / tiles;
+    if (pl.ks > MAX_KS) pl.ks = MAX_KS;
+    if (pl.ks > nchunk) pl.ks = nchunk;
+    if (pl.ks < 1) pl.ks = 1;
+    pl.cps = (nchunk + pl.ks - 1) / pl.ks;
+    pl.ks = (nchunk + pl.cps - 1) / pl.cps;
+    pl.bps = pl.cps * chb;
+    pl.raw_rs = ((pl.bps * bb + 15 + 15) / 16) * 16;
+    if ((pl.raw_rs / 16) % 2 == 0) pl.raw_rs += 16;    // odd multiple of 16 bytes: rows spread over the banks
+    pl.smem = (size_t)2 * 8 * pl.nbt * XS + (size_t)CTA_ROWS * pl.raw_rs;
+    return pl;
+}
+
+// Time of the two kernels here for one Q4_0 matrix, in ns (~0: not covered), fitted as lc_qgemm_tcl_estimate (qmatmul_tcl.cu) and
+// compared with it.  What decides: a tall matrix at short K is a second and third CTA per SM here, without a fixed cost per wave; with
+// fewer tiles than SMs, how often the splits' clusters have to share SMs.  From 33 rows the f32 scaling of every block doubles
+// this kernel's work, and it keeps the tall matrices only.
+static uint64_t wide_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uint32_t n) {
+    const uint64_t sms = (uint64_t)k->ctx->sm_count, tiles = (n + W_ROWS - 1) / W_ROWS;
+    if (m <= 32 || kk % W_CK != 0 || n < W_ROWS * sms || (size_t)W_STAGES * W_STAGE > k->ctx->smem_optin) return ~0ull;
+    return (tiles + sms - 1) / sms * (4000 + 5800 * (uint64_t)(kk / W_CK));
+}
+static uint64_t narrow_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uint32_t n) {
+    const uint64_t sms = (uint64_t)k->ctx->sm_count, tiles = (n + CTA_ROWS - 1) / CTA_ROWS, K = kk;
+    const MmaPlan pl = mma_plan(FMT_Q4_0, k, m, kk, (int)tiles);
+    if (pl.smem > k->ctx->smem_optin) return ~0ull;
+    const bool alone = 2 * (pl.smem + 1024) > 228 * 1024;   // one CTA fills an SM
+    if (tiles > sms) {
+        const uint64_t rounds = (tiles + sms - 1) / sms;
+        if (m <= 32) return rounds * (alone ? 2800 + 9 * K : 900 + 8 * K);
+        return rounds * (alone ? 3000 + 14 * K : 2600 + 9 * K);
+    }
+    const uint64_t ks = (uint64_t)pl.ks, cps = (uint64_t)pl.cps, ctas = tiles * ks, seen = ctas < sms ? ctas : sms;
+    if (m > 32) return ~0ull - 1;
+    const bool shared = ks > 1 && 10 * tiles > 9 * k->cluster_cap[ks];   // clusters meet on SMs
+    uint64_t t = 2600 + 900 * K / (256 * ks) + 1550 * seen * cps / sms;
+    if (ctas > sms) t += 1750 + (alone ? 950 * cps : 0) - (alone ? 0 : 550 * cps);
+    if (ks > 1) t += 300 * ks + 1200 * (ks == 2 && !shared ? 1 : cps) * seen / sms + (shared ? 950 : 0) - 270 * ks * seen / sms;
+    return t;
+}
+uint64_t lc_qgemm_mma_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uint32_t n) {
+    const uint64_t a = wide_estimate(k, m, kk, n), b = narrow_estimate(k, m, kk, n);
+    return a < b ? a : b;
+}
+
 // Grouped launch: `ng` weight matrices [ns[g], kk] sharing the activations `input` [m, kk], 8 < m <= 64.
 // Returns LC_OK after a launch, a positive status on error, or -1 when the shape is outside what this kernel
 // covers (the caller then uses another path).
 static int qgemm_mma_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng,
                             const lc_buf *const *weights, lc_buf *const *outputs, const uint32_t *ns, uint32_t m,
                             uint32_t kk, bool geglu) {
-    const int be = fmt == FMT_Q4_0 ? 32 : 256, bb = fmt == FMT_Q4_0 ? 18 : 66;
+    const int be = fmt == FMT_Q4_0 ? 32 : 256;
     if (m > 64 || ng < 1 || ng > MAX_GROUPS || kk % be != 0 || !lc_aligned(input->dptr, 16)) return -1;
     if (m <= 8) return -1;   // small batches: qmatvec_mma.cu / qmatvec.cu
     MmaParams p;
@@ -586,8 +642,7 @@ static int qgemm_mma_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, co
         if (g < ng) tiles += ((int)ns[g] + CTA_ROWS - 1) / CTA_ROWS;
         p.tile_end[g] = tiles;
     }
-    if (!geglu && fmt == FMT_Q4_0 && ng == 1 && m > 32 && kk % W_CK == 0 && ns[0] >= (uint32_t)(W_ROWS * k->ctx->sm_count) &&
-        (size_t)W_STAGES * W_STAGE <= k->ctx->smem_optin) {
+    if (!geglu && fmt == FMT_Q4_0 && ng == 1 && wide_estimate(k, m, kk, ns[0]) < narrow_estimate(k, m, kk, ns[0])) {
         WideParams wp;
         wp.w = (const uint8_t *)weights[0]->dptr;
         wp.out = outputs[0]->dptr;
@@ -601,25 +656,14 @@ static int qgemm_mma_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, co
     }
     p.geglu = geglu ? 1 : 0;
     if (geglu) tiles = ((int)ns[0] + CTA_ROWS / 2 - 1) / (CTA_ROWS / 2);
-    const int nbt = m <= 16 ? 2 : (m <= 32 ? 4 : 8);
-    // Split K (at most 8 ways: one cluster per tile) while the grid stays within 1.5 CTAs per SM (measured optimum:
-    // more splits cost more in the exchange than they gain in parallelism); whole 256-k chunks per
-    // split, and no more raw bytes per CTA than fit beside the activation buffers.
-    const int chb = CHUNK_K / be;                       // blocks per 256 k
-    const int nchunk = (p.nb + chb - 1) / chb;
-    int ks = (3 * k->ctx->sm_count / 2) / tiles;
-    if (ks > MAX_KS) ks = MAX_KS;
-    if (ks > nchunk) ks = nchunk;
-    if (ks < 1) ks = 1;
-    int cps = (nchunk + ks - 1) / ks;                   // chunks per split
-    ks = (nchunk + cps - 1) / cps;
-    p.ks = ks;
-    p.bps = cps * chb;
-    p.raw_rs = ((p.bps * bb + 15 + 15) / 16) * 16;
-    if ((p.raw_rs / 16) % 2 == 0) p.raw_rs += 16;      // odd multiple of 16 bytes: rows spread over the banks
-    const size_t smem = (size_t)2 * 8 * nbt * XS + (size_t)CTA_ROWS * p.raw_rs;
-    if (smem > k->ctx->smem_optin) return -1;           // K range too long for one CTA's raw rows (tcgen05 path instead)
-    dim3 grid(tiles, 1, ks);
+    const MmaPlan pl = mma_plan(fmt, k, m, kk, tiles);
+    if (pl.smem > k->ctx->smem_optin) return -1;        // (tcgen05 path instead)
+    const int nbt = pl.nbt;
+    const size_t smem = pl.smem;
+    p.ks = pl.ks;
+    p.bps = pl.bps;
+    p.raw_rs = pl.raw_rs;
+    dim3 grid(tiles, 1, pl.ks);
     if (fmt == FMT_Q4_0)
         return f32out ? launch_mma_nbt<FMT_Q4_0, float>(b, p, grid, smem, nbt) : launch_mma_nbt<FMT_Q4_0, __half>(b, p, grid, smem, nbt);
     return f32out ? launch_mma_nbt<FMT_TQ2_0, float>(b, p, grid, smem, nbt) : launch_mma_nbt<FMT_TQ2_0, __half>(b, p, grid, smem, nbt);

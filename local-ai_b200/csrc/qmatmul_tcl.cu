@@ -438,6 +438,51 @@ int launch_tcl(lc_batch *b, const TclParams &p, const CUtensorMap &x_map, int ti
 
 }  // namespace
 
+// Batch rows per CTA and K splits of a launch of `tiles` 128-row tiles: a step costs its tensor-memory stores (about 900 cycles)
+// or its MMAs (8 per column), whichever is more; a launch costs about 2500 cycles around its steps, the exchange of a split 3000
+// more.  Clusters cannot use every SM, other launches can.
+struct TclPlan {
+    int m_tiles, NB, ks, sps, steps;   // ks splits of sps steps
+    uint64_t waves;
+};
+static TclPlan tcl_plan(int fmt, const lc_kernels *k, uint32_t m, uint32_t kk, int tiles) {
+    const int step_k = fmt == FMT_Q4_0 ? TclFmt<FMT_Q4_0>::step_k : TclFmt<FMT_TQ2_0>::step_k;
+    TclPlan pl = {1, 16, 1, 1, ((int)kk + step_k - 1) / step_k, 1};
+    uint64_t best = ~0ull;
+    for (int mt = ((int)m + MAX_NB - 1) / MAX_NB; mt <= ((int)m + 47) / 48; mt++) {
+        const int nb = (((int)m + mt - 1) / mt + 15) / 16 * 16, real_mt = ((int)m + nb - 1) / nb;
+        for (int ks = 1; ks <= MAX_KS && (ks == 1 || 2 * ks <= pl.steps); ks++) {
+            const uint64_t at_once = ks > 1 ? k->cluster_cap[ks] : (uint64_t)k->ctx->sm_count, waves = ((uint64_t)tiles * real_mt + at_once - 1) / at_once;
+            const uint64_t cost = waves * (2500u + (uint64_t)((pl.steps + ks - 1) / ks) * (uint64_t)(8 * nb > 900 ? 8 * nb : 900) + (ks > 1 ? 3000u + 10u * nb : 0u));
+            if (cost < best) {
+                best = cost;
+                pl.m_tiles = real_mt;
+                pl.NB = nb;
+                pl.ks = ks;
+                pl.waves = waves;
+            }
+        }
+    }
+    pl.sps = (pl.steps + pl.ks - 1) / pl.ks;
+    pl.ks = (pl.steps + pl.sps - 1) / pl.sps;
+    return pl;
+}
+
+// What a launch over one Q4_0 matrix takes at 17 .. 64 rows, in ns, for the choice between this kernel and the register-direct one
+// (qmatmul_mma.cu).  Fitted to both kernels' times over 1100 shapes of n 300 .. 262144 and K 128 .. 8192 (6 % off on average): the
+// choice takes 0.4 % longer than the faster kernel on average, at most 16 % (0.4 us, K = 128).  A step takes about 1000; where a
+// second launch fits beside the first, its CTAs fetch and unpack their first steps meanwhile.
+uint64_t lc_qgemm_tcl_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uint32_t n) {
+    const uint64_t tiles = (n + ROWS - 1) / ROWS, sms = (uint64_t)k->ctx->sm_count;
+    const TclPlan pl = tcl_plan(FMT_Q4_0, k, m, kk, (int)tiles);
+    const uint64_t sps = (uint64_t)pl.sps, groups = tiles * pl.m_tiles, ctas = groups * pl.ks;
+    if (tiles > sms) return pl.waves * (4000 + 1000 * sps);
+    uint64_t t = 1850 + 1000 * sps + 2250 * (ctas < sms ? ctas : sms) / sms;
+    if (pl.ks > 1) t += 750 + 40 * pl.ks;
+    if (2 * groups <= (pl.ks > 1 ? k->cluster_cap[pl.ks] : sms)) t -= 350 * sps;
+    return pl.waves * t;
+}
+
 // Grouped launch: `ng` weight matrices [ns[g], kk] sharing the activations `input` [m, kk].  Returns LC_OK after a launch, a
 // positive status on error, or -1 when the shape is outside what this kernel covers (the caller then uses the CUDA-core path).
 int lc_qgemm_tcl_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng, const lc_buf *const *weights,
@@ -460,29 +505,12 @@ int lc_qgemm_tcl_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const 
     }
     if (tiles < 1) return -1;
     const int step_k = fmt == FMT_Q4_0 ? TclFmt<FMT_Q4_0>::step_k : TclFmt<FMT_TQ2_0>::step_k;
-    p.steps = ((int)kk + step_k - 1) / step_k;
-    // Batch rows per CTA and K splits: a step costs its tensor-memory stores (about 900 cycles) or its MMAs (8 per column),
-    // whichever is more; a launch costs about 2500 cycles around its steps, the exchange of a split 3000 more.  Clusters
-    // cannot use every SM, other launches can.
-    const int sms = k->ctx->sm_count;
-    uint64_t best = ~0ull;
-    p.m_tiles = 1;
-    p.ks = 1;
-    for (int mt = ((int)m + MAX_NB - 1) / MAX_NB; mt <= ((int)m + 47) / 48; mt++) {
-        const int nb = (((int)m + mt - 1) / mt + 15) / 16 * 16, real_mt = ((int)m + nb - 1) / nb;
-        for (int ks = 1; ks <= MAX_KS && (ks == 1 || 2 * ks <= p.steps); ks++) {
-            const uint64_t at_once = ks > 1 ? k->cluster_cap[ks] : (uint64_t)sms, waves = ((uint64_t)tiles * real_mt + at_once - 1) / at_once;
-            const uint64_t cost = waves * (2500u + (uint64_t)((p.steps + ks - 1) / ks) * (uint64_t)(8 * nb > 900 ? 8 * nb : 900) + (ks > 1 ? 3000u + 10u * nb : 0u));
-            if (cost < best) {
-                best = cost;
-                p.m_tiles = real_mt;
-                p.NB = nb;
-                p.ks = ks;
-            }
-        }
-    }
-    p.sps = (p.steps + p.ks - 1) / p.ks;
-    p.ks = (p.steps + p.sps - 1) / p.sps;
+    const TclPlan pl = tcl_plan(fmt, k, m, kk, tiles);
+    p.steps = pl.steps;
+    p.m_tiles = pl.m_tiles;
+    p.NB = pl.NB;
+    p.ks = pl.ks;
+    p.sps = pl.sps;
     if (p.m_tiles > 65535) return -1;
     p.status = k->dev_status;
     p.wait_limit = k->test_wait_expiry ? 4096u : WAIT_LIMIT;

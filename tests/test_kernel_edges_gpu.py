@@ -1,5 +1,7 @@
 """The tensor-core kernels at the sizes where their tiling can go wrong: tile edges, remainders, the smallest and the
 largest of each dispatch range, against the CPU oracle."""
+import time
+
 import numpy as np
 import pytest
 
@@ -187,3 +189,50 @@ def test_prefill_attention_keeps_large_value_norms_in_range(la, orc, ctx, kernel
     off = np.linalg.norm(got - back, axis=1)
     assert np.all(off <= tol * np.sqrt(hd) + 2.0 ** -11 * np.linalg.norm(back, axis=1)), off.max()
     device_status_ok(kernels)
+
+
+# Q4_0 at 17 .. 64 rows goes to the kernel that is estimated to take less: shapes of both, their clusters and edges
+Q4_0_ROUTES = [(17, 1024, 8200), (24, 4096, 4600), (32, 1536, 4100), (20, 256, 19001), (29, 768, 20737), (33, 128, 75777), (64, 256, 75900),
+               (45, 384, 19300), (32, 2048, 12300), (18, 160, 334)]
+
+
+@pytest.mark.parametrize("m,k,n", Q4_0_ROUTES)
+def test_q4_0_matmul_of_17_to_64_rows(la, orc, ctx, kernels, m, k, n):
+    raw = la.synth.q4_0_weights(n, k, 33)
+    a = la.synth.normal_f16((m, k), 34)
+    got = run_matmul(la, ctx, kernels, "matmul_nt_q4_0_into", a, raw, m, k, n).reshape(m, n)
+    rows = np.r_[0:200, n // 2:n // 2 + 200, n - 200:n] if n > 4000 else np.arange(n)   # (the oracle's time)
+    some = np.ascontiguousarray(raw.reshape(n, -1)[rows])
+    want = orc.matmul_nt(orc.Q4_0, a, some, m, k, rows.size).reshape(m, -1)
+    rel_close(got[:, rows], want, 1e-3, f"q4_0 m={m} k={k} n={n}")
+    assert np.isfinite(got).all() and got.std(axis=0).min() > 0
+    device_status_ok(kernels)
+
+
+@pytest.mark.parametrize("m,k,n", [(24, 512, 40000), (20, 256, 100000), (50, 256, 150000), (24, 4096, 6144), (40, 1536, 6144)])
+def test_q4_0_matmul_of_17_to_64_rows_is_not_the_slower_kernel(la, ctx, kernels, monkeypatch, m, k, n):
+    """The choice against the register-direct kernel alone (LOCAL_CUDA_DECODE_TC=0): at most 1.1 times its time, where a wrong
+    choice takes 1.16 to 1.9 times."""
+    monkeypatch.setenv("LOCAL_CUDA_DECODE_TC", "0")
+    other = la.Kernels.new(ctx)
+    w, x, out = la.CudaBuffer.empty(ctx, n * k // 32 * 18), la.CudaBuffer.empty(ctx, m * k * 2), la.CudaBuffer.empty(ctx, m * n * 2)
+    w.zero(), x.zero()
+    graphs = []
+    for kern in (kernels, other):
+        for begin in (la.CommandBatch.new, la.CommandBatch.capture):
+            b = begin(ctx)
+            for _ in range(20):
+                kern.matmul_nt_q4_0_into(b, x, w, out, m, k, n)
+            b.commit_and_wait() if begin == la.CommandBatch.new else graphs.append(b.end_capture())
+    best = [np.inf, np.inf]
+    for _ in range(8):
+        for i, g in enumerate(graphs):
+            ctx.synchronize()
+            t = time.perf_counter()
+            g.launch()
+            ctx.synchronize()
+            best[i] = min(best[i], time.perf_counter() - t)
+    for g in graphs:
+        g.destroy()
+    other.close()
+    assert best[0] <= 1.1 * best[1], best
