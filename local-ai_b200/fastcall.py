@@ -7,7 +7,8 @@ those of the ctypes binding, so they cannot drift from the C ABI.
 
 A handle argument is a `Handle` (or a subclass), an integer address or None; a scalar is anything with `__index__` /
 `__float__`; an array of handles is a list or tuple of handles.  A function that returns a status raises through the
-factory given to `bind` when the status is not 0 and returns None otherwise.
+factory given to `bind` when the status is not 0 and returns None otherwise.  The first call loads the library, by the
+function given to `on_first_call`.
 """
 from __future__ import annotations
 
@@ -51,6 +52,7 @@ def _function(ret: str, name: str, params: list[tuple[str, str]]) -> str:
         else:
             lines.append(f"    void *v{i}; if (to_ptr(a[{i}], &v{i})) return NULL;")
         call.append(f"({ty})v{i}" if stars else f"v{i}")
+    lines.append(f"    if (!fn_{name} && load()) return NULL;")
     types = ", ".join(t for t, _ in params) or "void"
     fn = f"(({ret} (*)({types}))fn_{name})({', '.join(call)})"
     if ret == "int":
@@ -92,7 +94,14 @@ typedef struct {
     void *h;
 } Handle;
 static PyTypeObject HandleType;
-static PyObject *error_factory, *str_value;
+static PyObject *error_factory, *loader, *str_value;
+
+static int load(void) {   // the library is loaded, and the functions bound, by the first call
+    PyObject *r = loader ? PyObject_CallNoArgs(loader) : NULL;
+    if (!r && !PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "liblocal_cuda.so is not loaded");
+    Py_XDECREF(r);
+    return r ? 0 : -1;
+}
 
 static int to_ptr(PyObject *o, void **out) {
     if (PyObject_TypeCheck(o, &HandleType)) { *out = ((Handle *)o)->h; return 0; }
@@ -182,7 +191,7 @@ static PyTypeObject HandleType = {
 static PyObject *begin(PyObject *self, PyObject *const *a, Py_ssize_t n) {   // begin(batch, ctx)
     void *ctx, *h = NULL;
     if (n != 2 || !PyObject_TypeCheck(a[0], &HandleType)) return wrong_count("begin", "batch, ctx", 2, n);
-    if (to_ptr(a[1], &ctx)) return NULL;
+    if (to_ptr(a[1], &ctx) || (!fn_lc_batch_begin && load())) return NULL;
     const int r = ((int (*)(lc_ctx *, lc_batch **))fn_lc_batch_begin)((lc_ctx *)ctx, (lc_batch **)&h);
     ((Handle *)a[0])->h = h;
     return status(r);
@@ -190,6 +199,7 @@ static PyObject *begin(PyObject *self, PyObject *const *a, Py_ssize_t n) {   // 
 static PyObject *commit(PyObject *self, PyObject *const *a, Py_ssize_t n) {   // commit(batch, pending): empties batch
     if (n != 2 || !PyObject_TypeCheck(a[0], &HandleType) || !PyObject_TypeCheck(a[1], &HandleType))
         return wrong_count("commit", "batch, pending", 2, n);
+    if (!fn_lc_batch_commit_async && load()) return NULL;
     void *b = ((Handle *)a[0])->h, *p = NULL;
     ((Handle *)a[0])->h = NULL;
     const int r = ((int (*)(lc_batch *, lc_pending **))fn_lc_batch_commit_async)((lc_batch *)b, (lc_pending **)&p);
@@ -218,6 +228,11 @@ static PyObject *bind(PyObject *self, PyObject *args) {   // bind({name: address
     Py_XSETREF(error_factory, factory);
     Py_RETURN_NONE;
 }
+static PyObject *on_first_call(PyObject *self, PyObject *f) {   // f() has to call bind
+    Py_INCREF(f);
+    Py_XSETREF(loader, f);
+    Py_RETURN_NONE;
+}
 // method(function): a function of this module as a method (the object becomes its first argument)
 static PyObject *method(PyObject *self, PyObject *f) { return PyInstanceMethod_New(f); }
 
@@ -226,6 +241,7 @@ static PyMethodDef own[] = {
     {"commit", (PyCFunction)(void (*)(void))commit, METH_FASTCALL, NULL},
     {"take", take, METH_O, NULL},
     {"bind", bind, METH_VARARGS, NULL},
+    {"on_first_call", on_first_call, METH_O, NULL},
     {"method", method, METH_O, NULL},
     {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", NULL, -1, own, NULL, NULL, NULL, NULL};

@@ -56,6 +56,7 @@ def _load():
 
 
 _load.bound = False
+_fast.on_first_call(_load)
 
 
 class CudaContext(Handle):

@@ -88,3 +88,22 @@ def test_product_never_imports_the_oracle():
     for f in list(pkg.glob("*.py")) + list((pkg / "csrc").glob("*")):
         text = f.read_text(errors="ignore")
         assert "oracle" not in text.lower(), f.name
+
+
+@pytest.mark.parametrize("call", ["la.PendingCommandBuffer().wait()", "la.Kernels.gelu_mul_into(None, None, None, None, None, 4)",
+                                  "la.kernels.tq_attention_noalloc_into(*[None] * 9, 256, 1, 0, 8, 1, 0, 2, 0, 1.0)"])
+def test_a_call_before_the_library_is_loaded_loads_it(call):
+    """The first call of a process may come before any context exists: it is an error of its arguments, not a crash."""
+    import pathlib
+    import subprocess
+    import sys
+    code = f"""
+import __graft_entry__ as g
+la = g.load_package()
+try:
+    {call}
+except la.Error as e:
+    print(e.kind)
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=pathlib.Path(__file__).resolve().parent.parent, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "InvalidArgument", (r.returncode, r.stdout, r.stderr[-500:])
