@@ -11,6 +11,7 @@ from __future__ import annotations
 import ctypes as C
 import importlib.util
 import re
+import warnings
 from pathlib import Path
 
 from . import build
@@ -67,12 +68,20 @@ _fast = None
 
 
 def fastcall():
-    """The generated CPython extension (fastcall.py): handles and calls without ctypes.  `load` binds its functions."""
+    """The generated CPython extension (fastcall.py): handles and calls without ctypes.  `load` binds its functions.  Where it is
+    not built and cannot be (no C compiler, no Python headers, a directory that cannot be written), the same calls through
+    ctypes: slower by some microseconds each, with the same results."""
     global _fast
     if _fast is None:
-        spec = importlib.util.spec_from_file_location("_fastcall", build.build_fastcall())
-        _fast = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(_fast)
+        try:
+            spec = importlib.util.spec_from_file_location("_fastcall", build.build_fastcall())
+            _fast = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(_fast)
+        except (RuntimeError, OSError, ImportError) as e:
+            from . import slowcall
+
+            warnings.warn(f"calls go through ctypes, which is slower: {e}", RuntimeWarning, stacklevel=2)
+            _fast = slowcall.Calls(declarations())
     return _fast
 
 

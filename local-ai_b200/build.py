@@ -4,7 +4,8 @@ The library is rebuilt when the hash of its sources (csrc/*.cu, csrc/*.h,
 include/local_cuda.h) differs from the hash recorded beside the built file,
 so a stale binary is never loaded.  Each .cu is compiled to an object file in
 parallel, then linked.  The CPython extension of fastcall.py (the argument
-conversion of the Python mirror) is generated from the header and built beside it.
+conversion of the Python mirror) is generated from the header and built beside it;
+a machine that cannot build it calls through ctypes (slowcall.py).
 """
 from __future__ import annotations
 
@@ -90,8 +91,7 @@ def build_fastcall(force: bool = False) -> Path:
 
 
 def build_library(force: bool = False, verbose: bool = False, extra_flags: list[str] | None = None) -> Path:
-    """Compile every CUDA source for sm_100a, link the shared library, build the CPython extension."""
-    build_fastcall(force)
+    """Compile every CUDA source for sm_100a and link the shared library."""
     if not force and is_current():
         return LIB
     nvcc = find_nvcc()
@@ -122,4 +122,5 @@ def build_library(force: bool = False, verbose: bool = False, extra_flags: list[
 
 
 if __name__ == "__main__":
+    print(build_fastcall(force="--force" in sys.argv))
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
