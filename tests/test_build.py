@@ -3,6 +3,7 @@ import os
 import shutil
 import subprocess
 import sys
+import time
 from pathlib import Path
 
 import pytest
@@ -17,7 +18,7 @@ def tree(tmp_path, la):
     shutil.copytree(ROOT / "local-ai_b200", t / "local-ai_b200", ignore=shutil.ignore_patterns("_fastcall.*", "build", "__pycache__", "liblocal_cuda.so"))
     shutil.copytree(ROOT / "include", t / "include")
     shutil.copy(ROOT / "__graft_entry__.py", t)
-    os.symlink(ROOT / "local-ai_b200" / "liblocal_cuda.so", t / "local-ai_b200" / "liblocal_cuda.so")
+    shutil.copy(ROOT / "local-ai_b200" / "liblocal_cuda.so", t / "local-ai_b200")
     return t
 
 
@@ -99,3 +100,49 @@ print(*[hashlib.sha256(o.as_slice(np.uint8)).hexdigest() for o in outs])
 def test_calls_through_ctypes_do_the_same_on_the_gpu(tree, tmp_path):
     out = with_and_without_a_compiler(tree, tmp_path, ON_THE_GPU)
     assert out["slow"] == out["fast"] and len(out["slow"].split()) == 3
+
+
+# a compiler that logs its links, leaves half a file under the output's name for a while, and then does its work
+SLOW_COMPILER = """#!/bin/sh
+out=; prev=
+for a in "$@"; do [ "$prev" = -o ] && out=$a; prev=$a; done
+case " $* " in *" -c "*) : > "$out"; exit 0;; esac
+echo link >> {log}
+printf half > "$out"
+sleep 0.7
+{work}
+"""
+BUILD = """
+import importlib.util, sys
+spec = importlib.util.spec_from_file_location("b", "local-ai_b200/build.py")
+b = importlib.util.module_from_spec(spec)
+spec.loader.exec_module(b)
+print(b.{call}())
+"""
+
+
+@pytest.mark.parametrize("compiler,call,product,work", [
+    ("gcc", "build_fastcall", "_fastcall.*.so", '{real} "$@"'), ("nvcc", "build_library", "liblocal_cuda.so", 'printf "whole library" > "$out"')])
+def test_processes_that_find_a_stale_build_build_it_once(tree, tmp_path, compiler, call, product, work):
+    bin_dir, log = tmp_path / "bin", tmp_path / "log"
+    bin_dir.mkdir()
+    script = bin_dir / compiler
+    script.write_text(SLOW_COMPILER.format(log=log, work=work.format(real=shutil.which(compiler) or "")))
+    script.chmod(0o755)
+    with open(tree / "include" / "local_cuda.h", "a") as f:
+        f.write("/* newer than what is built */\n")
+    before = {p: p.read_bytes() for p in (tree / "local-ai_b200").glob(product)}
+    ranks = [python(tree, BUILD.format(call=call), f"{bin_dir}:{os.environ['PATH']}") for _ in range(4)]
+    seen = set()
+    while any(r.poll() is None for r in ranks):
+        for p in (tree / "local-ai_b200").glob(product):
+            seen.add(p.read_bytes()[:64])
+        time.sleep(0.01)
+    for r in ranks:
+        stdout, stderr = r.communicate()
+        assert r.returncode == 0, stderr[-2000:]
+    (final,) = (tree / "local-ai_b200").glob(product)
+    assert log.read_text() == "link\n"                      # one process built, the others waited
+    assert seen <= {final.read_bytes()[:64], *(b[:64] for b in before.values())}   # and nobody could have loaded half a file
+    again = python(tree, BUILD.format(call=call), f"{bin_dir}:{os.environ['PATH']}")
+    assert again.communicate()[0].strip() and log.read_text() == "link\n"
