@@ -680,6 +680,8 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     p.n_lanes = n_lanes;
     p.counters = k->counters;
     p.pf_heads = pf_heads;
+    p.wait_limit = k->test_wait_expiry ? 4096u : 1u << 22;
+    p.extra_arrivals = k->test_wait_expiry ? 1u : 0u;
     p.cluster_merge = cluster_merge ? 1 : 0;
     p.partial = (float *)k->scratch;
     p.positions = positions ? (const uint32_t *)positions->dptr : nullptr;
@@ -957,6 +959,8 @@ extern "C" int lc_tq_attention_noalloc_into(lc_batch *b, const lc_buf *q, const 
     p.n_lanes = 1;
     p.counters = nullptr;
     p.pf_heads = 1;
+    p.wait_limit = 0;
+    p.extra_arrivals = 0;
     p.rq = nullptr;
     p.q = (const __half *)q->dptr;
     p.signs = (const float *)signs->dptr;

@@ -41,7 +41,10 @@ struct TqAttnParams {
     // most items a lane can have.
     uint32_t queue_chunk, n_lanes;   // n_lanes: lanes, or query rows of a prefill chunk
     unsigned int *counters;
-    uint32_t pf_heads;   // prefill kernel: MMA rows per query row (heads of a chunk, rounded up to a power of two)
+    // prefill kernel
+    uint32_t pf_heads;         // MMA rows per query row (heads of a chunk, rounded up to a power of two)
+    uint32_t wait_limit;
+    uint32_t extra_arrivals;   // 0; 1 in the expiry self-test: the "keys ready" barrier then expects an arrival nobody makes
 };
 constexpr uint32_t LC_ATTN_QUEUE_LANES = 512;   // most lanes of the queue form (its schedule lives in shared memory)
 

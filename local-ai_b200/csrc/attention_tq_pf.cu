@@ -25,7 +25,6 @@ namespace {
 
 constexpr int M = 128;
 constexpr int SMW = 8, DKW = 8, DVW = 4, MMA_WARP = SMW + DKW + DVW, PF_NT = (MMA_WARP + 1) * 32;   // softmax, K, V, issue
-constexpr uint32_t PF_WAIT_LIMIT = 1u << 22;
 // A weight is at most e^LAZY while the running maximum lags, and P, the weight times v_norm * gamma, is stored as f16: tiles with
 // a larger factor than LAZY_VMAX (e^8 * 21 = 62600 < 65504) move the maximum whenever it grows, which leaves P <= v_norm * gamma.
 // Unit normal V rows have 1 - 3, so the usual tile keeps the lag.
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid == 0) {
-        mbar_init(k_full, DKW);
+        mbar_init(k_full, DKW + p.extra_arrivals);
         mbar_init(v_full, DVW);
         mbar_init(p_full, SMW);
         mbar_init(pv_done, 1);
@@ -218,7 +217,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
     // ---- query rows: sign, transform, scale, split into two f16 operand tiles (K-major, 128-byte swizzle) ----
     auto warp_wait = [&](uint32_t bar, uint32_t parity) -> bool {
         uint32_t ok = 1;
-        if (lane == 0) ok = *abort_flag == 0u && mbar_wait(bar, parity, PF_WAIT_LIMIT) ? 1u : 0u;
+        if (lane == 0) ok = *abort_flag == 0u && mbar_wait(bar, parity, p.wait_limit) ? 1u : 0u;
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok || *abort_flag) {
             *abort_flag = 1;

@@ -66,14 +66,15 @@ struct lc_kernels {
     // GPC, so this is well below SMs / s: 74 pairs, but 45 triples, 33 fours and 15 eights on 148 SMs.  A launch of one more
     // runs a second wave and takes twice as long.
     uint32_t cluster_cap[9] = {0};
-    // LOCAL_CUDA_TEST_WAIT_EXPIRY=1 (read at creation): the tcgen05 matmul's barrier waits use a short limit and wait for
-    // an arrival that never comes, so the expiry path (status word, early exit, TMEM release) can be exercised on purpose.
+    // LOCAL_CUDA_TEST_WAIT_EXPIRY=1 (read at creation): the barrier waits of the matmuls (not of the streaming matvec) and of the
+    // prefill attention kernel use a short limit and wait for an arrival that never comes, so the expiry path (status word, early
+    // exit, TMEM release) can be exercised on purpose.
     bool test_wait_expiry = false;
 };
 
 // Values of the device-side status word (lc_kernels::dev_status).
-constexpr int LC_DEV_STATUS_WAIT_EXPIRED = 1;      // a bounded barrier wait ran out (large-batch matmul, prefill attention, streaming matvec)
-constexpr int LC_DEV_STATUS_WAIT_EXPIRED_TCD = 2;  // the same in the decode tcgen05 matmul
+constexpr int LC_DEV_STATUS_WAIT_EXPIRED = 1;      // a bounded barrier wait ran out (large-batch and vocabulary matmul, prefill attention, streaming matvec)
+constexpr int LC_DEV_STATUS_WAIT_EXPIRED_TCD = 2;  // the same in the small-batch and decode matmuls
 constexpr int LC_DEV_STATUS_POSITION = 3;          // a device-resident position pointed past its lane's pool rows
 
 // Record a failure for lc_last_error() and return `code`.

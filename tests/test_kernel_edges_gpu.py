@@ -236,3 +236,36 @@ def test_q4_0_matmul_of_17_to_64_rows_is_not_the_slower_kernel(la, ctx, kernels,
         g.destroy()
     other.close()
     assert best[0] <= 1.1 * best[1], best
+
+
+def test_expired_wait_in_prefill_attention_reports_timeout(la, orc, ctx, monkeypatch):
+    """LOCAL_CUDA_TEST_WAIT_EXPIRY=1: the prefill kernel's "keys ready" barrier expects an arrival nobody makes and its waits have a
+    short limit.  The launch returns, the status word reads Timeout, and a regular kernels object works afterwards."""
+    import ctypes as C
+    hd, n_q, n_kv, bits, rows, start = 256, 8, 1, 2, 150, 463
+    c = Cache(la, orc, ctx, hd, n_kv, bits, start + rows, seed=75)
+    c.fill_single(start + rows, 0)
+    kc, kn, vc, vn, lv, sg = c.device()
+    q = la.synth.normal_f16((rows, n_q, hd), 76)
+    monkeypatch.setenv("LOCAL_CUDA_TEST_WAIT_EXPIRY", "1")
+    expiring = la.Kernels.new(ctx)
+    monkeypatch.delenv("LOCAL_CUDA_TEST_WAIT_EXPIRY")
+    regular = la.Kernels.new(ctx)
+    out = Guarded(la, ctx, rows * n_q * hd * 2)
+    for k in (expiring, regular):
+        b = la.CommandBatch.new(ctx)
+        k.tq_attention_prefill_into(b, la.CudaBuffer.from_slice(ctx, q), kc, kn, vc, vn, lv, sg, out.view, hd, start + rows, start, rows, n_q,
+                                    n_kv, 0, bits, 0, 0.0625)
+        b.commit_and_wait()   # returns: no wait is endless
+        if k is expiring:
+            st = C.c_int(0)
+            with pytest.raises(la.Error) as ei:
+                k.kernels_device_status(C.addressof(st))
+            assert ei.value.kind == "Timeout" and st.value != 0
+    rq = orc.hadamard_rotate(q.astype(np.float32), c.signs, hd, rows * n_q, True, False)
+    want = orc.flash_attention_tq_prefill(rq, c.kc, c.kn, c.vc, c.vn, c.levels, hd, start + rows, start, rows, n_q, n_kv, 0, bits, 0, 0.0625)
+    back = orc.hadamard_rotate(want, c.signs, hd, rows * n_q, False, True)
+    rel_close(out.read(np.float16), back.astype(np.float16).astype(np.float32), 2e-3, "after an expired wait")
+    device_status_ok(regular)
+    expiring.close()
+    regular.close()

@@ -256,6 +256,29 @@ def test_expired_barrier_wait_reports_timeout(la, orc, ctx, monkeypatch):
     rel_close(got, orc.matmul_nt(orc.TQ2_0, a, raw, m, k, n), TC_TOL_TQ2, "after an expired wait")
 
 
+@pytest.mark.parametrize("fmt,m,k,n,f32", [("tq2_0", 16, 512, 600, False), ("q4_0", 3, 2048, 600, True)])
+def test_expired_wait_in_the_small_batch_kernel_reports_timeout(la, orc, ctx, monkeypatch, fmt, m, k, n, f32):
+    """The same for the kernel of up to 16 rows."""
+    import ctypes as C
+    raw = (la.synth.q4_0_weights if fmt == "q4_0" else la.synth.tq2_0_weights)(n, k, 85)
+    a = la.synth.normal_f16((m, k), 86)
+    entry = f"matmul_nt_{fmt}_f32out_into" if f32 else f"matmul_nt_{fmt}_into"
+    monkeypatch.setenv("LOCAL_CUDA_TEST_WAIT_EXPIRY", "1")
+    k2 = la.Kernels.new(ctx)
+    monkeypatch.delenv("LOCAL_CUDA_TEST_WAIT_EXPIRY")
+    run_matmul(la, ctx, k2, entry, a, raw, m, k, n, f32out=f32)   # returns: no wait is endless
+    st = C.c_int(0)
+    with pytest.raises(la.Error) as ei:
+        k2.kernels_device_status(C.addressof(st))
+    assert ei.value.kind == "Timeout" and st.value != 0
+    k2.close()
+    k3 = la.Kernels.new(ctx)
+    got = run_matmul(la, ctx, k3, entry, a, raw, m, k, n, f32out=f32)
+    device_status_ok(k3)
+    k3.close()
+    rel_close(got, orc.matmul_nt(orc.Q4_0 if fmt == "q4_0" else orc.TQ2_0, a, raw, m, k, n), 1e-3, "after an expired wait")
+
+
 @pytest.mark.parametrize("which", ["decode_matmul", "vocabulary"])
 def test_expired_wait_in_the_decode_kernels_reports_timeout(la, orc, ctx, monkeypatch, which):
     """The same self-test for the two tcgen05 kernels of the decode step: with LOCAL_CUDA_TEST_WAIT_EXPIRY=1 their
