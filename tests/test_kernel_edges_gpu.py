@@ -269,3 +269,32 @@ def test_expired_wait_in_prefill_attention_reports_timeout(la, orc, ctx, monkeyp
     device_status_ok(regular)
     expiring.close()
     regular.close()
+
+
+# Branches of the prefill kernel beside the usual one: signs other than +-1 (its query transform by shuffles), and rings, in which
+# a key tile wraps
+@pytest.mark.parametrize("hd,n_q,n_kv,bits,rows,start,window,ring,unit", [
+    (256, 8, 1, 2, 150, 463, 0, 0, False), (128, 8, 2, 3, 160, 95, 0, 0, False), (256, 8, 1, 4, 300, 500, 128, 0, False),
+    (128, 8, 1, 2, 310, 40, 0, 0, False),
+    (256, 8, 1, 2, 400, 1500, 512, 1024, True), (256, 8, 1, 4, 300, 777, 128, 512, True), (128, 12, 1, 3, 330, 1001, 200, 560, True),
+    (256, 8, 1, 2, 400, 1500, 512, 1024, False)])
+def test_prefill_attention_with_other_signs_and_rings(la, orc, ctx, kernels, hd, n_q, n_kv, bits, rows, start, window, ring, unit):
+    total = start + rows
+    c = Cache(la, orc, ctx, hd, n_kv, bits, ring or total, seed=70 + total)
+    c.fill_single(total, ring)
+    kc, kn, vc, vn, lv, _ = c.device()
+    signs = c.signs if unit else (c.signs * np.linspace(0.5, 1.5, hd)).astype(np.float32)
+    q = la.synth.normal_f16((rows, n_q, hd), 71)
+    rq = orc.hadamard_rotate(q.astype(np.float32), signs, hd, rows * n_q, True, False)
+    want = orc.flash_attention_tq_prefill(rq, c.kc, c.kn, c.vc, c.vn, c.levels, hd, total, start, rows, n_q, n_kv, window, bits, ring, 0.0625)
+    out, fused = Guarded(la, ctx, rows * n_q * hd * 4), Guarded(la, ctx, rows * n_q * hd * 2)
+    b = la.CommandBatch.new(ctx)
+    kernels.flash_attention_tq_prefill_into(b, la.CudaBuffer.from_slice(ctx, rq), kc, kn, vc, vn, lv, out.view, hd, total, start, rows,
+                                            n_q, n_kv, window, bits, ring, 0.0625)
+    kernels.tq_attention_prefill_into(b, la.CudaBuffer.from_slice(ctx, q), kc, kn, vc, vn, lv, la.CudaBuffer.from_slice(ctx, signs), fused.view,
+                                      hd, total, start, rows, n_q, n_kv, window, bits, ring, 0.0625)
+    b.commit_and_wait()
+    rel_close(out.read(np.float32), want, 1e-3, "prefill")
+    back = orc.hadamard_rotate(want, signs, hd, rows * n_q, False, True)
+    rel_close(fused.read(np.float16), back.astype(np.float16).astype(np.float32), 2e-3, "fused prefill")
+    device_status_ok(kernels)
