@@ -770,10 +770,9 @@ int lc_tq_attention_into(lc_kernels *k, lc_batch *b, const lc_buf *q, const lc_b
 
 // Prefill / multi-row verify over codes (shaders/attention_flash_tq.metal:290-556, kernels.rs:5259-5420): row r of the
 // chunk is a decode query at position start_pos + r over the one cache that already holds the chunk's rows.  Here both
-// reference kernels map onto the decode kernels with the chunk's rows as the grid's third dimension: the tensor-core
-// kernel already reads every K/V row once for all q-heads of a kv-head, and the rows of a chunk re-read the cache from
-// L2, which is what the reference's query-tiled kernel buys with its threadgroup tiles.  So the "tiled" entry point
-// is the same launch; it keeps the reference's name and argument list so callers can switch either way.
+// reference kernels map onto the same launch: the prefill kernel (attention_tq_pf.cu) for chunks that pay for it, else the
+// decode kernels with the chunk's rows as the grid's third dimension.  The "tiled" entry point keeps the reference's name
+// and argument list so callers can switch either way.
 int lc_flash_attention_tq_prefill_into(lc_kernels *k, lc_batch *b, const lc_buf *rq, const lc_buf *k_codes,
                                        const lc_buf *k_norms, const lc_buf *v_codes, const lc_buf *v_norms,
                                        const lc_buf *levels, lc_buf *out, uint32_t head_dim, uint32_t kv_len,

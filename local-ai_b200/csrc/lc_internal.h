@@ -50,10 +50,10 @@ struct lc_kernels {
     bool batchm = true;  // LOCAL_AI_BATCHM: register-resident small-M path
     bool smallm = true;  // LOCAL_AI_SMALLM
     bool mma = true;     // LOCAL_AI_MMA: tensor-core path for larger M
-    bool decode_tc = true;   // LOCAL_CUDA_DECODE_TC: lean tcgen05 kernel for TQ2_0 at small_m < M <= 64
+    bool decode_tc = true;   // LOCAL_CUDA_DECODE_TC: tcgen05 kernels at M <= 64 (TQ2_0 above small_m, Q4_0 from 17 rows), small-batch kernel for TQ2_0
     uint32_t small_m = 0;    // LOCAL_CUDA_SMALL_M (0..8): TQ2_0 matmuls of up to this many rows keep the CUDA-core kernel
     bool vocab_tc = true;    // LOCAL_CUDA_VOCAB_TC: persistent tcgen05 kernel for very tall Q4_0 matrices, f32 out, M <= 64
-    bool decode_mma = true;  // LOCAL_CUDA_DECODE_MMA: register-direct mma.sync path for 8 < M <= 64 (0: tcgen05 there too)
+    bool decode_mma = true;  // LOCAL_CUDA_DECODE_MMA: mma.sync kernels at M <= 64 (0: tcgen05 or CUDA cores there too)
     int kv_norm_mode = 0;  // LOCAL_CUDA_TQ_NORM: 0 sequential (Rust codec order), 1 tree (Metal order)
     // Library-owned scratch for split-K partials (grown outside graph capture).
     void *scratch = nullptr;
@@ -73,8 +73,8 @@ struct lc_kernels {
 };
 
 // Values of the device-side status word (lc_kernels::dev_status).
-constexpr int LC_DEV_STATUS_WAIT_EXPIRED = 1;      // a bounded barrier wait ran out (large-batch and vocabulary matmul, prefill attention, streaming matvec)
-constexpr int LC_DEV_STATUS_WAIT_EXPIRED_TCD = 2;  // the same in the small-batch and decode matmuls
+constexpr int LC_DEV_STATUS_WAIT_EXPIRED = 1;      // a bounded barrier wait ran out (large-batch matmul, prefill attention, streaming matvec)
+constexpr int LC_DEV_STATUS_WAIT_EXPIRED_TCD = 2;  // the same in the small-batch, decode and vocabulary matmuls
 constexpr int LC_DEV_STATUS_POSITION = 3;          // a device-resident position pointed past its lane's pool rows
 
 // Record a failure for lc_last_error() and return `code`.

@@ -1,18 +1,18 @@
 // Routing of the quantized batched matmul C[m, n] = A[m, k] x W[n, k]^T, the
 // stand-in for Kernels::matmul_nt_q4_0_into / matmul_nt_tq2_0_into
 // (local-metal/src/kernels.rs:6459-6563).  The reference picks between four
-// Metal kernels by m (batchm <= 4, smallm <= 8, simdgroup MMA, scalar tile);
-// here: for TQ2_0 with f16 output and m <= 64 the lean tcgen05 kernel
-// (qmatmul_tcd.cu; it is also the faster launch at m <= 8, LOCAL_CUDA_SMALL_M=8
-// keeps those on the CUDA-core kernel); otherwise the register-resident CUDA-core
-// path that streams the weights once for up to 16 rows (qmatvec.cu, m <= 8), the
-// register-direct mma.sync kernel for decode batches 8 < m <= 64 (qmatmul_mma.cu:
-// Q4_0, f32 out, shapes the tcgen05 kernel declines), and the large-batch tcgen05
-// kernel for larger m (qmatmul_tcl.cu).  The matvec entry points (lc_matvec_*) stay
-// on the CUDA-core kernels.
+// Metal kernels by m (batchm <= 4, smallm <= 8, simdgroup MMA, scalar tile); here
+//   m <= 8, two groups of 64 rows per SM or more: the streaming kernel (qmatvec_mma.cu);
+//   m <= 16: the small-batch kernel (qmatmul_sm.cu), but for wide Q4_0 outputs at short K;
+//   TQ2_0, 16 < m <= 64: the tcgen05 decode kernel (qmatmul_tcd.cu);
+//   Q4_0, f32 out, m > 8, 128 rows per SM or more: the vocabulary kernel (qmatmul_tcv.cu), 64 batch rows at a time;
+//   other Q4_0, 16 < m <= 64: the register-direct kernels (qmatmul_mma.cu) or the large-batch one, by their estimates;
+//   m > 64: the large-batch tcgen05 kernel (qmatmul_tcl.cu).
+// The matvec entry points (lc_matvec_*, qmatvec.cu) take the first two as well.  What a kernel declines falls through to the
+// next, and in the end to the CUDA-core kernels (qmatvec.cu).
 // LOCAL_AI_MMA=0 forces the CUDA-core path for every m, as it forces the non-MMA
-// kernels in the reference; LOCAL_CUDA_DECODE_TC=0 / LOCAL_CUDA_DECODE_MMA=0
-// switch the two decode kernels off (with both off, 8 < m <= 64 runs on
+// kernels in the reference; LOCAL_CUDA_SMALL_M=n keeps TQ2_0 of up to n rows on it (or the streaming kernel); LOCAL_CUDA_DECODE_TC=0 /
+// LOCAL_CUDA_DECODE_MMA=0 switch the tcgen05 and the mma.sync kernels of m <= 64 off (with both off, 8 < m <= 64 runs on
 // qmatmul_tcl.cu as well).
 #include <stdlib.h>
 #include "lc_internal.h"
@@ -33,7 +33,7 @@ int lc_qgemm_mma_grouped(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const
                          const lc_buf *const *weights, lc_buf *const *outputs, const uint32_t *ns, uint32_t m,
                          uint32_t kk);
 
-// qmatmul_tcd.cu: tcgen05 decode matmul (TQ2_0, f16 out, 8 < m <= 64); same return contract.
+// qmatmul_tcd.cu: tcgen05 decode matmul (TQ2_0, f16 out, m <= 64); same return contract.
 int lc_qgemm_tcd_launch(lc_kernels *k, lc_batch *b, const lc_buf *input, int ng, const lc_buf *const *weights,
                         lc_buf *const *outputs, const uint32_t *ns, uint32_t m, uint32_t kk, bool geglu);
 
