@@ -324,6 +324,7 @@ f16_attn_reduce_kernel(const float *__restrict__ pmax, const float *__restrict__
     const unsigned qh = blockIdx.x, cols = hd / 2, c = threadIdx.x % cols, r = threadIdx.x / cols, rows = blockDim.x / cols;
     const float *pm = pmax + (size_t)qh * num_splits, *ps = psum + (size_t)qh * num_splits;
     const float *pa = pacc + (size_t)qh * num_splits * hd + 2 * c;
+    const bool pairs = (reinterpret_cast<uintptr_t>(pacc) & 7) == 0;   // the caller's buffer may start at any float
     float gmax = -INFINITY;
     for (unsigned s = threadIdx.x; s < num_splits; s += blockDim.x) gmax = fmaxf(gmax, pm[s]);
 #pragma unroll
@@ -340,7 +341,8 @@ f16_attn_reduce_kernel(const float *__restrict__ pmax, const float *__restrict__
         for (int i = 0; i < 8; i++) {
             const unsigned s = s0 + i * rows;
             const bool ok = s < num_splits;
-            a[i] = ok ? *reinterpret_cast<const float2 *>(pa + (size_t)s * hd) : make_float2(0.f, 0.f);
+            const float *at = pa + (size_t)s * hd;
+            a[i] = !ok ? make_float2(0.f, 0.f) : pairs ? *reinterpret_cast<const float2 *>(at) : make_float2(at[0], at[1]);
             m[i] = ok ? pm[s] : -INFINITY;
             l[i] = ok ? ps[s] : 0.f;
         }
@@ -455,6 +457,8 @@ int lc_flash_attention_windowed_split_into(lc_kernels *k, lc_batch *b, const lc_
                    partial_acc->bytes >= parts * head_dim * 4,
                "flash_attention_windowed_split: partial buffers too small for %u heads x %u splits", num_q_heads,
                num_splits);
+    LC_REQUIRE(lc_aligned(partial_max->dptr, 4) && lc_aligned(partial_sum->dptr, 4) && lc_aligned(partial_acc->dptr, 4),
+               "flash_attention_windowed_split: partial buffers must be 4-byte aligned");
     return f16_attention("flash_attention_windowed_split", b, q, kk, v, output, (float *)partial_max->dptr,
                          (float *)partial_sum->dptr, (float *)partial_acc->dptr, head_dim, kv_len, current_pos,
                          num_q_heads, num_kv_heads, window, num_splits, 1.0f);

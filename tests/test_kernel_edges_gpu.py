@@ -136,6 +136,29 @@ def test_f16_attention_at_odd_lengths(la, orc, ctx, kernels, hd, n_q, n_kv, tota
     rel_close(out.read(np.float16), orc.attention_f16(q, k, v, hd, total, total - 1, n_q, n_kv, window).astype(np.float32), 2e-3, "f16")
 
 
+# the caller's partial buffers: at any float, refused at less
+@pytest.mark.parametrize("offset", [0, 4, 8, 12, 2])
+def test_windowed_split_with_partials_at_any_float(la, orc, ctx, kernels, offset):
+    hd, n_q, n_kv, total, window = 256, 8, 1, 700, 333
+    q, k, v = f16_case(la, hd, n_q, n_kv, total, 72)
+    splits = kernels.flash_split_count(window)
+    bufs = [la.CudaBuffer.empty(ctx, 16 + n_q * splits * d * 4) for d in (1, 1, hd)]
+    parts = [la.CudaBuffer.wrap(ctx, b.device_ptr + offset, b.nbytes - 16) for b in bufs]
+    out = Guarded(la, ctx, n_q * hd * 2)
+    f = lambda x: la.CudaBuffer.from_slice(ctx, x)
+    b = la.CommandBatch.new(ctx)
+    call = lambda: kernels.flash_attention_windowed_split_into(b, f(q), f(k), f(v), out.view, *parts, hd, total, total - 1, n_q, n_kv, window, splits)
+    if offset % 4:
+        with pytest.raises(la.Error) as ei:
+            call()
+        assert ei.value.kind == "InvalidArgument"
+        b.commit_and_wait()
+        return
+    call()
+    b.commit_and_wait()
+    rel_close(out.read(np.float16), orc.attention_f16(q, k, v, hd, total, total - 1, n_q, n_kv, window).astype(np.float32), 2e-3, "windowed split")
+
+
 @pytest.mark.parametrize("hd", [128, 256, 512])
 @pytest.mark.parametrize("rows", [1, 7, 9, 65])
 def test_encoder_rows_at_block_edges(la, orc, ctx, kernels, hd, rows):
