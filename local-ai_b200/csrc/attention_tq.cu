@@ -606,6 +606,11 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
             if (cost < grid_cost) { grid_cost = cost; n_splits = s; }
         }
     }
+    // The two forms below need room for partials where the splits above may need none, and scratch memory cannot grow while a graph
+    // is recorded: a call that was not made outside capture first keeps the splits.
+    auto partials_fit = [&](uint32_t splits, size_t counters) {
+        return !b->capturing || (qn / hd * splits * (size_t)(hd + 2) * sizeof(float) <= k->scratch_bytes && counters <= k->counters_len);
+    };
     // Queue form for pools of lanes that attend all of their keys.  Lanes differ in length, which the host cannot see, and
     // equal splits per lane leave most SMs waiting for the longest lane; so one persistent CTA per SM draws items of at
     // most `chunk` keys.  An item after a CTA's first costs about 620 keys' worth more, and a merge launch follows.  The chunk minimises
@@ -625,9 +630,10 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
             const uint64_t cost = full + (mean > per ? mean : per) + 2u * launch;
             if (cost < best_cost) { best_cost = cost; best_chunk = per + 64u; }   // (a few keys over do not make another item)
         }
-        if (best_cost < 2u * grid_cost) {
+        const uint32_t most = best_chunk ? (len_max + best_chunk - 1) / best_chunk : 1u;
+        if (best_cost < 2u * grid_cost && partials_fit(most, (size_t)n_kv * gchunks)) {
             chunk = best_chunk;
-            n_splits = (len_max + chunk - 1) / chunk;
+            n_splits = most;
         }
     }
     // Chunks of several rows: the prefill kernel shares each decoded key among 128 MMA rows, but takes 1900 keys' time (16 us)
@@ -649,7 +655,7 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
             if (splits > MERGE_ROWS_MAX_SPLITS) splits = MERGE_ROWS_MAX_SPLITS;
             const uint64_t waves = ((uint64_t)ctas * splits + sms - 1) / sms, steps = (key_tiles + splits - 1) / splits;
             const uint64_t merge = (uint64_t)n_rows * n_q * splits * hd / 6400u;   // partials: 25 KB of them in a key's time
-            if (waves * (in_keys(1900u) + steps * in_keys(bits == 2 ? 240u : 360u)) + in_keys((uint32_t)merge) < grid_cost)
+            if (waves * (in_keys(1900u) + steps * in_keys(bits == 2 ? 240u : 360u)) + in_keys((uint32_t)merge) < grid_cost && partials_fit(splits, 0))
                 n_splits = splits;
             else
                 pf_tiles = 0;

@@ -261,6 +261,39 @@ def test_q4_0_matmul_of_17_to_64_rows_is_not_the_slower_kernel(la, ctx, kernels,
     assert best[0] <= 1.1 * best[1], best
 
 
+@pytest.mark.parametrize("bits,rows,start", [(2, 256, 768), (4, 150, 1900)])
+def test_prefill_attention_captured_without_an_eager_call_first(la, orc, ctx, bits, rows, start):
+    """The prefill kernel's partials need scratch memory, which cannot grow while a graph is recorded: with none reserved the
+    chunk takes the decode kernel, which merges its splits itself.  After an eager call the graph holds the prefill kernel."""
+    hd, n_q, n_kv = 256, 8, 1
+    c = Cache(la, orc, ctx, hd, n_kv, bits, start + rows, seed=77)
+    c.fill_single(start + rows, 0)
+    kc, kn, vc, vn, lv, sg = c.device()
+    q = la.CudaBuffer.from_slice(ctx, la.synth.normal_f16((rows, n_q, hd), 78))
+    rq = orc.hadamard_rotate(q.as_slice(np.float16).astype(np.float32), c.signs, hd, rows * n_q, True, False)
+    want = orc.flash_attention_tq_prefill(rq, c.kc, c.kn, c.vc, c.vn, c.levels, hd, start + rows, start, rows, n_q, n_kv, 0, bits, 0, 0.0625)
+    back = orc.hadamard_rotate(want, c.signs, hd, rows * n_q, False, True).astype(np.float16).astype(np.float32)
+    k = la.Kernels.new(ctx)
+    launches = []
+    for eager_first in (False, True):
+        out = Guarded(la, ctx, rows * n_q * hd * 2)
+        call = lambda b: k.tq_attention_prefill_into(b, q, kc, kn, vc, vn, lv, sg, out.view, hd, start + rows, start, rows, n_q, n_kv, 0, bits, 0, 0.0625)
+        if eager_first:
+            b = la.CommandBatch.new(ctx)
+            call(b)
+            b.commit_and_wait()
+        b = la.CommandBatch.capture(ctx)
+        call(b)
+        launches.append(b.dispatch_count())
+        graph = b.end_capture()
+        graph.launch()
+        ctx.synchronize()
+        rel_close(out.read(np.float16), back, 2e-3, "captured prefill")
+        graph.destroy()
+    assert launches == [1, 2]
+    k.close()
+
+
 def test_expired_wait_in_prefill_attention_reports_timeout(la, orc, ctx, monkeypatch):
     """LOCAL_CUDA_TEST_WAIT_EXPIRY=1: the prefill kernel's "keys ready" barrier expects an arrival nobody makes and its waits have a
     short limit.  The launch returns, the status word reads Timeout, and a regular kernels object works afterwards."""
