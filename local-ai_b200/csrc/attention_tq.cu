@@ -587,10 +587,11 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     static const bool cluster_allowed = []() { const char *e = getenv("LOCAL_CUDA_ATTN_CLUSTER"); return !(e && e[0] == '0'); }();
     const bool clusters = use_mma && cluster_allowed && lc_aligned(out->dptr, 16) && (!fused || lc_aligned(signs->dptr, 16));
     uint64_t grid_cost = ~0ull;
-    auto in_keys = [&](uint32_t tq2_keys) -> uint32_t { return tq2_keys * (bits == 2 ? 8u : 5u) * 32u / hd; };
+    const bool one_part = bits == 2 && hd == 256;   // levels and P in one f16 (attention_tq_mma.cu)
+    auto in_keys = [&](uint32_t tq2_keys) -> uint32_t { return tq2_keys * (one_part ? 8u : 5u) * 32u / hd; };
     if (use_mma) {
         // One CTA per SM (shared memory), so the launch runs in whole waves.  Pick the split count that minimises their
-        // time, in keys of tq2 at head_dim 256 (8.5 ns each; more bits take 8/5 of that): 700 for the launch, 1050 for
+        // time, in keys of tq2 at head_dim 256 (8.5 ns each; others take 8/5 of that per 256 dims): 700 for the launch, 1050 for
         // every further wave, 640 for a merge launch.
         // Short contexts split down to two 32-key tiles per CTA (two warps that have the table's banks to themselves finish a
         // tile sooner than eight), but into no more splits than one launch merges; long ones to half the warps.
@@ -637,7 +638,7 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
         }
     }
     // Chunks of several rows: the prefill kernel shares each decoded key among 128 MMA rows, but takes 1900 keys' time (16 us)
-    // before and after its key tiles, of 240 (tq2; else 360) each.  Fewer than half a tile of rows, and chunks whose rows the decode
+    // before and after its key tiles, of 240 (operands in one part; else 360) each.  Fewer than half a tile of rows, and chunks whose rows the decode
     // kernel's CTAs finish sooner by the estimate above, stay there: 64 rows over 400 keys 9.7 us against 16.6, 256 over 330
     // 20.0 against 19.5, 256 over 4096 87 against 38.
     uint32_t pf_heads = 1, pf_tiles = 0;
@@ -655,7 +656,7 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
             if (splits > MERGE_ROWS_MAX_SPLITS) splits = MERGE_ROWS_MAX_SPLITS;
             const uint64_t waves = ((uint64_t)ctas * splits + sms - 1) / sms, steps = (key_tiles + splits - 1) / splits;
             const uint64_t merge = (uint64_t)n_rows * n_q * splits * hd / 6400u;   // partials: 25 KB of them in a key's time
-            if (waves * (in_keys(1900u) + steps * in_keys(bits == 2 ? 240u : 360u)) + in_keys((uint32_t)merge) < grid_cost && partials_fit(splits, 0))
+            if (waves * (in_keys(1900u) + steps * in_keys(one_part ? 240u : 360u)) + in_keys((uint32_t)merge) < grid_cost && partials_fit(splits, 0))
                 n_splits = splits;
             else
                 pf_tiles = 0;

@@ -4,7 +4,7 @@
 //
 // With 8 q-heads sharing every K/V row the CUDA-core kernel needs 16 x head_dim FMAs per key, which binds long before HBM
 // does.  Here both contractions run on tensor cores, with operands built in registers from the packed codes:
-//   * a shared-memory table maps one field of code bits (8 bits: four tq2 or two tq4 codes; 6 bits: two tq3 codes) to
+//   * a shared-memory table maps one field of code bits (8 bits: four tq2 or two tq4 codes; 6 or 4 bits: two tq3 or tq2 codes) to
 //     f16 levels with a single 8-byte load; it is replicated 16 times so that the lookups of a half-warp never collide;
 //   * S^T[16 keys x 8 heads] = K[16 x HD] . RQ^T: the contraction index (dims) is free to permute, so thread (g, t) of a
 //     warp feeds the MMA with the HD / 4 dims held in its own quarter of the code bytes of keys g, g + 8;
@@ -21,9 +21,11 @@
 // (tq4, from the CUDA-core kernel); 64 ragged lanes up to 8192 keys at tq4: 259 -> 49 us.
 //
 // Precision.  The query is split into an f16 and the f16 of the remainder (two MMAs), because logits reach |q||k| ~ head_dim
-// at softmax scale 1.  tq2: the table holds levels / gamma, with gamma searched (1024 mantissas) so that all four levels are
-// f16-representable to ~1e-6; gamma is folded into the row norms in f32.  tq3 / tq4 have too many levels for that: the
-// table holds each level as an f16 and the f16 of its remainder, and so is P (three MMAs per contraction step).
+// at softmax scale 1.  The table holds each level as an f16 and the f16 of its remainder, and so is P (three MMAs per contraction
+// step): the result is within 6e-6 of its norm against 64 bits.  Only tq2 at head_dim 256 makes do with one f16 each, P as it is and
+// levels / gamma, gamma searched (1024 mantissas) so that all four are f16-representable to ~2e-6 and folded into the row
+// norms in f32: 2e-4, mostly P's.  (64 lanes x 8192 keys of 128 took 31.6 us in that form, 46.8 in this one and 164 on CUDA cores,
+// whose error was 1e-6; behind an f16 output the single f16 showed as 3.0e-4 for 2.1e-4.)
 #include <math.h>
 #include <utility>
 
@@ -38,9 +40,9 @@ template <int HD_, int BITS_>
 struct AttnCfg {
     static constexpr int HD = HD_, BITS = BITS_;
     static constexpr int CB = HD * BITS / 8;            // code bytes per row
-    static constexpr int FB = BITS == 3 ? 6 : 8;        // table index bits
+    static constexpr bool HILO = BITS > 2 || HD != 256; // levels and P as an f16 and the f16 of the remainder
+    static constexpr int FB = HILO ? 2 * BITS : 8;      // table index bits
     static constexpr int NENT = 1 << FB;
-    static constexpr bool HILO = BITS > 2;
     static constexpr int MT = HD == 512 ? 1 : 2;        // 16-key MMA tiles per warp step
     static constexpr int KT = 16 * MT;
     static constexpr int NW = 8, NT = NW * 32;
@@ -154,9 +156,9 @@ __device__ __forceinline__ void split_h2(float x, float y, uint32_t &hi, uint32_
     const float2 h = unpack_h2(hi);
     lo = pack_h2(x - h.x, y - h.y);
 }
-template <int BITS>
+template <bool HILO>
 __device__ __forceinline__ float soft_exp(float x) {
-    return BITS == 2 ? __expf(x) : expf(x);
+    return HILO ? expf(x) : __expf(x);
 }
 
 // Walsh-Hadamard butterflies over 32 * DPL values held DPL per lane (lane owns consecutive dims), ascending stride.
@@ -594,7 +596,7 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
                 tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 8));
                 tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 16));
                 const float m_new = fmaxf(m_run[h], tm[h]);    // finite: key t0 is valid
-                resc[h] = soft_exp<C::BITS>(m_run[h] - m_new);
+                resc[h] = soft_exp<C::HILO>(m_run[h] - m_new);
                 m_run[h] = m_new;
                 l_part[h] *= resc[h];
             }
@@ -605,7 +607,7 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
 #pragma unroll
                 for (int r = 0; r < 2; r++) {
                     const float vn = __shfl_sync(0xffffffffu, nv, (KT == 32 ? 16 * mt : 0) + 8 * r + g);
-                    const float p0 = soft_exp<C::BITS>(sc[mt][r][0] - m_run[0]), p1 = soft_exp<C::BITS>(sc[mt][r][1] - m_run[1]);
+                    const float p0 = soft_exp<C::HILO>(sc[mt][r][0] - m_run[0]), p1 = soft_exp<C::HILO>(sc[mt][r][1] - m_run[1]);
                     l_part[0] += p0;
                     l_part[1] += p1;
                     if constexpr (!C::HILO) {
@@ -695,8 +697,8 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
                 g0 = fmaxf(g0, v.x);
                 g1 = fmaxf(g1, v.y);
             }
-            const float f0 = m_run[0] == -INFINITY ? 0.f : soft_exp<C::BITS>(m_run[0] - g0);
-            const float f1 = m_run[1] == -INFINITY ? 0.f : soft_exp<C::BITS>(m_run[1] - g1);
+            const float f0 = m_run[0] == -INFINITY ? 0.f : soft_exp<C::HILO>(m_run[0] - g0);
+            const float f1 = m_run[1] == -INFINITY ? 0.f : soft_exp<C::HILO>(m_run[1] - g1);
             if (g == 0) *reinterpret_cast<float2 *>(l_s + warp * G + 2 * t) = make_float2(f0 * l_part[0], f1 * l_part[1]);
             if (warp < nwa) {
                 float4 *dst = reinterpret_cast<float4 *>(acc_s) + warp * NS * 32 + lane;

@@ -12,8 +12,8 @@
 //     only when it has grown by more than LAZY (a rescale is a pass over the accumulator), or at all where a tile's value norms
 //     are so large that P could leave f16's range; P times the value norms goes back to tensor memory;
 //   * O[128 x HD] += P . V with P read from tensor memory.
-// Precision as in attention_tq_mma.cu: tq2 levels are f16-exact up to a factor gamma that is folded into the norms, P is an f16;
-// tq3 / tq4 levels and P are an f16 and the f16 of the remainder, which doubles the operand tiles.
+// Precision as in attention_tq_mma.cu: levels and P are an f16 and the f16 of the remainder, which doubles the operand tiles, but for tq2
+// at head_dim 256, whose levels are f16-exact up to a factor gamma that is folded into the norms and whose P is an f16.
 // Every barrier wait is bounded; on expiry the CTA records a status word and leaves.
 #include <math.h>
 #include <utility>
@@ -34,14 +34,14 @@ template <int HD_, int BITS_>
 struct PfCfg {
     static constexpr int HD = HD_, BITS = BITS_, CB = HD * BITS / 8;
     static constexpr int KN = HD == 256 && BITS > 2 ? 32 : 64;   // keys per tile (what fits beside the query)
-    static constexpr int PARTS = BITS > 2 ? 2 : 1;               // operand tiles per level: f16, remainder
+    static constexpr int PARTS = BITS > 2 || HD != 256 ? 2 : 1;  // operand tiles per level, and parts of P: f16, remainder
     static constexpr int NB = HD / 64;                           // 64-dim blocks (128 bytes: the swizzle's width)
     static constexpr int UN = HD / 32, UB = 4 * BITS;            // 32-dim units of a row, bytes of a unit
     static constexpr int NUK = KN * UN / (DKW * 32), NUV = KN * UN / (DVW * 32);   // units per decoding thread
-    static constexpr int FB = BITS == 3 ? 6 : 8, NENT = 1 << FB, COPIES = 8;
+    static constexpr int FB = 2 * BITS, NENT = 1 << FB, COPIES = 8;   // table of two codes
     static constexpr int Q_PART = NB * M * 128, KV_PART = NB * KN * 128;
     static constexpr int Q_OFF = 0, K_OFF = 2 * Q_PART, V_OFF = K_OFF + PARTS * KV_PART, LUT_OFF = V_OFF + PARTS * KV_PART;
-    static constexpr int LUT_BYTES = BITS > 2 ? NENT * COPIES * 8 : 0;
+    static constexpr int LUT_BYTES = PARTS == 2 ? NENT * COPIES * 8 : 0;
     static constexpr int NORM_OFF = LUT_OFF + LUT_BYTES, NORM_BYTES = 4 * 2 * KN * 4;   // [4 tiles][k, v][KN]
     static constexpr int STAGE = M * (HD + 4) * 4;               // results, reuses the operand tiles
     static constexpr int TAIL = NORM_OFF + NORM_BYTES;
@@ -77,8 +77,8 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t &hi, uint32_t 
     hi = *reinterpret_cast<const uint32_t *>(&h);
     lo = pack2(x - f.x, y - f.y);
 }
-template <int BITS>
-__device__ __forceinline__ float pf_exp(float x) { return BITS == 2 ? __expf(x) : expf(x); }
+template <int PARTS>
+__device__ __forceinline__ float pf_exp(float x) { return PARTS == 1 ? __expf(x) : expf(x); }
 __device__ __forceinline__ void sts16(uint32_t a, const uint32_t (&v)[4]) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(a), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
@@ -109,10 +109,10 @@ __device__ __forceinline__ void fwht_lanes(float (&x)[DPL], int lane) {
         }
     }
 }
-// Where dim d of a row sits in the operand tiles: tq2 keeps the order in which a byte table decodes sixteen dims.
-template <int BITS>
+// Where dim d of a row sits in the operand tiles: levels in one part keep the order in which a byte table decodes sixteen dims.
+template <int PARTS>
 __device__ __forceinline__ int tile_pos(int d) {
-    return BITS == 2 ? (d & ~15) + 4 * (d & 3) + ((d >> 2) & 3) : d;
+    return PARTS == 1 ? (d & ~15) + 4 * (d & 3) + ((d >> 2) & 3) : d;
 }
 
 template <typename C>
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
         ref = fmaxf(ref, fabsf(lvl[i]));
     }
     float gamma;
-    if constexpr (BITS == 2) {   // gamma such that every level / gamma is (almost) exactly an f16
+    if constexpr (C::PARTS == 1) {   // gamma such that every level / gamma is (almost) exactly an f16
         float best = INFINITY;
         int besti = 0;
         for (int j = tid; j < 1024; j += PF_NT) {
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
             }
         }
         for (int e = tid; e < 64 * 8; e += PF_NT) {   // H64 in the place of the first keys: row n is output dim tile_pos(n) (its own inverse)
-            const int n = e >> 3, c = e & 7, d = tile_pos<BITS>(n);
+            const int n = e >> 3, c = e & 7, d = tile_pos<C::PARTS>(n);
             uint32_t v[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
@@ -367,8 +367,8 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
                     }
                 }
             }
-            // tq2: sixteen dims (two lanes' at head_dim 256, four lanes' at 128) are stored in the order 4 (d % 4) + d / 4
-            if constexpr (BITS == 2 && DPL == 8) {   // the even lane takes dims d % 4 = 0, 1 of both, the odd lane 2, 3
+            // levels in one part: sixteen dims (two lanes') are stored in the order 4 (d % 4) + d / 4
+            if constexpr (C::PARTS == 1 && DPL == 8) {   // the even lane takes dims d % 4 = 0, 1 of both, the odd lane 2, 3
                 const bool odd = lane & 1;
                 float y[8];
 #pragma unroll
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
             } else {
 #pragma unroll
                 for (int i = 0; i < DPL; i++) {
-                    const int pos = tile_pos<BITS>(DPL * lane + i), nb = pos >> 6, c = (pos & 63) >> 3;
+                    const int pos = tile_pos<C::PARTS>(DPL * lane + i), nb = pos >> 6, c = (pos & 63) >> 3;
                     const uint32_t off = (uint32_t)(nb * M * 128 + r * 128 + ((c ^ (r & 7)) << 4) + (pos & 7) * 2);
                     const __half hi = __float2half_rn(x[i]), lo = __float2half_rn(x[i] - __half2float(hi));
                     *reinterpret_cast<__half *>(smem + C::Q_OFF + off) = hi;
@@ -441,8 +441,8 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
                 norm_next = key < k_end ? __half2float((dt < KN ? p.kn : p.vn)[slot_of(key)]) * gamma : 0.f;
             }
         };
-        [[maybe_unused]] uint32_t lut_lo = 0, lut_hi = 0;   // tq2: the four levels as a byte table for prmt
-        if constexpr (BITS == 2) {
+        [[maybe_unused]] uint32_t lut_lo = 0, lut_hi = 0;   // one part: the four levels as a byte table for prmt
+        if constexpr (C::PARTS == 1) {
             const uint32_t l01 = pack2(lvl[0] / gamma, lvl[1] / gamma), l23 = pack2(lvl[2] / gamma, lvl[3] / gamma);
             lut_lo = __byte_perm(l01, l23, 0x6420);
             lut_hi = __byte_perm(l01, l23, 0x7531);
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
             for (int j = 0; j < NU; j++) {
                 const int u = dt + j * ND, key = (u & 7) | ((u / (8 * C::UN)) << 3), unit = (u >> 3) % C::UN;
                 const uint32_t row = tile + (uint32_t)((unit >> 1) * (KN * 128) + key * 128), c0 = (uint32_t)(unit & 1) * 4u, sw = (uint32_t)key & 7u;
-                if constexpr (BITS == 2) {
+                if constexpr (C::PARTS == 1) {
 #pragma unroll
                     for (int w = 0; w < 2; w++) {
                         uint32_t v[8];   // sixteen dims: bit pair l of each byte, l = 0..3
@@ -623,7 +623,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
                 // the accumulator moves to the new maximum: PV of the tile before has to be complete
                 warp_wait(pv_done, (uint32_t)((t - 1) & 1));
                 tc_fence_after();
-                const float m_new = fmaxf(m_ref, mx), f = m_ref == -INFINITY ? 0.f : pf_exp<BITS>(m_ref - m_new);
+                const float m_new = fmaxf(m_ref, mx), f = m_ref == -INFINITY ? 0.f : pf_exp<C::PARTS>(m_ref - m_new);
 #pragma unroll 1
                 for (int c = half * (HD / 2); c < (half + 1) * (HD / 2); c += 16) {
                     uint32_t v[16];
@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
 #pragma unroll
             for (int i = 0; i < KH; i += 4) {
                 const float4 n4 = *reinterpret_cast<const float4 *>(vn + i);
-                const float e0 = pf_exp<BITS>(s[i] - mu), e1 = pf_exp<BITS>(s[i + 1] - mu), e2 = pf_exp<BITS>(s[i + 2] - mu), e3 = pf_exp<BITS>(s[i + 3] - mu);
+                const float e0 = pf_exp<C::PARTS>(s[i] - mu), e1 = pf_exp<C::PARTS>(s[i + 1] - mu), e2 = pf_exp<C::PARTS>(s[i + 2] - mu), e3 = pf_exp<C::PARTS>(s[i + 3] - mu);
                 l_sum += (e0 + e1) + (e2 + e3);
                 if (C::PARTS == 2) {
                     split2(e0 * n4.x, e1 * n4.y, ph[i / 2], pl[i / 2]);
@@ -695,12 +695,12 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
 #pragma unroll
                 for (int i = 0; i < 16; i++) v[i] = 0u;
             }
-            // sixteen columns are sixteen dims; tq2 keeps them in the order 4 (i % 4) + i / 4
+            // sixteen columns are sixteen dims; levels in one part keep them in the order 4 (i % 4) + i / 4
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 uint32_t o[4];
 #pragma unroll
-                for (int e = 0; e < 4; e++) o[e] = BITS == 2 ? v[4 * e + q] : v[4 * q + e];
+                for (int e = 0; e < 4; e++) o[e] = C::PARTS == 1 ? v[4 * e + q] : v[4 * q + e];
                 sts16(base + (uint32_t)((r * (HD + 4) + c + 4 * q) * 4), o);
             }
         }

@@ -354,3 +354,28 @@ def test_prefill_attention_with_other_signs_and_rings(la, orc, ctx, kernels, hd,
     back = orc.hadamard_rotate(want, signs, hd, rows * n_q, False, True)
     rel_close(fused.read(np.float16), back.astype(np.float16).astype(np.float32), 2e-3, "fused prefill")
     device_status_ok(kernels)
+
+
+@pytest.mark.parametrize("hd,rows,total", [(128, 0, 700), (512, 0, 700), (128, 0, 5000), (128, 256, 900)])
+def test_two_bit_attention_keeps_its_weights_in_32_bits(la, orc, ctx, kernels, hd, rows, total):
+    """At head_dim 128 and 512 tq2 attention ran with f32 levels and weights on CUDA cores; on tensor cores they are an f16 and the f16
+    of the remainder, 2^-22 of each.  An average over N keys of both signs is sqrt(N) times smaller than its terms, so 5000 keys turn
+    that into 2^-22 * 71 = 1.7e-5 at the very most (were all of it one way), and f32 sums stay below it: 1e-5 of the result's norm,
+    where weights in one f16 leave 2e-4."""
+    n_q, n_kv, bits = 8, 1, 2
+    c = Cache(la, orc, ctx, hd, n_kv, bits, total, seed=79)
+    c.fill_single(total, 0)
+    kc, kn, vc, vn, lv, _ = c.device()
+    rq = orc.hadamard_rotate(la.synth.normal(80, max(rows, 1) * n_q * hd).astype(np.float32), c.signs, hd, max(rows, 1) * n_q, True, False)
+    out = la.CudaBuffer.empty(ctx, rq.size * 4)
+    b = la.CommandBatch.new(ctx)
+    head = (b, la.CudaBuffer.from_slice(ctx, rq), kc, kn, vc, vn, lv, out, hd, total)
+    if rows:
+        kernels.flash_attention_tq_prefill_into(*head, total - rows, rows, n_q, n_kv, 0, bits, 0, 0.0625)
+        want = orc.flash_attention_tq_prefill(rq, c.kc, c.kn, c.vc, c.vn, c.levels, hd, total, total - rows, rows, n_q, n_kv, 0, bits, 0, 0.0625)
+    else:
+        kernels.flash_attention_tq_into(*head, total - 1, n_q, n_kv, 0, bits, 0, 0.0625)
+        want = orc.flash_attention_tq(rq, c.kc, c.kn, c.vc, c.vn, c.levels, hd, total, total - 1, n_q, n_kv, 0, bits, 0, 0.0625)
+    b.commit_and_wait()
+    off = out.as_slice(np.float32).astype(np.float64) - want
+    assert np.linalg.norm(off) <= 1e-5 * np.linalg.norm(want.astype(np.float64)), np.linalg.norm(off) / np.linalg.norm(want)
