@@ -6,7 +6,8 @@
 //   m <= 16: the small-batch kernel (qmatmul_sm.cu), but for wide Q4_0 outputs at short K;
 //   TQ2_0, 16 < m <= 64: the tcgen05 decode kernel (qmatmul_tcd.cu);
 //   Q4_0, f32 out, m > 8, 128 rows per SM or more: the vocabulary kernel (qmatmul_tcv.cu), 64 batch rows at a time;
-//   other Q4_0, 16 < m <= 64: the register-direct kernels (qmatmul_mma.cu) or the large-batch one, by their estimates;
+//   other Q4_0, 16 < m <= 64: f32 out the register-direct kernels (qmatmul_mma.cu), f16 out those or the large-batch one, by
+//     their estimates;
 //   m > 64: the large-batch tcgen05 kernel (qmatmul_tcl.cu).
 // The matvec entry points (lc_matvec_*, qmatvec.cu) take the first two as well.  What a kernel declines falls through to the
 // next, and in the end to the CUDA-core kernels (qmatvec.cu).
@@ -100,7 +101,8 @@ static int route(int fmt, bool f32out, const char *name, lc_kernels *k, lc_batch
         if (m <= 64) {
             // Q4_0 from 17 rows: whichever kernel's estimate is less.  40 x 6144 x 1536 9.4 us on the large-batch kernel, 15.3 on the
             // other; 24 x 6144 x 4096 20.0 and 17.2; 25 x 70991 x 512 30.8 and 20.2; 64 x 262144 x 256 93 and 61.
-            const bool choose = k->decode_tc && fmt == 0 && m > SM_MAX_M;
+            // f32 outputs keep the other: its sums, 32 k at a time, are within 1e-7 of 64 bits, the tcgen05 accumulators' within 1e-6.
+            const bool choose = k->decode_tc && fmt == 0 && m > SM_MAX_M && !f32out;
             if (k->decode_mma && (!choose || lc_qgemm_mma_estimate(k, m, kk, n) < lc_qgemm_tcl_estimate(k, m, kk, n))) {
                 st = lc_qgemm_mma_grouped(fmt, f32out, k, b, input, 1, ws, os, ns, m, kk);
                 if (st >= 0) return st;

@@ -232,6 +232,16 @@ def test_q4_0_matmul_of_17_to_64_rows(la, orc, ctx, kernels, m, k, n):
     device_status_ok(kernels)
 
 
+@pytest.mark.parametrize("m,k,n", [(17, 6144, 1536), (40, 1536, 6144), (64, 800, 3000)])
+def test_q4_0_matmul_with_f32_output_keeps_its_precision(la, orc, ctx, kernels, m, k, n):
+    """f32 outputs at 17 .. 64 rows: sums of f32-scaled 32-k blocks, K / 32 roundings of 2^-24 each in a walk, sqrt(192) 2^-24 = 8e-7 at
+    the most and 1e-7 as a rule; the tcgen05 accumulators are 9e-7 off."""
+    raw, a = la.synth.q4_0_weights(n, k, 35), la.synth.normal_f16((m, k), 36)
+    got = run_matmul(la, ctx, kernels, "matmul_nt_q4_0_f32out_into", a, raw, m, k, n, f32out=True).astype(np.float64)
+    want = orc.matmul_nt(orc.Q4_0, a, raw, m, k, n).astype(np.float64).reshape(m, n)
+    assert np.linalg.norm(got - want) <= 3e-7 * np.linalg.norm(want), np.linalg.norm(got - want) / np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("m,k,n", [(24, 512, 40000), (20, 256, 100000), (50, 256, 150000), (24, 4096, 6144), (40, 1536, 6144)])
 def test_q4_0_matmul_of_17_to_64_rows_is_not_the_slower_kernel(la, ctx, kernels, monkeypatch, m, k, n):
     """The choice against the register-direct kernel alone (LOCAL_CUDA_DECODE_TC=0): at most 1.1 times its time, where a wrong
