@@ -126,6 +126,7 @@ int lc_ctx_create(int device, lc_ctx **out) {
     cudaMemGetInfo(&fr, &tot);
     c->total_mem = tot;
     { const char *e = getenv("LOCAL_CUDA_PDL"); c->pdl = !(e && strcmp(e, "0") == 0); }
+    { const char *e = getenv("LOCAL_CUDA_OVERLAP"); c->side_by_side = !(e && strcmp(e, "0") == 0); }
     count_context(device, 1);
     *out = c;
     return LC_OK;
@@ -270,6 +271,59 @@ int lc_buf_fill(lc_buf *buf, size_t offset, size_t bytes, int value) {
     return LC_OK;
 }
 
+// ------------------------------------------------- launches side by side --
+LcOrder::LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, const lc_buf *const *weights, const size_t *w_bytes,
+                 lc_buf *const *outputs, const size_t *out_bytes)
+    : ctx(b->ctx), tracked(b->ctx->pdl && b->ctx->side_by_side && b->stream == b->ctx->stream) {
+    if (!tracked) {
+        serial = lc_count_launch(b);
+        return;
+    }
+    lc_overlap &o = ctx->overlap;
+    constexpr int MOST_READS = sizeof(o.reads) / sizeof(lc_range), MOST_WRITES = sizeof(o.writes) / sizeof(lc_range);
+    o.mu.lock();
+    before = ctx->launches.fetch_add(1);
+    if (before != o.seen) o.state = 0;
+    auto range = [](const lc_buf *buf, size_t bytes) { return lc_range{(uintptr_t)buf->dptr, (uintptr_t)buf->dptr + bytes}; };
+    auto meets = [](const lc_range &r, const lc_range *v, int n) {
+        for (int i = 0; i < n; i++)
+            if (r.lo < v[i].hi && v[i].lo < r.hi) return true;
+        return false;
+    };
+    const lc_range in = range(input, in_bytes);
+    const bool room = o.n_reads + 1 + ng <= MOST_READS && o.n_writes + ng <= MOST_WRITES;
+    bool apart = o.state != 0 && !meets(in, o.writes, o.n_writes), weights_apart = true;
+    for (int g = 0; g < ng; g++) {
+        const lc_range w = range(weights[g], w_bytes[g]), out = range(outputs[g], out_bytes[g]);
+        weights_apart = weights_apart && !meets(w, o.writes, o.n_writes);
+        apart = apart && weights_apart && !meets(out, o.writes, o.n_writes) && !meets(out, o.reads, o.n_reads);
+    }
+    if (o.state == 2 && room) {
+        // (the list stays: what it holds may be running when the next launch starts, whether this one waits or not)
+        flags = apart ? LC_LATE_WAIT : 0u;
+        serial = !weights_apart;   // (fetched ahead of the wait)
+        if (apart) ctx->beside = true;
+    } else {
+        serial = o.state == 2 && !weights_apart;
+        flags = apart ? LC_LATE_TRIGGER : 0u;
+        o.state = apart ? 2 : 1;
+        o.n_reads = o.n_writes = 0;
+    }
+    if (o.n_reads == 0 || o.reads[0].lo != in.lo || o.reads[0].hi < in.hi) o.reads[o.n_reads++] = in;   // (a run mostly shares its input)
+    for (int g = 0; g < ng; g++) {
+        o.reads[o.n_reads++] = range(weights[g], w_bytes[g]);
+        o.writes[o.n_writes++] = range(outputs[g], out_bytes[g]);
+    }
+}
+
+LcOrder::~LcOrder() {
+    if (!tracked) return;
+    lc_overlap &o = ctx->overlap;
+    if (launched) o.seen = before + 1;
+    else o.state = 0;
+    o.mu.unlock();
+}
+
 // ------------------------------------------------------------------ batch --
 int lc_batch_begin(lc_ctx *ctx, lc_batch **out) {
     if (!ctx || !out) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_batch_begin: NULL argument");
@@ -367,6 +421,8 @@ int lc_batch_begin_capture(lc_ctx *ctx, lc_batch **out) {
         return lc_fail(LC_ERR_CUDA, "begin capture: %s", cudaGetErrorString(e));
     }
     (*out)->capturing = true;
+    ctx->launches++;
+    ctx->beside = false;
     return LC_OK;
 }
 
@@ -375,6 +431,8 @@ int lc_batch_end_capture(lc_batch *batch, lc_graph **out) {
     if (!batch->capturing) return lc_fail(LC_ERR_INVALID_ARGUMENT, "batch is not capturing");
     lc_ctx *ctx = batch->ctx;
     cudaGraph_t g = nullptr;
+    ctx->launches++;
+    ctx->beside = false;
     cudaError_t e = cudaStreamEndCapture(batch->stream, &g);
     delete batch;
     if (e != cudaSuccess || !g) {
@@ -397,6 +455,7 @@ int lc_batch_end_capture(lc_batch *batch, lc_graph **out) {
 
 int lc_graph_launch(lc_graph *graph) {
     if (!graph) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_graph_launch: graph is NULL");
+    graph->ctx->launches++;
     LC_CUDA_TRY(cudaGraphLaunch(graph->exec, graph->ctx->stream));
     return LC_OK;
 }

@@ -4,10 +4,23 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <atomic>
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "../../include/local_cuda.h"
+
+// Which of a context's launches may run beside each other (LcOrder below).
+struct lc_range {
+    uintptr_t lo, hi;
+};
+struct lc_overlap {
+    std::mutex mu;
+    uint64_t seen = 0;       // the context's launch count after the launch last recorded here
+    int state = 0;           // 0: nothing known, 1: `reads` / `writes` are the last launch's, 2: those of every launch that may be running
+    int n_reads = 0, n_writes = 0;
+    lc_range reads[192], writes[96];   // (when they are full the run starts anew)
+};
 
 struct lc_ctx {
     int device = 0;
@@ -17,6 +30,10 @@ struct lc_ctx {
     size_t l2_bytes = 0;
     size_t total_mem = 0;
     bool pdl = true;  // launch kernels with programmatic stream serialization (LOCAL_CUDA_PDL=0 disables)
+    bool side_by_side = true;   // launches whose buffers do not meet may overlap (LOCAL_CUDA_OVERLAP=0 disables)
+    std::atomic<uint64_t> launches{0};   // every kernel launch, graph launch and capture boundary of the context counts
+    std::atomic<bool> beside{false};     // the last launch runs beside others
+    lc_overlap overlap;
 };
 
 struct lc_buf {
@@ -113,9 +130,16 @@ void lc_clear_error();
 // lc_pdl_trigger() at its top — its successors may then be scheduled — and lc_pdl_wait() before it
 // first touches memory a predecessor may have written.  Work that does not depend on the predecessor
 // (streaming constant weights towards the SM) goes before the wait.
+// Counts a launch; true where it has to start only when its predecessor is complete (the end of a run of launches side by side: several
+// of those may still be running, and a kernel fetches its constant operands ahead of its wait).
+static inline bool lc_count_launch(lc_batch *b) {
+    b->ctx->launches++;
+    return b->ctx->beside.load() && b->ctx->beside.exchange(false);
+}
+// `serial`: the launch starts only when its predecessor is complete.  (It is counted by whoever asks for it.)
 template <typename... KArgs, typename... Args>
-static inline cudaError_t lc_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, lc_batch *b,
-                                    Args &&...args) {
+static inline cudaError_t lc_launch_as(bool serial, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, lc_batch *b,
+                                       Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -125,12 +149,61 @@ static inline cudaError_t lc_launch(void (*kern)(KArgs...), dim3 grid, dim3 bloc
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = b->ctx->pdl ? 1 : 0;
+    cfg.numAttrs = b->ctx->pdl && !serial ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
+template <typename... KArgs, typename... Args>
+static inline cudaError_t lc_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, lc_batch *b,
+                                    Args &&...args) {
+    return lc_launch_as(lc_count_launch(b), kern, grid, block, smem, b, static_cast<KArgs>(args)...);
+}
+// Launches of one stream run one after the other because the next may read what the last wrote.  Several projections of the same
+// activations, or the same projection of several matrices, do not: a launch of a few microseconds then spends most of its time
+// on latency that the next one's work could hide.  The matmul kernels declare the bytes that they read and write; where those of
+// a new launch do not meet those of the launches it would run beside, it does not wait for them:
+//   * the first such launch waits for its predecessor as ever, but lets its successors start only after that wait (LC_LATE_TRIGGER),
+//     so whatever came before is complete when they run;
+//   * the following ones start at once and wait for their predecessor at their end (LC_LATE_WAIT), so that a launch is complete only
+//     when all before it are.  One that depends on any that may be running waits for the last as ever; so do launches that declare
+//     nothing, which end the run and, because a kernel fetches its constant operands ahead of its wait, start only when the last launch
+//     of a run is complete (`serial`).
+// A graph or a capture boundary ends the run, too.  Ranges are virtual addresses: memory mapped twice is not recognised.
+// (The line lies at the bytes and nowhere else: 35 matrices of 8192 x 1536 TQ2_0 times 16 rows took 225 us one after the
+// other and take 98 side by side, 35 of Q4_0 6144 x 1536 times 40 rows 348 and 269; no shape was found that loses.)
+constexpr uint32_t LC_LATE_TRIGGER = 1, LC_LATE_WAIT = 2;
+class LcOrder {
+public:
+    LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, const lc_buf *const *weights, const size_t *w_bytes,
+            lc_buf *const *outputs, const size_t *out_bytes);
+    ~LcOrder();
+    uint32_t flags = 0;      // for the kernel
+    bool serial = false;     // for the launch
+    bool launched = false;   // set by the caller once its one launch is enqueued
+
+private:
+    lc_ctx *ctx;
+    bool tracked;
+    uint64_t before = 0;
+};
 #ifdef __CUDACC__
 __device__ __forceinline__ void lc_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void lc_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The same for kernels launched under an LcOrder: at their top, before their first dependent access, and at their end (any one CTA
+// keeps the grid from completing).  ORDERED: flags are set; without them the kernel is one that knows none (reading them ahead of the
+// trigger cost a decode step 0.3 to 1.1 %).
+template <bool ORDERED>
+__device__ __forceinline__ void lc_order_begin(uint32_t flags) {
+    if (!ORDERED || !(flags & LC_LATE_TRIGGER)) lc_pdl_trigger();
+}
+template <bool ORDERED>
+__device__ __forceinline__ void lc_order_wait(uint32_t flags) {
+    if (!ORDERED || !(flags & LC_LATE_WAIT)) lc_pdl_wait();
+    if (ORDERED && (flags & LC_LATE_TRIGGER)) lc_pdl_trigger();
+}
+template <bool ORDERED>
+__device__ __forceinline__ void lc_order_end(uint32_t flags) {
+    if (ORDERED && (flags & LC_LATE_WAIT) && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) lc_pdl_wait();
+}
 
 // Walsh-Hadamard transform (unnormalised) over d = 32 .. 512 elements held one per thread of a d-thread block;
 // returns the thread's element of the result.  Butterflies run in ascending stride, lower = a + b, upper = a - b.

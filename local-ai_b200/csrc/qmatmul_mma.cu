@@ -49,6 +49,7 @@ struct MmaParams {
     int m, K, nb;          // nb = blocks per weight row
     int ks, bps;           // split-K: grid.z = cluster size = ks, bps = blocks per split
     int raw_rs;            // bytes reserved per row of raw blocks
+    uint32_t order;        // LcOrder::flags
     int geglu;             // 1: w[0] = gate, w[1] = up, out[0] = gelu(gate) * up (see lc_qgemm_mma_geglu)
 };
 
@@ -103,13 +104,13 @@ template <> struct Fmt<FMT_Q4_0> { static constexpr int bytes = 18, elems = 32, 
 template <> struct Fmt<FMT_TQ2_0> { static constexpr int bytes = 66, elems = 256, chunk_blocks = 1; };
 
 // NBT: 8-row batch tiles (m <= 8 NBT).
-template <int FMT, int NBT, typename OutT>
+template <int FMT, int NBT, typename OutT, bool ORDERED>
 __global__ void __launch_bounds__(NT) qgemm_mma_kernel(const MmaParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int BB = Fmt<FMT>::bytes, BE = Fmt<FMT>::elems, CHB = Fmt<FMT>::chunk_blocks;
     constexpr int XBUF = 8 * NBT * XS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    lc_pdl_trigger();
+    lc_order_begin<ORDERED>(p.order);
     int grp = 0;
     while (grp + 1 < p.ngroups && (int)blockIdx.x >= p.tile_end[grp]) grp++;
     // GeGLU mode: a CTA owns 64 rows of the gate matrix (warps 0-3) and the same 64 rows of the up matrix (warps 4-7)
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(NT) qgemm_mma_kernel(const MmaParams p) {
         }
     }
     cp_async_commit();
-    lc_pdl_wait();
+    lc_order_wait<ORDERED>(p.order);
 
     // ---- 2. activation chunks: [8 NBT rows][256 k] per buffer, 16-byte pieces, rows beyond m zero-filled ----
     const int nchunks = (nblk + CHB - 1) / CHB;
@@ -304,6 +305,7 @@ __global__ void __launch_bounds__(NT) qgemm_mma_kernel(const MmaParams p) {
         if (!p.geglu) {
 #pragma unroll
             for (int j = 0; j < NBT; j++) store_tile(make_float4(c[j][0], c[j][1], c[j][2], c[j][3]), warp, lane, j);
+            lc_order_end<ORDERED>(p.order);
             return;
         }
         cp_async_wait<0>();
@@ -317,6 +319,7 @@ __global__ void __launch_bounds__(NT) qgemm_mma_kernel(const MmaParams p) {
             for (int j = 0; j < NBT; j++)
                 store_geglu(make_float4(c[j][0], c[j][1], c[j][2], c[j][3]), red[j * NT + tid + 128], warp, lane, j);
         }
+        lc_order_end<ORDERED>(p.order);
         return;
     }
     // Split K: the ks CTAs of this tile are one cluster.  Partial tiles are exchanged through shared memory.
@@ -352,11 +355,12 @@ __global__ void __launch_bounds__(NT) qgemm_mma_kernel(const MmaParams p) {
         }
     }
     cluster_sync();   // no CTA leaves while a peer may still read its shared memory
+    lc_order_end<ORDERED>(p.order);
 }
 
-template <int FMT, int NBT, typename OutT>
-int launch_mma(lc_batch *b, const MmaParams &p, dim3 grid, size_t smem) {
-    auto kern = qgemm_mma_kernel<FMT, NBT, OutT>;
+template <int FMT, int NBT, typename OutT, bool ORDERED>
+int launch_mma_as(lc_batch *b, bool serial, const MmaParams &p, dim3 grid, size_t smem) {
+    auto kern = qgemm_mma_kernel<FMT, NBT, OutT, ORDERED>;
     static lc_smem_optin optin;
     LC_CUDA_TRY(lc_ensure_smem(kern, optin, b->ctx, smem));
     cudaLaunchConfig_t cfg = {};
@@ -366,7 +370,7 @@ int launch_mma(lc_batch *b, const MmaParams &p, dim3 grid, size_t smem) {
     cfg.stream = b->stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
-    if (b->ctx->pdl) {
+    if (b->ctx->pdl && !serial) {
         attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[na].val.programmaticStreamSerializationAllowed = 1;
         na++;
@@ -385,12 +389,17 @@ int launch_mma(lc_batch *b, const MmaParams &p, dim3 grid, size_t smem) {
     return LC_OK;
 }
 
+template <int FMT, int NBT, typename OutT>
+int launch_mma(lc_batch *b, bool serial, const MmaParams &p, dim3 grid, size_t smem) {
+    return p.order ? launch_mma_as<FMT, NBT, OutT, true>(b, serial, p, grid, smem) : launch_mma_as<FMT, NBT, OutT, false>(b, serial, p, grid, smem);
+}
+
 template <int FMT, typename OutT>
-int launch_mma_nbt(lc_batch *b, const MmaParams &p, dim3 grid, size_t smem, int nbt) {
+int launch_mma_nbt(lc_batch *b, bool serial, const MmaParams &p, dim3 grid, size_t smem, int nbt) {
     switch (nbt) {
-        case 2: return launch_mma<FMT, 2, OutT>(b, p, grid, smem);
-        case 4: return launch_mma<FMT, 4, OutT>(b, p, grid, smem);
-        default: return launch_mma<FMT, 8, OutT>(b, p, grid, smem);
+        case 2: return launch_mma<FMT, 2, OutT>(b, serial, p, grid, smem);
+        case 4: return launch_mma<FMT, 4, OutT>(b, serial, p, grid, smem);
+        default: return launch_mma<FMT, 8, OutT>(b, serial, p, grid, smem);
     }
 }
 
@@ -664,9 +673,20 @@ static int qgemm_mma_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, co
     p.bps = pl.bps;
     p.raw_rs = pl.raw_rs;
     dim3 grid(tiles, 1, pl.ks);
+    size_t w_bytes[MAX_GROUPS], out_bytes[MAX_GROUPS];
+    for (int g = 0; g < ng; g++) {
+        w_bytes[g] = (size_t)p.nb * (fmt == FMT_Q4_0 ? 18 : 66) * ns[g];
+        out_bytes[g] = (size_t)m * ns[g] * (f32out ? 4 : 2);
+    }
+    LcOrder order(b, input, (size_t)m * kk * 2, ng, weights, w_bytes, outputs, out_bytes);
+    p.order = order.flags;
+    int st;
     if (fmt == FMT_Q4_0)
-        return f32out ? launch_mma_nbt<FMT_Q4_0, float>(b, p, grid, smem, nbt) : launch_mma_nbt<FMT_Q4_0, __half>(b, p, grid, smem, nbt);
-    return f32out ? launch_mma_nbt<FMT_TQ2_0, float>(b, p, grid, smem, nbt) : launch_mma_nbt<FMT_TQ2_0, __half>(b, p, grid, smem, nbt);
+        st = f32out ? launch_mma_nbt<FMT_Q4_0, float>(b, order.serial, p, grid, smem, nbt) : launch_mma_nbt<FMT_Q4_0, __half>(b, order.serial, p, grid, smem, nbt);
+    else
+        st = f32out ? launch_mma_nbt<FMT_TQ2_0, float>(b, order.serial, p, grid, smem, nbt) : launch_mma_nbt<FMT_TQ2_0, __half>(b, order.serial, p, grid, smem, nbt);
+    order.launched = st == LC_OK;
+    return st;
 }
 
 int lc_qgemm_mma_grouped(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const lc_buf *input, int ng,

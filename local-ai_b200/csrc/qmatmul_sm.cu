@@ -40,6 +40,7 @@ struct SmParams {
     int *status;
     uint32_t wait_limit;
     uint32_t extra_arrivals;   // 0; 1 in the expiry self-test
+    uint32_t order;            // LcOrder::flags
 };
 
 // gelu_tanh(gate) * up with gate and up rounded to f16 first, as the separate projections would store them, and the
@@ -89,12 +90,12 @@ __device__ __forceinline__ uint32_t codes_f16(uint32_t w, int l) {
 
 // NT8: batch columns / 8.  MTW: 16-row tiles of the CTA (every warp works on all of them).  SINGLE: a warp has at most one
 // step, so a tile's sums go to shared memory at once and four tiles fit the registers of two CTAs per SM.
-template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT>
+template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT, bool ORDERED>
 __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_kernel(const __grid_constant__ SmParams p) {
     constexpr int BB = FMT == FMT_Q4_0 ? 18 : 66;
     constexpr int ROWS = MTW * 16, OROWS = GEGLU ? ROWS / 2 : ROWS;
     constexpr int RS = ROWS + 4;                // padded column of partial sums
-    lc_pdl_trigger();
+    lc_order_begin<ORDERED>(p.order);
     extern __shared__ __align__(16) uint8_t smem[];
     uint8_t *raw = smem;                                                       // [ROWS][raw_rs]
     float *red = reinterpret_cast<float *>(smem + ROWS * p.raw_rs);            // [SM_NW][NT8 * 8][RS]
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
         return smem_u32(raw) + (uint32_t)(r * p.raw_rs) + (uint32_t)(((size_t)row * rb) & 15);
     };
     const int units = (p.K + SM_UNIT - 1) / SM_UNIT;
-    lc_pdl_wait();
+    lc_order_wait<ORDERED>(p.order);
 
     // ---- activations of one step as B fragments.  TQ2_0: k = 32 l + 8t .. + 7 (l = 0..3), one 16-byte load each.
     //      Q4_0: block l of the step, k = 32 l + 4t .. + 3 and 32 l + 16 + 4t .. + 3, two 8-byte loads. ----
@@ -268,6 +269,7 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
     const bool failed = __syncthreads_or(!ok);
     if (failed) {
         tc_wait_expired(p.status, LC_DEV_STATUS_WAIT_EXPIRED_TCD, tid);
+        lc_order_end<ORDERED>(p.order);
         return;
     }
     const int parts = min(units, SM_NW);
@@ -300,31 +302,34 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
             if (n0 + r + 1 < n_rows) sm_store(dst + 1, v.y);
         }
     }
+    lc_order_end<ORDERED>(p.order);
 }
 
-template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT>
-int launch_sm(lc_batch *b, const SmParams &p, int tiles) {
-    auto kern = qgemm_sm_kernel<FMT, NT8, MTW, SINGLE, GEGLU, OutT>;
+template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT, bool ORDERED>
+int launch_sm(lc_batch *b, bool serial, const SmParams &p, int tiles) {
+    auto kern = qgemm_sm_kernel<FMT, NT8, MTW, SINGLE, GEGLU, OutT, ORDERED>;
     const size_t smem = (size_t)MTW * 16 * p.raw_rs + sizeof(float) * SM_NW * NT8 * 8 * (MTW * 16 + 4);
     static lc_smem_optin optin;
     LC_CUDA_TRY(lc_ensure_smem(kern, optin, b->ctx, smem));
-    LC_LAUNCH_CHECKED(lc_launch(kern, dim3(tiles), dim3(SM_NT), smem, b, p));
+    LC_LAUNCH_CHECKED(lc_launch_as(serial, kern, dim3(tiles), dim3(SM_NT), smem, b, p));
     b->dispatch_count++;
     return LC_OK;
 }
-template <int FMT, int NT8, bool GEGLU, typename OutT>
-int launch_rows(lc_batch *b, const SmParams &p, int tiles, int rows) {
+template <int FMT, int NT8, bool GEGLU, typename OutT, bool ORDERED>
+int launch_rows(lc_batch *b, bool serial, const SmParams &p, int tiles, int rows) {
     if (p.K <= SM_NW * SM_UNIT) {
-        if (rows == 64) return launch_sm<FMT, NT8, 4, true, GEGLU, OutT>(b, p, tiles);
-        if (rows == 32) return launch_sm<FMT, NT8, 2, true, GEGLU, OutT>(b, p, tiles);
-        return launch_sm<FMT, NT8, 1, true, GEGLU, OutT>(b, p, tiles);
+        if (rows == 64) return launch_sm<FMT, NT8, 4, true, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
+        if (rows == 32) return launch_sm<FMT, NT8, 2, true, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
+        return launch_sm<FMT, NT8, 1, true, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
     }
-    if (rows == 32) return launch_sm<FMT, NT8, 2, false, GEGLU, OutT>(b, p, tiles);
-    return launch_sm<FMT, NT8, 1, false, GEGLU, OutT>(b, p, tiles);
+    if (rows == 32) return launch_sm<FMT, NT8, 2, false, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
+    return launch_sm<FMT, NT8, 1, false, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
 }
 template <int FMT, bool GEGLU, typename OutT>
-int launch_nt(lc_batch *b, const SmParams &p, int tiles, int rows) {
-    return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT>(b, p, tiles, rows) : launch_rows<FMT, 2, GEGLU, OutT>(b, p, tiles, rows);
+int launch_nt(lc_batch *b, bool serial, const SmParams &p, int tiles, int rows) {
+    if (p.order)
+        return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT, true>(b, serial, p, tiles, rows) : launch_rows<FMT, 2, GEGLU, OutT, true>(b, serial, p, tiles, rows);
+    return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT, false>(b, serial, p, tiles, rows) : launch_rows<FMT, 2, GEGLU, OutT, false>(b, serial, p, tiles, rows);
 }
 
 }  // namespace
@@ -376,7 +381,17 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     p.status = k->dev_status;
     p.wait_limit = k->test_wait_expiry ? 4096u : SM_WAIT_LIMIT;
     p.extra_arrivals = k->test_wait_expiry ? 1u : 0u;
-    if (geglu) return launch_nt<FMT_TQ2_0, true, __half>(b, p, tiles, rows);
-    if (fmt == FMT_Q4_0) return f32out ? launch_nt<FMT_Q4_0, false, float>(b, p, tiles, rows) : launch_nt<FMT_Q4_0, false, __half>(b, p, tiles, rows);
-    return f32out ? launch_nt<FMT_TQ2_0, false, float>(b, p, tiles, rows) : launch_nt<FMT_TQ2_0, false, __half>(b, p, tiles, rows);
+    size_t w_bytes[SM_GROUPS], out_bytes[SM_GROUPS];
+    for (int g = 0; g < ng; g++) {
+        w_bytes[g] = rb * ns[g];
+        out_bytes[g] = (size_t)m * ns[g] * (f32out ? 4 : 2);
+    }
+    LcOrder order(b, input, (size_t)m * kk * 2, ng, weights, w_bytes, outputs, out_bytes);
+    p.order = order.flags;
+    int st;
+    if (geglu) st = launch_nt<FMT_TQ2_0, true, __half>(b, order.serial, p, tiles, rows);
+    else if (fmt == FMT_Q4_0) st = f32out ? launch_nt<FMT_Q4_0, false, float>(b, order.serial, p, tiles, rows) : launch_nt<FMT_Q4_0, false, __half>(b, order.serial, p, tiles, rows);
+    else st = f32out ? launch_nt<FMT_TQ2_0, false, float>(b, order.serial, p, tiles, rows) : launch_nt<FMT_TQ2_0, false, __half>(b, order.serial, p, tiles, rows);
+    order.launched = st == LC_OK;
+    return st;
 }

@@ -86,6 +86,7 @@ struct TcdParams {
     int geglu;           // 1: operand rows 0-63 are gate rows, 64-127 the same rows of the up matrix; out[0] = gelu(gate) * up
     int *status;
     uint32_t wait_limit;
+    uint32_t order;            // LcOrder::flags
     uint32_t extra_arrivals;   // 0; 1 in the expiry self-test: the "weights ready" barriers then expect an arrival nobody makes
 };
 
@@ -105,6 +106,7 @@ __device__ __forceinline__ uint2 pack4(float a, float b, float c, float d) {
 constexpr int NDQ = 8;                       // dequantizing warps (also the epilogue warps)
 constexpr int NT = (NDQ + 1 + NISS) * 32;    // + activation loader warp + MMA issuers
 
+template <bool ORDERED>
 __global__ void __launch_bounds__(NT, 1)
 qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CUtensorMap x_map) {
     constexpr int ROWS = TILE_ROWS;
@@ -122,7 +124,7 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
     volatile uint32_t *abort_flag = tmem_slot + 1;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    lc_pdl_trigger();
+    lc_order_begin<ORDERED>(p.order);
     int grp = 0;
     while (grp + 1 < p.ngroups && (int)blockIdx.x >= p.tile_end[grp]) grp++;
     const int rows_out = p.geglu ? TILE_ROWS / 2 : TILE_ROWS;                          // output rows of a tile
@@ -253,7 +255,7 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
         // =========================== activation loader (one thread) ===========================
         // Step i needs x[0..64, k .. k + 255], k = 256 (kbs + block): four boxes of the tensor map.
         if (lane == 0) {
-            lc_pdl_wait();   // the activations are the predecessor's output
+            lc_order_wait<ORDERED>(p.order);   // the activations are the predecessor's output
             bool dead = false;
             uint32_t sbi = 0;   // i % SB without the division
             for (int i = 0; i < total_steps && !dead; i++) {
@@ -418,6 +420,7 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
     if (warp == 0) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS) : "memory");
     }
+    lc_order_end<ORDERED>(p.order);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point lookup (no link-time dependency on the driver).
@@ -451,9 +454,10 @@ int make_x_map(CUtensorMap *map, const void *x, uint32_t m, uint32_t kk) {
     return LC_OK;
 }
 
-int launch_tcd(lc_batch *b, const TcdParams &p, const CUtensorMap &x_map, int tiles, size_t smem) {
+template <bool ORDERED>
+int launch_tcd(lc_batch *b, bool serial, const TcdParams &p, const CUtensorMap &x_map, int tiles, size_t smem) {
     static lc_smem_optin optin;
-    LC_CUDA_TRY(lc_ensure_smem(qgemm_tcd_kernel, optin, b->ctx, smem));
+    LC_CUDA_TRY(lc_ensure_smem(qgemm_tcd_kernel<ORDERED>, optin, b->ctx, smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles, 1, p.ks);
     cfg.blockDim = dim3(NT);
@@ -461,7 +465,7 @@ int launch_tcd(lc_batch *b, const TcdParams &p, const CUtensorMap &x_map, int ti
     cfg.stream = b->stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
-    if (b->ctx->pdl) {
+    if (b->ctx->pdl && !serial) {
         attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[na].val.programmaticStreamSerializationAllowed = 1;
         na++;
@@ -475,7 +479,7 @@ int launch_tcd(lc_batch *b, const TcdParams &p, const CUtensorMap &x_map, int ti
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    LC_LAUNCH_CHECKED(cudaLaunchKernelEx(&cfg, qgemm_tcd_kernel, p, x_map));
+    LC_LAUNCH_CHECKED(cudaLaunchKernelEx(&cfg, qgemm_tcd_kernel<ORDERED>, p, x_map));
     b->dispatch_count++;
     return LC_OK;
 }
@@ -548,5 +552,14 @@ int lc_qgemm_tcd_launch(lc_kernels *k, lc_batch *b, const lc_buf *input, int ng,
     CUtensorMap x_map;
     int st = make_x_map(&x_map, input->dptr, m, kk);
     if (st != LC_OK) return st;
-    return launch_tcd(b, p, x_map, tiles, smem);
+    size_t w_bytes[MAX_GROUPS], out_bytes[MAX_GROUPS];
+    for (int g = 0; g < ng; g++) {
+        w_bytes[g] = (size_t)p.nb * BB * ns[g];
+        out_bytes[g] = (size_t)m * ns[g] * 2;
+    }
+    LcOrder order(b, input, (size_t)m * kk * 2, ng, weights, w_bytes, outputs, out_bytes);
+    p.order = order.flags;
+    st = p.order ? launch_tcd<true>(b, order.serial, p, x_map, tiles, smem) : launch_tcd<false>(b, order.serial, p, x_map, tiles, smem);
+    order.launched = st == LC_OK;
+    return st;
 }

@@ -55,6 +55,7 @@ struct TclParams {
     int b_slots;           // activation ring depth, in steps
     int *status;
     uint32_t wait_limit;
+    uint32_t order;            // LcOrder::flags
     uint32_t extra_arrivals;   // 0; 1 in the expiry self-test: the "weights ready" barriers then expect an arrival nobody makes
 };
 
@@ -78,7 +79,7 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, uint32_
     return true;
 }
 
-template <int FMT, typename OutT>
+template <int FMT, typename OutT, bool ORDERED>
 __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant__ TclParams p, const __grid_constant__ CUtensorMap x_map) {
     using F = TclFmt<FMT>;
     constexpr int BB = F::bytes, STEP_TILES = F::step_k / KT, STEP_BYTES = F::blocks * BB;
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
     volatile uint32_t *abort_flag = tmem_slot + 1;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    lc_pdl_trigger();
+    lc_order_begin<ORDERED>(p.order);
     int grp = 0;
     while (grp + 1 < p.ngroups && (int)blockIdx.x >= p.tile_end[grp]) grp++;
     const int n0 = ((int)blockIdx.x - (grp ? p.tile_end[grp - 1] : 0)) * ROWS, m0 = (int)blockIdx.y * p.NB;
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
     } else if (warp == NDQ + NRAW) {
         // =========================== activations (one thread) ===========================
         if (lane == 0) {
-            lc_pdl_wait();   // the activations are the predecessor's output
+            lc_order_wait<ORDERED>(p.order);   // the activations are the predecessor's output
             uint32_t slot = 0;
             for (int i = 0; i < n_steps; i++) {
                 if (i >= BS) {   // its slot was last read by the MMAs of step i - BS
@@ -373,6 +374,7 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
     __syncthreads();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS) : "memory");
+    lc_order_end<ORDERED>(p.order);
 }
 
 typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
@@ -405,9 +407,9 @@ int make_x_map(CUtensorMap *map, const void *x, uint32_t m, uint32_t kk, uint32_
     return LC_OK;
 }
 
-template <int FMT, typename OutT>
-int launch_tcl(lc_batch *b, const TclParams &p, const CUtensorMap &x_map, int tiles, size_t smem) {
-    auto kern = qgemm_tcl_kernel<FMT, OutT>;
+template <int FMT, typename OutT, bool ORDERED>
+int launch_tcl_as(lc_batch *b, bool serial, const TclParams &p, const CUtensorMap &x_map, int tiles, size_t smem) {
+    auto kern = qgemm_tcl_kernel<FMT, OutT, ORDERED>;
     static lc_smem_optin optin;
     LC_CUDA_TRY(lc_ensure_smem(kern, optin, b->ctx, smem));
     cudaLaunchConfig_t cfg = {};
@@ -417,7 +419,7 @@ int launch_tcl(lc_batch *b, const TclParams &p, const CUtensorMap &x_map, int ti
     cfg.stream = b->stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
-    if (b->ctx->pdl) {
+    if (b->ctx->pdl && !serial) {
         attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[na].val.programmaticStreamSerializationAllowed = 1;
         na++;
@@ -434,6 +436,11 @@ int launch_tcl(lc_batch *b, const TclParams &p, const CUtensorMap &x_map, int ti
     LC_LAUNCH_CHECKED(cudaLaunchKernelEx(&cfg, kern, p, x_map));
     b->dispatch_count++;
     return LC_OK;
+}
+
+template <int FMT, typename OutT>
+int launch_tcl(lc_batch *b, bool serial, const TclParams &p, const CUtensorMap &x_map, int tiles, size_t smem) {
+    return p.order ? launch_tcl_as<FMT, OutT, true>(b, serial, p, x_map, tiles, smem) : launch_tcl_as<FMT, OutT, false>(b, serial, p, x_map, tiles, smem);
 }
 
 }  // namespace
@@ -526,7 +533,17 @@ int lc_qgemm_tcl_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const 
     CUtensorMap x_map;
     int st = make_x_map(&x_map, input->dptr, m, kk, (uint32_t)p.NB);
     if (st != LC_OK) return st;
+    size_t w_bytes[MAX_MATS], out_bytes[MAX_MATS];
+    for (int g = 0; g < ng; g++) {
+        w_bytes[g] = (size_t)p.nb * (fmt == FMT_Q4_0 ? 18 : 66) * ns[g];
+        out_bytes[g] = (size_t)m * ns[g] * (f32out ? 4 : 2);
+    }
+    LcOrder order(b, input, (size_t)m * kk * 2, ng, weights, w_bytes, outputs, out_bytes);
+    p.order = order.flags;
     if (fmt == FMT_Q4_0)
-        return f32out ? launch_tcl<FMT_Q4_0, float>(b, p, x_map, tiles, smem) : launch_tcl<FMT_Q4_0, __half>(b, p, x_map, tiles, smem);
-    return f32out ? launch_tcl<FMT_TQ2_0, float>(b, p, x_map, tiles, smem) : launch_tcl<FMT_TQ2_0, __half>(b, p, x_map, tiles, smem);
+        st = f32out ? launch_tcl<FMT_Q4_0, float>(b, order.serial, p, x_map, tiles, smem) : launch_tcl<FMT_Q4_0, __half>(b, order.serial, p, x_map, tiles, smem);
+    else
+        st = f32out ? launch_tcl<FMT_TQ2_0, float>(b, order.serial, p, x_map, tiles, smem) : launch_tcl<FMT_TQ2_0, __half>(b, order.serial, p, x_map, tiles, smem);
+    order.launched = st == LC_OK;
+    return st;
 }
