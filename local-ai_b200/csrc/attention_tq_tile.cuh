@@ -1,0 +1,385 @@
+// What the kernels that attend over TurboQuant codes on mma.sync share: the configuration, the table of levels and one warp's
+// step over a tile of keys (attention_tq_mma.cu explains the arithmetic; step_small.cu runs the same step inside the decode step).
+#pragma once
+#include <utility>
+
+#include "attention_tq.h"
+#include "tcgen05_util.cuh"
+
+namespace {
+
+constexpr int G = 8;             // q-heads per CTA (MMA N)
+constexpr int LUT_COPIES = 16;   // an 8-byte shared load is served per half-warp, so 16 copies are conflict-free
+
+template <int HD_, int BITS_>
+struct AttnCfg {
+    static constexpr int HD = HD_, BITS = BITS_;
+    static constexpr int CB = HD * BITS / 8;            // code bytes per row
+    static constexpr bool HILO = BITS > 2 || HD != 256; // levels and P as an f16 and the f16 of the remainder
+    static constexpr int FB = HILO ? 2 * BITS : 8;      // table index bits
+    static constexpr int NENT = 1 << FB;
+    static constexpr int MT = HD == 512 ? 1 : 2;        // 16-key MMA tiles per warp step
+    static constexpr int KT = 16 * MT;
+    static constexpr int NW = 8, NT = NW * 32;
+    static constexpr int NS = HD / 16;                  // k16 steps of QK, 16-dim tiles of PV
+    static constexpr int DPL = HD / 32;                 // dims per lane where a warp owns a head
+    static constexpr bool QSMEM = HD == 512;            // query fragments stay in shared memory (registers hold the accumulators)
+    // Row strides in the ring: chosen so that the fragment reads spread over the banks.
+    static constexpr int KRS = (BITS == 2 && HD == 256) ? CB : CB + 16;
+    static constexpr int VRS = CB + 16;
+    static constexpr int STAGE = KT * (KRS + VRS);
+    static constexpr int LUT_BYTES = NENT * LUT_COPIES * 8;
+    static constexpr int Q_BYTES = NS * 32 * 16;        // query: f32 [NS][32][4], then the packed fragments in place
+    static constexpr int ENT_BYTES = NENT * 8;
+    static constexpr int ACC_BYTES = NW * NS * 4 * 32 * 4;   // merge staging, reuses query and ring memory
+    static constexpr int RING_OFF = LUT_BYTES + Q_BYTES + ENT_BYTES;
+    // Merged rows (a head of one split): four floats of padding after every HD / 8 dims (their writers' lanes are HD / 8 dims
+    // apart).  A CTA of a cluster of n receives n rows for each of its ceil(8 / n) heads, at most 14.
+    static constexpr int CPS = HD + 40, ROWS = 14;
+    static constexpr int TAIL_BYTES = (2 * NW * G + 2 * ROWS) * 4 + ROWS * CPS * 4;  // (max, sum) of warps and rows, the rows
+    static __device__ __forceinline__ int cp_index(int row, int d) { return row * CPS + d + 4 * (d / (HD / 8)); }
+    static constexpr int RING_ROOM = 222 * 1024 - TAIL_BYTES - RING_OFF;
+    static constexpr int DEPTH_FIT = RING_ROOM / (NW * STAGE);
+    static constexpr int DEPTH = DEPTH_FIT > 4 ? 4 : DEPTH_FIT;   // ring slots per warp (DEPTH - 1 tiles in flight)
+    static constexpr int SMEM0 = RING_OFF + NW * DEPTH * STAGE;
+    static constexpr int TAIL_OFF = SMEM0 > LUT_BYTES + ACC_BYTES ? SMEM0 : LUT_BYTES + ACC_BYTES;
+    static constexpr int SMEM = TAIL_OFF + TAIL_BYTES;
+    static_assert(DEPTH >= 2, "the ring needs two slots");
+    static_assert(SMEM <= 224 * 1024, "shared memory, with room for the static part");
+};
+
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+// the same place in the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(addr), "r"(rank));
+    return ra;
+}
+__device__ __forceinline__ void st_cluster_f2(uint32_t a, float x, float y) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(a), "f"(x), "f"(y) : "memory");
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+// N 32-bit words of shared memory at an address aligned for the widest load that divides N
+template <int N>
+__device__ __forceinline__ void lds_words(uint32_t a, uint32_t (&w)[N]) {
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4)
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(w[i]), "=r"(w[i + 1]), "=r"(w[i + 2]), "=r"(w[i + 3]) : "r"(a + 4 * i));
+    } else if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 2)
+            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];\n" : "=r"(w[i]), "=r"(w[i + 1]) : "r"(a + 4 * i));
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i++) asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(w[i]) : "r"(a + 4 * i));
+    }
+}
+// f(integral_constant<0>) .. f(integral_constant<N - 1>)
+template <typename F, int... I>
+__device__ __forceinline__ void static_for_impl(F &&f, std::integer_sequence<int, I...>) {
+    (f(std::integral_constant<int, I>{}), ...);
+}
+template <int N, typename F>
+__device__ __forceinline__ void static_for(F &&f) {
+    static_for_impl(f, std::make_integer_sequence<int, N>{});
+}
+// Table address of the FB-bit field at bit O of a word run: lane base + index * 128 bytes.  The multiply-add goes to the
+// multiply pipe, which is idle here; the ALU pipe is the busy one.
+template <int FB, int O, int N>
+__device__ __forceinline__ uint32_t field_addr(const uint32_t (&w)[N], uint32_t lane_base) {
+    constexpr int i = O / 32, o = O % 32;
+    uint32_t idx, r;
+    if constexpr (FB == 8) idx = __byte_perm(w[i], 0u, 0x4440 + o / 8);
+    else if constexpr (o + FB > 32) idx = __funnelshift_r(w[i], w[i + 1 < N ? i + 1 : i], o) & ((1u << FB) - 1u);
+    else idx = (w[i] >> o) & ((1u << FB) - 1u);
+    asm("mad.lo.u32 %0, %1, %2, %3;\n" : "=r"(r) : "r"(idx), "n"(LUT_COPIES * 8), "r"(lane_base));
+    return r;
+}
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
+    uint32_t d;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(d) : "r"(a));
+    return d;
+}
+__device__ __forceinline__ uint32_t pack_h2(float x, float y) {
+    __half2 h = __floats2half2_rn(x, y);
+    return *reinterpret_cast<uint32_t *>(&h);
+}
+__device__ __forceinline__ float2 unpack_h2(uint32_t u) { return __half22float2(*reinterpret_cast<__half2 *>(&u)); }
+// f16 of the two values and f16 of what the rounding left
+__device__ __forceinline__ void split_h2(float x, float y, uint32_t &hi, uint32_t &lo) {
+    hi = pack_h2(x, y);
+    const float2 h = unpack_h2(hi);
+    lo = pack_h2(x - h.x, y - h.y);
+}
+template <bool HILO>
+__device__ __forceinline__ float soft_exp(float x) {
+    return HILO ? expf(x) : __expf(x);
+}
+
+// Walsh-Hadamard butterflies over 32 * DPL values held DPL per lane (lane owns consecutive dims), ascending stride.
+template <int DPL>
+__device__ __forceinline__ void warp_fwht(float (&x)[DPL], int lane) {
+#pragma unroll
+    for (int len = 1; len < DPL; len <<= 1) {
+#pragma unroll
+        for (int i = 0; i < DPL; i++) {
+            if (!(i & len)) {
+                const float a = x[i], b2 = x[i + len];
+                x[i] = a + b2;
+                x[i + len] = a - b2;
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) {
+        const bool upper = lane & m;
+#pragma unroll
+        for (int i = 0; i < DPL; i++) {
+            const float o2 = __shfl_xor_sync(0xffffffffu, x[i], m);
+            x[i] = upper ? o2 - x[i] : x[i] + o2;
+        }
+    }
+}
+
+// The table of levels at the start of shared memory and gamma, by the whole CTA; the levels are a constant operand.  The table is
+// complete for all threads after the caller's next barrier.
+template <typename C, int NW = C::NW, typename Sync = lc_block_sync>
+__device__ __forceinline__ float attn_table(const float *levels, uint2 *lut, uint2 *ent_s, int lane, int warp, Sync sync = {}) {
+    constexpr int NT = NW * 32;
+    __shared__ float gamma_s;
+    __shared__ float cand_err[NW];
+    __shared__ int cand_idx[NW];
+    if constexpr (!C::HILO) {
+        // gamma such that every level / gamma is (almost) exactly an f16
+        const float lv0 = levels[0], lv1 = levels[1], lv2 = levels[2], lv3 = levels[3];
+        const float ref = fmaxf(fmaxf(fabsf(lv0), fabsf(lv1)), fmaxf(fabsf(lv2), fabsf(lv3)));
+        const float ia0 = lv0 != 0.f ? 1.0f / fabsf(lv0) : 0.f, ia1 = lv1 != 0.f ? 1.0f / fabsf(lv1) : 0.f;
+        const float ia2 = lv2 != 0.f ? 1.0f / fabsf(lv2) : 0.f, ia3 = lv3 != 0.f ? 1.0f / fabsf(lv3) : 0.f;
+        float best = INFINITY;
+        int besti = 0;
+        for (int j = threadIdx.x; j < 1024; j += NT) {
+            const float gm = ref > 0.f ? ref / (1.0f + (float)j * (1.0f / 1024.0f)) : 1.0f;  // largest level -> [1, 2)
+            const float inv = __frcp_rn(gm);
+            float e = fabsf(__half2float(__float2half_rn(lv0 * inv)) * gm - lv0) * ia0;
+            e = fmaxf(e, fabsf(__half2float(__float2half_rn(lv1 * inv)) * gm - lv1) * ia1);
+            e = fmaxf(e, fabsf(__half2float(__float2half_rn(lv2 * inv)) * gm - lv2) * ia2);
+            e = fmaxf(e, fabsf(__half2float(__float2half_rn(lv3 * inv)) * gm - lv3) * ia3);
+            if (e < best) { best = e; besti = j; }
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {   // arg-min inside the warp, lowest index on ties
+            const float oe = __shfl_xor_sync(0xffffffffu, best, off);
+            const int oi = __shfl_xor_sync(0xffffffffu, besti, off);
+            if (oe < best || (oe == best && oi < besti)) { best = oe; besti = oi; }
+        }
+        if (lane == 0) { cand_err[warp] = best; cand_idx[warp] = besti; }
+        sync();
+        if (threadIdx.x == 0) {
+            float b2 = cand_err[0];
+            int bi = cand_idx[0];
+            for (int i = 1; i < NW; i++)
+                if (cand_err[i] < b2 || (cand_err[i] == b2 && cand_idx[i] < bi)) { b2 = cand_err[i]; bi = cand_idx[i]; }
+            gamma_s = ref > 0.f ? ref / (1.0f + (float)bi * (1.0f / 1024.0f)) : 1.0f;
+        }
+        sync();
+    } else {
+        // the largest level becomes 1; each level is stored as two f16
+        float ref = 0.f;
+#pragma unroll
+        for (int i = 0; i < (1 << C::BITS); i++) ref = fmaxf(ref, fabsf(levels[i]));
+        if (threadIdx.x == 0) gamma_s = ref > 0.f ? ref : 1.0f;
+        sync();
+    }
+    const float gamma = gamma_s;
+    for (int e = threadIdx.x; e < C::NENT; e += NT) {
+        uint2 v;
+        if constexpr (!C::HILO) {
+            v.x = pack_h2(levels[e & 3] / gamma, levels[(e >> 2) & 3] / gamma);
+            v.y = pack_h2(levels[(e >> 4) & 3] / gamma, levels[(e >> 6) & 3] / gamma);
+        } else {
+            constexpr int M = (1 << C::BITS) - 1;
+            split_h2(levels[e & M] / gamma, levels[(e >> C::BITS) & M] / gamma, v.x, v.y);   // {two high parts, two low parts}
+        }
+        ent_s[e] = v;
+    }
+    sync();
+#pragma unroll 8
+    for (int e = threadIdx.x; e < C::NENT * LUT_COPIES; e += NT) lut[e] = ent_s[e / LUT_COPIES];
+    return gamma;
+}
+
+// A warp's state over its tiles: O^T fragments, running maxima of heads 2t, 2t + 1 and this thread's part of the sums.
+template <typename C>
+struct AttnAcc {
+    float o[C::NS][4], m_run[2], l_part[2];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int s = 0; s < C::NS; s++) o[s][0] = o[s][1] = o[s][2] = o[s][3] = 0.f;
+        m_run[0] = m_run[1] = -INFINITY;
+        l_part[0] = l_part[1] = 0.f;
+    }
+};
+// One warp's step over the KT keys t0 .. t0 + KT - 1 (those below k_end count) whose codes lie at the shared-memory addresses ka
+// and va.  nk, nv: norms times gamma of key `lane`.  q_a: this lane's query fragments where they stay in shared memory.
+template <typename C, int NQ>
+__device__ __forceinline__ void attn_tile(AttnAcc<C> &st, uint32_t ka, uint32_t va, uint32_t t0, uint32_t k_end, float nk, float nv,
+                                          const uint32_t (&bq)[NQ][2], const uint32_t (&bql)[NQ][2], uint32_t q_a, uint32_t lut_lane, int lane) {
+    constexpr int CB = C::CB, KT = C::KT, MT = C::MT, NS = C::NS, FB = C::FB;
+    const int g = lane >> 2, t = lane & 3;
+    float(&o)[NS][4] = st.o;
+    float(&m_run)[2] = st.m_run, (&l_part)[2] = st.l_part;
+    // ---- S^T[KT keys x 8 heads] ----
+    constexpr int KW = CB / 16;   // words of one key in this thread's quarter row
+    uint32_t kw[MT][2][KW];
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++) {
+        lds_words<KW>(ka + (uint32_t)(mt * 16 + g) * C::KRS + (uint32_t)t * (KW * 4), kw[mt][0]);
+        lds_words<KW>(ka + (uint32_t)(mt * 16 + g + 8) * C::KRS + (uint32_t)t * (KW * 4), kw[mt][1]);
+    }
+    float c[MT][2][4];   // chains: high and low query parts
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) c[mt][0][i] = c[mt][1][i] = 0.f;
+    auto qk_step = [&](auto S) {
+        constexpr int s = decltype(S)::value;
+        uint32_t b0, b1, l0, l1;
+        if constexpr (C::QSMEM) {
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(b0), "=r"(b1), "=r"(l0), "=r"(l1) : "r"(q_a + s * 512));
+        } else {
+            b0 = bq[s][0]; b1 = bq[s][1]; l0 = bql[s][0]; l1 = bql[s][1];
+        }
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) {
+            if constexpr (!C::HILO) {
+                const uint2 x = lds64(field_addr<FB, s * 8>(kw[mt][0], lut_lane)), y = lds64(field_addr<FB, s * 8>(kw[mt][1], lut_lane));
+                const uint32_t a[4] = {x.x, y.x, x.y, y.y};
+                mma16816(c[mt][0], a, b0, b1);
+                mma16816(c[mt][1], a, l0, l1);
+            } else {
+                const uint2 x0 = lds64(field_addr<FB, 2 * s * FB>(kw[mt][0], lut_lane)), x1 = lds64(field_addr<FB, (2 * s + 1) * FB>(kw[mt][0], lut_lane));
+                const uint2 y0 = lds64(field_addr<FB, 2 * s * FB>(kw[mt][1], lut_lane)), y1 = lds64(field_addr<FB, (2 * s + 1) * FB>(kw[mt][1], lut_lane));
+                const uint32_t ah[4] = {x0.x, y0.x, x1.x, y1.x}, al[4] = {x0.y, y0.y, x1.y, y1.y};
+                mma16816(c[mt][0], ah, b0, b1);
+                mma16816(c[mt][1], ah, l0, l1);
+                mma16816(c[mt][1], al, b0, b1);
+            }
+        }
+    };
+    static_for<NS>(qk_step);
+
+    // ---- online softmax: logits of keys 16 mt + g (row 0), + 8 (row 1) for heads 2t, 2t+1 ----
+    float sc[MT][2][2], tm[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++) {
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int key = 16 * mt + 8 * r + g;
+            const float kn = __shfl_sync(0xffffffffu, nk, key);
+            const bool valid = t0 + key < k_end;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                sc[mt][r][h] = valid ? (c[mt][0][2 * r + h] + c[mt][1][2 * r + h]) * kn : -INFINITY;
+                tm[h] = fmaxf(tm[h], sc[mt][r][h]);
+            }
+        }
+    }
+    float resc[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 4));
+        tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 8));
+        tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 16));
+        const float m_new = fmaxf(m_run[h], tm[h]);    // finite: key t0 is valid
+        resc[h] = soft_exp<C::HILO>(m_run[h] - m_new);
+        m_run[h] = m_new;
+        l_part[h] *= resc[h];
+    }
+    // P (times the value norms) into the B operand: (key g | g+8; heads 2t, 2t+1) -> (keys 2t, 2t+1 | +8; head g)
+    uint32_t bp[MT][2], bpl[MT][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++) {
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const float vn = __shfl_sync(0xffffffffu, nv, (KT == 32 ? 16 * mt : 0) + 8 * r + g);
+            const float p0 = soft_exp<C::HILO>(sc[mt][r][0] - m_run[0]), p1 = soft_exp<C::HILO>(sc[mt][r][1] - m_run[1]);
+            l_part[0] += p0;
+            l_part[1] += p1;
+            if constexpr (!C::HILO) {
+                bp[mt][r] = movmatrix_trans(pack_h2(p0 * vn, p1 * vn));
+            } else {
+                uint32_t hi, lo;
+                split_h2(p0 * vn, p1 * vn, hi, lo);
+                bp[mt][r] = movmatrix_trans(hi);
+                bpl[mt][r] = movmatrix_trans(lo);
+            }
+        }
+    }
+    if (__any_sync(0xffffffffu, resc[0] != 1.0f || resc[1] != 1.0f)) {   // the running max moved for some head
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            o[s][0] *= resc[0]; o[s][1] *= resc[1]; o[s][2] *= resc[0]; o[s][3] *= resc[1];
+        }
+    }
+
+    // ---- O^T[HD dims x 8 heads] += V^T . P.  MMA tile j has rows (g, g + 8) = dims (g HD/8 + 2j, + 1). ----
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++) {
+        constexpr int VW = CB % 32 == 0 ? CB / 32 : 2;   // words of one key in this thread's eighth row
+        uint32_t vw[4][VW];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint32_t row = va + (uint32_t)(16 * mt + 2 * t + (q & 1) + 8 * (q >> 1)) * C::VRS;
+            if constexpr (CB % 32 == 0) {
+                lds_words<VW>(row + (uint32_t)g * (VW * 4), vw[q]);
+            } else {   // 6-byte pieces (tq3 at head_dim 128): two aligned words, shifted into place
+                const uint32_t a = row + (uint32_t)g * 6u, sh = (a & 2u) * 8u;
+                uint32_t w[2];
+                asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(w[0]) : "r"(a & ~3u));
+                asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(w[1]) : "r"((a & ~3u) + 4u));
+                vw[q][0] = __funnelshift_r(w[0], w[1], sh);
+                vw[q][1] = w[1] >> sh;
+            }
+        }
+        auto pv_step = [&](auto U) {
+            constexpr int u = decltype(U)::value;
+            const uint2 e0 = lds64(field_addr<FB, u * FB>(vw[0], lut_lane)), e1 = lds64(field_addr<FB, u * FB>(vw[1], lut_lane));   // keys 2t, 2t+1
+            const uint2 e2 = lds64(field_addr<FB, u * FB>(vw[2], lut_lane)), e3 = lds64(field_addr<FB, u * FB>(vw[3], lut_lane));   // keys 2t+8, 2t+9
+            // .x: first two dims (tq2) / high parts; .y: next two dims / low parts
+            const uint32_t ax[4] = {__byte_perm(e0.x, e1.x, 0x5410), __byte_perm(e0.x, e1.x, 0x7632), __byte_perm(e2.x, e3.x, 0x5410),
+                                    __byte_perm(e2.x, e3.x, 0x7632)};
+            const uint32_t ay[4] = {__byte_perm(e0.y, e1.y, 0x5410), __byte_perm(e0.y, e1.y, 0x7632), __byte_perm(e2.y, e3.y, 0x5410),
+                                    __byte_perm(e2.y, e3.y, 0x7632)};
+            if constexpr (!C::HILO) {
+                mma16816(o[2 * u], ax, bp[mt][0], bp[mt][1]);
+                mma16816(o[2 * u + 1], ay, bp[mt][0], bp[mt][1]);
+            } else {
+                mma16816(o[u], ax, bp[mt][0], bp[mt][1]);
+                mma16816(o[u], ax, bpl[mt][0], bpl[mt][1]);
+                mma16816(o[u], ay, bp[mt][0], bp[mt][1]);
+            }
+        };
+        static_for<(C::HILO ? NS : NS / 2)>(pv_step);
+    }
+}
+
+}  // namespace

@@ -23,6 +23,7 @@
 
 #include "lc_internal.h"
 #include "attention_tq.h"
+#include "step_small.h"
 
 int lc_matmul_nt_tq2_0_grouped(lc_kernels *k, lc_batch *b, const lc_buf *input, int ng, const lc_buf *const *weights,
                                lc_buf *const *outputs, const uint32_t *ns, uint32_t m, uint32_t kk);
@@ -47,6 +48,7 @@ struct lc_model {
     lc_buf *levels = nullptr, *signs = nullptr, *ones = nullptr;
     lc_buf *x = nullptr, *x2 = nullptr, *normed = nullptr, *q = nullptr, *qfrag = nullptr, *kbuf = nullptr, *vbuf = nullptr,
            *attn = nullptr, *resid = nullptr, *gate = nullptr, *up = nullptr, *ffn = nullptr, *logits = nullptr;
+    lc_buf *step_mail = nullptr;   // exchange buffers of the one-launch form of small steps (step_small.cu); NULL: not used
     std::vector<lc_buf *> owned;
     // lane-group chains (see chain_count): side streams, their own kernels objects (split-K scratch is per object) and
     // the fork / join events
@@ -136,6 +138,13 @@ int lc_model_create(lc_ctx *ctx, lc_kernels *k, const lc_model_config *cfg, lc_m
     const char *qf_env = getenv("LOCAL_CUDA_QFRAG");
     if (!(qf_env && qf_env[0] == '0') && lc_qfrag_supported(c.head_dim, c.kv_bits, c.n_q_heads, c.n_kv_heads))
         pieces.push_back({n * qd * 4, &m->qfrag});
+    // LOCAL_CUDA_STEP_ONE=0 keeps the launch-by-launch form of steps of a few lanes (for A/B timing and tests)
+    const char *one_env = getenv("LOCAL_CUDA_STEP_ONE");
+    if (!(one_env && one_env[0] == '0') && lc_step_small_supported(k, c.hidden, c.inter, c.n_q_heads, c.n_kv_heads, c.head_dim, c.kv_bits, c.n_layers)) {
+        std::vector<uint32_t> window, rows;
+        for (const lc_model_layer &L : m->layers) window.push_back(L.window), rows.push_back(L.lane_rows);
+        pieces.push_back({lc_step_small_mail_bytes(k, c.hidden, c.inter, c.n_q_heads, c.n_kv_heads, c.n_layers, c.max_lanes, window.data(), rows.data()), &m->step_mail});
+    }
     if ((st = place(m, pieces)) != LC_OK) return fail(st);
     if ((st = lc_buf_upload(m->levels, 0, lv.data(), lv.size() * 4)) ||
         (st = lc_buf_upload(m->signs, 0, sg.data(), sg.size() * 4)) ||
@@ -312,6 +321,43 @@ static int run_layers(lc_model *m, lc_kernels *k, lc_batch *b, const lc_buf *pos
     return LC_OK;
 }
 
+// The layers as one launch, embedding and first norm included (step_small.cu).  -1: this step is not one for it.
+static int run_layers_small(lc_model *m, lc_batch *b, const lc_buf *tokens, const lc_buf *positions, uint32_t n) {
+    const lc_kernels *k = m->k;
+    if (!m->step_mail || n > LC_STEP_MAX_LANES || !m->qfrag) return -1;
+    if (!(k->batchm && k->smallm && k->mma && k->decode_mma && k->decode_tc) || k->small_m || k->kv_norm_mode) return -1;
+    const lc_model_config &c = m->cfg;
+    LcStepParams p = {};
+    for (size_t i = 0; i < m->layers.size(); i++) {
+        const lc_model_layer &L = m->layers[i];
+        auto w = [](const lc_buf *t) { return (const uint8_t *)t->dptr; };
+        auto h = [](const lc_buf *t) { return (const __half *)t->dptr; };
+        p.layer[i] = {w(L.wq), w(L.wk), w(L.wv), w(L.wo), w(L.wgate), w(L.wup), w(L.wdown),
+                      h(L.attn_norm), h(L.q_norm), h(L.k_norm), h(L.post_attn_norm), h(L.ffn_norm), h(L.post_ffn_norm),
+                      (uint8_t *)L.k_codes->dptr, (uint8_t *)L.v_codes->dptr, (__half *)L.k_norms->dptr, (__half *)L.v_norms->dptr,
+                      L.window, L.ring, L.lane_rows, 0, 0};
+    }
+    p.m = (int)n;
+    p.n_layers = (int)c.n_layers;
+    p.hidden = (int)c.hidden;
+    p.inter = (int)c.inter;
+    p.n_q = (int)c.n_q_heads;
+    p.n_kv = (int)c.n_kv_heads;
+    p.embed = (const uint8_t *)m->embed->dptr;
+    p.tokens = (const uint32_t *)tokens->dptr;
+    p.positions = (const uint32_t *)positions->dptr;
+    p.embed_scale = c.embed_scale;
+    p.eps = c.rms_eps;
+    p.theta = c.rope_theta;
+    p.softmax_scale = c.softmax_scale;
+    p.final_norm = (const __half *)m->final_norm->dptr;
+    p.levels = (const float *)m->levels->dptr;
+    p.signs = (const float *)m->signs->dptr;
+    p.normed = (__half *)m->normed->dptr;
+    p.mail = (uint8_t *)m->step_mail->dptr;
+    return lc_step_small_launch(m->k, b, p, c.kv_bits);
+}
+
 // How many independent lane groups ("chains") the layers of a step are issued as.  The per-layer kernels of a decode
 // step are short and strictly dependent, so one chain leaves most SMs idle most of the time; lanes are independent
 // between the embedding and the vocabulary projection, so two or four chains on forked streams fill the gaps (each
@@ -337,10 +383,16 @@ int lc_model_decode_batch_step_into(lc_model *m, lc_batch *b, const lc_buf *toke
     const uint32_t H = c.hidden, n = n_lanes;
     int st;
 #define STEP(call) do { if ((st = (call)) != LC_OK) return st; } while (0)
-    STEP(lc_embed_rows_q4_0_into(k, b, m->embed, tokens, m->x, n, H, c.vocab, c.embed_scale));
-    STEP(lc_rms_norm_into(k, b, m->x, m->layers[0].attn_norm, m->normed, H, n, c.rms_eps));
+    const int small = run_layers_small(m, b, tokens, positions, n);
+    if (small > 0) return small;
+    if (small < 0) {
+        STEP(lc_embed_rows_q4_0_into(k, b, m->embed, tokens, m->x, n, H, c.vocab, c.embed_scale));
+        STEP(lc_rms_norm_into(k, b, m->x, m->layers[0].attn_norm, m->normed, H, n, c.rms_eps));
+    }
     const uint32_t chains = chain_count(m, n);
-    if (chains <= 1) {
+    if (small == LC_OK) {
+        // (done)
+    } else if (chains <= 1) {
         STEP(run_layers(m, k, b, positions, 0, n));
     } else {
         // fork: chain 0 stays on the batch's stream, chains 1.. run on the model's side streams (captured into the same

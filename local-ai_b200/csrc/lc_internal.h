@@ -213,10 +213,13 @@ __device__ __forceinline__ void lc_order_end(uint32_t flags) {
 // to them, with one barrier in all instead of two per stage.  No thread may still be reading `sh` from earlier code
 // when the block enters (callers that used it since their last barrier place one), and callers that reuse `sh`
 // afterwards synchronise first.
-template <int P>
-__device__ __forceinline__ float lc_fwht_cross_warp(float v, float *sh, unsigned t) {
+struct lc_block_sync {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+template <int P, typename Sync = lc_block_sync>
+__device__ __forceinline__ float lc_fwht_cross_warp(float v, float *sh, unsigned t, Sync sync = {}) {
     sh[t] = v;
-    __syncthreads();
+    sync();
     float a[P];
 #pragma unroll
     for (int j = 0; j < P; j++) a[j] = sh[t ^ ((unsigned)j << 5)];

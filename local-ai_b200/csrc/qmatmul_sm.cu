@@ -20,7 +20,7 @@
 #include <stdlib.h>
 
 #include "lc_internal.h"
-#include "tcgen05_util.cuh"
+#include "qm_codes.cuh"
 
 namespace {
 
@@ -43,51 +43,10 @@ struct SmParams {
     uint32_t order;            // LcOrder::flags
 };
 
-// gelu_tanh(gate) * up with gate and up rounded to f16 first, as the separate projections would store them, and the
-// element-wise kernel's arithmetic (shaders/gelu.metal:23-37)
-__device__ __forceinline__ float geglu_f(float gate, float up) {
-    const float x = __half2float(__float2half_rn(gate)), u = __half2float(__float2half_rn(up));
-    float inner = 0.7978845608f * (x + 0.044715f * (x * x * x));
-    inner = fminf(fmaxf(inner, -10.0f), 10.0f);
-    return 0.5f * x * (1.0f + tanhf(inner)) * u;
-}
 __device__ __forceinline__ void sm_store(__half *p, float v) { *p = __float2half_rn(v); }
 __device__ __forceinline__ void sm_store(float *p, float v) { *p = v; }
 __device__ __forceinline__ void sm_store2(__half *p, float2 v) { *reinterpret_cast<__half2 *>(p) = __floats2half2_rn(v.x, v.y); }
 __device__ __forceinline__ void sm_store2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
-__device__ __forceinline__ void sm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// N consecutive 32-bit words at a 2-byte aligned shared-memory address, the bytes of each in the order 0, 2, 1, 3: a mask
-// then pairs neighbouring codes in the halves of a register.
-template <int N>
-__device__ __forceinline__ void lds_codes(uint32_t a, uint32_t (&w)[N]) {
-    const uint32_t sel = (a & 2u) ? 0x5342u : 0x3120u, base = a & ~3u;
-    uint32_t r[N + 1];
-#pragma unroll
-    for (int i = 0; i <= N; i++) r[i] = lds32(base + 4 * i);
-#pragma unroll
-    for (int i = 0; i < N; i++) w[i] = __byte_perm(r[i], r[i + 1], sel);
-}
-__device__ __forceinline__ uint32_t lds16(uint32_t a) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(v) : "r"(a));
-    return v;
-}
-
-// two codes, BITS wide at bit BITS * l of each half of w, as f16 (q - Z) 2^-9
-template <int BITS, int Z>
-__device__ __forceinline__ uint32_t codes_f16(uint32_t w, int l) {
-    constexpr uint32_t one = (1u << BITS) - 1u;
-    const uint32_t v = w & ((one | one << 16) << (BITS * l));      // q 2^(BITS l - 24)
-    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&v), __float2half2_rn((float)(1 << (15 - BITS * l))),
-                              __float2half2_rn(-(float)Z / 512.0f));
-    return *reinterpret_cast<const uint32_t *>(&r);
-}
-
 // NT8: batch columns / 8.  MTW: 16-row tiles of the CTA (every warp works on all of them).  SINGLE: a warp has at most one
 // step, so a tile's sums go to shared memory at once and four tiles fit the registers of two CTAs per SM.
 template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT, bool ORDERED>
@@ -133,11 +92,11 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
             mbar_arrive(bar);
         }
     }
-    // this lane's operand rows: 16 mt + g and + 8
+    // this lane's operand rows, 16 mt + g and + 8: where their blocks start in `raw`
     auto row_at = [&](int mt, int h, bool &ok_) -> uint32_t {
         const int r = mt * 16 + h * 8 + g, row = n0 + (GEGLU ? r % OROWS : r);
         ok_ = row < n_rows;
-        return smem_u32(raw) + (uint32_t)(r * p.raw_rs) + (uint32_t)(((size_t)row * rb) & 15);
+        return (uint32_t)(r * p.raw_rs) + (uint32_t)(((size_t)row * rb) & 15);
     };
     const int units = (p.K + SM_UNIT - 1) / SM_UNIT;
     lc_order_wait<ORDERED>(p.order);
@@ -182,10 +141,10 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const uint32_t a = ra[h] + (uint32_t)((u >> 1) * BB);
-                lds_codes<2>(a + (uint32_t)(32 * (u & 1) + 8 * t), cw[h]);
+                lds_codes<2>(raw, a + (uint32_t)(32 * (u & 1) + 8 * t), cw[h]);
                 sh[h][0] = cw[h][0] >> 8;
                 sh[h][1] = cw[h][1] >> 8;
-                d[h] = rok[h] ? __half2float(__ushort_as_half((unsigned short)lds16(a + 64u))) * 512.0f : 0.f;
+                d[h] = rok[h] ? __half2float(__ushort_as_half((unsigned short)lds16(raw, a + 64u))) * 512.0f : 0.f;
             }
             float c[2][NT8][4] = {};
 #pragma unroll
@@ -213,10 +172,10 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
                 for (int h = 0; h < 2; h++) {
                     const uint32_t a = ra[h] + (uint32_t)(blk * BB);
                     uint32_t w[1];
-                    lds_codes<1>(a + 2u + (uint32_t)(4 * t), w);
+                    lds_codes<1>(raw, a + 2u + (uint32_t)(4 * t), w);
                     cw[h] = w[0];
                     sh[h] = w[0] >> 8;
-                    d[h] = rok[h] ? __half2float(__ushort_as_half((unsigned short)lds16(a))) * 512.0f : 0.f;
+                    d[h] = rok[h] ? __half2float(__ushort_as_half((unsigned short)lds16(raw, a))) * 512.0f : 0.f;
                 }
 #pragma unroll
                 for (int nt = 0; nt < NT8; nt++) {

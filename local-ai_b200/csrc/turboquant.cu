@@ -16,6 +16,7 @@
 
 #include "lc_internal.h"
 #include "attention_tq.h"
+#include "tq_rows.cuh"
 
 namespace {
 
@@ -139,68 +140,6 @@ __global__ void encode_kv_kernel(const __half *__restrict__ input, const float *
                &norm_sh);
 }
 
-// Rotates x (HD / 32 consecutive dims per lane): Walsh-Hadamard butterflies in ascending stride, lower = a + b, upper = a - b.
-template <int DPL>
-__device__ __forceinline__ void fwht_warp_row(float (&x)[DPL], int lane) {
-#pragma unroll
-    for (int len = 1; len < DPL; len <<= 1)
-#pragma unroll
-        for (int i = 0; i < DPL; i++)
-            if (!(i & len)) {
-                const float a = x[i], b = x[i + len];
-                x[i] = __fadd_rn(a, b);
-                x[i + len] = __fsub_rn(a, b);
-            }
-#pragma unroll
-    for (int m = 1; m < 32; m <<= 1) {
-        const bool upper = lane & m;
-#pragma unroll
-        for (int i = 0; i < DPL; i++) {
-            const float o = __shfl_xor_sync(0xffffffffu, x[i], m);
-            x[i] = upper ? __fsub_rn(o, x[i]) : __fadd_rn(x[i], o);
-        }
-    }
-}
-// Encodes one row held by a warp, HD / 32 consecutive dims per lane, whose norm is known (TurboQuant::encode_into).
-template <int HD, int BITS>
-__device__ __forceinline__ void encode_warp_row(float (&x)[HD / 32], float norm, const float (&lv)[1 << BITS], const float (&sg)[HD / 32],
-                                                int lane, uint8_t *dst, __half *norm_out) {
-    constexpr int DPL = HD / 32, NLEV = 1 << BITS;
-    const float inv = norm > 0.f ? __fdiv_rn(1.0f, norm) : 0.f;
-#pragma unroll
-    for (int i = 0; i < DPL; i++) x[i] = __fmul_rn(norm > 0.f ? __fmul_rn(x[i], inv) : x[i], sg[i]);
-    fwht_warp_row<DPL>(x, lane);
-    const float inv_sqrt_d = __fdiv_rn(1.0f, __fsqrt_rn((float)HD));
-    unsigned long long word = 0;   // this lane's DPL codes, LSB first
-#pragma unroll
-    for (int i = 0; i < DPL; i++) {
-        const float v = __fmul_rn(x[i], inv_sqrt_d);
-        unsigned best = 0;
-        float bd = INFINITY;
-#pragma unroll
-        for (int j = 0; j < NLEV; j++) {
-            const float dd = fabsf(__fsub_rn(v, lv[j]));
-            if (dd < bd) { bd = dd; best = (unsigned)j; }
-        }
-        word |= (unsigned long long)best << (BITS * i);
-    }
-    constexpr int LB = DPL * BITS;   // bits of one lane: 8 .. 64, or 12 (tq3 at head_dim 128)
-    if constexpr (LB == 12) {        // two lanes share three bytes
-        const unsigned w = (unsigned)word | (__shfl_down_sync(0xffffffffu, (unsigned)word, 1) << 12);
-        if (!(lane & 1)) {
-            dst += (lane >> 1) * 3;
-            dst[0] = (uint8_t)w;
-            dst[1] = (uint8_t)(w >> 8);
-            dst[2] = (uint8_t)(w >> 16);
-        }
-    } else {
-        dst += lane * (LB / 8);
-#pragma unroll
-        for (int i = 0; i < LB / 8; i++) dst[i] = (uint8_t)(word >> (8 * i));
-    }
-    if (lane == 0) *norm_out = __float2half_rn(norm);
-}
-
 // The same rows for head_dim 128 / 256 / 512 and the sequential norm, a warp per row and eight rows per CTA: what one row
 // takes is the dependent chain of the norm's head_dim additions (about a microsecond at 256), so eight of them run side
 // by side in the lanes of one warp, and the rest of a row needs no further barrier.  grid.y = 1 or 2: the K rows and the V
@@ -249,16 +188,7 @@ __global__ void __launch_bounds__(ENC_ROWS * 32) encode_rows_kernel(const Encode
         *reinterpret_cast<float4 *>(&sq[warp][DPL * lane + i]) =
             make_float4(__fmul_rn(x[i], x[i]), __fmul_rn(x[i + 1], x[i + 1]), __fmul_rn(x[i + 2], x[i + 2]), __fmul_rn(x[i + 3], x[i + 3]));
     __syncthreads();
-    if (warp == 0 && lane < ENC_ROWS) {   // the reference's sequential f32 sum, in index order
-        const float4 *r4 = reinterpret_cast<const float4 *>(sq[lane]);
-        float s = 0.f;
-#pragma unroll 8
-        for (int i = 0; i < HD / 4; i++) {
-            const float4 a = r4[i];
-            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a.x), a.y), a.z), a.w);
-        }
-        norm_s[lane] = __fsqrt_rn(s);
-    }
+    if (warp == 0 && lane < ENC_ROWS) norm_s[lane] = sequential_norm<HD>(sq[lane]);
     __syncthreads();
     if (!live) return;
     size_t slot;
@@ -274,7 +204,8 @@ __global__ void __launch_bounds__(ENC_ROWS * 32) encode_rows_kernel(const Encode
         const unsigned logical = p.position + row;
         slot = (size_t)(p.ring ? logical % p.ring : logical) * p.n_kv + head;
     }
-    encode_warp_row<HD, BITS>(x, norm_s[warp], lv, sg, lane, p.packed[y] + slot * (HD * BITS / 8), p.norms[y] + slot);
+    store_warp_codes<HD, BITS>(encode_warp_row<HD, BITS>(x, norm_s[warp], lv, sg, lane), lane, p.packed[y] + slot * (HD * BITS / 8));
+    if (lane == 0) *(p.norms[y] + slot) = __float2half_rn(norm_s[warp]);
 }
 template <int HD, bool BATCHED>
 cudaError_t launch_encode_rows(lc_batch *b, const EncodeRows &p, unsigned tensors, unsigned bits) {
@@ -461,36 +392,8 @@ __global__ void __launch_bounds__(ENC_ROWS * 32) kv_write_rows_kernel(const __gr
             x[2 * i + 1] = f.y;
         }
     }
-    // mean square: 32-dim groups as shuffle trees (strides 16, 8 across lanes; 4, 2, 1 inside), then the groups in order
-    float tot = 0.f;
-    {
-        float s[DPL];
-#pragma unroll
-        for (int e = 0; e < DPL; e++) {
-            s[e] = x[e] * x[e];
-            s[e] += __shfl_xor_sync(0xffffffffu, s[e], 2);
-            s[e] += __shfl_xor_sync(0xffffffffu, s[e], 1);
-        }
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-            for (int e = 0; e < o; e++) s[e] += s[e + o];
-#pragma unroll
-        for (int g = 0; g < 8; g++) tot += __shfl_sync(0xffffffffu, s[0], 4 * g);
-    }
-    const float rms = rsqrtf(tot / (float)HD + p.eps);
-#pragma unroll
-    for (int e = 0; e < DPL; e++) x[e] = __half2float(__float2half_rn(x[e] * rms * w[e]));
-    if (role != 2) {
-#pragma unroll
-        for (int e = 0; e < DPL; e++) {
-            const float other = __shfl_xor_sync(0xffffffffu, x[e], 16);
-            const bool low = lane < 16;
-            const float x0 = low ? x[e] : other, x1 = low ? other : x[e];
-            const float v = low ? x0 * cs[e] - x1 * sn[e] : x0 * sn[e] + x1 * cs[e];
-            if (((unsigned)(DPL * lane + e) & (HD / 2 - 1)) < angles) x[e] = __half2float(__float2half_rn(v));
-        }
-    }
+    warp_head_norm(x, w, p.eps);
+    if (role != 2) warp_rope(x, cs, sn, angles, lane);
     if (role == 0) {
         if (!live) return;
         uint4 raw;
@@ -499,23 +402,11 @@ __global__ void __launch_bounds__(ENC_ROWS * 32) kv_write_rows_kernel(const __gr
         for (int i = 0; i < DPL / 2; i++) h[i] = __floats2half2_rn(x[2 * i], x[2 * i + 1]);
         *reinterpret_cast<uint4 *>(qrow) = raw;
         if (p.qfrag) {
-            // the tensor-core attention kernel's first steps (see kv_write_kernel): sign, transform, scale, split
-#pragma unroll
-            for (int e = 0; e < DPL; e++) x[e] = __fmul_rn(x[e], sg[e]);
-            fwht_warp_row<DPL>(x, lane);
-            const float f = __fdiv_rn(p.q_scale, __fsqrt_rn((float)HD));
-            unsigned hi[DPL / 2], lo[DPL / 2];
-#pragma unroll
-            for (int i = 0; i < DPL / 2; i++) {
-                const float v0 = __fmul_rn(x[2 * i], f), v1 = __fmul_rn(x[2 * i + 1], f);
-                const __half2 a = __floats2half2_rn(v0, v1);
-                const __half2 b = __floats2half2_rn(__fsub_rn(v0, __low2float(a)), __fsub_rn(v1, __high2float(a)));
-                hi[i] = *reinterpret_cast<const unsigned *>(&a);
-                lo[i] = *reinterpret_cast<const unsigned *>(&b);
-            }
+            uint4 f[2];
+            warp_query_frag(x, sg, p.q_scale, lane, f);
             uint4 *dst = p.qfrag + ((size_t)row * (p.n_q >> 3) + (head >> 3)) * 512 + 4 * (head & 7) + (lane >> 3);
-            dst[((lane & 7) * 2) * 32] = make_uint4(hi[0], hi[1], lo[0], lo[1]);
-            dst[((lane & 7) * 2 + 1) * 32] = make_uint4(hi[2], hi[3], lo[2], lo[3]);
+            dst[((lane & 7) * 2) * 32] = f[0];
+            dst[((lane & 7) * 2 + 1) * 32] = f[1];
         }
         return;
     }
@@ -524,16 +415,7 @@ __global__ void __launch_bounds__(ENC_ROWS * 32) kv_write_rows_kernel(const __gr
         *reinterpret_cast<float4 *>(&sq[warp][DPL * lane + i]) =
             make_float4(__fmul_rn(x[i], x[i]), __fmul_rn(x[i + 1], x[i + 1]), __fmul_rn(x[i + 2], x[i + 2]), __fmul_rn(x[i + 3], x[i + 3]));
     __syncthreads();
-    if (warp == 0 && lane < ENC_ROWS) {   // the reference's sequential f32 sum, in index order
-        const float4 *r4 = reinterpret_cast<const float4 *>(sq[lane]);
-        float s = 0.f;
-#pragma unroll 8
-        for (int i = 0; i < HD / 4; i++) {
-            const float4 a = r4[i];
-            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a.x), a.y), a.z), a.w);
-        }
-        norm_s[lane] = __fsqrt_rn(s);
-    }
+    if (warp == 0 && lane < ENC_ROWS) norm_s[lane] = sequential_norm<HD>(sq[lane]);
     __syncthreads();
     if (!live) return;
     const unsigned ppos = p.ring ? pos % p.ring : pos;
@@ -542,7 +424,8 @@ __global__ void __launch_bounds__(ENC_ROWS * 32) kv_write_rows_kernel(const __gr
         return;
     }
     const size_t slot = ((size_t)row * p.lane_capacity + ppos) * p.n_kv + head;
-    encode_warp_row<HD, BITS>(x, norm_s[warp], lv, sg, lane, p.packed[role - 1] + slot * (HD * BITS / 8), p.norms[role - 1] + slot);
+    store_warp_codes<HD, BITS>(encode_warp_row<HD, BITS>(x, norm_s[warp], lv, sg, lane), lane, p.packed[role - 1] + slot * (HD * BITS / 8));
+    if (lane == 0) *(p.norms[role - 1] + slot) = __float2half_rn(norm_s[warp]);
 }
 
 // dequantize_kv.metal:132-189. grid = n_kv * (num_tokens - token_start).
