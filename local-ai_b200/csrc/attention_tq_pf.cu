@@ -57,11 +57,6 @@ __device__ __forceinline__ void umma_ss(uint32_t d, uint64_t a, uint64_t b, uint
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-    uint32_t on;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(on));
-    return on != 0;
-}
 // Operand descriptor of a tile whose rows (64 elements, 128-byte swizzle) run along the MMA's K: 1024 bytes between groups of
 // eight rows, `block` bytes between blocks of 64 elements of the other dimension.
 __device__ __forceinline__ uint64_t make_desc_mn(uint32_t saddr, uint32_t block) {
@@ -215,16 +210,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
     lc_pdl_wait();
 
     // ---- query rows: sign, transform, scale, split into two f16 operand tiles (K-major, 128-byte swizzle) ----
-    auto warp_wait = [&](uint32_t bar, uint32_t parity) -> bool {
-        uint32_t ok = 1;
-        if (lane == 0) ok = *abort_flag == 0u && mbar_wait(bar, parity, p.wait_limit) ? 1u : 0u;
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok || *abort_flag) {
-            *abort_flag = 1;
-            return false;
-        }
-        return true;
-    };
+    auto warp_wait = [&](uint32_t bar, uint32_t parity) -> bool { return mbar_wait_warp(bar, parity, p.wait_limit, abort_flag); };
     // The transform of 128 rows by shuffles took 13 of this kernel's 61 thousand cycles (16 rows over 2000 keys 21.0 -> 19.1 us
     // without it, 256 over 4096 39.4 -> 37.8).  With signs of +-1 the signed row is an f16 still, exactly, and 64 dims of it at a
     // time go through the tensor cores: D = A . H64 (Sylvester's matrix, its rows in the order of the operand tiles), then butterflies over the 64-dim blocks when a row is read back.

@@ -189,13 +189,7 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
             }
             if (!counted) mbar_arrive(bar);
         }
-        bool dead = false;
-        {
-            uint32_t ok = 1;
-            if (lane == 0) ok = mbar_wait(smem_u32(raw_full), 0u, p.wait_limit) ? 1u : 0u;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) { *abort_flag = 1; dead = true; }
-        }
+        bool dead = !mbar_wait_warp(smem_u32(raw_full), 0u, p.wait_limit, abort_flag);
         // This thread's share of every step: operand row 32 (warp & 3) + lane and, of each 32-byte half h of the row's
         // block, the 16 code bytes 16 bq .. + 15 (bq = warp >> 2): 128 weights.
         const int r = 32 * (warp & 3) + lane, bq = warp >> 2;
@@ -235,11 +229,8 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
                     }
                 }
                 if (h == 0 && i >= SA) {   // the MMAs that read this slot SA steps ago have completed
-                    uint32_t ok = 1;
                     const int u = i - SA;
-                    if (lane == 0) ok = mbar_wait(smem_u32(&step_done[u % NBAR]), (uint32_t)((u / NBAR) & 1), p.wait_limit) ? 1u : 0u;
-                    ok = __shfl_sync(0xffffffffu, ok, 0);
-                    if (!ok || *abort_flag) { *abort_flag = 1; dead = true; break; }
+                    if (!mbar_wait_warp(smem_u32(&step_done[u % NBAR]), (uint32_t)((u / NBAR) & 1), p.wait_limit, abort_flag)) { dead = true; break; }
                     tc_fence_after();
                 }
 #pragma unroll

@@ -67,18 +67,6 @@ __device__ __forceinline__ void store_c4(__half *p, float4 v) {
 }
 __device__ __forceinline__ void store_c4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
 
-// whole-warp bounded wait: lane 0 polls
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, uint32_t limit, int lane, volatile uint32_t *abort_flag) {
-    uint32_t ok = 1;
-    if (lane == 0) ok = mbar_wait(bar, parity, limit) ? 1u : 0u;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    if (!ok || *abort_flag) {
-        *abort_flag = 1;
-        return false;
-    }
-    return true;
-}
-
 template <int FMT, typename OutT, bool ORDERED>
 __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant__ TclParams p, const __grid_constant__ CUtensorMap x_map) {
     using F = TclFmt<FMT>;
@@ -139,7 +127,7 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
         const uint32_t ta = tmem_base + ((uint32_t)(32 * (wq & 3)) << 16) + (uint32_t)(A_BASE + group * A_COLS);
         for (int i = group; i < n_steps; i += GROUPS) {
             const int rs = i % RAW_SLOTS;
-            if (!warp_wait(smem_u32(&raw_full[rs]), (uint32_t)((i / RAW_SLOTS) & 1), p.wait_limit, lane, abort_flag)) break;
+            if (!mbar_wait_warp(smem_u32(&raw_full[rs]), (uint32_t)((i / RAW_SLOTS) & 1), p.wait_limit, abort_flag)) break;
             const size_t g0 = (size_t)row * rb + (size_t)(s0 + i) * STEP_BYTES;
             const uint32_t ra = smem_u32(raw + rs * RAW_SLOT + r * RAW_RS) + (uint32_t)(g0 & 15);
             // sixteen code bytes, 2-byte aligned: five aligned words, funnel-shifted into place
@@ -160,7 +148,7 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
             auto slot_free = [&]() -> bool {
                 if (i < GROUPS) return true;
                 const int u = i - GROUPS;
-                if (!warp_wait(smem_u32(&step_done[u % NBAR]), (uint32_t)((u / NBAR) & 1), p.wait_limit, lane, abort_flag)) return false;
+                if (!mbar_wait_warp(smem_u32(&step_done[u % NBAR]), (uint32_t)((u / NBAR) & 1), p.wait_limit, abort_flag)) return false;
                 tc_fence_after();
                 return true;
             };
@@ -239,7 +227,7 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
         }
         for (int i = 0; i < n_steps; i++) {
             const int rs = i % RAW_SLOTS;
-            if (i >= RAW_SLOTS && !warp_wait(smem_u32(&raw_empty[rs]), (uint32_t)((i / RAW_SLOTS - 1) & 1), p.wait_limit, lane, abort_flag)) break;
+            if (i >= RAW_SLOTS && !mbar_wait_warp(smem_u32(&raw_empty[rs]), (uint32_t)((i / RAW_SLOTS - 1) & 1), p.wait_limit, abort_flag)) break;
 #pragma unroll
             for (int j = 0; j < PER_LANE; j++) {
                 const int idx = (j * NRAW + w) * 32 + lane, pc = idx % PIECES;

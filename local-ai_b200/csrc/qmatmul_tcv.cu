@@ -61,12 +61,6 @@ struct TcvParams {
     uint32_t extra_arrivals;   // 0; 1 in the expiry self-test: the readiness barriers then expect an arrival nobody makes
 };
 
-// bounded wait by lane 0, result shared with the warp
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, uint32_t limit, int lane) {
-    uint32_t ok = 1;
-    if (lane == 0) ok = mbar_wait(bar, parity, limit) ? 1u : 0u;
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
-}
 __device__ __forceinline__ uint32_t lds16(uint32_t addr) {
     uint32_t v;
     asm volatile("ld.shared.u16 %0, [%1];\n" : "=r"(v) : "r"(addr));
@@ -138,7 +132,7 @@ qgemm_tcv_kernel(const __grid_constant__ TcvParams p, const __grid_constant__ CU
         bool dead = false;
         for (int g = grp; g < total && !dead; g += 2) {
             const int cg = g >> 1, rs = cg % V_RS;
-            if (!warp_wait(smem_u32(&raw_full[rs]), (uint32_t)((cg / V_RS) & 1), p.wait_limit, lane) || *abort_flag) { *abort_flag = 1; dead = true; break; }
+            if (!mbar_wait_warp(smem_u32(&raw_full[rs]), (uint32_t)((cg / V_RS) & 1), p.wait_limit, abort_flag)) { dead = true; break; }
 #pragma unroll
             for (int bi = 0; bi < 2; bi++) {
                 // block 4 grp + 2 bq + bi of the box: f16 scale, then 16 bytes of nibbles (2-byte aligned)
@@ -169,7 +163,7 @@ qgemm_tcv_kernel(const __grid_constant__ TcvParams p, const __grid_constant__ CU
                 if (bi == 0 && g >= V_SA) {
                     // the first block is in registers; the stores have to wait for the MMAs that read this slot two steps ago
                     const int u = g - V_SA;
-                    if (!warp_wait(smem_u32(&step_done[u % V_NBAR]), (uint32_t)((u / V_NBAR) & 1), p.wait_limit, lane)) { *abort_flag = 1; dead = true; break; }
+                    if (!mbar_wait_warp(smem_u32(&step_done[u % V_NBAR]), (uint32_t)((u / V_NBAR) & 1), p.wait_limit, abort_flag)) { dead = true; break; }
                     tc_fence_after();
                 }
                 if (bi == 1) {   // every lane of this warp has read its bytes of the box
@@ -271,7 +265,7 @@ qgemm_tcv_kernel(const __grid_constant__ TcvParams p, const __grid_constant__ CU
         const int qtr = warp & 3;
         bool dead = false;
         for (int j = 0; j < my_tiles && !dead; j++) {
-            if (!warp_wait(smem_u32(acc_full), (uint32_t)(j & 1), p.wait_limit, lane) || *abort_flag) { dead = true; break; }
+            if (!mbar_wait_warp(smem_u32(acc_full), (uint32_t)(j & 1), p.wait_limit, abort_flag)) { dead = true; break; }
             tc_fence_after();
             // The sums go to shared memory first (a warp writes 32 consecutive floats per batch column), so that the
             // accumulators are handed back after the loads alone; the stores to global memory, 16 bytes per thread,
