@@ -265,40 +265,41 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
         }
         __syncwarp();
     } else {
-        // =========================== MMA issue (four warps, one thread each) ===========================
+        // =========================== MMA issue (four warps) ===========================
         // Issuer iw owns TMEM accumulator iw (columns 64 iw ..) and takes K = 16 slice iw of each of the four 64-k tiles of
         // every step: weights from tensor memory (eight columns per slice), activations from shared memory.
-        // One thread per issuer runs the loop: every instruction in it (barrier test, MMA, commit) costs its thread on
-        // the order of a hundred cycles or more, so nothing warp-wide is added.
+        // The whole warp runs the loop, so that descriptors stay in uniform registers, and one lane issues: an MMA costs its warp 33
+        // cycles, a loop of one lane 46 and more around its waits (a step of 64 lanes at 2048 keys 1887 -> 1830 us).
         const int iw = warp - NDQ - 1;
-        if (lane == 0) {
-            const uint64_t bdesc0 = make_desc(smem_u32(b_s) + (uint32_t)(iw * 32));
-            const uint32_t tmem_acc = tmem_base + (uint32_t)(iw * NB);
-            const uint32_t ta0 = tmem_base + (uint32_t)(A_BASE + 8 * iw);
-            const uint32_t af0 = smem_u32(a_full), bf0 = smem_u32(b_full), sd0 = smem_u32(step_done);
-            bool dead = false;
-            // counters instead of divisions by the (run-time) ring depth: this thread's loop is the pace of the CTA
-            uint32_t sbi = 0, sbp = 0;   // activation slot of step i and the parity of its barrier's phase
-            for (int i = 0; i < total_steps; i++) {
-                const uint32_t sa = (uint32_t)i & (SA - 1);
-                if (!mbar_wait(af0 + 8u * sa, ((uint32_t)i / SA) & 1u, p.wait_limit) || !mbar_wait(bf0 + 8u * sbi, sbp, p.wait_limit)) { dead = true; break; }
-                tc_fence_after();
-                const uint32_t ta = ta0 + sa * (uint32_t)A_COLS;
-                const uint64_t bd = bdesc0 + (uint64_t)((sbi * (uint32_t)B_SLOT) >> 4);
+        const bool leader = elect_one();
+        const uint64_t bdesc0 = make_desc(smem_u32(b_s) + (uint32_t)(iw * 32));
+        const uint32_t tmem_acc = tmem_base + (uint32_t)(iw * NB);
+        const uint32_t ta0 = tmem_base + (uint32_t)(A_BASE + 8 * iw);
+        const uint32_t af0 = smem_u32(a_full), bf0 = smem_u32(b_full), sd0 = smem_u32(step_done);
+        bool dead = false;
+        // counters instead of divisions by the (run-time) ring depth: this thread's loop is the pace of the CTA
+        uint32_t sbi = 0, sbp = 0;   // activation slot of step i and the parity of its barrier's phase
+        for (int i = 0; i < total_steps; i++) {
+            const uint32_t sa = (uint32_t)i & (SA - 1);
+            if (!mbar_wait_warp(af0 + 8u * sa, ((uint32_t)i / SA) & 1u, p.wait_limit, abort_flag) || !mbar_wait_warp(bf0 + 8u * sbi, sbp, p.wait_limit, abort_flag)) { dead = true; break; }
+            tc_fence_after();
+            const uint32_t ta = ta0 + sa * (uint32_t)A_COLS;
+            const uint64_t bd = bdesc0 + (uint64_t)((sbi * (uint32_t)B_SLOT) >> 4);
+            if (leader) {
 #pragma unroll
                 for (int lp = 0; lp < STEP_TILES; lp++)
                     umma_f16_ta(tmem_acc, ta + (uint32_t)(32 * lp), bd + (uint64_t)((uint32_t)(lp * B_TILE) >> 4), idesc, (i > 0 || lp > 0) ? 1u : 0u);
                 umma_commit(sd0 + 8u * ((uint32_t)i & (NBAR - 1)));
-                if (++sbi == (uint32_t)SB) { sbi = 0; sbp ^= 1u; }
             }
-            // drain: the last step's barrier completes when all four issuers' MMAs are done
-            if (!dead && total_steps > 0) {
-                const int last = total_steps - 1;
-                dead = !mbar_wait(smem_u32(&step_done[last % NBAR]), (uint32_t)((last / NBAR) & 1), p.wait_limit);
-            }
-            if (dead) *abort_flag = 1;
+            __syncwarp();
+            if (++sbi == (uint32_t)SB) { sbi = 0; sbp ^= 1u; }
         }
-        __syncwarp();
+        // drain: the last step's barrier completes when all four issuers' MMAs are done
+        if (!dead && total_steps > 0) {
+            const int last = total_steps - 1;
+            dead = !mbar_wait_warp(smem_u32(&step_done[last % NBAR]), (uint32_t)((last / NBAR) & 1), p.wait_limit, abort_flag);
+        }
+        if (dead) *abort_flag = 1;
     }
     tc_fence_before();
     __syncthreads();
