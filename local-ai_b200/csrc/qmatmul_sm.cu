@@ -47,6 +47,29 @@ __device__ __forceinline__ void sm_store(__half *p, float v) { *p = __float2half
 __device__ __forceinline__ void sm_store(float *p, float v) { *p = v; }
 __device__ __forceinline__ void sm_store2(__half *p, float2 v) { *reinterpret_cast<__half2 *>(p) = __floats2half2_rn(v.x, v.y); }
 __device__ __forceinline__ void sm_store2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
+__device__ __forceinline__ void sm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// N consecutive 32-bit words at a 2-byte aligned shared-memory address, the bytes of each in the order 0, 2, 1, 3: a mask
+// then pairs neighbouring codes in the halves of a register.
+template <int N>
+__device__ __forceinline__ void lds_codes(uint32_t a, uint32_t (&w)[N]) {
+    const uint32_t sel = (a & 2u) ? 0x5342u : 0x3120u, base = a & ~3u;
+    uint32_t r[N + 1];
+#pragma unroll
+    for (int i = 0; i <= N; i++) r[i] = lds32(base + 4 * i);
+#pragma unroll
+    for (int i = 0; i < N; i++) w[i] = __byte_perm(r[i], r[i + 1], sel);
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t a) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(v) : "r"(a));
+    return v;
+}
+
 // NT8: batch columns / 8.  MTW: 16-row tiles of the CTA (every warp works on all of them).  SINGLE: a warp has at most one
 // step, so a tile's sums go to shared memory at once and four tiles fit the registers of two CTAs per SM.
 template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT, bool ORDERED>
@@ -92,11 +115,11 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
             mbar_arrive(bar);
         }
     }
-    // this lane's operand rows, 16 mt + g and + 8: where their blocks start in `raw`
+    // this lane's operand rows: 16 mt + g and + 8
     auto row_at = [&](int mt, int h, bool &ok_) -> uint32_t {
         const int r = mt * 16 + h * 8 + g, row = n0 + (GEGLU ? r % OROWS : r);
         ok_ = row < n_rows;
-        return (uint32_t)(r * p.raw_rs) + (uint32_t)(((size_t)row * rb) & 15);
+        return smem_u32(raw) + (uint32_t)(r * p.raw_rs) + (uint32_t)(((size_t)row * rb) & 15);
     };
     const int units = (p.K + SM_UNIT - 1) / SM_UNIT;
     lc_order_wait<ORDERED>(p.order);
@@ -141,10 +164,10 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const uint32_t a = ra[h] + (uint32_t)((u >> 1) * BB);
-                lds_codes<2>(raw, a + (uint32_t)(32 * (u & 1) + 8 * t), cw[h]);
+                lds_codes<2>(a + (uint32_t)(32 * (u & 1) + 8 * t), cw[h]);
                 sh[h][0] = cw[h][0] >> 8;
                 sh[h][1] = cw[h][1] >> 8;
-                d[h] = rok[h] ? __half2float(__ushort_as_half((unsigned short)lds16(raw, a + 64u))) * 512.0f : 0.f;
+                d[h] = rok[h] ? __half2float(__ushort_as_half((unsigned short)lds16(a + 64u))) * 512.0f : 0.f;
             }
             float c[2][NT8][4] = {};
 #pragma unroll
@@ -172,10 +195,10 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
                 for (int h = 0; h < 2; h++) {
                     const uint32_t a = ra[h] + (uint32_t)(blk * BB);
                     uint32_t w[1];
-                    lds_codes<1>(raw, a + 2u + (uint32_t)(4 * t), w);
+                    lds_codes<1>(a + 2u + (uint32_t)(4 * t), w);
                     cw[h] = w[0];
                     sh[h] = w[0] >> 8;
-                    d[h] = rok[h] ? __half2float(__ushort_as_half((unsigned short)lds16(raw, a))) * 512.0f : 0.f;
+                    d[h] = rok[h] ? __half2float(__ushort_as_half((unsigned short)lds16(a))) * 512.0f : 0.f;
                 }
 #pragma unroll
                 for (int nt = 0; nt < NT8; nt++) {

@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(NT, 1) qgemv_mma_stream_kernel(const __grid_co
     __syncthreads();          // the activations have landed, the barriers are ready
     bool alive = true;   // no wait of this warp has run out
     auto warp_wait = [&](uint32_t bar, uint32_t parity) -> bool {
-        if (alive && !__all_sync(0xffffffffu, mbar_wait(bar, parity, STREAM_WAIT_LIMIT))) {
+        if (alive && !mbar_wait_warp(bar, parity, STREAM_WAIT_LIMIT)) {
             alive = false;
             *abort_flag = 1;
         }

@@ -83,6 +83,26 @@ __device__ __forceinline__ uint4 gather8(float v) {
     return make_uint4(w, __shfl_down_sync(0xffffffffu, w, 2), __shfl_down_sync(0xffffffffu, w, 4), __shfl_down_sync(0xffffffffu, w, 6));
 }
 
+// (Neither the MMA nor the loads are volatile: the compiler overlaps the steps of an unrolled loop.)
+__device__ __forceinline__ void sm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// N consecutive 32-bit words at byte `at` (even) of a 4-byte aligned array in shared memory, the bytes of each in the order 0, 2, 1, 3: a
+// mask then pairs neighbouring codes in the halves of a register.
+template <int N>
+__device__ __forceinline__ void lds_codes(const uint8_t *smem, uint32_t at, uint32_t (&w)[N]) {
+    const uint32_t sel = (at & 2u) ? 0x5342u : 0x3120u;
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(smem + (at & ~3u));
+    uint32_t r[N + 1];
+#pragma unroll
+    for (int i = 0; i <= N; i++) r[i] = src[i];
+#pragma unroll
+    for (int i = 0; i < N; i++) w[i] = __byte_perm(r[i], r[i + 1], sel);
+}
+__device__ __forceinline__ uint32_t lds16(const uint8_t *smem, uint32_t at) { return *reinterpret_cast<const uint16_t *>(smem + at); }
+
 // acc += a step's product: 16 weight rows (a: byte of this lane's row g of the tile in w, rb8: eight rows on) times 128 k (unit u) of
 // the activations, x: this lane's k = 8t .. + 7 of column g, 32 apart.
 __device__ __forceinline__ void step_mma(float (&acc)[4], const uint8_t *w, uint32_t a, uint32_t rb8, int u, int t, const uint4 *x, bool col) {
@@ -287,7 +307,7 @@ __global__ void __launch_bounds__(ST_NT + 32, 1) step_layers_kernel(const __grid
         for (int h = 0;; h++) {
             const int ffn = h & 1, n = h < halves ? an[ffn] : 0, rows = ffn ? 8 : 16, pieces = ffn ? 2 * n : n;
             const LcStepLayer &L = layer_s[(h >> 1) % 3], &before = layer_s[((h >> 1) + 2) % 3];
-            if (h > 0 && !__all_sync(0xffffffffu, mbar_wait(free_a, (uint32_t)(h - 1) & 1u, p.wait_limit))) break;   // (expired)
+            if (h > 0 && !mbar_wait_warp(free_a, (uint32_t)(h - 1) & 1u, p.wait_limit)) break;   // (expired)
             if (lane == 0) mbar_arrive_expect_tx(bar_a, (uint32_t)(n * 16 * rb_h + (h > 0 ? 4 : 2) * H));
             __syncwarp();
             const uint32_t dst = smem_u32(wa_s);
@@ -314,7 +334,7 @@ __global__ void __launch_bounds__(ST_NT + 32, 1) step_layers_kernel(const __grid
             }
             __syncwarp();
             if (h < halves && bn > 0) {
-                if (h > 0 && !__all_sync(0xffffffffu, mbar_wait(free_b, (uint32_t)(h - 1) & 1u, p.wait_limit))) break;   // (expired)
+                if (h > 0 && !mbar_wait_warp(free_b, (uint32_t)(h - 1) & 1u, p.wait_limit)) break;   // (expired)
                 if (lane == 0) {
                     const uint32_t bytes = (uint32_t)(16 * (ffn ? rb_i : rb_q));
                     mbar_arrive_expect_tx(bar_b, bytes);
@@ -328,7 +348,7 @@ __global__ void __launch_bounds__(ST_NT + 32, 1) step_layers_kernel(const __grid
         tc_wait_expired(p.status, LC_DEV_STATUS_WAIT_EXPIRED, lane);
         return;
     }
-    auto weights = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.wait_limit)); };
+    auto weights = [&](uint32_t bar, uint32_t parity) -> bool { return mbar_wait_warp(bar, parity, p.wait_limit); };
     auto here = [&](const uint4 &v) -> bool { return v.x != 0xffffffffu && !p.never; };
 
     // ---- once: table of levels, signs, rotations of every lane's position, embedding rows ----

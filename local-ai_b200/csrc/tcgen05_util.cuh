@@ -63,6 +63,22 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t addr, uint32_t parity, u
     *abort_flag = 1;
     return false;
 }
+// The same without roles that may give up.  (Not for the small-batch matmul: one wait by all twelve warps at once, where the weights may
+// still be on their way, cost a step of eight lanes 5 %.)
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t addr, uint32_t parity, uint32_t limit) {
+    for (uint32_t i = 0; i < limit; i++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(addr), "r"(parity)
+            : "memory");
+        if (__all_sync(0xffffffffu, ok)) return true;
+    }
+    return false;
+}
 __device__ __forceinline__ bool elect_one() {
     uint32_t on;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(on));
