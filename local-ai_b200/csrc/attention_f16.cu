@@ -10,6 +10,7 @@
 #include <math.h>
 
 #include "lc_internal.h"
+#include "split_merge.cuh"
 
 namespace {
 
@@ -367,6 +368,30 @@ f16_attn_reduce_kernel(const float *__restrict__ pmax, const float *__restrict__
     }
 }
 
+// The same with a cluster of CTAs per head (split_merge.cuh): many splits, few heads.  8191 keys, 64 splits of 8 heads: 10.4 -> 9.2 us with
+// the launch before it.
+__global__ void __launch_bounds__(MC_THREADS)
+f16_attn_reduce_cluster_kernel(const float *__restrict__ pmax, const float *__restrict__ psum, const float *__restrict__ pacc,
+                               __half *__restrict__ out, unsigned hd, unsigned num_splits) {
+    lc_pdl_trigger();
+    __shared__ ClusterMerge sh;
+    const size_t qh = blockIdx.x / MC;
+    const float *pm = pmax + qh * num_splits, *ps = psum + qh * num_splits, *pa = pacc + qh * num_splits * hd;
+    const bool pairs = (reinterpret_cast<uintptr_t>(pacc) & 7) == 0;   // the caller's buffer may start at any float
+    float2 o;
+    float gsum;
+    const bool mine = cluster_merge(
+        sh, hd, num_splits, [&](unsigned s) { return make_float2(pm[s], ps[s]); },
+        [&](unsigned s, unsigned c) {
+            const float *at = pa + (size_t)s * hd + 2 * c;
+            return pairs ? *reinterpret_cast<const float2 *>(at) : make_float2(at[0], at[1]);
+        }, o, gsum);
+    if (!mine) return;
+    const float inv = gsum > 0.f ? 1.f / gsum : 0.f;
+    out[qh * hd + 2 * threadIdx.x] = __float2half_rn(gsum > 0.f ? o.x * inv : 0.f);
+    out[qh * hd + 2 * threadIdx.x + 1] = __float2half_rn(gsum > 0.f ? o.y * inv : 0.f);
+}
+
 template <int HD>
 int launch_mma(lc_batch *b, const __half *q, const __half *k, const __half *v, float *pmax, float *psum, float *pacc, uint32_t kv_len,
                uint32_t current_pos, uint32_t n_q, uint32_t n_kv, uint32_t window, uint32_t num_splits, float scale) {
@@ -415,7 +440,11 @@ int f16_attention(const char *name, lc_batch *b, const lc_buf *q, const lc_buf *
     b->dispatch_count++;
     uint32_t rows = 2048 / hd;   // rows of splits that the block's 1024 threads hold
     if (rows > (num_splits + 7) / 8) rows = (num_splits + 7) / 8;
-    LC_LAUNCH_CHECKED(lc_launch(f16_attn_reduce_kernel, dim3(n_q), dim3(rows * (hd / 2)), 0, b, (const float *)pmax, (const float *)psum,
+    if (cluster_merge_fits(b->ctx, n_q, num_splits, hd))
+        LC_LAUNCH_CHECKED(launch_cluster_merge(f16_attn_reduce_cluster_kernel, n_q, b, (const float *)pmax, (const float *)psum, (const float *)pacc,
+                                               (__half *)output->dptr, hd, num_splits));
+    else
+        LC_LAUNCH_CHECKED(lc_launch(f16_attn_reduce_kernel, dim3(n_q), dim3(rows * (hd / 2)), 0, b, (const float *)pmax, (const float *)psum,
                                 (const float *)pacc, (__half *)output->dptr, hd, num_splits));
     LC_CHECK_LAUNCH(name);
     b->dispatch_count++;
