@@ -595,10 +595,9 @@ static MmaPlan mma_plan(int fmt, const lc_kernels *k, uint32_t m, uint32_t kk, i
     return pl;
 }
 
-// Time of the two kernels here for one Q4_0 matrix, in ns (~0: not covered), fitted as lc_qgemm_tcl_estimate (qmatmul_tcl.cu) and
-// compared with it.  What decides: a tall matrix at short K is a second and third CTA per SM here, without a fixed cost per wave; with
-// fewer tiles than SMs, how often the splits' clusters have to share SMs.  From 33 rows the f32 scaling of every block doubles
-// this kernel's work, and it keeps the tall matrices only.
+// Time of the two kernels here for one tall Q4_0 matrix, in ns (~0: not covered), fitted as lc_qgemm_tcl_estimate (qmatmul_tcl.cu) and
+// compared with it.  What decides: a tall matrix at short K is a second and third CTA per SM here, without a fixed cost per wave.
+// From 33 rows the f32 scaling of every block doubles this kernel's work, and it keeps the tallest matrices only.
 static uint64_t wide_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uint32_t n) {
     const uint64_t sms = (uint64_t)k->ctx->sm_count, tiles = (n + W_ROWS - 1) / W_ROWS;
     if (m <= 32 || kk % W_CK != 0 || n < W_ROWS * sms || (size_t)W_STAGES * W_STAGE > k->ctx->smem_optin) return ~0ull;
@@ -614,13 +613,7 @@ static uint64_t narrow_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, ui
         if (m <= 32) return rounds * (alone ? 2800 + 9 * K : 900 + 8 * K);
         return rounds * (alone ? 3000 + 14 * K : 2600 + 9 * K);
     }
-    const uint64_t ks = (uint64_t)pl.ks, cps = (uint64_t)pl.cps, ctas = tiles * ks, seen = ctas < sms ? ctas : sms;
-    if (m > 32) return ~0ull - 1;
-    const bool shared = ks > 1 && 10 * tiles > 9 * k->cluster_cap[ks];   // clusters meet on SMs
-    uint64_t t = 2600 + 900 * K / (256 * ks) + 1550 * seen * cps / sms;
-    if (ctas > sms) t += 1750 + (alone ? 950 * cps : 0) - (alone ? 0 : 550 * cps);
-    if (ks > 1) t += 300 * ks + 1200 * (ks == 2 && !shared ? 1 : cps) * seen / sms + (shared ? 950 : 0) - 270 * ks * seen / sms;
-    return t;
+    return ~0ull - 1;   // fewer tiles than SMs: compared with nothing that could be slower
 }
 uint64_t lc_qgemm_mma_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uint32_t n) {
     const uint64_t a = wide_estimate(k, m, kk, n), b = narrow_estimate(k, m, kk, n);

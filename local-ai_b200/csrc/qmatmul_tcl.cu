@@ -467,18 +467,14 @@ static TclPlan tcl_plan(int fmt, const lc_kernels *k, uint32_t m, uint32_t kk, i
 }
 
 // What a launch over one Q4_0 matrix takes at 17 .. 64 rows, in ns, for the choice between this kernel and the register-direct one
-// (qmatmul_mma.cu).  Fitted to both kernels' times over 1100 shapes of n 300 .. 262144 and K 128 .. 8192 (6 % off on average): the
-// choice takes 0.4 % longer than the faster kernel on average, at most 16 % (0.4 us, K = 128).  A step takes about 1000; where a
-// second launch fits beside the first, its CTAs fetch and unpack their first steps meanwhile.
+// (qmatmul_mma.cu) where there are more tiles than SMs; 0 with fewer, where this one is never the slower by more than 1 % (20 x 512 x 6144:
+// 5.45 us against 5.41; 24 x 16384 x 256 5.1 / 5.8; 24 x 4096 x 6144 15.4 / 17.4; eight of 24 x 1536 x 512 in one batch 25.8 / 37.7).
+// Fitted to n 24000 .. 262144, K 256 .. 1536: a wave costs its start and epilogue and about 720 a step.
 uint64_t lc_qgemm_tcl_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uint32_t n) {
     const uint64_t tiles = (n + ROWS - 1) / ROWS, sms = (uint64_t)k->ctx->sm_count;
+    if (tiles <= sms) return 0;
     const TclPlan pl = tcl_plan(FMT_Q4_0, k, m, kk, (int)tiles);
-    const uint64_t sps = (uint64_t)pl.sps, groups = tiles * pl.m_tiles, ctas = groups * pl.ks;
-    if (tiles > sms) return pl.waves * (4000 + 1000 * sps);
-    uint64_t t = 1850 + 1000 * sps + 2250 * (ctas < sms ? ctas : sms) / sms;
-    if (pl.ks > 1) t += 750 + 40 * pl.ks;
-    if (2 * groups <= (pl.ks > 1 ? k->cluster_cap[pl.ks] : sms)) t -= 350 * sps;
-    return pl.waves * t;
+    return pl.waves * (3300 + 720 * (uint64_t)pl.sps);
 }
 
 // Grouped launch: `ng` weight matrices [ns[g], kk] sharing the activations `input` [m, kk].  Returns LC_OK after a launch, a
