@@ -204,8 +204,12 @@ __global__ void __launch_bounds__(ENC_ROWS * 32) encode_rows_kernel(const Encode
         const unsigned logical = p.position + row;
         slot = (size_t)(p.ring ? logical % p.ring : logical) * p.n_kv + head;
     }
-    store_warp_codes<HD, BITS>(encode_warp_row<HD, BITS>(x, norm_s[warp], lv, sg, lane), lane, p.packed[y] + slot * (HD * BITS / 8));
-    if (lane == 0) *(p.norms[y] + slot) = __float2half_rn(norm_s[warp]);
+    // addresses ahead of the search for the codes: 1950 x 2 rows of 2-bit codes 9.7 us, 10.5 with them after it (8 registers fewer)
+    uint8_t *const dst = p.packed[y] + slot * (HD * BITS / 8);
+    __half *const norm_out = p.norms[y] + slot;
+    const float norm = norm_s[warp];
+    store_warp_codes<HD, BITS>(encode_warp_row<HD, BITS>(x, norm, lv, sg, lane), lane, dst);
+    if (lane == 0) *norm_out = __float2half_rn(norm);
 }
 template <int HD, bool BATCHED>
 cudaError_t launch_encode_rows(lc_batch *b, const EncodeRows &p, unsigned tensors, unsigned bits) {
@@ -424,8 +428,11 @@ __global__ void __launch_bounds__(ENC_ROWS * 32) kv_write_rows_kernel(const __gr
         return;
     }
     const size_t slot = ((size_t)row * p.lane_capacity + ppos) * p.n_kv + head;
-    store_warp_codes<HD, BITS>(encode_warp_row<HD, BITS>(x, norm_s[warp], lv, sg, lane), lane, p.packed[role - 1] + slot * (HD * BITS / 8));
-    if (lane == 0) *(p.norms[role - 1] + slot) = __float2half_rn(norm_s[warp]);
+    uint8_t *const dst = p.packed[role - 1] + slot * (HD * BITS / 8);
+    __half *const norm_out = p.norms[role - 1] + slot;
+    const float norm = norm_s[warp];
+    store_warp_codes<HD, BITS>(encode_warp_row<HD, BITS>(x, norm, lv, sg, lane), lane, dst);
+    if (lane == 0) *norm_out = __float2half_rn(norm);
 }
 
 // dequantize_kv.metal:132-189. grid = n_kv * (num_tokens - token_start).
