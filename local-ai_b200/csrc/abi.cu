@@ -285,18 +285,20 @@ LcOrder::LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, cons
     before = ctx->launches.fetch_add(1);
     if (before != o.seen) o.state = 0;
     auto range = [](const lc_buf *buf, size_t bytes) { return lc_range{(uintptr_t)buf->dptr, (uintptr_t)buf->dptr + bytes}; };
-    auto meets = [](const lc_range &r, const lc_range *v, int n) {
+    // (most ranges lie outside of what all those of the list span: the call costs the host less than a walk over it)
+    auto meets = [](const lc_range &r, const lc_range &span, const lc_range *v, int n) {
+        if (n == 0 || r.lo >= span.hi || span.lo >= r.hi) return false;
         for (int i = 0; i < n; i++)
             if (r.lo < v[i].hi && v[i].lo < r.hi) return true;
         return false;
     };
     const lc_range in = range(input, in_bytes);
     const bool room = o.n_reads + 1 + ng <= MOST_READS && o.n_writes + ng <= MOST_WRITES;
-    bool apart = o.state != 0 && !meets(in, o.writes, o.n_writes), weights_apart = true;
+    bool apart = o.state != 0 && !meets(in, o.write_span, o.writes, o.n_writes), weights_apart = true;
     for (int g = 0; g < ng; g++) {
         const lc_range w = range(weights[g], w_bytes[g]), out = range(outputs[g], out_bytes[g]);
-        weights_apart = weights_apart && !meets(w, o.writes, o.n_writes);
-        apart = apart && weights_apart && !meets(out, o.writes, o.n_writes) && !meets(out, o.reads, o.n_reads);
+        weights_apart = weights_apart && !meets(w, o.write_span, o.writes, o.n_writes);
+        apart = apart && weights_apart && !meets(out, o.write_span, o.writes, o.n_writes) && !meets(out, o.read_span, o.reads, o.n_reads);
     }
     if (o.state == 2 && room) {
         // (the list stays: what it holds may be running when the next launch starts, whether this one waits or not)
@@ -309,10 +311,14 @@ LcOrder::LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, cons
         o.state = apart ? 2 : 1;
         o.n_reads = o.n_writes = 0;
     }
-    if (o.n_reads == 0 || o.reads[0].lo != in.lo || o.reads[0].hi < in.hi) o.reads[o.n_reads++] = in;   // (a run mostly shares its input)
+    auto add = [](const lc_range &r, lc_range &span, lc_range *v, int &n) {
+        span = n == 0 ? r : lc_range{r.lo < span.lo ? r.lo : span.lo, r.hi > span.hi ? r.hi : span.hi};
+        v[n++] = r;
+    };
+    if (o.n_reads == 0 || o.reads[0].lo != in.lo || o.reads[0].hi < in.hi) add(in, o.read_span, o.reads, o.n_reads);   // (a run mostly shares its input)
     for (int g = 0; g < ng; g++) {
-        o.reads[o.n_reads++] = range(weights[g], w_bytes[g]);
-        o.writes[o.n_writes++] = range(outputs[g], out_bytes[g]);
+        add(range(weights[g], w_bytes[g]), o.read_span, o.reads, o.n_reads);
+        add(range(outputs[g], out_bytes[g]), o.write_span, o.writes, o.n_writes);
     }
 }
 

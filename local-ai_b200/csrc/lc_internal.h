@@ -20,6 +20,7 @@ struct lc_overlap {
     int state = 0;           // 0: nothing known, 1: `reads` / `writes` are the last launch's, 2: those of every launch that may be running
     int n_reads = 0, n_writes = 0;
     lc_range reads[192], writes[96];   // (when they are full the run starts anew)
+    lc_range read_span = {}, write_span = {};   // what the lists span together
 };
 
 struct lc_ctx {
@@ -169,7 +170,9 @@ static inline cudaError_t lc_launch(void (*kern)(KArgs...), dim3 grid, dim3 bloc
 //     of a run is complete (`serial`).
 // A graph or a capture boundary ends the run, too.  Ranges are virtual addresses: memory mapped twice is not recognised.
 // (The line lies at the bytes and nowhere else: 35 matrices of 8192 x 1536 TQ2_0 times 16 rows took 225 us one after the
-// other and take 98 side by side, 35 of Q4_0 6144 x 1536 times 40 rows 348 and 269; no shape was found that loses.)
+// other and take 98 side by side, 35 of Q4_0 6144 x 1536 times 40 rows 348 and 269, 35 of Q4_0 8192 x
+// 1536 times one row 206 and 113.  Where the host sets the pace, at matrices of a megabyte or so and one row, the look at the ranges costs about 0.07
+// us a launch: 35 of 3740 x 768 in 139.0 us and 139.9, of 1024 x 512 in 97.6 and 101.8.)
 constexpr uint32_t LC_LATE_TRIGGER = 1, LC_LATE_WAIT = 2;
 class LcOrder {
 public:
