@@ -996,6 +996,7 @@ def main() -> None:
         wl = WORKLOADS[args.workload](la, ctx, kernels)
     wl.prepare()
     stream = torch.cuda.ExternalStream(ctx.stream, device=torch.device("cuda", local_rank))
+    ctx.set_overlap(True)   # (only events are recorded there)
 
     def barrier(collective: bool = True):
         ctx.synchronize()

@@ -84,8 +84,13 @@ LC_API void lc_ctx_destroy(lc_ctx *ctx);
  * CTA, L2 bytes, total device memory. Any out pointer may be NULL. */
 LC_API int lc_ctx_caps(const lc_ctx *ctx, int *sm_count, size_t *smem_per_cta,
                        size_t *l2_bytes, size_t *total_mem);
-/* The context's stream as a cudaStream_t, for callers that time with events. */
+/* The context's stream as a cudaStream_t.  The library cannot see what a caller puts there, so from this call on
+ * every matmul waits for the work before it; see lc_ctx_set_overlap. */
 LC_API void *lc_ctx_stream(const lc_ctx *ctx);
+/* Matmul launches whose buffers do not meet run beside each other (1, the start unless LOCAL_CUDA_OVERLAP=0) or one
+ * after the other (0).  A caller of lc_ctx_stream that puts nothing but events there may switch it on again; one
+ * that puts kernels or copies there must not while they and dispatches of this library follow one another. */
+LC_API int lc_ctx_set_overlap(lc_ctx *ctx, uint32_t on);
 LC_API int lc_ctx_synchronize(lc_ctx *ctx);
 
 /* -------------------------------------------------------------- buffer -- */
@@ -110,6 +115,9 @@ LC_API int lc_buf_fill(lc_buf *buf, size_t offset, size_t bytes, int value);
 /* --------------------------------------------------------------- batch -- */
 LC_API int lc_batch_begin(lc_ctx *ctx, lc_batch **out);           /* CommandBatch::new batch.rs:160-172 */
 LC_API uint32_t lc_batch_dispatch_count(const lc_batch *batch);   /* batch.rs:174-182 */
+/* How the batch's last dispatch stands to those before it: 0 behind them, 1 the first of a run side by side, 2 beside
+ * those of a run (for tests and tuning). */
+LC_API uint32_t lc_batch_last_order(const lc_batch *batch);
 /* CommandBatch::blit_buffer_copies (batch.rs:196-226), one copy per call. */
 LC_API int lc_batch_copy(lc_batch *batch, const lc_buf *src, size_t src_off, lc_buf *dst,
                          size_t dst_off, size_t bytes);

@@ -126,7 +126,8 @@ int lc_ctx_create(int device, lc_ctx **out) {
     cudaMemGetInfo(&fr, &tot);
     c->total_mem = tot;
     { const char *e = getenv("LOCAL_CUDA_PDL"); c->pdl = !(e && strcmp(e, "0") == 0); }
-    { const char *e = getenv("LOCAL_CUDA_OVERLAP"); c->side_by_side = !(e && strcmp(e, "0") == 0); }
+    { const char *e = getenv("LOCAL_CUDA_OVERLAP"); c->overlap_wanted = !(e && strcmp(e, "0") == 0); }
+    c->side_by_side = c->overlap_wanted;
     count_context(device, 1);
     *out = c;
     return LC_OK;
@@ -153,7 +154,18 @@ int lc_ctx_caps(const lc_ctx *ctx, int *sm_count, size_t *smem_per_cta, size_t *
     return LC_OK;
 }
 
-void *lc_ctx_stream(const lc_ctx *ctx) { return ctx ? (void *)ctx->stream : nullptr; }
+void *lc_ctx_stream(const lc_ctx *ctx) {
+    if (!ctx) return nullptr;
+    ctx->side_by_side = false;   // (what the caller will put there is unknown)
+    return (void *)ctx->stream;
+}
+
+int lc_ctx_set_overlap(lc_ctx *ctx, uint32_t on) {
+    if (!ctx) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_ctx_set_overlap: ctx is NULL");
+    lc_order_break(ctx, true);
+    ctx->side_by_side = on && ctx->overlap_wanted;
+    return LC_OK;
+}
 
 int lc_ctx_synchronize(lc_ctx *ctx) {
     if (!ctx) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_ctx_synchronize: ctx is NULL");
@@ -175,6 +187,7 @@ int lc_buf_alloc(lc_ctx *ctx, size_t bytes, lc_buf **out) {
         return lc_fail(LC_ERR_BUFFER_ALLOCATION, "size=%zu: %s", bytes, cudaGetErrorString(e));
     }
     e = cudaMemsetAsync(p, 0, n, ctx->stream);
+    lc_order_break(ctx);
     if (e != cudaSuccess) {
         cudaFree(p);
         return lc_fail(LC_ERR_CUDA, "memset: %s", cudaGetErrorString(e));
@@ -240,6 +253,7 @@ int lc_buf_upload(lc_buf *buf, size_t offset, const void *src, size_t bytes) {
     if (!src) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_buf_upload: src is NULL");
     cudaStream_t s = buf->ctx->stream;
     LC_CUDA_TRY(cudaMemcpyAsync((char *)buf->dptr + offset, src, bytes, cudaMemcpyHostToDevice, s));
+    lc_order_break(buf->ctx);
     LC_CUDA_TRY(cudaStreamSynchronize(s));
     return LC_OK;
 }
@@ -251,6 +265,7 @@ int lc_buf_download(const lc_buf *buf, size_t offset, void *dst, size_t bytes) {
     if (!dst) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_buf_download: dst is NULL");
     cudaStream_t s = buf->ctx->stream;
     LC_CUDA_TRY(cudaMemcpyAsync(dst, (const char *)buf->dptr + offset, bytes, cudaMemcpyDeviceToHost, s));
+    lc_order_break(buf->ctx);
     LC_CUDA_TRY(cudaStreamSynchronize(s));
     return LC_OK;
 }
@@ -260,6 +275,7 @@ int lc_buf_zero(lc_buf *buf, size_t offset, size_t bytes) {
     if (st != LC_OK) return st;
     if (!bytes) return LC_OK;
     LC_CUDA_TRY(cudaMemsetAsync((char *)buf->dptr + offset, 0, bytes, buf->ctx->stream));
+    lc_order_break(buf->ctx);
     return LC_OK;
 }
 
@@ -268,22 +284,27 @@ int lc_buf_fill(lc_buf *buf, size_t offset, size_t bytes, int value) {
     if (st != LC_OK) return st;
     if (!bytes) return LC_OK;
     LC_CUDA_TRY(cudaMemsetAsync((char *)buf->dptr + offset, value & 0xFF, bytes, buf->ctx->stream));
+    lc_order_break(buf->ctx);
     return LC_OK;
 }
 
 // ------------------------------------------------- launches side by side --
 LcOrder::LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, const lc_buf *const *weights, const size_t *w_bytes,
                  lc_buf *const *outputs, const size_t *out_bytes)
-    : ctx(b->ctx), tracked(b->ctx->pdl && b->ctx->side_by_side && b->stream == b->ctx->stream) {
-    if (!tracked) {
-        serial = lc_count_launch(b);
-        return;
-    }
+    : ctx(b->ctx) {
     lc_overlap &o = ctx->overlap;
     constexpr int MOST_READS = sizeof(o.reads) / sizeof(lc_range), MOST_WRITES = sizeof(o.writes) / sizeof(lc_range);
     o.mu.lock();
-    before = ctx->launches.fetch_add(1);
-    if (before != o.seen) o.state = 0;
+    b->last_order = 0;
+    const bool own = b->stream == ctx->stream, tracked = own && ctx->pdl && ctx->side_by_side.load(std::memory_order_relaxed);
+    if (!tracked) {
+        o.state = 0;
+        if (own) {
+            serial = o.beside;
+            o.beside = false;
+        }
+        return;
+    }
     auto range = [](const lc_buf *buf, size_t bytes) { return lc_range{(uintptr_t)buf->dptr, (uintptr_t)buf->dptr + bytes}; };
     // (most ranges lie outside of what all those of the list span: the call costs the host less than a walk over it)
     auto meets = [](const lc_range &r, const lc_range &span, const lc_range *v, int n) {
@@ -304,13 +325,17 @@ LcOrder::LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, cons
         // (the list stays: what it holds may be running when the next launch starts, whether this one waits or not)
         flags = apart ? LC_LATE_WAIT : 0u;
         serial = !weights_apart;   // (fetched ahead of the wait)
-        if (apart) ctx->beside = true;
+        if (apart) o.beside = true;
     } else {
-        serial = o.state == 2 && !weights_apart;
+        // The list starts anew with this launch, so what it held has to be complete when the next one starts.  (`beside` in state 0: another
+        // library's kernel stands behind a run.)
+        serial = o.state == 2 ? !apart : o.beside;
+        o.beside = false;
         flags = apart ? LC_LATE_TRIGGER : 0u;
         o.state = apart ? 2 : 1;
         o.n_reads = o.n_writes = 0;
     }
+    b->last_order = flags;
     auto add = [](const lc_range &r, lc_range &span, lc_range *v, int &n) {
         span = n == 0 ? r : lc_range{r.lo < span.lo ? r.lo : span.lo, r.hi > span.hi ? r.hi : span.hi};
         v[n++] = r;
@@ -323,11 +348,8 @@ LcOrder::LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, cons
 }
 
 LcOrder::~LcOrder() {
-    if (!tracked) return;
-    lc_overlap &o = ctx->overlap;
-    if (launched) o.seen = before + 1;
-    else o.state = 0;
-    o.mu.unlock();
+    if (!launched) ctx->overlap.state = 0;
+    ctx->overlap.mu.unlock();
 }
 
 // ------------------------------------------------------------------ batch --
@@ -342,6 +364,7 @@ int lc_batch_begin(lc_ctx *ctx, lc_batch **out) {
 }
 
 uint32_t lc_batch_dispatch_count(const lc_batch *batch) { return batch ? batch->dispatch_count : 0; }
+uint32_t lc_batch_last_order(const lc_batch *batch) { return batch ? batch->last_order : 0; }
 
 int lc_batch_copy(lc_batch *batch, const lc_buf *src, size_t src_off, lc_buf *dst, size_t dst_off,
                   size_t bytes) {
@@ -353,6 +376,7 @@ int lc_batch_copy(lc_batch *batch, const lc_buf *src, size_t src_off, lc_buf *ds
     if (!bytes) return LC_OK;
     LC_CUDA_TRY(cudaMemcpyAsync((char *)dst->dptr + dst_off, (const char *)src->dptr + src_off, bytes,
                                 cudaMemcpyDeviceToDevice, batch->stream));
+    lc_order_break(batch->ctx);
     batch->dispatch_count++;
     return LC_OK;
 }
@@ -365,6 +389,7 @@ int lc_batch_upload(lc_batch *batch, lc_buf *dst, size_t dst_off, const void *sr
     if (!src) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_batch_upload: src is NULL");
     LC_CUDA_TRY(cudaMemcpyAsync((char *)dst->dptr + dst_off, src, bytes, cudaMemcpyHostToDevice,
                                 batch->stream));
+    lc_order_break(batch->ctx);
     return LC_OK;
 }
 
@@ -376,6 +401,7 @@ int lc_batch_download(lc_batch *batch, const lc_buf *src, size_t src_off, void *
     if (!dst) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_batch_download: dst is NULL");
     LC_CUDA_TRY(cudaMemcpyAsync(dst, (const char *)src->dptr + src_off, bytes, cudaMemcpyDeviceToHost,
                                 batch->stream));
+    lc_order_break(batch->ctx);
     return LC_OK;
 }
 
@@ -427,8 +453,7 @@ int lc_batch_begin_capture(lc_ctx *ctx, lc_batch **out) {
         return lc_fail(LC_ERR_CUDA, "begin capture: %s", cudaGetErrorString(e));
     }
     (*out)->capturing = true;
-    ctx->launches++;
-    ctx->beside = false;
+    lc_order_break(ctx);
     return LC_OK;
 }
 
@@ -437,8 +462,7 @@ int lc_batch_end_capture(lc_batch *batch, lc_graph **out) {
     if (!batch->capturing) return lc_fail(LC_ERR_INVALID_ARGUMENT, "batch is not capturing");
     lc_ctx *ctx = batch->ctx;
     cudaGraph_t g = nullptr;
-    ctx->launches++;
-    ctx->beside = false;
+    lc_order_break(ctx);
     cudaError_t e = cudaStreamEndCapture(batch->stream, &g);
     delete batch;
     if (e != cudaSuccess || !g) {
@@ -461,8 +485,8 @@ int lc_batch_end_capture(lc_batch *batch, lc_graph **out) {
 
 int lc_graph_launch(lc_graph *graph) {
     if (!graph) return lc_fail(LC_ERR_INVALID_ARGUMENT, "lc_graph_launch: graph is NULL");
-    graph->ctx->launches++;
     LC_CUDA_TRY(cudaGraphLaunch(graph->exec, graph->ctx->stream));
+    lc_order_break(graph->ctx);
     return LC_OK;
 }
 
@@ -515,6 +539,7 @@ int lc_kernels_create(lc_ctx *ctx, lc_kernels **out) {
     lc_cluster_capacity(ctx, k->cluster_cap);
     cudaError_t e = cudaMalloc((void **)&k->dev_status, 128);  // status word + tuning stamps
     if (e == cudaSuccess) e = cudaMemsetAsync(k->dev_status, 0, 128, ctx->stream);
+    lc_order_break(ctx);
     if (e != cudaSuccess) {
         delete k;
         return lc_fail(LC_ERR_PIPELINE_CREATION, "status word: %s", cudaGetErrorString(e));
@@ -583,6 +608,7 @@ int lc_reserve_scratch(lc_kernels *k, lc_batch *b, size_t bytes, size_t counters
         // zeroed in stream order, before any kernel that is enqueued after this call can use them
         cudaStream_t s = b ? b->stream : k->ctx->stream;
         e = cudaMemsetAsync(fresh, 0, want * sizeof(unsigned int), s);
+        lc_order_break(k->ctx);
         if (e != cudaSuccess) {
             cudaFree(fresh);
             return lc_fail(LC_ERR_CUDA, "counters memset: %s", cudaGetErrorString(e));

@@ -513,8 +513,8 @@ int launch(lc_batch *b, const TqAttnParams &p, dim3 grid) {
     cfg.stream = b->stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
-    const bool serial = lc_count_launch(b);
-    if (b->ctx->pdl && !serial) {
+    LcPlain plain(b);
+    if (b->ctx->pdl && !plain.serial) {
         attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[na].val.programmaticStreamSerializationAllowed = 1;
         na++;

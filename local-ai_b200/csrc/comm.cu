@@ -186,6 +186,7 @@ int lc_comm_all_gather_into(lc_batch *b, lc_comm *c, const lc_buf *send, size_t 
     if (!a->handle) return lc_comm_available();
     const int rc = a->all_gather((const uint8_t *)send->dptr + send_offset, recv->dptr, bytes_per_rank, NCCL_UINT8, c->comm,
                                  b->stream);
+    lc_order_break(b->ctx, true);
     if (rc != 0) return nccl_fail(a, "ncclAllGather", rc);
     b->dispatch_count++;
     return LC_OK;

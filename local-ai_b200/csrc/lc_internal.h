@@ -15,8 +15,8 @@ struct lc_range {
     uintptr_t lo, hi;
 };
 struct lc_overlap {
-    std::mutex mu;
-    uint64_t seen = 0;       // the context's launch count after the launch last recorded here
+    std::mutex mu;           // held from the decision about a launch until it is enqueued
+    bool beside = false;     // the last launch runs beside others
     int state = 0;           // 0: nothing known, 1: `reads` / `writes` are the last launch's, 2: those of every launch that may be running
     int n_reads = 0, n_writes = 0;
     lc_range reads[192], writes[96];   // (when they are full the run starts anew)
@@ -31,9 +31,10 @@ struct lc_ctx {
     size_t l2_bytes = 0;
     size_t total_mem = 0;
     bool pdl = true;  // launch kernels with programmatic stream serialization (LOCAL_CUDA_PDL=0 disables)
-    bool side_by_side = true;   // launches whose buffers do not meet may overlap (LOCAL_CUDA_OVERLAP=0 disables)
-    std::atomic<uint64_t> launches{0};   // every kernel launch, graph launch and capture boundary of the context counts
-    std::atomic<bool> beside{false};     // the last launch runs beside others
+    // Launches whose buffers do not meet may overlap.  LOCAL_CUDA_OVERLAP=0 disables, and so does handing out the stream: work that
+    // others put there is not seen here (lc_ctx_set_overlap).
+    bool overlap_wanted = true;
+    mutable std::atomic<bool> side_by_side{true};
     lc_overlap overlap;
 };
 
@@ -48,6 +49,7 @@ struct lc_batch {
     lc_ctx *ctx = nullptr;
     cudaStream_t stream = nullptr;
     uint32_t dispatch_count = 0;
+    uint32_t last_order = 0;   // LcOrder::flags of the last launch, 0 where it declares nothing
     bool capturing = false;
 };
 
@@ -131,13 +133,33 @@ void lc_clear_error();
 // lc_pdl_trigger() at its top — its successors may then be scheduled — and lc_pdl_wait() before it
 // first touches memory a predecessor may have written.  Work that does not depend on the predecessor
 // (streaming constant weights towards the SM) goes before the wait.
-// Counts a launch; true where it has to start only when its predecessor is complete (the end of a run of launches side by side: several
-// of those may still be running, and a kernel fetches its constant operands ahead of its wait).
-static inline bool lc_count_launch(lc_batch *b) {
-    b->ctx->launches++;
-    return b->ctx->beside.load() && b->ctx->beside.exchange(false);
+// A launch that declares nothing ends a run of launches side by side (LcOrder below); it lives until its launch is enqueued.  `serial`: the
+// launch has to start only when its predecessor is complete (several of a run may still be running, and a kernel fetches its
+// constant operands ahead of its wait).
+class LcPlain {
+public:
+    explicit LcPlain(lc_batch *b) : lock(b->ctx->overlap.mu) {
+        lc_overlap &o = b->ctx->overlap;
+        o.state = 0;
+        b->last_order = 0;
+        if (b->stream == b->ctx->stream) {   // (runs are that stream's)
+            serial = o.beside;
+            o.beside = false;
+        }
+    }
+    bool serial = false;
+
+private:
+    std::lock_guard<std::mutex> lock;
+};
+// After work that is no launch of this library's kernels: what LcOrder knows is no longer all that may be running.  `foreign`: a kernel
+// of another library, which may let its successors start early; copies, memsets and graphs are complete before a later launch starts.
+static inline void lc_order_break(lc_ctx *ctx, bool foreign = false) {
+    std::lock_guard<std::mutex> lock(ctx->overlap.mu);
+    ctx->overlap.state = 0;
+    if (!foreign) ctx->overlap.beside = false;
 }
-// `serial`: the launch starts only when its predecessor is complete.  (It is counted by whoever asks for it.)
+// `serial`: the launch starts only when its predecessor is complete.
 template <typename... KArgs, typename... Args>
 static inline cudaError_t lc_launch_as(bool serial, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, lc_batch *b,
                                        Args &&...args) {
@@ -156,7 +178,8 @@ static inline cudaError_t lc_launch_as(bool serial, void (*kern)(KArgs...), dim3
 template <typename... KArgs, typename... Args>
 static inline cudaError_t lc_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, lc_batch *b,
                                     Args &&...args) {
-    return lc_launch_as(lc_count_launch(b), kern, grid, block, smem, b, static_cast<KArgs>(args)...);
+    LcPlain plain(b);
+    return lc_launch_as(plain.serial, kern, grid, block, smem, b, static_cast<KArgs>(args)...);
 }
 // Launches of one stream run one after the other because the next may read what the last wrote.  Several projections of the same
 // activations, or the same projection of several matrices, do not: a launch of a few microseconds then spends most of its time
@@ -168,7 +191,8 @@ static inline cudaError_t lc_launch(void (*kern)(KArgs...), dim3 grid, dim3 bloc
 //     when all before it are.  One that depends on any that may be running waits for the last as ever; so do launches that declare
 //     nothing, which end the run and, because a kernel fetches its constant operands ahead of its wait, start only when the last launch
 //     of a run is complete (`serial`).
-// A graph or a capture boundary ends the run, too.  Ranges are virtual addresses: memory mapped twice is not recognised.
+// Whatever else the library puts on the stream ends the run, too (lc_order_break: copies, memsets, collectives, graphs, capture
+// boundaries), and a program that takes the stream for work of its own has no runs at all (lc_ctx_stream).  Ranges are virtual addresses: memory mapped twice is not recognised.
 // (The line lies at the bytes and nowhere else: 35 matrices of 8192 x 1536 TQ2_0 times 16 rows took 225 us one after the
 // other and take 98 side by side, 35 of Q4_0 6144 x 1536 times 40 rows 348 and 269, 35 of Q4_0 8192 x
 // 1536 times one row 206 and 113.  Where the host sets the pace, at matrices of a megabyte or so and one row, the look at the ranges costs about 0.07
@@ -185,8 +209,6 @@ public:
 
 private:
     lc_ctx *ctx;
-    bool tracked;
-    uint64_t before = 0;
 };
 #ifdef __CUDACC__
 __device__ __forceinline__ void lc_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -106,9 +106,9 @@ cudaError_t launch_cluster_merge(void (*kern)(KArgs...), unsigned heads, lc_batc
     attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
-    const bool serial = lc_count_launch(b);
+    LcPlain plain(b);
     cfg.attrs = attr;
-    cfg.numAttrs = b->ctx->pdl && !serial ? 2 : 1;
+    cfg.numAttrs = b->ctx->pdl && !plain.serial ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 // Whether a merge of `n` splits of `heads` heads is one for it.  Few heads: all CTAs have an SM each (16384 keys, cluster against one CTA a head:

@@ -825,7 +825,7 @@ int launch_step(lc_kernels *k, lc_batch *b, LcStepParams &p) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    lc_count_launch(b);
+    LcPlain plain(b);   // (without the programmatic attribute it starts when its predecessor is complete)
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
     if (e == cudaErrorCooperativeLaunchTooLarge) {   // (part of the device only)
         cudaGetLastError();

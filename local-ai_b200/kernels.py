@@ -82,6 +82,9 @@ class CudaContext(Handle):
     def stream(self) -> int:
         return self._lib.lc_ctx_stream(self._h) or 0
 
+    def set_overlap(self, on: bool) -> None:
+        _check(self._lib.lc_ctx_set_overlap(self._h, int(on)))
+
     synchronize = _fast.method(_fast.lc_ctx_synchronize)
 
     def close(self) -> None:
@@ -196,6 +199,9 @@ class CommandBatch(Handle):
 
     def dispatch_count(self) -> int:
         return self._lib.lc_batch_dispatch_count(self._h)
+
+    def last_order(self) -> int:
+        return self._lib.lc_batch_last_order(self._h)
 
     def blit_buffer_copy(self, src: CudaBuffer, src_off: int, dst: CudaBuffer, dst_off: int, nbytes: int) -> None:
         _fast.lc_batch_copy(self, src, src_off, dst, dst_off, nbytes)

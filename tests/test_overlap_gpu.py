@@ -108,6 +108,74 @@ def test_other_launches_end_a_run(la, ctx, kernels):
             assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("work", ["none", "copy", "upload", "download", "zero", "fill", "as_slice", "from_bytes", "alloc", "gather", "graph", "add"])
+def test_order_behind_other_work(la, ctx, kernels, work):
+    """A matmul runs beside those before it only while nothing but matmuls stands between: behind every other kind of work on the stream it
+    waits, also where that work declares no buffers of its own."""
+    m, n = 16, 512
+    x = la.CudaBuffer.from_slice(ctx, la.synth.normal_f16((m, K), 95))
+    ws = [la.CudaBuffer.from_slice(ctx, la.synth.tq2_0_weights(n, K, seed=96 + i)) for i in range(3)]
+    outs = [la.CudaBuffer.empty(ctx, m * n * 2) for _ in range(4)]
+    other = la.CudaBuffer.empty(ctx, m * n * 2)
+    host = np.zeros(m * n, np.uint16)
+    if work == "gather":
+        import torch  # noqa: F401  (brings the NCCL that it links; the system's, loaded first, would be in its way)
+    comm = la.Communicator(ctx, la.Communicator.unique_id(), 0, 1) if work == "gather" else None
+    b = la.CommandBatch.capture(ctx)
+    kernels.residual_add_into(b, other, other, other, m * n)
+    graph = b.end_capture()
+    b = la.CommandBatch.new(ctx)
+    kernels.residual_add_into(b, other, other, other, m * n)
+    orders = []
+    for i in range(3):
+        kernels.matmul_nt_tq2_0_into(b, x, ws[i], outs[i], m, K, n)
+        orders.append(b.last_order())
+    assert orders == [0, 1, 2]
+    {"none": lambda: None,
+     "copy": lambda: b.blit_buffer_copy(outs[2], 0, other, 0, m * n * 2),
+     "upload": lambda: b.upload(other, 0, host.ctypes.data, m * n * 2),
+     "download": lambda: b.download(outs[2], 0, host.ctypes.data, m * n * 2),
+     "zero": lambda: other.zero(),
+     "fill": lambda: other.fill(1),
+     "as_slice": lambda: outs[2].as_slice(np.uint16),
+     "from_bytes": lambda: other.copy_from_bytes(host),
+     "alloc": lambda: la.CudaBuffer.empty(ctx, 4096),
+     "gather": lambda: comm.all_gather_into(b, outs[2], 0, other, m * n * 2),
+     "graph": lambda: graph.launch(),
+     "add": lambda: kernels.residual_add_into(b, other, other, other, m * n)}[work]()
+    kernels.matmul_nt_tq2_0_into(b, x, ws[0], outs[3], m, K, n)
+    assert b.last_order() == (2 if work == "none" else 0)
+    b.commit_and_wait()
+    graph.destroy()
+    if comm:
+        comm.close()
+
+
+def test_no_runs_once_the_stream_is_out(la):
+    own = la.CudaContext.new(0)
+    kernels = la.Kernels.new(own)
+    x, w = la.CudaBuffer.from_slice(own, la.synth.normal_f16((16, K), 97)), la.CudaBuffer.from_slice(own, la.synth.tq2_0_weights(512, K, seed=98))
+    outs = [la.CudaBuffer.empty(own, 16 * 512 * 2) for _ in range(3)]
+
+    def orders():
+        b, got = la.CommandBatch.new(own), []
+        for o in outs:
+            kernels.matmul_nt_tq2_0_into(b, x, w, o, 16, K, 512)
+            got.append(b.last_order())
+        b.commit_and_wait()
+        return got
+
+    assert orders()[1:] == [1, 2]
+    assert own.stream
+    assert orders() == [0, 0, 0]
+    own.set_overlap(True)
+    assert orders() == [0, 1, 2]
+    for o in outs + [x, w]:
+        o.free()
+    kernels.close()
+    own.close()
+
+
 def test_weights_written_two_dispatches_before(la, ctx, kernels):
     """The header's rule for constant operands built on the device: any dispatch in between is enough, also where both are projections that
     run beside others."""
