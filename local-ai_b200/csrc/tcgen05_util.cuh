@@ -44,7 +44,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity, uint32
     }
     return false;
 }
-// The same by a whole warp, all of whose lanes ask; false on expiry or where another role of the CTA has given up.  (Lane 0 asking and
+// The same by a whole warp, all of whose lanes ask; on expiry false, and the CTA's other roles are told.  The vote alone ends the loop: lanes that
+// each looked at the flag here could leave it without the others, which would wait for them in the next vote.  (A vote on the flag, too, cost prefill
+// attention of 256 rows over 4096 keys 1 %; a role that waits while another gives up runs into its own limit.)  (Lane 0 asking and
 // a shuffle behind its loop took about 400 cycles on a phase that was complete, this takes about 200: with several such waits in
 // the path of every step 509 x 1536 x 6144 Q4_0 went from 31.4 to 27.2 us.)
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t addr, uint32_t parity, uint32_t limit, volatile uint32_t *abort_flag) {
@@ -58,7 +60,6 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t addr, uint32_t parity, u
             : "r"(addr), "r"(parity)
             : "memory");
         if (__all_sync(0xffffffffu, ok)) return true;
-        if (*abort_flag) break;
     }
     *abort_flag = 1;
     return false;
