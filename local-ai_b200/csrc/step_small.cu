@@ -39,6 +39,7 @@ constexpr int PROW = 260;              // floats of a head's partial: {max, sum,
 constexpr int MAX_HIDDEN = 2048;       // two 16-byte pieces of a row per thread at four lanes
 constexpr int RED_COL = 20, RED_PART = 8 * RED_COL + 16;   // a warp's sums of a tile, floats: [column][16 rows + padding] + padding
 constexpr int MAX_TILES = 16;          // of a CTA in one phase
+constexpr int FEW_SPLITS = 32, FULL_SPLIT = 4;   // more splits than the former only with this many blocks of keys in each
 
 // The exchange buffers of a layer: the counts of posts to O and to down (128 bytes each), rows of Q, K, V; attention; O; down;
 // gate * up; partials.
@@ -414,8 +415,9 @@ __global__ void __launch_bounds__(ST_NT + 32, 1) step_layers_kernel(const __grid
                 const uint32_t end = r.newest ? r.pos : L.lane_rows;   // (a position past the lane's rows is clamped and reported)
                 r.begin = L.window > 0u && r.pos + 1u > L.window ? r.pos + 1u - L.window : 0u;
                 r.old_keys = end > r.begin ? end - r.begin : 0u;
-                r.per = ((r.old_keys + (uint32_t)S - 1u) / (uint32_t)S + (KB - 1)) & ~(uint32_t)(KB - 1);
-                if (r.per < (uint32_t)KB) r.per = KB;
+                auto keys_of = [&](uint32_t n) -> uint32_t { return max(((r.old_keys + n - 1u) / n + (KB - 1)) & ~(uint32_t)(KB - 1), (uint32_t)KB); };
+                r.per = keys_of(min((uint32_t)S, (uint32_t)FEW_SPLITS));
+                if (r.per > FULL_SPLIT * KB) r.per = max(keys_of((uint32_t)S), (uint32_t)(FULL_SPLIT * KB));   // (long ones: all the splits)
                 return r;
             };
             uint8_t *scratch = work + STAGES * W::STAGE;
@@ -595,30 +597,34 @@ __global__ void __launch_bounds__(ST_NT + 32, 1) step_layers_kernel(const __grid
                 auto at = [&](int j) -> const float * { return part + (size_t)(j < n_old ? j : S) * 8 * PROW; };
                 float m_run = -INFINITY, l_run = 0.f;
                 float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-                uint4 ml, v;
-                if (grp < n) {
-                    ml = take16(at(grp));
-                    v = take16(at(grp) + 4 + 4 * d4);
-                }
+                constexpr int AT_ONCE = 4;   // splits whose trips pass together
                 uint32_t tries = 0;
 #pragma unroll 1
-                for (int j = grp; j < n; j += 8) {
+                for (int j0 = grp; j0 < n; j0 += 8 * AT_ONCE) {
+                    uint4 ml[AT_ONCE], v[AT_ONCE];
+                    bool fail;
 #pragma unroll 1
-                    while (!(here(ml) && here(v)) && tries < p.wait_limit) {
-                        ml = take16(at(j));
-                        v = take16(at(j) + 4 + 4 * d4);
-                        tries++;
+                    do {
+                        fail = false;
+#pragma unroll
+                        for (int u = 0; u < AT_ONCE; u++) {
+                            const float *src = at(min(j0 + 8 * u, n - 1));
+                            ml[u] = take16(src);
+                            v[u] = take16(src + 4 + 4 * d4);
+                        }
+#pragma unroll
+                        for (int u = 0; u < AT_ONCE; u++) fail = fail || !(here(ml[u]) && here(v[u]));
+                    } while (fail && ++tries < p.wait_limit);
+#pragma unroll
+                    for (int u = 0; u < AT_ONCE; u++) {
+                        if (j0 + 8 * u >= n) break;
+                        const float4 x = as_f4(v[u]);
+                        const float mj = __uint_as_float(ml[u].x), lj = __uint_as_float(ml[u].y);
+                        const float m_new = fmaxf(m_run, mj), f0 = m_run == -INFINITY ? 0.f : expf(m_run - m_new), f1 = mj == -INFINITY ? 0.f : expf(mj - m_new);
+                        a.x = a.x * f0 + x.x * f1; a.y = a.y * f0 + x.y * f1; a.z = a.z * f0 + x.z * f1; a.w = a.w * f0 + x.w * f1;
+                        l_run = l_run * f0 + lj * f1;
+                        m_run = m_new;
                     }
-                    const float4 x = as_f4(v);
-                    const float mj = __uint_as_float(ml.x), lj = __uint_as_float(ml.y);
-                    if (j + 8 < n) {   // (the next one's trip passes meanwhile)
-                        ml = take16(at(j + 8));
-                        v = take16(at(j + 8) + 4 + 4 * d4);
-                    }
-                    const float m_new = fmaxf(m_run, mj), f0 = m_run == -INFINITY ? 0.f : expf(m_run - m_new), f1 = mj == -INFINITY ? 0.f : expf(mj - m_new);
-                    a.x = a.x * f0 + x.x * f1; a.y = a.y * f0 + x.y * f1; a.z = a.z * f0 + x.z * f1; a.w = a.w * f0 + x.w * f1;
-                    l_run = l_run * f0 + lj * f1;
-                    m_run = m_new;
                 }
                 float *grp_s = reinterpret_cast<float *>(work);   // [8]: {max, sum, -, -}, 256 sums; then room for the transform
                 *reinterpret_cast<float4 *>(grp_s + grp * PROW + 4 + 4 * d4) = a;
@@ -764,15 +770,29 @@ expired:   // a wait ran out: this CTA leaves, and the waits of the others run o
 
 int cdiv(int a, int b) { return (a + b - 1) / b; }
 
-// Splits of a layer's keys: a block of 64 per split where the window is short and lanes are few; never more than 32 (the merge takes
-// its time, too) nor more than there are CTAs.
+// Blocks of 64 keys that a layer's attention reads of a lane at most.
+int blocks_of(uint32_t window, uint32_t lane_rows) { return (int)(((window && window < lane_rows ? window : lane_rows) + 63u) / 64u); }
+// Splits of a layer's keys: a block per split where the window is short and lanes are few; up to 32 of them, and for more than four
+// blocks in each as many as there are CTAs.  (Never more than 32: a step of one lane at 131072 keys took 1589 us, now 1025; at 32768 1023 and 899.)
 int splits_of(int ctas, int m, int n_q, uint32_t window, uint32_t lane_rows) {
-    const uint32_t span = window && window < lane_rows ? window : lane_rows;
-    const int most = ctas / (m * n_q / 8) - 1, blocks = (int)((span + 63) / 64);
+    const int most = ctas / (m * n_q / 8) - 1, blocks = blocks_of(window, lane_rows);
     int s = blocks <= 8 && m > 2 ? (blocks + 1) / 2 : blocks;
-    if (s > 32) s = 32;
+    if (s > FEW_SPLITS) s = blocks > FEW_SPLITS * FULL_SPLIT ? cdiv(blocks, FULL_SPLIT) : FEW_SPLITS;
     if (s > most) s = most;
     return s < 1 ? 1 : s;
+}
+// Whether the launches of run_layers take less time at full contexts, which is what the host knows of them.  A block of keys of a split takes
+// 1.05 us from the fifth on, more than the attention launch needs for its share of them; a layer saves 7.5 us of hand-over for one and two lanes,
+// 5.6 for three and 4.8 for four.  (One launch and launches, 35 layers of which 7 are full, tq2: two lanes x 131072 1189 and 1263 us; three x 65536
+// 1187 and 1251, x 131072 1434 and 1345; four x 32768 1124 and 1209, x 65536 1284 and 1272, x 131072 1611 and 1406.)
+bool launches_faster(int ctas, int m, int n_q, const LcStepLayer *layers, int n_layers) {
+    const float saved = (m <= 2 ? 7.5f : (m == 3 ? 5.6f : 4.8f)) * (float)n_layers;
+    int over = 0;
+    for (int i = 0; i < n_layers; i++) {
+        const int per = cdiv(blocks_of(layers[i].window, layers[i].lane_rows), splits_of(ctas, m, n_q, layers[i].window, layers[i].lane_rows));
+        over += per > FULL_SPLIT ? per - FULL_SPLIT : 0;
+    }
+    return 1.05f * (float)over > saved;
 }
 size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 
@@ -786,7 +806,7 @@ int launch_step(lc_kernels *k, lc_batch *b, LcStepParams &p) {
     const int rb_h = H / 256 * 66, rb_o = (p.inter > p.n_q * HD ? p.inter : p.n_q * HD) / 256 * 66;
     const int ta = p.inter / 8 > (p.n_q + 2 * p.n_kv) * 16 ? p.inter / 8 : (p.n_q + 2 * p.n_kv) * 16;
     const int na = cdiv(ta, ctas);
-    if (H / 16 > ctas) return -1;
+    if (H / 16 > ctas || launches_faster(ctas, m, p.n_q, p.layer, p.n_layers)) return -1;
     int at = C::LUT_BYTES + C::Q_BYTES + HD * 4 + up(4 * H + na * 16 * rb_h);
     p.off_b = at;
     at += up(16 * rb_o);

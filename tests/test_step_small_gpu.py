@@ -44,38 +44,80 @@ def differing_bytes(gm, om):
                for i, pool in enumerate(om.pools) for name in ("k_codes", "v_codes", "k_norms", "v_norms"))
 
 
+def check_step(la, orc, ctx, gm, om, tokens, positions):
+    """One step against the oracle's from the same pools; whether the rows that it wrote came out byte-identical."""
+    cfg, lanes = gm.cfg, len(tokens)
+    sync_pools(gm, om)
+    want, want_h = om.decode_batch_step(tokens, positions)
+    b = la.CommandBatch.new(ctx)
+    tb, pb, nt = la.CudaBuffer.from_slice(ctx, tokens), la.CudaBuffer.from_slice(ctx, positions), la.CudaBuffer.empty(ctx, lanes * 4)
+    gm.decode_batch_step_into(b, tb, pb, lanes, True, nt)
+    assert b.dispatch_count() == 3   # the layers, vocabulary, argmax
+    b.commit_and_wait()
+    got = gm.logits_buffer().as_slice(np.float32, lanes * cfg.vocab).reshape(lanes, cfg.vocab)
+    got_h = gm.hidden_buffer().as_slice(np.float16, lanes * cfg.hidden).reshape(lanes, cfg.hidden).astype(np.float32)
+    mism = differing_bytes(gm, om)
+    assert np.all(np.isfinite(got))
+    scale = max(1.0, float(np.abs(want).max()))
+    tol = 2e-3 if mism == 0 else 0.15
+    err = float(np.abs(got - want).max()) / scale
+    assert err <= tol, f"logits off by {err:.3e} of scale with {mism} differing KV bytes"
+    argmax_consistent(nt.as_slice(np.uint32), want, tol * scale)
+    assert mism <= 0.01 * cfg.n_layers * 2 * lanes * cfg.n_kv_heads * (cfg.head_dim * cfg.kv_bits // 8 + 2) + 4
+    if mism == 0:
+        assert np.abs(got_h - want_h.astype(np.float32)).max() <= 4e-3 * max(1.0, float(np.abs(want_h.astype(np.float32)).max()))
+    return mism == 0
+
+
 @pytest.mark.parametrize("lanes,bits,n_kv", [(1, 2, 1), (2, 2, 1), (3, 2, 2), (4, 2, 1), (1, 3, 1), (4, 3, 1), (2, 4, 2), (4, 4, 1)])
 def test_against_the_oracle(la, orc, ctx, kernels, lanes, bits, n_kv):
-    """Positions: the first key of a lane, a tile's edges, a split's edges (256 keys), a ring before and after it wrapped."""
+    """Positions: the first key of a lane, the edges of blocks of 64 keys (a split is one or two of them), a ring before and after it wrapped."""
     cfg = cfg_of(la, lanes, bits, n_kv)
     gm, om = models(la, orc, ctx, kernels, cfg, 650)
     rng = np.random.default_rng(40 + lanes)
-    edges = [0, 1, 31, 32, 255, 256, 257, 511, 512, 513, 649]
+    edges = [0, 1, 63, 64, 255, 256, 257, 511, 512, 513, 649]
     exact = 0
     for step in range(5):
         tokens = rng.integers(0, cfg.vocab, lanes).astype(np.uint32)
         positions = np.array([edges[(step * lanes + i) % len(edges)] for i in range(lanes)], np.uint32)
-        sync_pools(gm, om)
-        want, want_h = om.decode_batch_step(tokens, positions)
-        b = la.CommandBatch.new(ctx)
-        tb, pb, nt = la.CudaBuffer.from_slice(ctx, tokens), la.CudaBuffer.from_slice(ctx, positions), la.CudaBuffer.empty(ctx, lanes * 4)
-        gm.decode_batch_step_into(b, tb, pb, lanes, True, nt)
-        assert b.dispatch_count() == 3   # the layers, vocabulary, argmax
-        b.commit_and_wait()
-        got = gm.logits_buffer().as_slice(np.float32, lanes * cfg.vocab).reshape(lanes, cfg.vocab)
-        got_h = gm.hidden_buffer().as_slice(np.float16, lanes * cfg.hidden).reshape(lanes, cfg.hidden).astype(np.float32)
-        mism = differing_bytes(gm, om)
-        assert np.all(np.isfinite(got))
-        scale = max(1.0, float(np.abs(want).max()))
-        tol = 2e-3 if mism == 0 else 0.15
-        err = float(np.abs(got - want).max()) / scale
-        assert err <= tol, f"step {step}: logits off by {err:.3e} of scale with {mism} differing KV bytes"
-        argmax_consistent(nt.as_slice(np.uint32), want, tol * scale)
-        assert mism <= 0.01 * cfg.n_layers * 2 * lanes * n_kv * (cfg.head_dim * bits // 8 + 2) + 4
-        if mism == 0:
-            exact += 1
-            assert np.abs(got_h - want_h.astype(np.float32)).max() <= 4e-3 * max(1.0, float(np.abs(want_h.astype(np.float32)).max()))
+        exact += check_step(la, orc, ctx, gm, om, tokens, positions)
     assert exact >= 1 or lanes * n_kv > 1   # (a written coordinate in a thousand sits on a level's edge)
+    device_status_ok(kernels)
+
+
+@pytest.mark.parametrize("lanes,n_kv,context,positions,bits", [
+    # eight splits of up to eight blocks: more than the ring of blocks in shared memory holds (five at two bits, three above)
+    (4, 4, 4096, ((4095, 4000, 2049, 3), (64, 1700, 4095, 511)), 2),
+    (4, 4, 4096, ((4095, 4000, 2049, 3), (64, 1700, 4095, 511)), 3),
+    (4, 4, 4096, ((4095, 4000, 2049, 3), (64, 1700, 4095, 511)), 4),
+    # more than 32 splits: 64 of four blocks, 147 of five (the last ones empty); short contexts of the same lane keep few
+    (1, 1, 16384, ((16383,), (8193,), (8192,), (300,)), 2),
+    (1, 1, 40000, ((39999,), (38000,), (0,)), 2),
+    (1, 1, 40000, ((39999,), (9001,)), 4),
+    (2, 1, 30000, ((29999, 17), (12000, 29000)), 3),
+])
+def test_long_contexts(la, orc, ctx, kernels, lanes, n_kv, context, positions, bits):
+    cfg = cfg_of(la, lanes, bits, n_kv, context=context)
+    gm, om = models(la, orc, ctx, kernels, cfg, context)
+    rng = np.random.default_rng(60 + lanes)
+    for row in positions:
+        check_step(la, orc, ctx, gm, om, rng.integers(0, cfg.vocab, lanes).astype(np.uint32), np.array(row, np.uint32))
+    device_status_ok(kernels)
+
+
+@pytest.mark.parametrize("lanes,context,one", [(4, 4096, True), (4, 65536, False), (2, 65536, False), (2, 16384, True), (1, 65536, True)])
+def test_full_layers_whose_keys_the_launches_read_sooner(la, ctx, kernels, lanes, context, one):
+    """All layers full: the form follows from the most keys that a split can have."""
+    cfg = cfg_of(la, lanes, context=context, ring=0, window=0, n_layers=2)
+    gm = la.DecodeModel(ctx, kernels, cfg)
+    for i in range(cfg.n_layers):
+        gm.set_layer(i, la.model.synth_layer(cfg, i, seed=31))
+    gm.set_embedding(*la.model.synth_embedding(cfg, seed=31))
+    b = la.CommandBatch.new(ctx)
+    gm.decode_batch_step_into(b, la.CudaBuffer.from_slice(ctx, np.zeros(lanes, np.uint32)), la.CudaBuffer.from_slice(ctx, np.zeros(lanes, np.uint32)), lanes)
+    assert (b.dispatch_count() == 2) == one
+    b.commit_and_wait()
+    gm.close()
     device_status_ok(kernels)
 
 
