@@ -290,7 +290,7 @@ int lc_buf_fill(lc_buf *buf, size_t offset, size_t bytes, int value) {
 
 // ------------------------------------------------- launches side by side --
 LcOrder::LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, const lc_buf *const *weights, const size_t *w_bytes,
-                 lc_buf *const *outputs, const size_t *out_bytes)
+                 lc_buf *const *outputs, const size_t *out_bytes, bool brief)
     : ctx(b->ctx) {
     lc_overlap &o = ctx->overlap;
     constexpr int MOST_READS = sizeof(o.reads) / sizeof(lc_range), MOST_WRITES = sizeof(o.writes) / sizeof(lc_range);
@@ -315,7 +315,8 @@ LcOrder::LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, cons
     };
     const lc_range in = range(input, in_bytes);
     const bool room = o.n_reads + 1 + ng <= MOST_READS && o.n_writes + ng <= MOST_WRITES;
-    bool apart = o.state != 0 && !meets(in, o.write_span, o.writes, o.n_writes), weights_apart = true;
+    const bool starts = b->capturing || !(brief && o.brief);
+    bool apart = (o.state == 2 || (o.state == 1 && starts)) && !meets(in, o.write_span, o.writes, o.n_writes), weights_apart = true;
     for (int g = 0; g < ng; g++) {
         const lc_range w = range(weights[g], w_bytes[g]), out = range(outputs[g], out_bytes[g]);
         weights_apart = weights_apart && !meets(w, o.write_span, o.writes, o.n_writes);
@@ -335,6 +336,7 @@ LcOrder::LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, cons
         o.state = apart ? 2 : 1;
         o.n_reads = o.n_writes = 0;
     }
+    o.brief = brief;
     b->last_order = flags;
     auto add = [](const lc_range &r, lc_range &span, lc_range *v, int &n) {
         span = n == 0 ? r : lc_range{r.lo < span.lo ? r.lo : span.lo, r.hi > span.hi ? r.hi : span.hi};

@@ -17,6 +17,7 @@ struct lc_range {
 struct lc_overlap {
     std::mutex mu;           // held from the decision about a launch until it is enqueued
     bool beside = false;     // the last launch runs beside others
+    bool brief = false;      // the last launch recorded here takes the host longer than the GPU
     int state = 0;           // 0: nothing known, 1: `reads` / `writes` are the last launch's, 2: those of every launch that may be running
     int n_reads = 0, n_writes = 0;
     lc_range reads[192], writes[96];   // (when they are full the run starts anew)
@@ -193,15 +194,16 @@ static inline cudaError_t lc_launch(void (*kern)(KArgs...), dim3 grid, dim3 bloc
 //     of a run is complete (`serial`).
 // Whatever else the library puts on the stream ends the run, too (lc_order_break: copies, memsets, collectives, graphs, capture
 // boundaries), and a program that takes the stream for work of its own has no runs at all (lc_ctx_stream).  Ranges are virtual addresses: memory mapped twice is not recognised.
-// (The line lies at the bytes and nowhere else: 35 matrices of 8192 x 1536 TQ2_0 times 16 rows took 225 us one after the
+// (35 matrices of 8192 x 1536 TQ2_0 times 16 rows took 225 us one after the
 // other and take 98 side by side, 35 of Q4_0 6144 x 1536 times 40 rows 348 and 269, 35 of Q4_0 8192 x
-// 1536 times one row 206 and 113.  Where the host sets the pace, at matrices of a megabyte or so and one row, the look at the ranges costs about 0.07
-// us a launch: 35 of 3740 x 768 in 139.0 us and 139.9, of 1024 x 512 in 97.6 and 101.8.)
+// 1536 times one row 206 and 113.  `brief`: outside a capture the host takes longer to enqueue the launch than the GPU to run it, so there is
+// nothing to hide, while launches side by side cost the host 0.05 to 0.1 us each, of which the look at the ranges is 0.015; two such launches
+// start no run.  35 of 1024 x 512 TQ2_0 times one row 94.7 us one after the other, 101 side by side.)
 constexpr uint32_t LC_LATE_TRIGGER = 1, LC_LATE_WAIT = 2;
 class LcOrder {
 public:
     LcOrder(lc_batch *b, const lc_buf *input, size_t in_bytes, int ng, const lc_buf *const *weights, const size_t *w_bytes,
-            lc_buf *const *outputs, const size_t *out_bytes);
+            lc_buf *const *outputs, const size_t *out_bytes, bool brief = false);
     ~LcOrder();
     uint32_t flags = 0;      // for the kernel
     bool serial = false;     // for the launch

@@ -368,7 +368,13 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
         w_bytes[g] = rb * ns[g];
         out_bytes[g] = (size_t)m * ns[g] * (f32out ? 4 : 2);
     }
-    LcOrder order(b, input, (size_t)m * kk * 2, ng, weights, w_bytes, outputs, out_bytes);
+    // Weights up to which 35 such launches one after the other keep up with the host (2.5 us each).  On the lines' two sides, side by side against
+    // that: Q4_0, 2.1 M 1.02 / 3.1 M 0.77 at up to four rows, 1.6 M 1.02 / 2.1 M 0.79 at eight, 0.5 M 0.89 at sixteen; TQ2_0, 3.1 M 1.02 / 4.2 M 0.94 at up to
+    // eight, 1.6 M 1.04 / 2.1 M 0.98 at sixteen.
+    const size_t host_paced = fmt == FMT_Q4_0 ? (m <= 4 ? 5u << 19 : m <= 8 ? 7u << 18 : 3u << 17) : (m <= 8 ? 7u << 19 : 7u << 18);
+    size_t n_all = 0;
+    for (int g = 0; g < ng; g++) n_all += ns[g];
+    LcOrder order(b, input, (size_t)m * kk * 2, ng, weights, w_bytes, outputs, out_bytes, n_all * kk <= host_paced);
     p.order = order.flags;
     int st;
     if (geglu) st = launch_nt<FMT_TQ2_0, true, __half>(b, order.serial, p, tiles, rows);

@@ -20,13 +20,14 @@ int main() {
         uint32_t flags = 0, serial = 0;
         if (kind == 'm') {
             size_t at[3];
+            int brief;
             lc_buf bufs[3];
-            if (scanf("%zu %zu %zu", &at[0], &at[1], &at[2]) != 3) return 1;
+            if (scanf("%zu %zu %zu %d", &at[0], &at[1], &at[2], &brief) != 4) return 1;
             for (int i = 0; i < 3; i++) bufs[i].dptr = (void *)(at[i] * 16 + 4096);
             const lc_buf *w = &bufs[1];
             lc_buf *out = &bufs[2];
             const size_t n = 16;
-            LcOrder o(&b, &bufs[0], n, 1, &w, &n, &out, &n);
+            LcOrder o(&b, &bufs[0], n, 1, &w, &n, &out, &n, brief);
             flags = o.flags;
             serial = o.serial;
             o.launched = true;
@@ -76,13 +77,13 @@ def conflicts(ops, orders):
             data, trig, end = i, start, i
         if op[0] == "m":
             for j in range(data, i):
-                if ops[j][0] in "pf" or {op[1], op[2]} & {ops[j][3]} or op[3] in ops[j][1:]:
+                if ops[j][0] in "pf" or ops[j][3] in op[1:3] or op[3] in ops[j][1:4]:
                     bad.append((i, j))
     return bad
 
 
 def matmul(rng, spots):
-    return ("m", rng.randrange(spots), 1000 + rng.randrange(3), rng.randrange(spots))
+    return ("m", rng.randrange(spots), 1000 + rng.randrange(3), rng.randrange(spots), int(rng.random() < 0.3))
 
 
 @pytest.mark.parametrize("spots", [4, 12, 400])
@@ -98,7 +99,7 @@ def test_nothing_meets(decide, spots):
 
 
 def test_other_work_ends_a_run(decide):
-    run = [("m", 1, 1000, 10 + i) for i in range(4)]
+    run = [("m", 1, 1000, 10 + i, 0) for i in range(4)]
     for kind in "pcf":
         orders = decide(run + [(kind,)] + run)
         assert [f for f, _ in orders] == [0, 1, 2, 2, 0, 0, 1, 2, 2]
@@ -109,8 +110,16 @@ def test_other_work_ends_a_run(decide):
 def test_a_full_list(decide):
     """The lists hold 96 writes.  A launch that finds them full and meets the run starts when the run is complete, since the next one
     knows only of it."""
-    ops = [("m", 1, 1000, 10 + i) for i in range(97)]
-    ops += [("m", 50, 1000, 200), ("m", 1, 60, 300)]
+    ops = [("m", 1, 1000, 10 + i, 0) for i in range(97)]
+    ops += [("m", 50, 1000, 200, 0), ("m", 1, 60, 300, 0)]
     orders = decide(ops)
     assert [f for f, _ in orders][:97] == [0] + [1] + [2] * 95
     assert not conflicts(ops, orders) and orders[97] == (0, 1)
+
+
+def test_brief_launches_start_no_run(decide):
+    """Two launches that the host enqueues more slowly than the GPU runs them stay one behind the other; beside a longer one they do not."""
+    run = [("m", 1, 1000, 10 + i, 1) for i in range(4)]
+    assert decide(run) == [(0, 0)] * 4
+    assert [f for f, _ in decide([("m", 1, 1000, 9, 0)] + run)] == [0, 1, 2, 2, 2]
+    assert [f for f, _ in decide(run + [("m", 1, 1000, 9, 0)] + run[:2])] == [0, 0, 0, 0, 1, 2, 2]

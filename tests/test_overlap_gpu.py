@@ -112,7 +112,7 @@ def test_other_launches_end_a_run(la, ctx, kernels):
 def test_order_behind_other_work(la, ctx, kernels, work):
     """A matmul runs beside those before it only while nothing but matmuls stands between: behind every other kind of work on the stream it
     waits, also where that work declares no buffers of its own."""
-    m, n = 16, 512
+    m, n = 16, 4096
     x = la.CudaBuffer.from_slice(ctx, la.synth.normal_f16((m, K), 95))
     ws = [la.CudaBuffer.from_slice(ctx, la.synth.tq2_0_weights(n, K, seed=96 + i)) for i in range(3)]
     outs = [la.CudaBuffer.empty(ctx, m * n * 2) for _ in range(4)]
@@ -154,13 +154,13 @@ def test_order_behind_other_work(la, ctx, kernels, work):
 def test_no_runs_once_the_stream_is_out(la):
     own = la.CudaContext.new(0)
     kernels = la.Kernels.new(own)
-    x, w = la.CudaBuffer.from_slice(own, la.synth.normal_f16((16, K), 97)), la.CudaBuffer.from_slice(own, la.synth.tq2_0_weights(512, K, seed=98))
-    outs = [la.CudaBuffer.empty(own, 16 * 512 * 2) for _ in range(3)]
+    x, w = la.CudaBuffer.from_slice(own, la.synth.normal_f16((16, K), 97)), la.CudaBuffer.from_slice(own, la.synth.tq2_0_weights(4096, K, seed=98))
+    outs = [la.CudaBuffer.empty(own, 16 * 4096 * 2) for _ in range(3)]
 
     def orders():
         b, got = la.CommandBatch.new(own), []
         for o in outs:
-            kernels.matmul_nt_tq2_0_into(b, x, w, o, 16, K, 512)
+            kernels.matmul_nt_tq2_0_into(b, x, w, o, 16, K, 4096)
             got.append(b.last_order())
         b.commit_and_wait()
         return got
