@@ -1,5 +1,5 @@
-// Quantized weights on mma.sync at few batch rows (qmatmul_sm.cu; step_small.cu): two codes to two f16 in two instructions, and the
-// GeGLU epilogue.
+// Quantized weights on mma.sync (the streaming matvec, the small-batch matmul and the one-launch step): two codes to two f16 in two
+// instructions; and the GeGLU epilogue of every kernel that has one.
 #pragma once
 #include "tcgen05_util.cuh"
 
@@ -13,7 +13,8 @@ __device__ __forceinline__ float geglu_f(float gate, float up) {
     inner = fminf(fmaxf(inner, -10.0f), 10.0f);
     return 0.5f * x * (1.0f + tanhf(inner)) * u;
 }
-// two codes, BITS wide at bit BITS * l of each half of w, as f16 (q - Z) 2^-9
+// two codes, BITS wide at bit BITS * l of each half of w, as f16 (q - Z) 2^-9: in place they are the f16 subnormals
+// q 2^(BITS l - 24), which one multiply-add moves to the common scale, exactly
 template <int BITS, int Z>
 __device__ __forceinline__ uint32_t codes_f16(uint32_t w, int l) {
     constexpr uint32_t one = (1u << BITS) - 1u;

@@ -26,6 +26,7 @@
 // the weights keep the f32 value d (q - 8) the reference's kernels use (shaders/matvec_quant.metal:25,477-506).
 // Accumulation is f32.
 #include "lc_internal.h"
+#include "qm_codes.cuh"
 
 namespace {
 
@@ -53,7 +54,6 @@ struct MmaParams {
     int geglu;             // 1: w[0] = gate, w[1] = up, out[0] = gelu(gate) * up (see lc_qgemm_mma_geglu)
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t src_bytes = 16u) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
@@ -77,16 +77,6 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(addr));
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ float4 ld_dsmem_f4(uint32_t local_addr, uint32_t rank) {
-    uint32_t ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(local_addr), "r"(rank));
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ra));
-    return v;
 }
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t *>(&h); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<__half2 *>(&u); }
@@ -283,21 +273,13 @@ __global__ void __launch_bounds__(NT) qgemm_mma_kernel(const MmaParams p) {
             if (row < n_rows && col < p.m) store_c(out + (size_t)col * n_rows + row, e4[e]);
         }
     };
-    // GeGLU: gate and up are rounded to f16 as the separate projections would store them, then
-    // gelu_tanh(gate) * up exactly as the element-wise kernel computes it (gelu.metal, layer.rs:825-838)
-    auto geglu = [](float gate, float up) {
-        const float x = __half2float(__float2half_rn(gate)), u = __half2float(__float2half_rn(up));
-        float inner = 0.7978845608f * (x + 0.044715f * (x * x * x));
-        inner = fminf(fmaxf(inner, -10.0f), 10.0f);
-        return 0.5f * x * (1.0f + tanhf(inner)) * u;
-    };
     auto store_geglu = [&](const float4 gt, const float4 up, int w, int ln, int j) {   // w = 0..3: gate warp
         const int row0 = (int)blockIdx.x * (CTA_ROWS / 2) + w * WROWS + (ln >> 2), col0 = 8 * j + 2 * (ln & 3);
         const float g4[4] = {gt.x, gt.y, gt.z, gt.w}, u4[4] = {up.x, up.y, up.z, up.w};
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             const int row = row0 + 8 * (e >> 1), col = col0 + (e & 1);
-            if (row < n_rows && col < p.m) store_c(out + (size_t)col * n_rows + row, geglu(g4[e], u4[e]));
+            if (row < n_rows && col < p.m) store_c(out + (size_t)col * n_rows + row, geglu_f(g4[e], u4[e]));
         }
     };
     float4 *red = reinterpret_cast<float4 *>(x_s);           // [NBT][NT]

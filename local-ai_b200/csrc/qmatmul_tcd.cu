@@ -48,6 +48,7 @@
 #include <stdlib.h>
 
 #include "lc_internal.h"
+#include "qm_codes.cuh"
 #include "tcgen05_util.cuh"
 
 namespace {
@@ -90,14 +91,6 @@ struct TcdParams {
     uint32_t extra_arrivals;   // 0; 1 in the expiry self-test: the "weights ready" barriers then expect an arrival nobody makes
 };
 
-// gelu_tanh(gate) * up with gate and up rounded to f16 first, as the separate projections would store them, and the
-// element-wise kernel's arithmetic (shaders/gelu.metal:23-37)
-__device__ __forceinline__ float geglu_f(float gate, float up) {
-    const float x = __half2float(__float2half_rn(gate)), u = __half2float(__float2half_rn(up));
-    float inner = 0.7978845608f * (x + 0.044715f * (x * x * x));
-    inner = fminf(fmaxf(inner, -10.0f), 10.0f);
-    return 0.5f * x * (1.0f + tanhf(inner)) * u;
-}
 __device__ __forceinline__ uint2 pack4(float a, float b, float c, float d) {
     __half2 lo = __floats2half2_rn(a, b), hi = __floats2half2_rn(c, d);
     return make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));

@@ -284,8 +284,8 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
                     const uint64_t bj = bd + (uint64_t)(((uint32_t)((j >> 1) * B_TILE) + (uint32_t)((j & 1) * 64)) >> 4);
                     umma_f16_ta(acc, ta + (uint32_t)(16 * j), bj, idesc, (i > 0 || j > 0) ? 1u : 0u);
                     if (FMT == FMT_Q4_0) umma_f16_ta(acc, ta + (uint32_t)(64 + 16 * j), bj, idesc, 1u);
-            }
-            umma_commit(smem_u32(&step_done[i % NBAR]));
+                }
+                umma_commit(smem_u32(&step_done[i % NBAR]));
             }
             __syncwarp();
         }

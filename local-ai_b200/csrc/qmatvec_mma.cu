@@ -20,6 +20,7 @@
 // TQ2_0 gains more, as its conversion had a permute and a multiply per two weights: 90 matrices of 8192 x 1536 in one
 // launch 2.4 -> 1.6 us each.
 #include "lc_internal.h"
+#include "qm_codes.cuh"
 #include "tcgen05_util.cuh"
 
 namespace {
@@ -61,15 +62,6 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
 }
 __device__ __forceinline__ void ldmatrix_x2(uint32_t &b0, uint32_t &b1, uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];\n" : "=r"(b0), "=r"(b1) : "r"(addr));
-}
-// two codes, BITS wide at bit BITS * l of each half of w, as f16 (q - Z) 2^-9: in place they are the f16 subnormals
-// q 2^(BITS l - 24), which one multiply-add moves to the common scale, exactly
-template <int BITS, int Z>
-__device__ __forceinline__ uint32_t codes_f16(uint32_t w, int l) {
-    constexpr uint32_t one = (1u << BITS) - 1u;
-    const uint32_t v = w & ((one | one << 16) << (BITS * l));
-    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&v), __float2half2_rn((float)(1 << (15 - BITS * l))), __float2half2_rn(-(float)Z / 512.0f));
-    return *reinterpret_cast<const uint32_t *>(&r);
 }
 __device__ __forceinline__ void store_c(__half *p, float v) { *p = __float2half_rn(v); }
 __device__ __forceinline__ void store_c(float *p, float v) { *p = v; }
