@@ -22,11 +22,14 @@
  *    of batches that belong to different devices.
  *  - Kernels start copying their constant operands (weights, norm weights,
  *    levels, signs) while the previous kernel of the stream is still running
- *    (programmatic dependent launch).  Such a buffer must therefore not be
- *    written by the kernel enqueued immediately before the call that reads it as
- *    a constant operand; callers that build weights on the device in the preceding
- *    dispatch set LOCAL_CUDA_PDL=0 (no early start) or enqueue any other dispatch
- *    in between.  Activations, positions and KV pools carry no such rule.
+ *    (programmatic dependent launch), and a kernel lets its successor start before
+ *    it has waited itself.  Such a buffer must therefore not be written by a kernel
+ *    that may still be running when the call that reads it as a constant operand
+ *    starts, the one enqueued immediately before above all; callers that build
+ *    weights on the device wait for that batch, let a copy, a memset or a graph
+ *    launch stand in between (each is complete before the next kernel starts), or
+ *    set LOCAL_CUDA_PDL=0 (no early start).  Activations, positions and KV pools
+ *    carry no such rule.
  *  - Split-K scratch owned by an `lc_kernels` grows on demand, outside graph
  *    capture only.  A block that was handed out once stays allocated until
  *    lc_kernels_destroy, so a captured graph keeps working after later, larger

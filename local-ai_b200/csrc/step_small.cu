@@ -7,8 +7,8 @@
 //   norms, Q/K/V | attention over splits of the keys, K and V rows encoded on the way | merge of the splits | O | norms, gate, up | down
 //   * Every exchange buffer is written once per step, in 16-byte pieces, and starts out as all ones, which no piece of data is (f16
 //     and f32 conversions give no such NaN).  A consumer reads the pieces it needs until they are there.  There is no fence and no
-//     second trip for the data, and nothing is written twice, so nothing can be overwritten early.  (With a counter per phase, a
-//     release by every producer and an acquire by every consumer an exchange took 3700 cycles from the last store to the data;
+//     second trip for the data, and nothing is written twice, so nothing can be overwritten early.  (148 CTAs that post 32 bytes each
+//     and read all of them: 1960 cycles; 3050 with a counter, a release by every producer and an acquire by every consumer, since
 //     a fence waits for the stores' acknowledgements.)
 //   * The weights of a phase are brought into shared memory by bulk copies while the phases before it run (two regions: one for
 //     Q/K/V and gate/up, one for O and down), so HBM is read while the chain of small phases waits on itself.
@@ -17,12 +17,12 @@
 //   * Queries are normalised, turned, rotated and split where attention needs them, and the newest key is a split of its
 //     own, whose CTA encodes the row first: the KV-write launch is gone from the chain, too.
 //   * Code is kept short, its loops rolled: what a layer runs through once comes out of the instruction caches at one instruction
-//     per cycle from 8 KB, per 3 cycles from about 32 KB and per 5.6 cycles beyond (measured with straight runs of FFMA), whatever the
-//     number of warps.
-// What bounds it: latency, twelve times a layer (load, multiply, add up, post), about 22 us a layer.  35 layers at context 8192, with
-// the vocabulary and the greedy choice, before and now: 1145 and 870 us for one lane, 1140 and 857 for two, 1160 and 982 for four.  At
-// eight lanes it takes 1270 us and the launches 1258 (the norms of eight rows in every CTA, and the gate's rows, 98 KB, into each):
-// the line lies at four.
+//     per cycle from 8 KB, per 1.5 to 2.4 cycles from 16 to 32 KB and per 6 cycles from 64 KB (measured with straight runs of FFMA),
+//     whatever the number of warps.
+// What bounds it: latency, twelve times a layer (load, multiply, add up, post), about 23 us a layer.  35 layers at context 8192, with
+// the vocabulary and the greedy choice, as launches and as one: 1143 and 878 us for one lane, 1147 and 883 for two, 1163 and 967 for three, 1159
+// and 991 for four.  At eight lanes the launches are ahead, 1258 us against 1270 when that was measured (the norms of eight rows in every
+// CTA, and the gate's rows, 98 KB, into each): the line lies at four, and for long contexts below (launches_faster).
 // The arithmetic and its f16 rounding points are those of the launches; sums may be added in another order.
 #include <math.h>
 #include <stdlib.h>

@@ -76,7 +76,7 @@ def test_same_as_one_after_the_other(la, ctx, kernels, m, fmt, captured):
 
 
 def test_other_launches_end_a_run(la, ctx, kernels):
-    """Between projections on disjoint buffers stand launches that declare nothing (an addition in place, a copy): what follows them sees
+    """Between projections on disjoint buffers stand launches that declare nothing (additions, one in place): what follows them sees
     their results, and they see those of every projection before."""
     m, n = 16, 8192
     x = la.CudaBuffer.from_slice(ctx, la.synth.normal_f16((m, K), 70))
@@ -177,8 +177,8 @@ def test_no_runs_once_the_stream_is_out(la):
 
 
 def test_weights_written_two_dispatches_before(la, ctx, kernels):
-    """The header's rule for constant operands built on the device: any dispatch in between is enough, also where both are projections that
-    run beside others."""
+    """Constant operands written by a dispatch with another in between, where both are projections that run beside others: the launch behind the run
+    starts when all of them are complete."""
     m, n = 16, 4096
     x = la.CudaBuffer.from_slice(ctx, la.synth.normal_f16((m, K), 90))
     ws = [la.CudaBuffer.from_slice(ctx, la.synth.tq2_0_weights(n, K, seed=91 + i)) for i in range(6)]
