@@ -40,7 +40,13 @@ struct PfCfg {
     static constexpr int NUK = KN * UN / (DKW * 32), NUV = KN * UN / (DVW * 32);   // units per decoding thread
     static constexpr int FB = 2 * BITS, NENT = 1 << FB, COPIES = 8;   // table of two codes
     static constexpr int Q_PART = NB * M * 128, KV_PART = NB * KN * 128;
-    static constexpr int Q_OFF = 0, K_OFF = 2 * Q_PART, V_OFF = K_OFF + PARTS * KV_PART, LUT_OFF = V_OFF + PARTS * KV_PART;
+    // The query's f16 parts are A operands in tensor memory, but for the remainder at head_dim 256, which has no room there.
+    // K and V tiles have two buffers each.
+    static constexpr bool QL_SMEM = HD == 256;
+    static constexpr int SIDE = PARTS * KV_PART;                 // one tile of K or V
+    static constexpr int QL_OFF = 0, K_OFF = QL_SMEM ? Q_PART : 0, V_OFF = K_OFF + 2 * SIDE, LUT_OFF = V_OFF + 2 * SIDE;
+    // Before the first tile: signed query rows (until the transform has read them), and query parts on their way to tensor memory.
+    static constexpr int RAW_OFF = QL_SMEM ? QL_OFF : V_OFF, QST_OFF = K_OFF;
     static constexpr int LUT_BYTES = PARTS == 2 ? NENT * COPIES * 8 : 0;
     static constexpr int NORM_OFF = LUT_OFF + LUT_BYTES, NORM_BYTES = 4 * 2 * KN * 4;   // [4 tiles][k, v][KN]
     static constexpr int STAGE = M * (HD + 4) * 4;               // results, reuses the operand tiles
@@ -48,7 +54,10 @@ struct PfCfg {
     static constexpr int SMEM = (TAIL > STAGE ? TAIL : STAGE) + 256 + 1024;
     static constexpr int NVW = KN / 32;                          // warps that fetch a tile's V norms, one lane per key
     static_assert(NUK >= 1 && NUV >= 1 && SMEM <= 226 * 1024, "shared memory");
-    static constexpr int S_COL = 0, P_COL = 128, PL_COL = 160, O_COL = 256;   // tensor memory: S x 2, P, remainder of P, O
+    static_assert((QL_SMEM ? 1 : 2) * Q_PART <= 4 * SIDE && Q_PART <= 2 * SIDE && 64 * 128 <= 2 * SIDE, "what K's and V's place holds at first");
+    // Tensor memory: S x 2 (P and its remainder replace the S they come from), the query's two parts, O.
+    static constexpr int S_COL = 0, QH_COL = 128, QL_COL = 192, O_COL = 256;
+    static_assert(2 * KN <= QH_COL && QH_COL + HD / 2 <= (QL_SMEM ? O_COL : QL_COL) && O_COL + HD <= 512, "tensor memory");
 };
 
 __device__ __forceinline__ void umma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
@@ -77,6 +86,14 @@ __device__ __forceinline__ float pf_exp(float x) { return PARTS == 1 ? __expf(x)
 __device__ __forceinline__ void sts16(uint32_t a, const uint32_t (&v)[4]) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(a), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
+__device__ __forceinline__ void lds128(uint32_t a, uint32_t (&v)[4]) {
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a));
+}
+// four columns of this thread's row
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&v)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ uint2 lds64(uint32_t a) {
     uint2 v;
     asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "r"(a));
@@ -120,8 +137,11 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
     float *norms = reinterpret_cast<float *>(smem + C::NORM_OFF);
     constexpr int BAR_OFF = C::TAIL > C::STAGE ? C::TAIL : C::STAGE;
     const uint32_t bars = base + BAR_OFF;
-    const uint32_t k_full = bars, v_full = bars + 8, p_full = bars + 16, pv_done = bars + 24, qk_done = bars + 32, rot_done = bars + 56;   // qk_done: two
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + BAR_OFF + 48);
+    // two of each, of even and odd tiles: a side may be a tile ahead of a role that waits for it
+    const uint32_t k_full = bars, v_full = bars + 16, p_full = bars + 32, pv_done = bars + 48, qk_done = bars + 64, rot_done = bars + 80;
+    auto of_tile = [](uint32_t bar, int t) -> uint32_t { return bar + 8u * (uint32_t)(t & 1); };
+    auto phase_of = [](int t) -> uint32_t { return (uint32_t)((t >> 1) & 1); };
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + BAR_OFF + 96);
     volatile uint32_t *abort_flag = tmem_slot + 1;
     __shared__ float m_s[M], l_s[2][M], mx_s[2][2][M], vmax_s[4][C::NVW], gamma_s, cand_err[PF_NT / 32];
     __shared__ int cand_idx[PF_NT / 32];
@@ -148,12 +168,13 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid == 0) {
-        mbar_init(k_full, DKW + p.extra_arrivals);
-        mbar_init(v_full, DVW);
-        mbar_init(p_full, SMW);
-        mbar_init(pv_done, 1);
-        mbar_init(qk_done, 1);
-        mbar_init(qk_done + 8, 1);
+        for (uint32_t i = 0; i < 16; i += 8) {
+            mbar_init(k_full + i, DKW + p.extra_arrivals);
+            mbar_init(v_full + i, DVW);
+            mbar_init(p_full + i, SMW);
+            mbar_init(pv_done + i, 1);
+            mbar_init(qk_done + i, 1);
+        }
         mbar_init(rot_done, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -248,7 +269,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
 #pragma unroll
                     for (int i = 0; i < DPL / 4; i++) {
                         const int d = DPL * lane + 4 * i;
-                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(base + (uint32_t)(C::Q_OFF + (d >> 6) * M * 128 + r * 128 + ((((d & 63) >> 3) ^ (r & 7)) << 4) + (d & 4) * 2)),
+                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(base + (uint32_t)(C::RAW_OFF + (d >> 6) * M * 128 + r * 128 + ((((d & 63) >> 3) ^ (r & 7)) << 4) + (d & 4) * 2)),
                                      "r"(raw[j][i].x ^ flip[2 * i]), "r"(raw[j][i].y ^ flip[2 * i + 1])
                                      : "memory");
                     }
@@ -278,7 +299,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
                 for (int nb = 0; nb < NB; nb++)
 #pragma unroll
                     for (int j = 0; j < 4; j++)
-                        umma_ss(d_tmem + 64u * nb, make_desc(base + C::Q_OFF + nb * M * 128) + 2 * j, make_desc(base + C::K_OFF) + 2 * j, idesc, j > 0 ? 1u : 0u);
+                        umma_ss(d_tmem + 64u * nb, make_desc(base + C::RAW_OFF + nb * M * 128) + 2 * j, make_desc(base + C::K_OFF) + 2 * j, idesc, j > 0 ? 1u : 0u);
                 umma_commit(rot_done);
             }
             __syncwarp();
@@ -312,11 +333,12 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
                     uint32_t hi[4], lo[4];
 #pragma unroll
                     for (int i = 0; i < 4; i++) split2(__uint_as_float(v[nb][2 * i]) * f, __uint_as_float(v[nb][2 * i + 1]) * f, hi[i], lo[i]);
-                    const uint32_t off = base + (uint32_t)(C::Q_OFF + nb * M * 128 + r * 128 + ((c ^ (r & 7)) << 4));
-                    sts16(off, hi);
-                    sts16(off + C::Q_PART, lo);
+                    tmem_st4(tq - C::O_COL + C::QH_COL + 32 * nb + 4 * c, hi);
+                    if (C::QL_SMEM) sts16(base + (uint32_t)(C::QL_OFF + nb * M * 128 + r * 128 + ((c ^ (r & 7)) << 4)), lo);
+                    else tmem_st4(tq - C::O_COL + C::QL_COL + 32 * nb + 4 * c, lo);
                 }
             }
+            tmem_st_wait();
         }
     } else if (warp < MMA_WARP) {   // queries rotated already, or other signs
 #pragma unroll 1
@@ -373,19 +395,39 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
                 uint32_t hi[4], lo[4];
 #pragma unroll
                 for (int i = 0; i < 4; i++) split2(x[2 * i], x[2 * i + 1], hi[i], lo[i]);
-                const uint32_t off = base + (uint32_t)(C::Q_OFF + (lane >> 3) * M * 128 + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
-                sts16(off, hi);
-                sts16(off + C::Q_PART, lo);
+                const uint32_t off = base + (uint32_t)((lane >> 3) * M * 128 + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+                sts16(off + C::QST_OFF, hi);
+                sts16(off + (C::QL_SMEM ? C::QL_OFF : C::QST_OFF + C::Q_PART), lo);
             } else {
 #pragma unroll
                 for (int i = 0; i < DPL; i++) {
                     const int pos = tile_pos<C::PARTS>(DPL * lane + i), nb = pos >> 6, c = (pos & 63) >> 3;
                     const uint32_t off = (uint32_t)(nb * M * 128 + r * 128 + ((c ^ (r & 7)) << 4) + (pos & 7) * 2);
                     const __half hi = __float2half_rn(x[i]), lo = __float2half_rn(x[i] - __half2float(hi));
-                    *reinterpret_cast<__half *>(smem + C::Q_OFF + off) = hi;
-                    *reinterpret_cast<__half *>(smem + C::Q_OFF + C::Q_PART + off) = lo;
+                    *reinterpret_cast<__half *>(smem + C::QST_OFF + off) = hi;
+                    *reinterpret_cast<__half *>(smem + (C::QL_SMEM ? C::QL_OFF : C::QST_OFF + C::Q_PART) + off) = lo;
                 }
             }
+        }
+    }
+    if (!unit) {   // (the same for every warp)
+        __syncthreads();
+        if (warp < SMW) {   // into tensor memory: two threads per row, half of each block's columns each
+            const int half = warp >> 2, r = (warp & 3) * 32 + lane;
+            const uint32_t tq = *tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16);
+#pragma unroll 1
+            for (int e = 0; e < 4 * NB; e++) {
+                const int nb = e >> 2, c = 4 * half + (e & 3);
+                const uint32_t off = base + (uint32_t)(C::QST_OFF + nb * M * 128 + r * 128 + ((c ^ (r & 7)) << 4));
+                uint32_t v[4];
+                lds128(off, v);
+                tmem_st4(tq + C::QH_COL + 32 * nb + 4 * c, v);
+                if (!C::QL_SMEM) {
+                    lds128(off + C::Q_PART, v);
+                    tmem_st4(tq + C::QL_COL + 32 * nb + 4 * c, v);
+                }
+            }
+            tmem_st_wait();
         }
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -396,9 +438,9 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
 
     float m_ref = -INFINITY, l_sum = 0.f;   // softmax threads: reference maximum and sum of this thread's row
     // =========================== decoding warps: codes -> f16 operand tiles ===========================
-    // One side (K or V) by WARPS warps from warp `first`: `free_bar` completes when the side's tile of the step before has been
-    // read, `full` when this one's is in place.
-    auto decode_side = [&](auto WARPS, int first, const uint8_t *codes, bool with_norms, uint32_t tile, uint32_t full, auto free_wait) {
+    // One side (K or V) by WARPS warps from warp `first`, into two buffers at `tiles_at`: `read` completes when a tile has been read,
+    // `full` when one is in place.
+    auto decode_side = [&](auto WARPS, int first, const uint8_t *codes, bool with_norms, uint32_t tiles_at, uint32_t full, uint32_t read) {
         constexpr int ND = decltype(WARPS)::value * 32, NU = KN * C::UN / ND, W = C::UB / 4;   // threads, units of a thread, words of a unit
         const int dt = tid - first * 32;
         uint32_t raw[NU][W];
@@ -434,7 +476,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
             lut_hi = __byte_perm(l01, l23, 0x7531);
         }
         [[maybe_unused]] const uint32_t lut_lane = base + (uint32_t)C::LUT_OFF + (uint32_t)(lane & (C::COPIES - 1)) * 8u;
-        auto decode = [&](const uint32_t (&raw)[NU][W]) {
+        auto decode = [&](const uint32_t (&raw)[NU][W], uint32_t tile) {
 #pragma unroll
             for (int j = 0; j < NU; j++) {
                 const int u = dt + j * ND, key = (u & 7) | ((u / (8 * C::UN)) << 3), unit = (u >> 3) % C::UN;
@@ -488,27 +530,26 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
             for (int j = 0; j < NU; j++)
 #pragma unroll
                 for (int i = 0; i < W; i++) now[j][i] = raw[j][i];
-            if (with_norms && dt < 2 * KN) {   // (read before QK of tile t + 2 was issued)
-                norms[(t & 3) * 2 * KN + dt] = norm_next;
+            const float norm_now = norm_next;
+            if (t + 1 < tiles) fetch(t + 1);
+            if (t > 1 && !warp_wait(of_tile(read, t), phase_of(t - 2))) break;
+            if (with_norms && dt < 2 * KN) {   // (QK of tile t - 2 was issued after P of tile t - 4 was there: nobody reads that tile's norms)
+                norms[(t & 3) * 2 * KN + dt] = norm_now;
                 if (dt >= KN) {   // whole warps: the largest magnitude (as integers, so that a NaN is the largest)
-                    const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(norm_next)));
+                    const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(norm_now)));
                     if (lane == 0) vmax_s[t & 3][(dt - KN) / 32] = __uint_as_float(most);
                 }
             }
-            if (t + 1 < tiles) fetch(t + 1);
-            if (t > 0 && !free_wait(t - 1)) break;
-            decode(now);
+            decode(now, tiles_at + (uint32_t)((t & 1) * C::SIDE));
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(full);
+            if (lane == 0) mbar_arrive(of_tile(full, t));
         }
     };
     if (warp >= SMW && warp < SMW + DKW) {
-        decode_side(std::integral_constant<int, DKW>{}, SMW, p.kc, true, base + (uint32_t)C::K_OFF, k_full,
-                    [&](int t) { return warp_wait(qk_done + 8 * (t & 1), (uint32_t)((t >> 1) & 1)); });
+        decode_side(std::integral_constant<int, DKW>{}, SMW, p.kc, true, base + (uint32_t)C::K_OFF, k_full, qk_done);
     } else if (warp >= SMW + DKW && warp < MMA_WARP) {
-        decode_side(std::integral_constant<int, DVW>{}, SMW + DKW, p.vc, false, base + (uint32_t)C::V_OFF, v_full,
-                    [&](int t) { return warp_wait(pv_done, (uint32_t)(t & 1)); });
+        decode_side(std::integral_constant<int, DVW>{}, SMW + DKW, p.vc, false, base + (uint32_t)C::V_OFF, v_full, pv_done);
     } else if (warp == MMA_WARP) {
         // =========================== MMA issue ===========================
         // The whole warp runs the loop, so that descriptors stay in uniform registers; one lane issues (33 cycles per MMA at
@@ -519,44 +560,48 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
             const uint32_t id_pv = (1u << 4) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(M >> 4) << 24);   // B transposed
             bool dead = false;
             auto qk = [&](int t) {
-                if (!warp_wait(k_full, (uint32_t)(t & 1))) { dead = true; return; }
+                if (!warp_wait(of_tile(k_full, t), phase_of(t))) { dead = true; return; }
+                // S of tile t takes the place of P of tile t - 2, which PV reads
+                if (t > 1 && !warp_wait(of_tile(pv_done, t), phase_of(t - 2))) { dead = true; return; }
                 tc_fence_after();
-                const uint32_t s = tmem + (uint32_t)(C::S_COL + (t & 1) * KN);
+                const uint32_t s = tmem + (uint32_t)(C::S_COL + (t & 1) * KN), k_at = base + (uint32_t)(C::K_OFF + (t & 1) * C::SIDE);
 #pragma unroll
                 for (int nb = 0; nb < NB; nb++) {
-                    const uint64_t qh = make_desc(base + C::Q_OFF + nb * M * 128), ql = make_desc(base + C::Q_OFF + C::Q_PART + nb * M * 128);
-                    const uint64_t kh = make_desc(base + C::K_OFF + nb * KN * 128), kl = make_desc(base + C::K_OFF + C::KV_PART + nb * KN * 128);
+                    const uint64_t ql = make_desc(base + C::QL_OFF + nb * M * 128), kh = make_desc(k_at + nb * KN * 128), kl = make_desc(k_at + C::KV_PART + nb * KN * 128);
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {   // K = 16 slices: 32 bytes of the rows
+                    for (int j = 0; j < 4; j++) {   // K = 16 slices: 32 bytes of the rows, eight columns of tensor memory
                         if (leader) {
-                            umma_ss(s, qh + 2 * j, kh + 2 * j, id_qk, nb > 0 || j > 0 ? 1u : 0u);
-                            umma_ss(s, ql + 2 * j, kh + 2 * j, id_qk, 1u);
-                            if (C::PARTS == 2) umma_ss(s, qh + 2 * j, kl + 2 * j, id_qk, 1u);
+                            const uint32_t qc = tmem + (uint32_t)(C::QH_COL + 32 * nb + 8 * j);
+                            umma_f16_ta(s, qc, kh + 2 * j, id_qk, nb > 0 || j > 0 ? 1u : 0u);
+                            if constexpr (C::QL_SMEM) umma_ss(s, ql + 2 * j, kh + 2 * j, id_qk, 1u);
+                            else umma_f16_ta(s, qc - C::QH_COL + C::QL_COL, kh + 2 * j, id_qk, 1u);
+                            if (C::PARTS == 2) umma_f16_ta(s, qc, kl + 2 * j, id_qk, 1u);
                         }
                     }
                 }
-                if (leader) umma_commit(qk_done + 8 * (t & 1));
+                if (leader) umma_commit(of_tile(qk_done, t));
                 __syncwarp();
             };
             qk(0);
             for (int t = 0; t < tiles && !dead; t++) {
                 if (t + 1 < tiles) qk(t + 1);
-                if (dead || !warp_wait(v_full, (uint32_t)(t & 1)) || !warp_wait(p_full, (uint32_t)(t & 1))) { dead = true; break; }
+                if (dead || !warp_wait(of_tile(v_full, t), phase_of(t)) || !warp_wait(of_tile(p_full, t), phase_of(t))) { dead = true; break; }
                 tc_fence_after();
-                const uint64_t vh = make_desc_mn(base + C::V_OFF, KN * 128), vl = make_desc_mn(base + C::V_OFF + C::KV_PART, KN * 128);
+                const uint32_t v_at = base + (uint32_t)(C::V_OFF + (t & 1) * C::SIDE), pc = tmem + (uint32_t)(C::S_COL + (t & 1) * KN);
+                const uint64_t vh = make_desc_mn(v_at, KN * 128), vl = make_desc_mn(v_at + C::KV_PART, KN * 128);
 #pragma unroll
                 for (int j = 0; j < KN / 16; j++) {   // K = 16 keys: two groups of eight rows
                     const uint64_t off = (uint64_t)(2048 >> 4) * j;
                     if (leader) {
-                        umma_f16_ta(tmem + C::O_COL, tmem + C::P_COL + 8 * j, vh + off, id_pv, t > 0 || j > 0 ? 1u : 0u);
-                        if (C::PARTS == 2) umma_f16_ta(tmem + C::O_COL, tmem + C::PL_COL + 8 * j, vh + off, id_pv, 1u);
-                        if (C::PARTS == 2) umma_f16_ta(tmem + C::O_COL, tmem + C::P_COL + 8 * j, vl + off, id_pv, 1u);
+                        umma_f16_ta(tmem + C::O_COL, pc + 8 * j, vh + off, id_pv, t > 0 || j > 0 ? 1u : 0u);
+                        if (C::PARTS == 2) umma_f16_ta(tmem + C::O_COL, pc + KN / 2 + 8 * j, vh + off, id_pv, 1u);
+                        if (C::PARTS == 2) umma_f16_ta(tmem + C::O_COL, pc + 8 * j, vl + off, id_pv, 1u);
                     }
                 }
-                if (leader) umma_commit(pv_done);
+                if (leader) umma_commit(of_tile(pv_done, t));
                 __syncwarp();
             }
-            if (!dead) dead = !warp_wait(pv_done, (uint32_t)((tiles - 1) & 1));
+            if (!dead) dead = !warp_wait(of_tile(pv_done, tiles - 1), phase_of(tiles - 1));
             if (dead) *abort_flag = 1;
         }
         __syncwarp();
@@ -571,7 +616,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
         const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
         // (an expired wait does not leave the loop: the other softmax warps count on this one at their barrier)
         for (int t = 0; t < tiles; t++) {
-            warp_wait(qk_done + 8 * (t & 1), (uint32_t)((t >> 1) & 1));
+            warp_wait(of_tile(qk_done, t), phase_of(t));
             tc_fence_after();
             float s[KH];
             {
@@ -601,13 +646,15 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
             for (int i = 0; i < KH; i++) mx = fmaxf(mx, s[i]);
             // the row's other half (two buffers: a warp may be a tile ahead)
             mx_s[t & 1][half][r] = mx;
+            tc_fence_before();
             asm volatile("bar.sync 1, %0;\n" ::"n"(SMW * 32) : "memory");
+            tc_fence_after();
             mx = fmaxf(mx, mx_s[t & 1][half ^ 1][r]);
             if (t == 0) {
                 m_ref = mx;
             } else if (__any_sync(0xffffffffu, mx > m_ref + lag)) {
                 // the accumulator moves to the new maximum: PV of the tile before has to be complete
-                warp_wait(pv_done, (uint32_t)((t - 1) & 1));
+                warp_wait(of_tile(pv_done, t - 1), phase_of(t - 1));
                 tc_fence_after();
                 const float m_new = fmaxf(m_ref, mx), f = m_ref == -INFINITY ? 0.f : pf_exp<C::PARTS>(m_ref - m_new);
 #pragma unroll 1
@@ -619,7 +666,7 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
                     for (int i = 0; i < 16; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
                     tmem_st16(tq + (uint32_t)(C::O_COL + c), v);
                 }
-                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                tmem_st_wait();
                 l_sum *= f;
                 m_ref = m_new;
             }
@@ -638,26 +685,24 @@ __global__ void __launch_bounds__(PF_NT, 1) tq_attn_prefill_kernel(const TqAttnP
                     ph[i / 2 + 1] = pack2(e2 * n4.z, e3 * n4.w);
                 }
             }
-            if (t > 0) {   // P's columns are free
-                warp_wait(pv_done, (uint32_t)((t - 1) & 1));
-                tc_fence_after();
-            }
+            // P in the place of S, which every softmax warp has read (the barrier above)
+            const uint32_t pc = tq + (uint32_t)(C::S_COL + (t & 1) * KN + half * (KH / 2));
 #pragma unroll
             for (int c = 0; c < KH / 2; c += 8) {
                 uint32_t v[8];
 #pragma unroll
                 for (int i = 0; i < 8; i++) v[i] = ph[c + i];
-                tmem_st8(tq + (uint32_t)(C::P_COL + half * (KH / 2) + c), v);
+                tmem_st8(pc + c, v);
                 if constexpr (C::PARTS == 2) {
 #pragma unroll
                     for (int i = 0; i < 8; i++) v[i] = pl[c + i];
-                    tmem_st8(tq + (uint32_t)(C::PL_COL + half * (KH / 2) + c), v);
+                    tmem_st8(pc + KN / 2 + c, v);
                 }
             }
-            asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(p_full);
+            if (lane == 0) mbar_arrive(of_tile(p_full, t));
         }
         if (half == 0) m_s[r] = m_ref;
         l_s[half][r] = l_sum;
