@@ -50,6 +50,7 @@
 #include "lc_internal.h"
 #include "qm_codes.cuh"
 #include "tcgen05_util.cuh"
+#include "tensor_map.h"
 
 namespace {
 
@@ -408,25 +409,10 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
     lc_order_end<ORDERED>(p.order);
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point lookup (no link-time dependency on the driver).
-typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                    const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-encode_tiled_fn encode_tiled() {
-    static encode_tiled_fn fn = []() -> encode_tiled_fn {
-        void *ptr = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qr) != cudaSuccess || qr != cudaDriverEntryPointSuccess)
-            return nullptr;
-        return reinterpret_cast<encode_tiled_fn>(ptr);
-    }();
-    return fn;
-}
-
 // The activations x[m, K] (f16, row-major) as a 2-D tensor map: boxes of 64 k x 64 rows land as 64 rows of 128 bytes
 // with the 128-byte swizzle; rows beyond m read as zero.
 int make_x_map(CUtensorMap *map, const void *x, uint32_t m, uint32_t kk) {
-    encode_tiled_fn fn = encode_tiled();
+    lc_encode_tiled_fn fn = lc_encode_tiled();
     if (!fn) return lc_fail(LC_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
     const cuuint64_t dims[2] = {kk, m};
     const cuuint64_t strides[1] = {(cuuint64_t)kk * 2};

@@ -28,6 +28,7 @@
 
 #include "lc_internal.h"
 #include "tcgen05_util.cuh"
+#include "tensor_map.h"
 
 namespace {
 
@@ -322,20 +323,6 @@ qgemm_tcv_kernel(const __grid_constant__ TcvParams p, const __grid_constant__ CU
     }
 }
 
-typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                    const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-encode_tiled_fn encode_tiled() {
-    static encode_tiled_fn fn = []() -> encode_tiled_fn {
-        void *ptr = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qr) != cudaSuccess || qr != cudaDriverEntryPointSuccess)
-            return nullptr;
-        return reinterpret_cast<encode_tiled_fn>(ptr);
-    }();
-    return fn;
-}
-
 }  // namespace
 
 // One Q4_0 matrix [n, kk] against activations [m, kk], m <= 64, f32 out.  Returns LC_OK after a launch, a positive
@@ -349,7 +336,7 @@ int lc_qgemm_tcv_launch(lc_kernels *k, lc_batch *b, const lc_buf *input, const l
     if (n < (uint32_t)(V_ROWS * k->ctx->sm_count)) return -1;
     const size_t smem = (size_t)V_SB * V_B_SLOT + (size_t)V_RS * V_RAW_SLOT + (size_t)V_NB * V_ROWS * 4 + (2 * V_RS + V_SB + V_NBAR + 2) * 8 + 16 + 1024;
     if (smem > k->ctx->smem_optin) return -1;
-    encode_tiled_fn fn = encode_tiled();
+    lc_encode_tiled_fn fn = lc_encode_tiled();
     if (!fn) return -1;
     CUtensorMap x_map, w_map;
     {

@@ -396,6 +396,22 @@ def test_q4_0_wide_matrix_small_batch_keeps_exact_weights(la, orc, ctx, kernels,
         rel_close(y, want[0], 2e-4, "matvec_q4_0_f32out on a wide table")
 
 
+@pytest.mark.parametrize("m,k,n", [(1, 128, 18945), (1, 512, 18881), (1, 1920, 19001), (1, 2048, 18944), (2, 640, 19037), (2, 2048, 18945),
+                                   (3, 1024, 19000), (4, 1664, 18943), (5, 1536, 18945), (8, 2048, 18882)])
+def test_q4_0_streaming_columns(la, orc, ctx, kernels, m, k, n):
+    """The streaming kernel's MMA columns shared by 1, 2, 4 and 8 vectors and as many blocks as that leaves; quarters of K that end
+    inside a run of blocks or hold none; row pitches with and without the wider box; ragged last groups.  f32 sums over at most 2048
+    products against f64: 2e-4 of max(|want|, 1), as for the other widths."""
+    raw = la.synth.q4_0_weights(n, k, 63)
+    a = la.synth.normal_f16((m, k), 64)
+    x, w, out = la.CudaBuffer.from_slice(ctx, a), la.CudaBuffer.from_slice(ctx, raw), Guarded(la, ctx, m * n * 4)
+    b = la.CommandBatch.new(ctx)
+    kernels.matmul_nt_q4_0_f32out_into(b, x, w, out.view, m, k, n)
+    assert b.dispatch_count() == 1
+    b.commit_and_wait()
+    rel_close(out.read(np.float32), orc.matmul_nt(orc.Q4_0, a, raw, m, k, n), 2e-4, "streaming q4_0")
+
+
 @pytest.mark.parametrize("m,k,n", [(1, 256, 19000), (8, 512, 20001), (2, 1536, 19100)])
 def test_tq2_0_streaming_small_batch(la, orc, ctx, kernels, m, k, n):
     """Batch <= 8 over a TQ2_0 matrix with enough rows for the streaming tensor-core kernel (ragged last group)."""
