@@ -3,21 +3,23 @@
 // matmul_nt_{q4_0,tq2_0}_mma (shaders/matvec_quant.metal:447-577) at those sizes.
 //
 // A CTA computes 128 weight rows (the MMA's M) x NB <= 128 batch rows (its N) over a range of K, in steps that fill one weight
-// slot of 128 tensor-memory columns: 256 k of TQ2_0, or 128 k of Q4_0 as two f16 operands (the rounded weight and what the
+// slot of 64 tensor-memory columns: 128 k of TQ2_0, or 64 k of Q4_0 as two f16 operands (the rounded weight and what the
 // rounding dropped; their MMAs add up to the product with the exact weight).
-//   * two warps bring in the raw blocks of each step with 16-byte cp.async (rows are only 2-byte aligned: the enclosing
-//     16-byte range) into a ring of four slots.  (A bulk copy per row and step is too small for the copy engine: 128 of them
-//     took 9000 cycles.);
-//   * two groups of eight warps take alternate steps and turn raw blocks into f16 weights in the group's own slot of tensor
+//   * four warps bring in the raw blocks of two steps at a time with 16-byte cp.async (rows are only 2-byte aligned: the enclosing
+//     16-byte range) into a ring of four slots, from the kernel's first instruction on.  (A bulk copy per row is too small for the
+//     copy engine: 128 of them took 9000 cycles.);
+//   * four groups of four warps take a step in turn and turn raw blocks into f16 weights in the group's own slot of tensor
 //     memory (tcgen05.st; the MMA reads its A operand there, so the weights never pass through shared memory again);
 //   * one thread requests the step's activations, TMA boxes of 64 k x NB rows with the 128-byte swizzle;
-//   * two issuing threads, an accumulator of NB columns each, take alternate K = 16 slices and commit to the step's barrier.
-// Tensor memory: 2 x 128 accumulator columns + 2 x 128 weight columns.  Everything but the activations is independent of the
+//   * two issuing warps, an accumulator of NB columns each, take alternate steps and commit to the step's barrier.
+// Tensor memory: 2 x 128 accumulator columns + 4 x 64 weight columns.  Everything but the activations is independent of the
 // previous kernel and starts before the dependency wait.  Small outputs split K over a thread-block cluster; the partial tiles
 // are exchanged through distributed shared memory and added in split order (deterministic).
 //
-// What bounds it: a step's MMAs take 16 x 64 cycles at NB = 128, its stores into tensor memory about 900; the kernel this one
-// replaced unpacked through shared memory, ran every Q4_0 tile in two passes and reached 10 % of the tensor peak.
+// What bounds it: 512 x 16384 x 8192 TQ2_0 at 124 us (141 with two raw-block warps, two slots of twice the columns, shifts in place of
+// multiplies and results stored from tensor memory), 106 without the conversion, 122 without the MMAs, 127 without the stores into
+// tensor memory, 96 without conversion and MMAs: the activations, which every tile of rows fetches from L2, and the conversion's
+// integer instructions.  Small launches are bound by their fixed part, some 7000 cycles.
 // Every wait is bounded; on expiry the CTA records a status word and leaves.
 #include <stdlib.h>
 
@@ -31,19 +33,19 @@ constexpr int FMT_Q4_0 = 0, FMT_TQ2_0 = 1;
 constexpr int ROWS = 128;            // weight rows per CTA
 constexpr int MAX_NB = 128;
 constexpr int KT = 64;               // k per activation tile (128 bytes per row: the swizzle's width)
-constexpr int GROUPS = 2, GROUP_WARPS = 8, NDQ = GROUPS * GROUP_WARPS;
-constexpr int NISS = 2, NRAW = 2;
+constexpr int GROUPS = 4, GROUP_WARPS = 4, NDQ = GROUPS * GROUP_WARPS;
+constexpr int NISS = 2, NRAW = 4;
 constexpr int NT = (NDQ + NRAW + 1 + NISS) * 32;   // + raw loaders, activation loader, issuers
-constexpr int A_BASE = NISS * MAX_NB, A_COLS = 128, TMEM_COLS = A_BASE + GROUPS * A_COLS;   // 512
-constexpr int RAW_RS = 112;          // bytes per row and step: at most 72 data + 15 skew, rounded up; an odd multiple of 16
+constexpr int A_BASE = NISS * MAX_NB, A_COLS = 64, TMEM_COLS = A_BASE + GROUPS * A_COLS;   // 512
+constexpr int RAW_RS = 112;          // bytes per row and unit of two steps: at most 72 data + 15 skew, rounded up; an odd multiple of 16
 constexpr int RAW_SLOTS = 4, RAW_SLOT = ROWS * RAW_RS;
-constexpr int NBAR = 4;              // step barriers: more than the steps in flight
+constexpr int NBAR = 8;              // step barriers: more than the steps in flight
 constexpr int MAX_MATS = 3, MAX_KS = 8;
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 
 template <int FMT> struct TclFmt;
-template <> struct TclFmt<FMT_Q4_0> { static constexpr int step_k = 128, blocks = 4, bytes = 18, elems = 32; };
-template <> struct TclFmt<FMT_TQ2_0> { static constexpr int step_k = 256, blocks = 1, bytes = 66, elems = 256; };
+template <> struct TclFmt<FMT_Q4_0> { static constexpr int step_k = 64, unit_bytes = 4 * 18, block_bytes = 18; };
+template <> struct TclFmt<FMT_TQ2_0> { static constexpr int step_k = 128, unit_bytes = 66, block_bytes = 66; };
 
 struct TclParams {
     const uint8_t *w[MAX_MATS];
@@ -68,15 +70,60 @@ __device__ __forceinline__ void store_c4(__half *p, float4 v) {
 }
 __device__ __forceinline__ void store_c4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
 
+// The raw blocks of a step, by 16-byte cp.async: piece idx is number idx % 6 of row idx / 6 (six pieces hold 72 bytes at any alignment; the
+// last is left out where the row's skew lets five hold them).  Four warps and 32-bit addresses: two warps that checked each piece's end
+// took 1150 - 1900 cycles for what the rest of the kernel did in 800 (509 x 1536 x 6144 Q4_0 24.7 -> 21.5 us).
+template <int FMT>
+struct RawLoader {
+    static constexpr int UNIT_BYTES = TclFmt<FMT>::unit_bytes, PIECES = 6, PER_LANE = ROWS * PIECES / 32 / NRAW;
+    const uint8_t *tile;       // the tile's first row, 16-byte aligned: 128 rows of an even number of bytes
+    size_t left;               // bytes from there to the matrix's end
+    uint32_t off[PER_LANE];    // where the row's bytes of the next step start
+    uint32_t dst[PER_LANE], piece[PER_LANE];
+    bool inside;               // no piece reaches past the matrix
+    __device__ __forceinline__ void start(const uint8_t *w, size_t rb, int n0, int n_rows, int u0, int n_units, uint32_t raw, int t) {
+        tile = w + (size_t)n0 * rb;
+        left = (size_t)(n_rows - n0) * rb;
+        inside = (((size_t)(ROWS - 1) * rb + (size_t)(u0 + n_units) * UNIT_BYTES + 15) & ~(size_t)15) <= left;
+#pragma unroll
+        for (int j = 0; j < PER_LANE; j++) {
+            const int idx = j * NRAW * 32 + t, r = idx / PIECES, pc = idx - r * PIECES;
+            off[j] = (uint32_t)r * (uint32_t)rb + (uint32_t)(u0 * UNIT_BYTES);
+            dst[j] = raw + (uint32_t)(r * RAW_RS + pc * 16);
+            piece[j] = (uint32_t)(pc * 16);
+        }
+    }
+    __device__ __forceinline__ void unit(int slot, uint32_t bar) {
+        const uint32_t at_slot = (uint32_t)(slot * RAW_SLOT);
+        if (inside) {
+#pragma unroll
+            for (int j = 0; j < PER_LANE; j++) {
+                if (piece[j] < (off[j] & 15u) + UNIT_BYTES)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst[j] + at_slot), "l"(tile + ((off[j] & ~15u) + piece[j])) : "memory");
+                off[j] += UNIT_BYTES;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < PER_LANE; j++) {
+                const size_t at = (size_t)((off[j] & ~15u) + piece[j]), rest = at < left ? left - at : 0;   // past the matrix: zeros
+                const uint32_t n = rest < 16 ? (uint32_t)rest : 16u;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst[j] + at_slot), "l"(tile + (n ? at : 0)), "r"(n) : "memory");
+                off[j] += UNIT_BYTES;
+            }
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
+    }
+};
+
 template <int FMT, typename OutT, bool ORDERED>
 __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant__ TclParams p, const __grid_constant__ CUtensorMap x_map) {
     using F = TclFmt<FMT>;
-    constexpr int BB = F::bytes, STEP_TILES = F::step_k / KT, STEP_BYTES = F::blocks * BB;
+    constexpr int BB = F::block_bytes, STEP_TILES = F::step_k / KT, UNIT_BYTES = F::unit_bytes;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // operand tiles start on 1024-byte boundaries
     const int B_TILE = p.NB * KT * 2, B_SLOT = STEP_TILES * B_TILE, BS = p.b_slots;
-    uint8_t *b_s = smem;                                                   // [BS][B_SLOT]; reused by the split exchange
-    uint8_t *raw = b_s + max(BS * B_SLOT, p.ks > 1 ? ROWS * p.NB * 4 : 0); // [RAW_SLOTS][RAW_SLOT]
+    uint8_t *b_s = smem;                                                   // [BS][B_SLOT]; reused by the results
+    uint8_t *raw = b_s + max(BS * B_SLOT, ROWS * p.NB * 4); // [RAW_SLOTS][RAW_SLOT]
     uint64_t *raw_full = reinterpret_cast<uint64_t *>(raw + RAW_SLOTS * RAW_SLOT);   // [RAW_SLOTS]
     uint64_t *raw_empty = raw_full + RAW_SLOTS;
     uint64_t *a_full = raw_empty + RAW_SLOTS;                              // [GROUPS]
@@ -92,45 +139,57 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
     const int n0 = ((int)blockIdx.x - (grp ? p.tile_end[grp - 1] : 0)) * ROWS, m0 = (int)blockIdx.y * p.NB;
     const int n_rows = p.n[grp];
     const uint8_t *wmat = p.w[grp];
-    const size_t rb = (size_t)p.nb * BB, w_bytes = rb * (size_t)n_rows;
-    const int s0 = (int)blockIdx.z * p.sps, n_steps = max(0, min(p.steps, s0 + p.sps) - s0);   // this CTA's steps
+    const size_t rb = (size_t)p.nb * BB;
+    const int s0 = (int)blockIdx.z * p.sps, n_steps = max(0, min(p.steps, s0 + p.sps) - s0);   // this CTA's steps; s0 is even
+    const int u0 = s0 / 2, n_units = (n_steps + 1) / 2;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    if (tid == 0) {
-        for (int i = 0; i < RAW_SLOTS; i++) {
-            mbar_init(smem_u32(&raw_full[i]), 32 * NRAW);
-            mbar_init(smem_u32(&raw_empty[i]), GROUP_WARPS);
+    const bool raw_warp = warp >= NDQ && warp < NDQ + NRAW;
+    RawLoader<FMT> loader;
+    if (raw_warp) {   // the first raw blocks leave ahead of everything else; these warps do not wait for the others
+        if (tid == NDQ * 32) {
+            for (int i = 0; i < RAW_SLOTS; i++) {
+                mbar_init(smem_u32(&raw_full[i]), 32 * NRAW);
+                mbar_init(smem_u32(&raw_empty[i]), 2 * GROUP_WARPS);
+            }
+            *abort_flag = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
-        for (int i = 0; i < GROUPS; i++) mbar_init(smem_u32(&a_full[i]), GROUP_WARPS + p.extra_arrivals);
-        for (int i = 0; i < NBAR; i++) {
-            mbar_init(smem_u32(&b_full[i]), 1);
-            mbar_init(smem_u32(&step_done[i]), NISS);
+        asm volatile("bar.sync 1, %0;\n" ::"n"(NRAW * 32) : "memory");
+        asm volatile("bar.arrive 2, %0;\n" ::"n"(NT) : "memory");
+        loader.start(wmat, rb, n0, n_rows, u0, n_units, smem_u32(raw), tid - NDQ * 32);
+    } else {
+        if (tid == 0) {
+            for (int i = 0; i < GROUPS; i++) mbar_init(smem_u32(&a_full[i]), GROUP_WARPS + p.extra_arrivals);
+            for (int i = 0; i < NBAR; i++) {
+                mbar_init(smem_u32(&b_full[i]), 1);
+                mbar_init(smem_u32(&step_done[i]), 1);
+            }
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
-        *abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        tc_fence_before();
+        asm volatile("bar.sync 2, %0;\n" ::"n"(NT) : "memory");
+        tc_fence_after();
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = raw_warp ? 0u : *tmem_slot;
     const uint32_t idesc = (1u << 4) | ((uint32_t)(p.NB >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
 
     if (warp < NDQ) {
         // =========================== dequantizing warps ===========================
-        const int group = warp / GROUP_WARPS, wq = warp % GROUP_WARPS;
-        const int r = 32 * (wq & 3) + lane, bq = wq >> 2;     // operand row; which half of the step's bytes
+        const int group = warp / GROUP_WARPS, quarter = warp % GROUP_WARPS, half = group & 1;   // steps group, group + 4, ..: always this half of a unit
+        const int r = 32 * quarter + lane;     // operand row
         const int row = n0 + r;
         const bool rvalid = row < n_rows;
-        const uint32_t ta = tmem_base + ((uint32_t)(32 * (wq & 3)) << 16) + (uint32_t)(A_BASE + group * A_COLS);
+        const uint32_t ta = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(A_BASE + group * A_COLS);
         for (int i = group; i < n_steps; i += GROUPS) {
-            const int rs = i % RAW_SLOTS;
-            if (!mbar_wait_warp(smem_u32(&raw_full[rs]), (uint32_t)((i / RAW_SLOTS) & 1), p.wait_limit, abort_flag)) break;
-            const size_t g0 = (size_t)row * rb + (size_t)(s0 + i) * STEP_BYTES;
-            const uint32_t ra = smem_u32(raw + rs * RAW_SLOT + r * RAW_RS) + (uint32_t)(g0 & 15);
+            const int u = i / 2, rs = u % RAW_SLOTS;
+            if (!mbar_wait_warp(smem_u32(&raw_full[rs]), (uint32_t)((u / RAW_SLOTS) & 1), p.wait_limit, abort_flag)) break;
+            const uint32_t g0 = (uint32_t)r * (uint32_t)rb + (uint32_t)((u0 + u) * UNIT_BYTES);   // (of the tile, which starts on 16 bytes)
+            const uint32_t ra = smem_u32(raw + rs * RAW_SLOT + r * RAW_RS) + (g0 & 15u);
             // sixteen code bytes, 2-byte aligned: five aligned words, funnel-shifted into place
             auto codes16 = [&](uint32_t a, uint32_t (&cw)[4]) {
                 const uint32_t sh = (a & 3u) * 8u, wa = a & ~3u;
@@ -145,15 +204,20 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
                 asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(v) : "r"(a));
                 return __ushort_as_half(v);
             };
-            // the MMAs that read this slot a step of this group ago
+            // the step is in registers: its raw bytes may go, and the weights go in when the MMAs that read this slot a step of this group ago
+            // are done
+            bool dead = false;
+            auto release = [&]() {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&raw_empty[rs]));
+            };
             auto slot_free = [&]() -> bool {
                 if (i < GROUPS) return true;
-                const int u = i - GROUPS;
-                if (!mbar_wait_warp(smem_u32(&step_done[u % NBAR]), (uint32_t)((u / NBAR) & 1), p.wait_limit, abort_flag)) return false;
+                const int j = i - GROUPS;
+                if (!mbar_wait_warp(smem_u32(&step_done[j % NBAR]), (uint32_t)((j / NBAR) & 1), p.wait_limit, abort_flag)) return false;
                 tc_fence_after();
                 return true;
             };
-            bool dead = false;
             if constexpr (FMT == FMT_TQ2_0) {
                 const __half d = rvalid ? half_at(ra + 64u) : __float2half(0.0f);
                 // the four weights a code can mean, (q - 1) d, as a byte table for prmt
@@ -161,85 +225,66 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
                 const uint32_t p23 = (uint32_t)__half_as_ushort(d) | ((uint32_t)__half_as_ushort(__hadd(d, d)) << 16);
                 const uint32_t lut_lo = __byte_perm(p01, p23, 0x6420), lut_hi = __byte_perm(p01, p23, 0x7531);
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
+                for (int bi = 0; bi < 2; bi++) {
                     uint32_t cw[4], v[4][8];
-                    codes16(ra + (uint32_t)(32 * h + 16 * bq), cw);
+                    codes16(ra + (uint32_t)(32 * half + 16 * bi), cw);
 #pragma unroll
                     for (int l = 0; l < 4; l++)
 #pragma unroll
                         for (int q = 0; q < 4; q++) {
-                            const uint32_t sel = ((cw[q] >> (2 * l)) & 0x03030303u) * 0x11u + 0x40404040u;
-                            v[l][2 * q] = __byte_perm(lut_lo, lut_hi, sel);
-                            v[l][2 * q + 1] = __byte_perm(lut_lo, lut_hi, sel >> 16);
+                            const uint32_t c = (cw[q] >> (2 * l)) & 0x03030303u;
+                            uint32_t sel_hi;
+                            asm("mad.hi.u32 %0, %1, 0x110000, 0x4040;\n" : "=r"(sel_hi) : "r"(c));
+                            v[l][2 * q] = __byte_perm(lut_lo, lut_hi, c * 0x11u + 0x40404040u);
+                            v[l][2 * q + 1] = __byte_perm(lut_lo, lut_hi, sel_hi);
                         }
-                    if (h == 0 && !slot_free()) { dead = true; break; }
-                    // element k = 128 h + 32 l + j is bit pair l of code byte 32 h + j: eight columns from k / 2
+                    if (bi == 0 && !slot_free()) { dead = true; break; }
+                    if (bi == 1) release();
 #pragma unroll
-                    for (int l = 0; l < 4; l++) tmem_st8(ta + (uint32_t)(64 * h + 16 * l + 8 * bq), v[l]);
+                    for (int l = 0; l < 4; l++) tmem_st8(ta + (uint32_t)(16 * l + 8 * bi), v[l]);
                 }
             } else {
-                const __half2 c1032 = __float2half2_rn(1032.0f);
+                const __half2 offset[2] = {__float2half2_rn(1032.0f), __float2half2_rn(72.0f)};
 #pragma unroll
                 for (int bi = 0; bi < 2; bi++) {
-                    const int b = 2 * bq + bi;
-                    const bool ok = rvalid && (s0 + i) * F::blocks + b < p.nb;
+                    const int b = 2 * half + bi;
+                    const bool ok = rvalid && (u0 + u) * 4 + b < p.nb;
                     uint32_t cw[4], hi[16], lo[16];
                     codes16(ra + (uint32_t)(b * BB + 2), cw);
                     const __half2 d2 = __half2half2(ok ? half_at(ra + (uint32_t)(b * BB)) : __float2half(0.0f));
-                    // byte j: k = j in the low nibble, k = j + 16 in the high one
+                    // byte j: k = j in the low nibble, k = j + 16 in the high one; under an exponent in place they are 1024 + q and 64 + q
 #pragma unroll
                     for (int q = 0; q < 4; q++)
 #pragma unroll
-                        for (int nib = 0; nib < 2; nib++)
+                        for (int e = 0; e < 2; e++) {
+                            const uint32_t c = __byte_perm(cw[q], 0u, e ? 0x4342 : 0x4140);
 #pragma unroll
-                            for (int e = 0; e < 2; e++) {
-                                const uint32_t c = __byte_perm(nib ? cw[q] >> 4 : cw[q], 0u, e ? 0x4342 : 0x4140);
-                                const uint32_t u = (c & 0x000F000Fu) | 0x64006400u;                           // 1024 + q
-                                const __half2 q8 = __hsub2(*reinterpret_cast<const __half2 *>(&u), c1032);     // q - 8, exact
+                            for (int nib = 0; nib < 2; nib++) {
+                                const uint32_t v = nib ? (c & 0x00F000F0u) | 0x54005400u : (c & 0x000F000Fu) | 0x64006400u;
+                                const __half2 q8 = __hsub2(*reinterpret_cast<const __half2 *>(&v), offset[nib]);   // q - 8, exact
                                 const __half2 w = __hmul2(q8, d2), rem = __hfma2(q8, d2, __hneg2(w));          // rounded weight, remainder
                                 hi[8 * nib + 2 * q + e] = *reinterpret_cast<const uint32_t *>(&w);
                                 lo[8 * nib + 2 * q + e] = *reinterpret_cast<const uint32_t *>(&rem);
                             }
+                        }
                     if (bi == 0 && !slot_free()) { dead = true; break; }
-                    tmem_st16(ta + (uint32_t)(16 * b), hi);
-                    tmem_st16(ta + (uint32_t)(64 + 16 * b), lo);
+                    if (bi == 1) release();
+                    tmem_st16(ta + (uint32_t)(16 * bi), hi);
+                    tmem_st16(ta + (uint32_t)(32 + 16 * bi), lo);
                 }
             }
             if (dead) break;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&raw_empty[rs]));   // the raw bytes are in registers
             asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&a_full[group]));
         }
-    } else if (warp < NDQ + NRAW) {
+    } else if (raw_warp) {
         // =========================== raw blocks ===========================
-        // piece idx of a step: 16 bytes number idx % 6 of row idx / 6 (six pieces hold 72 bytes at any alignment)
-        constexpr int PIECES = 6, PER_LANE = ROWS * PIECES / 32 / NRAW;
-        const int w = warp - NDQ;
-        size_t off[PER_LANE];   // where the row's bytes of the next step start, in the matrix; past its end for rows that do not exist
-        uint32_t dst[PER_LANE];
-#pragma unroll
-        for (int j = 0; j < PER_LANE; j++) {
-            const int idx = (j * NRAW + w) * 32 + lane, r = idx / PIECES, pc = idx - r * PIECES;
-            off[j] = n0 + r < n_rows ? (size_t)(n0 + r) * rb + (size_t)s0 * STEP_BYTES : w_bytes;
-            dst[j] = smem_u32(raw) + (uint32_t)(r * RAW_RS + pc * 16);
-        }
-        for (int i = 0; i < n_steps; i++) {
-            const int rs = i % RAW_SLOTS;
-            if (i >= RAW_SLOTS && !mbar_wait_warp(smem_u32(&raw_empty[rs]), (uint32_t)((i / RAW_SLOTS - 1) & 1), p.wait_limit, abort_flag)) break;
-#pragma unroll
-            for (int j = 0; j < PER_LANE; j++) {
-                const int idx = (j * NRAW + w) * 32 + lane, pc = idx % PIECES;
-                const size_t at = (off[j] & ~(size_t)15) + (size_t)(pc * 16);
-                const size_t left = at < w_bytes ? w_bytes - at : 0;   // nothing is read past the matrix: the rest is zero-filled
-                const uint32_t n = left < 16 ? (uint32_t)left : 16u;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst[j] + (uint32_t)(rs * RAW_SLOT)), "l"(wmat + (n ? at : 0)), "r"(n)
-                             : "memory");
-                off[j] += STEP_BYTES;
-            }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(&raw_full[rs])) : "memory");
+        for (int u = 0; u < n_units; u++) {
+            const int rs = u % RAW_SLOTS;
+            if (u >= RAW_SLOTS && !mbar_wait_warp(smem_u32(&raw_empty[rs]), (uint32_t)((u / RAW_SLOTS - 1) & 1), p.wait_limit, abort_flag)) break;
+            loader.unit(rs, smem_u32(&raw_full[rs]));
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
     } else if (warp == NDQ + NRAW) {
@@ -266,32 +311,33 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
         // 509 x 1536 x 6144 Q4_0 took 27.2 instead of 25.5 us).
         const int iw = warp - NDQ - NRAW - 1;
         const bool leader = elect_one();
-        const uint64_t bdesc0 = make_desc(smem_u32(b_s) + (uint32_t)(iw * 32));
-        const uint32_t acc = tmem_base + (uint32_t)(iw * MAX_NB), ta0 = tmem_base + (uint32_t)(A_BASE + 8 * iw);
+        const uint64_t bdesc0 = make_desc(smem_u32(b_s));
+        const uint32_t acc = tmem_base + (uint32_t)(iw * MAX_NB), ta0 = tmem_base + (uint32_t)A_BASE;
         bool dead = false;
-        uint32_t slot = 0;
-        for (int i = 0; i < n_steps; i++) {
+        int slot = iw < BS ? iw : 0;
+        for (int i = iw; i < n_steps; i += NISS) {   // every other step, into this warp's accumulator
             const uint32_t sa = (uint32_t)i % GROUPS;
+            // (the activations first, which come ahead of time: a wait takes some 250 cycles even so, and weights are turned over in a loop)
             if (!mbar_wait_warp(smem_u32(&a_full[sa]), (uint32_t)((i / GROUPS) & 1), p.wait_limit, abort_flag) ||
                 !mbar_wait_warp(smem_u32(&b_full[i % NBAR]), (uint32_t)((i / NBAR) & 1), p.wait_limit, abort_flag)) { dead = true; break; }
             tc_fence_after();
             const uint32_t ta = ta0 + sa * (uint32_t)A_COLS;
-            const uint64_t bd = bdesc0 + (uint64_t)((slot * (uint32_t)B_SLOT) >> 4);
-            if (++slot == (uint32_t)BS) slot = 0;
-            // K = 16 slices iw, iw + 2, ..: slice s of the step is 32 bytes (s % 4) of activation tile s / 4
+            const uint64_t bd = bdesc0 + (uint64_t)(((uint32_t)slot * (uint32_t)B_SLOT) >> 4);
+            for (slot += NISS; slot >= BS;) slot -= BS;
+            // slice s of 16 k is 32 bytes (s % 4) of activation tile s / 4
             if (leader) {
 #pragma unroll
-                for (int j = 0; j < STEP_TILES * 2; j++) {
-                    const uint64_t bj = bd + (uint64_t)(((uint32_t)((j >> 1) * B_TILE) + (uint32_t)((j & 1) * 64)) >> 4);
-                    umma_f16_ta(acc, ta + (uint32_t)(16 * j), bj, idesc, (i > 0 || j > 0) ? 1u : 0u);
-                    if (FMT == FMT_Q4_0) umma_f16_ta(acc, ta + (uint32_t)(64 + 16 * j), bj, idesc, 1u);
+                for (int j = 0; j < STEP_TILES * 4; j++) {
+                    const uint64_t bj = bd + (uint64_t)(((uint32_t)((j >> 2) * B_TILE) + (uint32_t)((j & 3) * 32)) >> 4);
+                    umma_f16_ta(acc, ta + (uint32_t)(8 * j), bj, idesc, (i > iw || j > 0) ? 1u : 0u);
+                    if (FMT == FMT_Q4_0) umma_f16_ta(acc, ta + (uint32_t)(32 + 8 * j), bj, idesc, 1u);
                 }
                 umma_commit(smem_u32(&step_done[i % NBAR]));
             }
             __syncwarp();
         }
-        if (!dead && n_steps > 0) {   // drain: the last step's barrier completes when both issuers' MMAs are done
-            const int last = n_steps - 1;
+        if (!dead && n_steps > iw) {   // drain: this warp's last step
+            const int last = iw + (n_steps - 1 - iw) / NISS * NISS;
             dead = !mbar_wait_warp(smem_u32(&step_done[last % NBAR]), (uint32_t)((last / NBAR) & 1), p.wait_limit, abort_flag);
         }
         if (dead) *abort_flag = 1;
@@ -303,7 +349,7 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
 
     // ---- results.  Dequantizing warp w reads TMEM lanes 32 (w & 3) .. + 31 (one weight row per thread) and every fourth group
     //      of 16 batch columns; the two accumulators are added ----
-    float *red = reinterpret_cast<float *>(b_s);   // split exchange: [NB cols][128 rows]
+    float *red = reinterpret_cast<float *>(b_s);   // [NB cols][128 rows]
     OutT *out = reinterpret_cast<OutT *>(p.out[grp]);
     if (warp < NDQ) {
         const int lrow = 32 * (warp & 3) + lane;
@@ -316,30 +362,33 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
                 tmem_ld16(t + MAX_NB, a1);
                 tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 16; j++) v[j] = __uint_as_float(a0[j]) + __uint_as_float(a1[j]);
+                for (int j = 0; j < 16; j++) v[j] = __uint_as_float(a0[j]) + (n_steps > 1 ? __uint_as_float(a1[j]) : 0.f);   // (one step: one accumulator)
             } else {
 #pragma unroll
                 for (int j = 0; j < 16; j++) v[j] = 0.f;
             }
-            if (p.ks > 1) {
 #pragma unroll
-                for (int j = 0; j < 16; j++) red[(c0 + j) * ROWS + lrow] = v[j];
-            } else if (n0 + lrow < n_rows && !failed) {
-#pragma unroll
-                for (int j = 0; j < 16; j++)
-                    if (m0 + c0 + j < p.m) store_c(out + (size_t)(m0 + c0 + j) * n_rows + n0 + lrow, v[j]);
-            }
+            for (int j = 0; j < 16; j++) red[(c0 + j) * ROWS + lrow] = v[j];
         }
     }
+    const int cols = min(p.NB, p.m - m0), r4 = lane * 4;
+    auto store_rows = [&](int col, float4 a) {   // a warp finishes a column: 32 x 4 rows
+        OutT *dst = out + (size_t)(m0 + col) * n_rows + n0 + r4;
+        if (n0 + r4 + 3 < n_rows && (((uintptr_t)dst) & (4 * sizeof(OutT) - 1)) == 0) {
+            store_c4(dst, a);
+        } else {
+            const float e[4] = {a.x, a.y, a.z, a.w};
+            for (int q = 0; q < 4; q++)
+                if (n0 + r4 + q < n_rows) store_c(dst + q, e[q]);
+        }
+    };
     if (p.ks > 1) {
-        // The ks CTAs of this tile are one cluster.  An item is four consecutive output rows of one batch column; CTA `rank`
-        // finishes every ks-th run of 32 items: adds the partials in split order and stores.
+        // The ks CTAs of this tile are one cluster; CTA `rank` finishes every ks-th column: adds the partials in split order and stores.
         cluster_sync();
-        const int rank = (int)blockIdx.z, cols = min(p.NB, p.m - m0);
+        const int rank = (int)blockIdx.z;
         const uint32_t red_a = smem_u32(red);
         if (!failed) {
-            for (int col = rank + p.ks * warp; col < cols; col += p.ks * (NT / 32)) {   // a warp finishes a column: 32 x 4 rows
-                const int r4 = lane * 4;
+            for (int col = rank + p.ks * warp; col < cols; col += p.ks * (NT / 32)) {
                 const uint32_t la = red_a + (uint32_t)((col * ROWS + r4) * 4);
                 float4 pv[MAX_KS];
 #pragma unroll
@@ -349,17 +398,15 @@ __global__ void __launch_bounds__(NT, 1) qgemm_tcl_kernel(const __grid_constant_
                 for (int sp = 0; sp < MAX_KS; sp++) {
                     a.x += pv[sp].x; a.y += pv[sp].y; a.z += pv[sp].z; a.w += pv[sp].w;
                 }
-                OutT *dst = out + (size_t)(m0 + col) * n_rows + n0 + r4;
-                if (n0 + r4 + 3 < n_rows && (((uintptr_t)dst) & (4 * sizeof(OutT) - 1)) == 0) {
-                    store_c4(dst, a);
-                } else {
-                    const float e[4] = {a.x, a.y, a.z, a.w};
-                    for (int q = 0; q < 4; q++)
-                        if (n0 + r4 + q < n_rows) store_c(dst + q, e[q]);
-                }
+                store_rows(col, a);
             }
         }
         cluster_sync();   // no CTA leaves while a peer may still read its shared memory
+    } else {
+        // (through shared memory: stored straight from tensor memory, 64 bytes a warp, a 96-column tile took 3500 cycles)
+        __syncthreads();
+        if (!failed)
+            for (int col = warp; col < cols; col += NT / 32) store_rows(col, *reinterpret_cast<const float4 *>(red + col * ROWS + r4));
     }
     if (failed) tc_wait_expired(p.status, LC_DEV_STATUS_WAIT_EXPIRED, tid);
     tc_fence_before();
@@ -423,22 +470,24 @@ int launch_tcl(lc_batch *b, bool serial, const TclParams &p, const CUtensorMap &
 
 }  // namespace
 
-// Batch rows per CTA and K splits of a launch of `tiles` 128-row tiles: a step costs its tensor-memory stores (about 900 cycles)
-// or its MMAs (8 per column), whichever is more; a launch costs about 2500 cycles around its steps, the exchange of a split 3000
-// more.  Clusters cannot use every SM, other launches can.
+// Batch rows per CTA and K splits of a launch of `tiles` 128-row tiles, the cheapest by an estimate in cycles fitted to all plans of 113
+// shapes (17 .. 512 rows, K 512 .. 8192, n 512 .. 16384, with and without an overlap of launches): the plan it picks takes 0.5 % longer
+// than the best one in the mean, 10 % at most.  352 x 1530 x 2048 TQ2_0 9.5 -> 7.9 us against a rule without a launch's true fixed part.
+// Clusters cannot use every SM, other launches can.
 struct TclPlan {
-    int m_tiles, NB, ks, sps, steps;   // ks splits of sps steps
+    int m_tiles, NB, ks, ups, units;   // ks splits of ups units of two steps
     uint64_t waves;
 };
 static TclPlan tcl_plan(int fmt, const lc_kernels *k, uint32_t m, uint32_t kk, int tiles) {
     const int step_k = fmt == FMT_Q4_0 ? TclFmt<FMT_Q4_0>::step_k : TclFmt<FMT_TQ2_0>::step_k;
-    TclPlan pl = {1, 16, 1, 1, ((int)kk + step_k - 1) / step_k, 1};
+    TclPlan pl = {1, 16, 1, 1, ((int)kk + 2 * step_k - 1) / (2 * step_k), 1};
     uint64_t best = ~0ull;
     for (int mt = ((int)m + MAX_NB - 1) / MAX_NB; mt <= ((int)m + 47) / 48; mt++) {
         const int nb = (((int)m + mt - 1) / mt + 15) / 16 * 16, real_mt = ((int)m + nb - 1) / nb;
-        for (int ks = 1; ks <= MAX_KS && (ks == 1 || 2 * ks <= pl.steps); ks++) {
+        for (int ks = 1; ks <= MAX_KS && (ks == 1 || 2 * ks <= pl.units); ks++) {
             const uint64_t at_once = ks > 1 ? k->cluster_cap[ks] : (uint64_t)k->ctx->sm_count, waves = ((uint64_t)tiles * real_mt + at_once - 1) / at_once;
-            const uint64_t cost = waves * (2500u + (uint64_t)((pl.steps + ks - 1) / ks) * (uint64_t)(8 * nb > 900 ? 8 * nb : 900) + (ks > 1 ? 3000u + 10u * nb : 0u));
+            const uint64_t unit = 910u + (fmt == FMT_Q4_0 ? 4u : 7u) * (uint64_t)nb;
+            const uint64_t cost = waves * (6900u + (uint64_t)((pl.units + ks - 1) / ks) * unit + 9u * (uint64_t)nb + (ks > 1 ? 2000u + 100u * (uint64_t)ks : 0u));
             if (cost < best) {
                 best = cost;
                 pl.m_tiles = real_mt;
@@ -448,8 +497,8 @@ static TclPlan tcl_plan(int fmt, const lc_kernels *k, uint32_t m, uint32_t kk, i
             }
         }
     }
-    pl.sps = (pl.steps + pl.ks - 1) / pl.ks;
-    pl.ks = (pl.steps + pl.sps - 1) / pl.sps;
+    pl.ups = (pl.units + pl.ks - 1) / pl.ks;
+    pl.ks = (pl.units + pl.ups - 1) / pl.ups;
     return pl;
 }
 
@@ -461,7 +510,7 @@ uint64_t lc_qgemm_tcl_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uin
     const uint64_t tiles = (n + ROWS - 1) / ROWS, sms = (uint64_t)k->ctx->sm_count;
     if (tiles <= sms) return 0;
     const TclPlan pl = tcl_plan(FMT_Q4_0, k, m, kk, (int)tiles);
-    return pl.waves * (3300 + 720 * (uint64_t)pl.sps);
+    return pl.waves * (3300 + 720 * (uint64_t)pl.ups);
 }
 
 // Grouped launch: `ng` weight matrices [ns[g], kk] sharing the activations `input` [m, kk].  Returns LC_OK after a launch, a
@@ -487,11 +536,11 @@ int lc_qgemm_tcl_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const 
     if (tiles < 1) return -1;
     const int step_k = fmt == FMT_Q4_0 ? TclFmt<FMT_Q4_0>::step_k : TclFmt<FMT_TQ2_0>::step_k;
     const TclPlan pl = tcl_plan(fmt, k, m, kk, tiles);
-    p.steps = pl.steps;
+    p.steps = ((int)kk + step_k - 1) / step_k;
     p.m_tiles = pl.m_tiles;
     p.NB = pl.NB;
     p.ks = pl.ks;
-    p.sps = pl.sps;
+    p.sps = 2 * pl.ups;
     if (p.m_tiles > 65535) return -1;
     p.status = k->dev_status;
     p.wait_limit = k->test_wait_expiry ? 4096u : WAIT_LIMIT;
@@ -501,7 +550,7 @@ int lc_qgemm_tcl_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const 
     if (p.b_slots > NBAR) p.b_slots = NBAR;
     if (p.b_slots > p.sps) p.b_slots = p.sps;
     size_t b_bytes = b_slot * p.b_slots;
-    if (p.ks > 1 && b_bytes < (size_t)ROWS * p.NB * 4) b_bytes = (size_t)ROWS * p.NB * 4;
+    if (b_bytes < (size_t)ROWS * p.NB * 4) b_bytes = (size_t)ROWS * p.NB * 4;
     const size_t smem = fixed + b_bytes;
     if (smem > k->ctx->smem_optin) return -1;
     CUtensorMap x_map;

@@ -232,6 +232,20 @@ def test_matmul_nt_q4_0_tensor_core(la, orc, ctx, tc_kernels, m, k, n):
     device_status_ok(kernels)
 
 
+@pytest.mark.parametrize("fmt,m,k,n", [("q4_0", 70, 32, 128), ("q4_0", 66, 96, 129), ("q4_0", 97, 160, 257), ("q4_0", 129, 192, 127), ("q4_0", 300, 704, 256),
+                                       ("q4_0", 65, 5216, 130), ("tq2_0", 66, 256, 129), ("tq2_0", 113, 768, 127), ("tq2_0", 300, 1280, 385),
+                                       ("tq2_0", 65, 5888, 200)])
+def test_matmul_nt_large_batch_steps(la, orc, ctx, kernels, fmt, m, k, n):
+    """The large-batch kernel's steps: one of them, an odd number, half of one, as many as its rings hold and more, split over a cluster;
+    raw blocks that end with the matrix, on and off a 16-byte boundary.  Tolerances as above."""
+    raw = (la.synth.q4_0_weights if fmt == "q4_0" else la.synth.tq2_0_weights)(n, k, 17)
+    a = la.synth.normal_f16((m, k), 18)
+    want = orc.matmul_nt(orc.Q4_0 if fmt == "q4_0" else orc.TQ2_0, a, raw, m, k, n)
+    got = run_matmul(la, ctx, kernels, f"matmul_nt_{fmt}_into", a, raw, m, k, n)
+    rel_close(got, want, TC_TOL_Q4 if fmt == "q4_0" else TC_TOL_TQ2, f"large-batch {fmt} m={m} k={k} n={n}")
+    device_status_ok(kernels)
+
+
 def test_expired_barrier_wait_reports_timeout(la, orc, ctx, monkeypatch):
     """Every barrier wait of the tcgen05 matmul is bounded.  LOCAL_CUDA_TEST_WAIT_EXPIRY=1 gives a kernels object
     whose launches wait (with a short limit) for an arrival nobody makes: the launch must come back by itself, leave
