@@ -32,7 +32,8 @@
 
 namespace {
 
-template <typename C>
+// QUEUE: the queue form (TqAttnParams::queue_chunk), an instantiation of its own so that the others' code stays short.
+template <typename C, bool QUEUE>
 __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p) {
     constexpr int HD = C::HD, CB = C::CB, NW = C::NW, NT = C::NT, KT = C::KT, NS = C::NS, DPL = C::DPL;
     lc_pdl_trigger();
@@ -42,8 +43,9 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
     uint2 *lut = reinterpret_cast<uint2 *>(smem);                       // [NENT][16 copies]
     float *rq_s = reinterpret_cast<float *>(smem + C::LUT_BYTES);       // [NS][32 lanes][4] rotated, scaled query
     uint2 *ent_s = reinterpret_cast<uint2 *>(smem + C::LUT_BYTES + C::Q_BYTES);   // one table copy
-    __shared__ uint32_t q_first[LC_ATTN_QUEUE_LANES + 1];               // queue form: first item of each lane
-    __shared__ uint32_t q_ticket, q_lane;
+    __shared__ uint32_t q_first[QUEUE ? LC_ATTN_QUEUE_LANES + 1 : 1];               // queue form: first item of each lane
+    __shared__ uint32_t q_pos[QUEUE ? LC_ATTN_QUEUE_LANES : 1];                     // and its position
+    __shared__ uint32_t q_ticket;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -61,14 +63,13 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
     // itself comes from the predecessor.  A caller that also guarantees that `positions` was written before the
     // predecessor kernels started (the decode step: it is an input of the step) sets early_kv, and the first tiles'
     // copies are then in flight while the predecessor finishes.
-    const bool queue = p.queue_chunk != 0u;
-    const bool early = p.early_kv != 0u && p.positions != nullptr && p.row_positions == 0u && !queue;
-    if (!early && !(queue && p.early_kv)) lc_pdl_wait();
+    const bool early = p.early_kv != 0u && p.positions != nullptr && p.row_positions == 0u && !QUEUE;
+    if (!early && !(QUEUE && p.early_kv)) lc_pdl_wait();
 
     // keys [win_start, seq_len) of a lane
-    auto lane_range = [&](uint32_t li, uint32_t &pos, uint32_t &seq_len, uint32_t &win_start, bool report) {
+    auto lane_range = [&](uint32_t li, uint32_t &pos, uint32_t &seq_len, uint32_t &win_start, bool report, bool in_smem) {
         if (p.positions) {
-            pos = p.positions[li];
+            pos = in_smem ? q_pos[li] : p.positions[li];
             seq_len = pos + 1u;
             if (p.ring == 0u && seq_len > p.lane_capacity) {   // never read past the lane's rows
                 seq_len = p.lane_capacity;
@@ -81,10 +82,11 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
         win_start = (p.window > 0u && pos + 1u > p.window) ? (pos + 1u - p.window) : 0u;
     };
     uint32_t n_items = 0;
-    if (queue) {
+    if (QUEUE) {
         for (uint32_t li = threadIdx.x; li < p.n_lanes; li += NT) {
             uint32_t pos, seq_len, ws;
-            lane_range(li, pos, seq_len, ws, false);
+            lane_range(li, pos, seq_len, ws, false, false);
+            q_pos[li] = pos;
             const uint32_t n = seq_len > ws ? seq_len - ws : 0u;
             q_first[li + 1] = lc_attn_items(n, p.queue_chunk);   // (an empty lane is one item and stores zeros)
         }
@@ -109,33 +111,27 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
         n_items = q_first[p.n_lanes];
         if (p.early_kv) lc_pdl_wait();
     }
-    uint32_t ticket = 0;   // thread 0: the item drawn
-    const uint32_t items_all = n_items + gridDim.x;
-    if (queue && threadIdx.x == 0) ticket = atomicAdd(&p.counters[blockIdx.y], 1u);
+    // A CTA's first item is its own number; it draws the others one after the other.
+    uint32_t item = blockIdx.x;
+    uint32_t ticket = 0;   // thread 0
+    auto draw = [&]() { ticket = atomicAdd(&p.counters[blockIdx.y], 1u); };
 
     // The item at hand: keys [k_begin, k_end) of lane lane_idx, its part number `split`.
     uint32_t lane_idx = blockIdx.z, split = blockIdx.x, pos = 0, k_begin = 0, k_end = 0;
-    auto next_item = [&]() -> bool {   // (a barrier at the end: every thread has read the schedule's words)
-        if (queue) {
-            if (threadIdx.x == 0) q_ticket = ticket;
-            __syncthreads();
-            const uint32_t item = q_ticket;
-            if (item >= n_items) {
-                // every CTA has drawn its last: zero again for the next launch
-                if (item == items_all - 1u && threadIdx.x == 0) p.counters[blockIdx.y] = 0u;
-                return false;
-            }
-            for (uint32_t li = threadIdx.x; li < p.n_lanes; li += NT)
-                if (q_first[li] <= item && item < q_first[li + 1]) q_lane = li;
-            __syncthreads();
-            lane_idx = q_lane;
+    auto next_item = [&]() -> bool {
+        if (QUEUE) {
+            if (item >= n_items) return false;
+            uint32_t before = 0;   // lanes whose items all come first
+            for (uint32_t l0 = 0; l0 < p.n_lanes; l0 += 32)
+                before += __popc(__ballot_sync(0xffffffffu, l0 + lane < p.n_lanes && q_first[l0 + lane + 1] <= item));
+            lane_idx = before;
             split = item - q_first[lane_idx];
         }
         uint32_t seq_len, win_start;
-        lane_range(lane_idx, pos, seq_len, win_start, true);
+        lane_range(lane_idx, pos, seq_len, win_start, true, QUEUE);
         const uint32_t n_keys = seq_len > win_start ? seq_len - win_start : 0u;
         uint32_t per;
-        if (queue) {
+        if (QUEUE) {
             per = lc_attn_item_keys(n_keys, p.queue_chunk);
         } else {
             per = (n_keys + p.n_splits - 1) / p.n_splits;
@@ -199,6 +195,23 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
         }
         load_norms(k_begin + warp * KT, nk_raw, nv_raw);
     };
+    // warp w's share of the query: head w's dims DPL lane .., as they are
+    const bool have_frag = p.qfrag != nullptr;   // the launch that wrote q left the fragments ready (group % 8 == 0)
+    uint4 q_raw[DPL / 4];
+    auto load_query = [&]() {
+        if (have_frag || warp >= gvalid) return;
+        const size_t q_row = ((size_t)lane_idx * p.n_q + qh0 + warp) * HD + DPL * lane;
+#pragma unroll
+        for (int i = 0; i < DPL; i += 4) {
+            if (p.fused_q) {
+                const uint2 v = *reinterpret_cast<const uint2 *>(p.q + q_row + i);
+                q_raw[i / 4].x = v.x;
+                q_raw[i / 4].y = v.y;
+            } else {
+                q_raw[i / 4] = *reinterpret_cast<const uint4 *>(p.rq + q_row + i);
+            }
+        }
+    };
     bool more = next_item();
     if (more) {
         t_issue = k_begin + warp * KT;
@@ -219,6 +232,7 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
             lc_pdl_wait();
         }
         start_item(issued);
+        load_query();
     }
 
     while (more) {
@@ -226,7 +240,6 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
         //      It is the one operand f16 cannot hold well enough: a high f16 part and the f16 of the remainder. ----
         constexpr int NQ = C::QSMEM ? 1 : NS;
         uint32_t bq[NQ][2], bql[NQ][2];
-        const bool have_frag = p.qfrag != nullptr;   // the launch that wrote q left the fragments ready (group % 8 == 0)
         if (C::QSMEM && have_frag) {
             const uint4 *src = p.qfrag + ((size_t)lane_idx * (p.n_q >> 3) + (qh0 >> 3)) * (NS * 32);
             for (int e = threadIdx.x; e < NS * 32; e += NT) *reinterpret_cast<uint4 *>(rq_s + e * 4) = src[e];
@@ -245,11 +258,10 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
 #pragma unroll
             for (int i = 0; i < DPL; i++) x[i] = 0.f;
             if (warp < gvalid) {
-                const size_t q_row = ((size_t)lane_idx * p.n_q + qh0 + warp) * HD + DPL * lane;
                 if (p.fused_q) {
 #pragma unroll
                     for (int i = 0; i < DPL; i += 4) {
-                        const uint2 raw = *reinterpret_cast<const uint2 *>(p.q + q_row + i);
+                        const uint4 raw = q_raw[i / 4];
                         const float4 sg = *reinterpret_cast<const float4 *>(p.signs + DPL * lane + i);
                         const float2 f0 = unpack_h2(raw.x), f1 = unpack_h2(raw.y);
                         x[i] = f0.x * sg.x;
@@ -264,11 +276,11 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
                 } else {
 #pragma unroll
                     for (int i = 0; i < DPL; i += 4) {
-                        const float4 r = *reinterpret_cast<const float4 *>(p.rq + q_row + i);
-                        x[i] = r.x * p.scale;
-                        x[i + 1] = r.y * p.scale;
-                        x[i + 2] = r.z * p.scale;
-                        x[i + 3] = r.w * p.scale;
+                        const uint4 r = q_raw[i / 4];
+                        x[i] = __uint_as_float(r.x) * p.scale;
+                        x[i + 1] = __uint_as_float(r.y) * p.scale;
+                        x[i + 2] = __uint_as_float(r.z) * p.scale;
+                        x[i + 3] = __uint_as_float(r.w) * p.scale;
                     }
                 }
             }
@@ -303,11 +315,11 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
         // ---- main loop: each warp takes every 8th tile of this split ----
         AttnAcc<C> acc;
         acc.clear();
-        float(&o)[NS][4] = acc.o;
         float(&m_run)[2] = acc.m_run, (&l_part)[2] = acc.l_part;
 
         int stage = 0;
         for (uint32_t t0 = k_begin + warp * KT; t0 < k_end; t0 += NW * KT) {
+            if (QUEUE && threadIdx.x == 0 && t0 + NW * KT >= k_end) draw();   // as late as a tile hides the round trip
             cp_async_wait<C::DEPTH - 2>();   // tile t0 is the oldest group in flight
             __syncwarp();                    // ... for every lane; and every lane is done with the tile before
             const float nk = __half2float(nk_raw) * gamma, nv = __half2float(nv_raw) * gamma;
@@ -324,8 +336,11 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
             attn_tile<C>(acc, ka, va, t0, k_end, nk, nv, bq, bql, q_a, lut_lane, lane);
         }
 
-        // the next ticket, drawn as late as hides the round trip: items are then handed out in the order of need
-        if (queue && threadIdx.x == 0) ticket = atomicAdd(&p.counters[blockIdx.y], 1u);
+        if (QUEUE && threadIdx.x == 0) {
+            if (k_begin >= k_end) draw();
+            if (ticket == n_items - 1u) p.counters[blockIdx.y] = 0u;   // every CTA has drawn its last: zero again for the next launch
+            q_ticket = gridDim.x + ticket;
+        }
 
         // ---- merge the warps that had keys; query and ring memory is reused for their accumulators.  A step of the decode
         //      model comes here after one or two tiles per warp, with this code cold in the instruction cache: it is
@@ -359,7 +374,10 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
             if (warp < nwa) {
                 float4 *dst = reinterpret_cast<float4 *>(acc_s) + warp * NS * 32 + lane;
 #pragma unroll
-                for (int s = 0; s < NS; s++) dst[s * 32] = make_float4(o[s][0] * f0, o[s][1] * f1, o[s][2] * f0, o[s][3] * f1);
+                for (int s = 0; s < NS; s++) {
+                    const float4 v = acc.result(s);
+                    dst[s * 32] = make_float4(v.x * f0, v.y * f1, v.z * f0, v.w * f1);
+                }
             }
         }
         // Head h's row: of this CTA alone row h; in a cluster row (h / n) * n + split of CTA h mod n, which finishes head h.
@@ -383,6 +401,10 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
         }
         const size_t part_row = HD + 2;
         const uint32_t it_lane = lane_idx, it_split = split;
+        if (QUEUE) {   // what comes next, and its query on the way
+            item = q_ticket;
+            if (next_item()) load_query();
+        }
         // where head h's partial of this split goes
         auto part_of = [&](int h, uint32_t sp) -> float * {
             const size_t qh = (size_t)it_lane * p.n_q + qh0 + h;
@@ -475,14 +497,10 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
             return;
         }
         __syncthreads();   // the tile is complete; the ring is free
-        if (queue) {
-            more = next_item();
-            if (more) {
-                t_issue = k_begin + warp * KT;
-                start_item(0);
-            }
-        } else {
-            more = false;
+        more = QUEUE && item < n_items;
+        if (more) {
+            t_issue = k_begin + warp * KT;
+            start_item(0);
         }
         // a merge launch follows (unless there is nothing to merge)
         for (int e = threadIdx.x; e < gvalid * (HD / 2); e += NT) {
@@ -502,10 +520,10 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
     }
 }
 
-template <typename C>
-int launch(lc_batch *b, const TqAttnParams &p, dim3 grid) {
+template <typename C, bool QUEUE>
+int launch_as(lc_batch *b, const TqAttnParams &p, dim3 grid) {
     static lc_smem_optin optin;
-    LC_CUDA_TRY(lc_ensure_smem(tq_attn_mma_kernel<C>, optin, b->ctx, C::SMEM));
+    LC_CUDA_TRY(lc_ensure_smem(tq_attn_mma_kernel<C, QUEUE>, optin, b->ctx, C::SMEM));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(C::NT);
@@ -528,9 +546,14 @@ int launch(lc_batch *b, const TqAttnParams &p, dim3 grid) {
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    LC_LAUNCH_CHECKED(cudaLaunchKernelEx(&cfg, tq_attn_mma_kernel<C>, p));
+    LC_LAUNCH_CHECKED(cudaLaunchKernelEx(&cfg, tq_attn_mma_kernel<C, QUEUE>, p));
     b->dispatch_count++;
     return LC_OK;
+}
+
+template <typename C>
+int launch(lc_batch *b, const TqAttnParams &p, dim3 grid) {
+    return p.queue_chunk != 0u ? launch_as<C, true>(b, p, grid) : launch_as<C, false>(b, p, grid);
 }
 
 template <int HD>
@@ -557,7 +580,7 @@ int lc_tq_attn_mma_launch(lc_batch *b, const TqAttnParams &p, dim3 grid, uint32_
 // (asked of one of the kernels that fill an SM's shared memory; the others that do differ in nothing that counts here)
 void lc_cluster_capacity(const lc_ctx *ctx, uint32_t (&cap)[9]) {
     using C = AttnCfg<256, 2>;
-    auto kern = tq_attn_mma_kernel<C>;
+    auto kern = tq_attn_mma_kernel<C, false>;
     cap[0] = 0;
     cap[1] = (uint32_t)ctx->sm_count;
     const bool ready = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) == cudaSuccess;

@@ -23,7 +23,9 @@ struct AttnCfg {
     static constexpr int NW = 8, NT = NW * 32;
     static constexpr int NS = HD / 16;                  // k16 steps of QK, 16-dim tiles of PV
     static constexpr int DPL = HD / 32;                 // dims per lane where a warp owns a head
-    static constexpr bool QSMEM = HD == 512;            // query fragments stay in shared memory (registers hold the accumulators)
+    static constexpr bool PAIRS = HD <= 256;            // V lookups serve two keys at once (attn_tile); at 512 dims two parts of them leave no registers
+    static constexpr int NO = HILO && PAIRS ? 2 * NS : NS;   // accumulator tiles of a warp
+    static constexpr bool QSMEM = NO > 16;              // query fragments stay in shared memory (registers hold the accumulators)
     // Row strides in the ring: chosen so that the fragment reads spread over the banks.
     static constexpr int KRS = (BITS == 2 && HD == 256) ? CB : CB + 16;
     static constexpr int VRS = CB + 16;
@@ -227,89 +229,142 @@ __device__ __forceinline__ float attn_table(const float *levels, uint2 *lut, uin
     return gamma;
 }
 
+// The fields of two packed rows side by side: every second BITS-wide field of the word run, from the first on, of `a` next to the same
+// of `b` (in lo), and those between (in hi); so a table field of two codes takes one of either row.
+template <int WIDTH, int N>
+__device__ __forceinline__ void pair_rows(const uint32_t (&a)[N], const uint32_t (&b)[N], uint32_t (&lo)[N], uint32_t (&hi)[N]) {
+    static_for<N>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        constexpr uint32_t mask = [] {
+            uint32_t m = 0;
+            for (int j = 0; j < 32; j++)
+                if ((32 * i + j) / WIDTH % 2 == 0) m |= 1u << j;
+            return m;
+        }();
+        uint32_t up, down;   // (a field may cross into the next word)
+        if constexpr (32 % (2 * WIDTH) == 0) {
+            up = b[i] << WIDTH;
+            down = a[i] >> WIDTH;
+        } else {
+            up = __funnelshift_l(i > 0 ? b[i > 0 ? i - 1 : 0] : 0u, b[i], WIDTH);
+            down = __funnelshift_r(a[i], i + 1 < N ? a[i + 1 < N ? i + 1 : i] : 0u, WIDTH);
+        }
+        lo[i] = (a[i] & mask) | (up & ~mask);
+        hi[i] = (down & mask) | (b[i] & ~mask);
+    });
+}
+
 // A warp's state over its tiles: O^T fragments, running maxima of heads 2t, 2t + 1 and this thread's part of the sums.
 template <typename C>
 struct AttnAcc {
-    float o[C::NS][4], m_run[2], l_part[2];
+    float o[C::NO][4], m_run[2], l_part[2];
     __device__ __forceinline__ void clear() {
 #pragma unroll
-        for (int s = 0; s < C::NS; s++) o[s][0] = o[s][1] = o[s][2] = o[s][3] = 0.f;
+        for (int s = 0; s < C::NO; s++) o[s][0] = o[s][1] = o[s][2] = o[s][3] = 0.f;
         m_run[0] = m_run[1] = -INFINITY;
         l_part[0] = l_part[1] = 0.f;
+    }
+    // O^T of dims (HD / 8) g + 2 s (heads 2t, 2t + 1), + 1 (the same)
+    __device__ __forceinline__ float4 result(int s) const {
+        if constexpr (!C::PAIRS) return make_float4(o[s][0], o[s][1], o[s][2], o[s][3]);
+        else if constexpr (C::HILO) return make_float4(o[2 * s][0] + o[2 * s][2], o[2 * s][1] + o[2 * s][3], o[2 * s + 1][0] + o[2 * s + 1][2], o[2 * s + 1][1] + o[2 * s + 1][3]);
+        else return s % 2 == 0 ? make_float4(o[s][0], o[s][1], o[s | 1][0], o[s | 1][1]) : make_float4(o[s & ~1][2], o[s & ~1][3], o[s][2], o[s][3]);
     }
 };
 // One warp's step over the KT keys t0 .. t0 + KT - 1 (those below k_end count) whose codes lie at the shared-memory addresses ka
 // and va.  nk, nv: norms times gamma of key `lane`.  q_a: this lane's query fragments where they stay in shared memory.
+//
+// A lookup's eight bytes land in two neighbouring registers, and an MMA's A operand is four in a row, of which the first two (and the last
+// two) are operand rows g and g + 8 at the same k.  So what a lookup returns is arranged to be such a pair, which saves the moves and
+// permutes that put operands together (15 of 54 instructions per key at 4 bits):
+//   * S^T, two parts: rows g and g + 8 are the high and the low part of one key.  One part: two keys, their codes side by side (pair_rows);
+//   * O^T, two parts: the high and low part of one dim, at two adjacent keys, whose codes lie side by side; the two parts' sums stay apart
+//     until the end.  One part: two dims, at two adjacent keys.
+// 64 lanes x 8192 keys: tq2 @@ us, tq3 @@, tq4 @@.
 template <typename C, int NQ>
 __device__ __forceinline__ void attn_tile(AttnAcc<C> &st, uint32_t ka, uint32_t va, uint32_t t0, uint32_t k_end, float nk, float nv,
                                           const uint32_t (&bq)[NQ][2], const uint32_t (&bql)[NQ][2], uint32_t q_a, uint32_t lut_lane, int lane) {
-    constexpr int CB = C::CB, KT = C::KT, MT = C::MT, NS = C::NS, FB = C::FB;
+    constexpr int CB = C::CB, KT = C::KT, MT = C::MT, NS = C::NS, FB = C::FB, NO = C::NO;
     const int g = lane >> 2, t = lane & 3;
-    float(&o)[NS][4] = st.o;
+    float(&o)[NO][4] = st.o;
     float(&m_run)[2] = st.m_run, (&l_part)[2] = st.l_part;
     // ---- S^T[KT keys x 8 heads] ----
-    constexpr int KW = CB / 16;   // words of one key in this thread's quarter row
-    uint32_t kw[MT][2][KW];
+    constexpr int KG = KT / 8, KW = CB / 16;   // words of one key in this thread's quarter row
+    float sc[KG][2];   // logits of keys 8 kg + g for heads 2t, 2t + 1, less the key's norm
+    {
+        uint32_t kw[KG][KW];
 #pragma unroll
-    for (int mt = 0; mt < MT; mt++) {
-        lds_words<KW>(ka + (uint32_t)(mt * 16 + g) * C::KRS + (uint32_t)t * (KW * 4), kw[mt][0]);
-        lds_words<KW>(ka + (uint32_t)(mt * 16 + g + 8) * C::KRS + (uint32_t)t * (KW * 4), kw[mt][1]);
-    }
-    float c[MT][2][4];   // chains: high and low query parts
+        for (int kg = 0; kg < KG; kg++) lds_words<KW>(ka + (uint32_t)(8 * kg + g) * C::KRS + (uint32_t)t * (KW * 4), kw[kg]);
+        constexpr int NC = C::HILO ? KG : MT;
+        float c[NC][2][4];   // chains: high and low query parts
 #pragma unroll
-    for (int mt = 0; mt < MT; mt++)
+        for (int i = 0; i < NC; i++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) c[mt][0][i] = c[mt][1][i] = 0.f;
-    auto qk_step = [&](auto S) {
-        constexpr int s = decltype(S)::value;
-        uint32_t b0, b1, l0, l1;
-        if constexpr (C::QSMEM) {
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(b0), "=r"(b1), "=r"(l0), "=r"(l1) : "r"(q_a + s * 512));
-        } else {
-            b0 = bq[s][0]; b1 = bq[s][1]; l0 = bql[s][0]; l1 = bql[s][1];
+            for (int e = 0; e < 4; e++) c[i][0][e] = c[i][1][e] = 0.f;
+        if constexpr (!C::HILO) {
+            // bytes of two codes of key g and the same two of key g + 8: four dims of a k-step are a byte of either run
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++) {
+                uint32_t lo[KW], hi[KW];
+                pair_rows<4>(kw[2 * mt], kw[2 * mt + 1], lo, hi);
+#pragma unroll
+                for (int w = 0; w < KW; w++) { kw[2 * mt][w] = lo[w]; kw[2 * mt + 1][w] = hi[w]; }
+            }
         }
-#pragma unroll
-        for (int mt = 0; mt < MT; mt++) {
-            if constexpr (!C::HILO) {
-                const uint2 x = lds64(field_addr<FB, s * 8>(kw[mt][0], lut_lane)), y = lds64(field_addr<FB, s * 8>(kw[mt][1], lut_lane));
-                const uint32_t a[4] = {x.x, y.x, x.y, y.y};
-                mma16816(c[mt][0], a, b0, b1);
-                mma16816(c[mt][1], a, l0, l1);
+        static_for<NS>([&](auto S) {
+            constexpr int s = decltype(S)::value;
+            uint32_t b0, b1, l0, l1;
+            if constexpr (C::QSMEM) {
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(b0), "=r"(b1), "=r"(l0), "=r"(l1) : "r"(q_a + s * 512));
             } else {
-                const uint2 x0 = lds64(field_addr<FB, 2 * s * FB>(kw[mt][0], lut_lane)), x1 = lds64(field_addr<FB, (2 * s + 1) * FB>(kw[mt][0], lut_lane));
-                const uint2 y0 = lds64(field_addr<FB, 2 * s * FB>(kw[mt][1], lut_lane)), y1 = lds64(field_addr<FB, (2 * s + 1) * FB>(kw[mt][1], lut_lane));
-                const uint32_t ah[4] = {x0.x, y0.x, x1.x, y1.x}, al[4] = {x0.y, y0.y, x1.y, y1.y};
-                mma16816(c[mt][0], ah, b0, b1);
-                mma16816(c[mt][1], ah, l0, l1);
-                mma16816(c[mt][1], al, b0, b1);
+                b0 = bq[s][0]; b1 = bq[s][1]; l0 = bql[s][0]; l1 = bql[s][1];
             }
-        }
-    };
-    static_for<NS>(qk_step);
+#pragma unroll
+            for (int i = 0; i < NC; i++) {
+                uint2 x, y;
+                if constexpr (!C::HILO) {
+                    x = lds64(field_addr<FB, s * FB>(kw[2 * i], lut_lane));
+                    y = lds64(field_addr<FB, s * FB>(kw[2 * i + 1], lut_lane));
+                } else {
+                    x = lds64(field_addr<FB, 2 * s * FB>(kw[i], lut_lane));
+                    y = lds64(field_addr<FB, (2 * s + 1) * FB>(kw[i], lut_lane));
+                }
+                const uint32_t a[4] = {x.x, x.y, y.x, y.y};
+                mma16816(c[i][0], a, b0, b1);
+                mma16816(c[i][1], a, l0, l1);
+            }
+        });
+#pragma unroll
+        for (int kg = 0; kg < KG; kg++)
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                sc[kg][h] = C::HILO ? c[kg % NC][0][h] + (c[kg % NC][0][2 + h] + c[kg % NC][1][h] + c[kg % NC][1][2 + h])
+                                    : c[kg / 2][0][2 * (kg % 2) + h] + c[kg / 2][1][2 * (kg % 2) + h];
+    }
 
-    // ---- online softmax: logits of keys 16 mt + g (row 0), + 8 (row 1) for heads 2t, 2t+1 ----
-    float sc[MT][2][2], tm[2] = {-INFINITY, -INFINITY};
+    // ---- online softmax ----
+    float tm[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-    for (int mt = 0; mt < MT; mt++) {
+    for (int kg = 0; kg < KG; kg++) {
+        const int key = 8 * kg + g;
+        const float kn = __shfl_sync(0xffffffffu, nk, key);
+        const bool valid = t0 + key < k_end;
 #pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const int key = 16 * mt + 8 * r + g;
-            const float kn = __shfl_sync(0xffffffffu, nk, key);
-            const bool valid = t0 + key < k_end;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                sc[mt][r][h] = valid ? (c[mt][0][2 * r + h] + c[mt][1][2 * r + h]) * kn : -INFINITY;
-                tm[h] = fmaxf(tm[h], sc[mt][r][h]);
-            }
+        for (int h = 0; h < 2; h++) {
+            sc[kg][h] = valid ? sc[kg][h] * kn : -INFINITY;
+            tm[h] = fmaxf(tm[h], sc[kg][h]);
         }
     }
     float resc[2];
+    // Where P has two parts the running maximum may lag by 8, so the accumulators are hardly ever rescaled: weights reach e^8, and norms
+    // above 21, which could take P past an f16, move it at once.
+    const float lag = C::HILO && !__any_sync(0xffffffffu, fabsf(nv) > 21.0f) ? 8.0f : 0.0f;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 4));
         tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 8));
         tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 16));
-        const float m_new = fmaxf(m_run[h], tm[h]);    // finite: key t0 is valid
+        const float m_new = C::HILO ? (tm[h] > m_run[h] + lag ? tm[h] : m_run[h]) : fmaxf(m_run[h], tm[h]);    // finite: key t0 is valid
         resc[h] = soft_exp<C::HILO>(m_run[h] - m_new);
         m_run[h] = m_new;
         l_part[h] *= resc[h];
@@ -321,7 +376,7 @@ __device__ __forceinline__ void attn_tile(AttnAcc<C> &st, uint32_t ka, uint32_t 
 #pragma unroll
         for (int r = 0; r < 2; r++) {
             const float vn = __shfl_sync(0xffffffffu, nv, (KT == 32 ? 16 * mt : 0) + 8 * r + g);
-            const float p0 = soft_exp<C::HILO>(sc[mt][r][0] - m_run[0]), p1 = soft_exp<C::HILO>(sc[mt][r][1] - m_run[1]);
+            const float p0 = soft_exp<C::HILO>(sc[2 * mt + r][0] - m_run[0]), p1 = soft_exp<C::HILO>(sc[2 * mt + r][1] - m_run[1]);
             l_part[0] += p0;
             l_part[1] += p1;
             if constexpr (!C::HILO) {
@@ -336,16 +391,16 @@ __device__ __forceinline__ void attn_tile(AttnAcc<C> &st, uint32_t ka, uint32_t 
     }
     if (__any_sync(0xffffffffu, resc[0] != 1.0f || resc[1] != 1.0f)) {   // the running max moved for some head
 #pragma unroll
-        for (int s = 0; s < NS; s++) {
+        for (int s = 0; s < NO; s++) {
             o[s][0] *= resc[0]; o[s][1] *= resc[1]; o[s][2] *= resc[0]; o[s][3] *= resc[1];
         }
     }
 
-    // ---- O^T[HD dims x 8 heads] += V^T . P.  MMA tile j has rows (g, g + 8) = dims (g HD/8 + 2j, + 1). ----
+    // ---- O^T[HD dims x 8 heads] += V^T . P (AttnAcc::result says which dims a tile's rows g, g + 8 are) ----
 #pragma unroll
     for (int mt = 0; mt < MT; mt++) {
         constexpr int VW = CB % 32 == 0 ? CB / 32 : 2;   // words of one key in this thread's eighth row
-        uint32_t vw[4][VW];
+        uint32_t vw[4][VW];   // keys 2t, 2t + 1, 2t + 8, 2t + 9
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const uint32_t row = va + (uint32_t)(16 * mt + 2 * t + (q & 1) + 8 * (q >> 1)) * C::VRS;
@@ -360,25 +415,35 @@ __device__ __forceinline__ void attn_tile(AttnAcc<C> &st, uint32_t ka, uint32_t 
                 vw[q][1] = w[1] >> sh;
             }
         }
-        auto pv_step = [&](auto U) {
-            constexpr int u = decltype(U)::value;
-            const uint2 e0 = lds64(field_addr<FB, u * FB>(vw[0], lut_lane)), e1 = lds64(field_addr<FB, u * FB>(vw[1], lut_lane));   // keys 2t, 2t+1
-            const uint2 e2 = lds64(field_addr<FB, u * FB>(vw[2], lut_lane)), e3 = lds64(field_addr<FB, u * FB>(vw[3], lut_lane));   // keys 2t+8, 2t+9
-            // .x: first two dims (tq2) / high parts; .y: next two dims / low parts
-            const uint32_t ax[4] = {__byte_perm(e0.x, e1.x, 0x5410), __byte_perm(e0.x, e1.x, 0x7632), __byte_perm(e2.x, e3.x, 0x5410),
-                                    __byte_perm(e2.x, e3.x, 0x7632)};
-            const uint32_t ay[4] = {__byte_perm(e0.y, e1.y, 0x5410), __byte_perm(e0.y, e1.y, 0x7632), __byte_perm(e2.y, e3.y, 0x5410),
-                                    __byte_perm(e2.y, e3.y, 0x7632)};
-            if constexpr (!C::HILO) {
-                mma16816(o[2 * u], ax, bp[mt][0], bp[mt][1]);
-                mma16816(o[2 * u + 1], ay, bp[mt][0], bp[mt][1]);
-            } else {
+        if constexpr (C::PAIRS) {
+            uint32_t pw[2][2][VW];   // [keys 2t .. | 2t + 8 ..][codes 0, 2, 4 .. | 1, 3, 5 ..]
+#pragma unroll
+            for (int q = 0; q < 2; q++) pair_rows<C::BITS>(vw[2 * q], vw[2 * q + 1], pw[q][0], pw[q][1]);
+            static_for<(C::HILO ? NS : NS / 2)>([&](auto U) {   // one dim (two parts) or dims d, d + 2 of either run of codes
+                constexpr int u = decltype(U)::value;
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const uint2 x = lds64(field_addr<FB, u * FB>(pw[0][e], lut_lane)), y = lds64(field_addr<FB, u * FB>(pw[1][e], lut_lane));
+                    const uint32_t a[4] = {x.x, x.y, y.x, y.y};
+                    mma16816(o[2 * u + e], a, bp[mt][0], bp[mt][1]);
+                    if constexpr (C::HILO) mma16816(o[2 * u + e], a, bpl[mt][0], bpl[mt][1]);
+                }
+            });
+        } else {
+            static_for<NS>([&](auto U) {
+                constexpr int u = decltype(U)::value;
+                const uint2 e0 = lds64(field_addr<FB, u * FB>(vw[0], lut_lane)), e1 = lds64(field_addr<FB, u * FB>(vw[1], lut_lane));   // keys 2t, 2t+1
+                const uint2 e2 = lds64(field_addr<FB, u * FB>(vw[2], lut_lane)), e3 = lds64(field_addr<FB, u * FB>(vw[3], lut_lane));   // keys 2t+8, 2t+9
+                // .x: high parts of two dims; .y: low parts
+                const uint32_t ax[4] = {__byte_perm(e0.x, e1.x, 0x5410), __byte_perm(e0.x, e1.x, 0x7632), __byte_perm(e2.x, e3.x, 0x5410),
+                                        __byte_perm(e2.x, e3.x, 0x7632)};
+                const uint32_t ay[4] = {__byte_perm(e0.y, e1.y, 0x5410), __byte_perm(e0.y, e1.y, 0x7632), __byte_perm(e2.y, e3.y, 0x5410),
+                                        __byte_perm(e2.y, e3.y, 0x7632)};
                 mma16816(o[u], ax, bp[mt][0], bp[mt][1]);
                 mma16816(o[u], ax, bpl[mt][0], bpl[mt][1]);
                 mma16816(o[u], ay, bp[mt][0], bp[mt][1]);
-            }
-        };
-        static_for<(C::HILO ? NS : NS / 2)>(pv_step);
+            });
+        }
     }
 }
 
