@@ -42,7 +42,6 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
     const uint32_t base_a = smem_u32(smem);
     uint2 *lut = reinterpret_cast<uint2 *>(smem);                       // [NENT][16 copies]
     float *rq_s = reinterpret_cast<float *>(smem + C::LUT_BYTES);       // [NS][32 lanes][4] rotated, scaled query
-    uint2 *ent_s = reinterpret_cast<uint2 *>(smem + C::LUT_BYTES + C::Q_BYTES);   // one table copy
     __shared__ uint32_t q_first[QUEUE ? LC_ATTN_QUEUE_LANES + 1 : 1];               // queue form: first item of each lane
     __shared__ uint32_t q_pos[QUEUE ? LC_ATTN_QUEUE_LANES : 1];                     // and its position
     __shared__ uint32_t q_ticket;
@@ -55,8 +54,9 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
     const uint32_t qh0 = kv_head * p.group + gchunk * G;
 
     // ---- before the dependency wait: everything that depends on the codec's levels only (a constant operand): gamma and
-    //      the table.  A CTA that becomes resident while its predecessor drains does this part for free. ----
-    const float gamma = attn_table<C>(p.levels, lut, ent_s, lane, warp);
+    //      the table.  A CTA that becomes resident while its predecessor drains does this part for free (and where there is no
+    //      predecessor, built while the first loads were on their way it took as long). ----
+    const float gamma = attn_table<C>(p.levels, lut, lane, warp);
     const uint32_t lut_lane = base_a + (uint32_t)(lane & (LUT_COPIES - 1)) * 8u;
 
     // Codes and norms of keys below the lanes' positions were written by earlier steps; only the key at the position
@@ -213,24 +213,24 @@ __global__ void __launch_bounds__(C::NT) tq_attn_mma_kernel(const TqAttnParams p
         }
     };
     bool more = next_item();
-    if (more) {
-        t_issue = k_begin + warp * KT;
-        // With early_kv the first tiles leave before the dependency wait, up to the tile that holds the key the
-        // predecessor is writing (position pos: the last key of the last split); that tile and the ones after it follow
-        // the wait.  Groups are committed in tile order either way.
-        int issued = 0;
-        if (early) {
+    t_issue = k_begin + warp * KT;
+    // With early_kv the first tiles leave before the dependency wait, up to the tile that holds the key the
+    // predecessor is writing (position pos: the last key of the last split); that tile and the ones after it follow
+    // the wait.  Groups are committed in tile order either way.
+    int issued = 0;
+    if (early) {
 #pragma unroll
-            for (int i = 0; i < C::DEPTH - 1; i++) {
-                if (issued == i && !(t_issue <= pos && pos < t_issue + KT)) {
-                    if (t_issue < k_end) issue(t_issue, i);
-                    cp_async_commit();
-                    t_issue += NW * KT;
-                    issued = i + 1;
-                }
+        for (int i = 0; i < C::DEPTH - 1; i++) {
+            if (issued == i && !(t_issue <= pos && pos < t_issue + KT)) {
+                if (t_issue < k_end) issue(t_issue, i);
+                cp_async_commit();
+                t_issue += NW * KT;
+                issued = i + 1;
             }
-            lc_pdl_wait();
         }
+        lc_pdl_wait();
+    }
+    if (more) {
         start_item(issued);
         load_query();
     }

@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(ST_NT + 32, 1) step_layers_kernel(const __grid
     auto here = [&](const uint4 &v) -> bool { return v.x != 0xffffffffu && !p.never; };
 
     // ---- once: table of levels, signs, rotations of every lane's position, embedding rows ----
-    const float gamma = attn_table<C, ST_NW>(p.levels, lut, reinterpret_cast<uint2 *>(work), lane, warp, [] { wide_sync(); });
+    const float gamma = attn_table<C, ST_NW>(p.levels, lut, lane, warp, [] { wide_sync(); });
     const uint2 *lut_lane = lut + (lane & (LUT_COPIES - 1));
     if (tid < HD) sg_s[tid] = p.signs[tid];
 #pragma unroll 1
@@ -821,7 +821,7 @@ int launch_step(lc_kernels *k, lc_batch *b, LcStepParams &p) {
     const int red = (ST_NW + na) * RED_PART * 4, rows_a = m * (H * 2 + 64), rows_b = m * (units_b * UNIT * 2 + 64);
     p.off_red = up(rows_a > rows_b ? rows_a : rows_b);
     int work = p.off_red + red;
-    for (int w : {STAGES * W::STAGE + W::SCRATCH + STAGES * 2 * W::KB * 4, (8 * PROW + ST_NT) * 4, C::ENT_BYTES}) work = w > work ? w : work;
+    for (int w : {STAGES * W::STAGE + W::SCRATCH + STAGES * 2 * W::KB * 4, (8 * PROW + ST_NT) * 4}) work = w > work ? w : work;
     const size_t smem = (size_t)at + up(work);
     if (smem + 3072 > k->ctx->smem_optin) return -1;
     size_t mail = 0;
