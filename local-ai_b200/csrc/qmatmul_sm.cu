@@ -5,7 +5,7 @@
 // Such a projection is a few megabytes that sit behind the kernel before it, so what counts is the chain after that kernel
 // has finished: read the activations, multiply, add up, store.  The chain here has no shared-memory staging of the
 // activations, no tensor memory and no exchange between CTAs:
-//   * a CTA owns 16 / 32 / 64 weight rows and all of K; its raw blocks come in by one bulk copy per row before the
+//   * a CTA owns 16 / 32 / 64 weight rows and all of K; its raw blocks come in by bulk copy (COPY_ROWS .. below) before the
 //     dependency wait, and the CTA is small enough that the next launch's CTAs become resident and fetch theirs meanwhile;
 //   * the twelve warps split K into 128-k steps: a warp reads its part of the activations straight into MMA fragments,
 //     16 bytes per lane, all of them in flight together; K is permuted so that a lane's weights come from the code bytes it
@@ -21,6 +21,7 @@
 
 #include "lc_internal.h"
 #include "qm_codes.cuh"
+#include "tensor_map.h"
 
 namespace {
 
@@ -28,6 +29,14 @@ constexpr int FMT_Q4_0 = 0, FMT_TQ2_0 = 1;
 constexpr int SM_NW = 12, SM_NT = SM_NW * 32, SM_UNIT = 128;   // warps (each a part of K), threads, k per step of a warp
 constexpr int SM_GROUPS = 3;
 constexpr uint32_t SM_WAIT_LIMIT = 1u << 22;
+// A bulk copy takes the copy engine some 70 cycles however short it is, and a CTA has up to 64 rows: rows below 2 KB come in together, as the
+// one range that they are, or, where rows an even number of 16-byte pieces long would start in the same banks, as a box of a tensor map
+// 16 bytes wider than the matrix.  (35 matrices in a graph: TQ2_0 8192 x 1536 at one row 109 -> 100 us, at 16 rows 154 -> 144; Q4_0 6144 x 1536 at
+// one row 115 -> 102, 4000 x 2048 at four 126 -> 116.)  Kernels of their own: decided at run time it cost CTAs of 16 rows 3 %.
+constexpr int COPY_ROWS = 0, COPY_RANGE = 1, COPY_BOX = 2;
+struct NoMap {};
+template <int COPY> struct SmMap { typedef NoMap type; };
+template <> struct SmMap<COPY_BOX> { typedef CUtensorMap type; };
 
 struct SmParams {
     const uint8_t *w[SM_GROUPS];
@@ -36,7 +45,7 @@ struct SmParams {
     int ngroups;
     const __half *x;
     int m, K, nb;          // nb = blocks per weight row
-    int raw_rs;            // bytes reserved per row of raw blocks
+    int raw_rs;            // bytes from row to row of raw blocks
     int *status;
     uint32_t wait_limit;
     uint32_t extra_arrivals;   // 0; 1 in the expiry self-test
@@ -70,17 +79,21 @@ __device__ __forceinline__ uint32_t lds16(uint32_t a) {
     return v;
 }
 
+__host__ __device__ __forceinline__ int raw_bytes(int rows, int rs) { return (rows * rs + 15) / 16 * 16; }
+
 // NT8: batch columns / 8.  MTW: 16-row tiles of the CTA (every warp works on all of them).  SINGLE: a warp has at most one
 // step, so a tile's sums go to shared memory at once and four tiles fit the registers of two CTAs per SM.
-template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT, bool ORDERED>
-__global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_kernel(const __grid_constant__ SmParams p) {
+template <int FMT, int NT8, int MTW, bool SINGLE, int COPY, bool GEGLU, typename OutT, bool ORDERED>
+__global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2)
+qgemm_sm_kernel(const __grid_constant__ SmParams p, const __grid_constant__ typename SmMap<COPY>::type w_map) {
     constexpr int BB = FMT == FMT_Q4_0 ? 18 : 66;
     constexpr int ROWS = MTW * 16, OROWS = GEGLU ? ROWS / 2 : ROWS;
     constexpr int RS = ROWS + 4;                // padded column of partial sums
     lc_order_begin<ORDERED>(p.order);
-    extern __shared__ __align__(16) uint8_t smem[];
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    uint8_t *smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
     uint8_t *raw = smem;                                                       // [ROWS][raw_rs]
-    float *red = reinterpret_cast<float *>(smem + ROWS * p.raw_rs);            // [SM_NW][NT8 * 8][RS]
+    float *red = reinterpret_cast<float *>(smem + raw_bytes(ROWS, p.raw_rs));  // [SM_NW][NT8 * 8][RS]
     __shared__ __align__(8) uint64_t raw_full;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     int grp = 0;
@@ -93,33 +106,54 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
     // ---- before the dependency wait: the raw blocks (constant operands) ----
     const uint32_t bar = smem_u32(&raw_full);
     if (tid == 0) {
-        mbar_init(bar, ROWS + p.extra_arrivals);
+        mbar_init(bar, (COPY == COPY_ROWS ? ROWS : 1) + p.extra_arrivals);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        if constexpr (COPY == COPY_BOX) {
+            mbar_arrive_expect_tx(bar, (uint32_t)(ROWS * p.raw_rs));
+            tma_load_2d(smem_u32(raw), &w_map, 0, n0, bar);
+        } else if constexpr (COPY == COPY_RANGE) {   // (a tile starts on a multiple of 8 rows of an even number of bytes)
+            const uint32_t want = (uint32_t)(min(OROWS, n_rows - n0) * (int)rb);
+            const size_t a0 = (size_t)n0 * rb;
+            uint32_t bytes = (want + 15u) & ~15u;
+            const bool past = a0 + bytes > w_bytes;   // the last bytes of the matrix: nothing is read past its end
+            if (past) {
+                bytes -= 16;
+                for (int h = 0; h < (GEGLU ? 2 : 1); h++)
+#pragma unroll 1
+                    for (uint32_t i = bytes; i < want; i++) raw[h * OROWS * (int)rb + i] = p.w[GEGLU ? h : grp][a0 + i];
+            }
+            mbar_arrive_expect_tx(bar, bytes * (GEGLU ? 2u : 1u));
+#pragma unroll
+            for (int h = 0; h < (GEGLU ? 2 : 1); h++)
+                if (bytes) bulk_g2s(smem_u32(raw) + (uint32_t)(h * OROWS * (int)rb), p.w[GEGLU ? h : grp] + a0, bytes, bar);
+        }
     }
     __syncthreads();
-    if (tid < ROWS) {
-        const int row = n0 + (GEGLU ? tid % OROWS : tid);
-        const uint8_t *wm = p.w[GEGLU ? tid / OROWS : grp];
-        if (row < n_rows) {
-            const size_t g0 = (size_t)row * rb, a0 = g0 & ~(size_t)15;
-            uint32_t bytes = (uint32_t)(((g0 + rb - a0) + 15) & ~(size_t)15);
-            uint8_t *dst = raw + tid * p.raw_rs;
-            if (a0 + bytes > w_bytes) {   // the last bytes of the matrix: nothing is read past its end
-                bytes -= 16;
+    if constexpr (COPY == COPY_ROWS) {
+        if (tid < ROWS) {
+            const int row = n0 + (GEGLU ? tid % OROWS : tid);
+            const uint8_t *wm = p.w[GEGLU ? tid / OROWS : grp];
+            if (row < n_rows) {
+                const size_t g0 = (size_t)row * rb, a0 = g0 & ~(size_t)15;
+                uint32_t bytes = (uint32_t)(((g0 + rb - a0) + 15) & ~(size_t)15);
+                uint8_t *dst = raw + tid * p.raw_rs;
+                if (a0 + bytes > w_bytes) {   // the last bytes of the matrix: nothing is read past its end
+                    bytes -= 16;
 #pragma unroll 1
-                for (uint32_t i = 0; i < 16; i++) dst[bytes + i] = (a0 + bytes + i < w_bytes) ? wm[a0 + bytes + i] : 0;
+                    for (uint32_t i = 0; i < 16; i++) dst[bytes + i] = (a0 + bytes + i < w_bytes) ? wm[a0 + bytes + i] : 0;
+                }
+                mbar_arrive_expect_tx(bar, bytes);
+                if (bytes) bulk_g2s(smem_u32(dst), wm + a0, bytes, bar);
+            } else {
+                mbar_arrive(bar);
             }
-            mbar_arrive_expect_tx(bar, bytes);
-            if (bytes) bulk_g2s(smem_u32(dst), wm + a0, bytes, bar);
-        } else {
-            mbar_arrive(bar);
         }
     }
     // this lane's operand rows: 16 mt + g and + 8
     auto row_at = [&](int mt, int h, bool &ok_) -> uint32_t {
         const int r = mt * 16 + h * 8 + g, row = n0 + (GEGLU ? r % OROWS : r);
         ok_ = row < n_rows;
-        return smem_u32(raw) + (uint32_t)(r * p.raw_rs) + (uint32_t)(((size_t)row * rb) & 15);
+        return smem_u32(raw) + (uint32_t)(r * p.raw_rs) + (COPY == COPY_ROWS ? (uint32_t)(((size_t)row * rb) & 15) : 0u);
     };
     const int units = (p.K + SM_UNIT - 1) / SM_UNIT;
     lc_order_wait<ORDERED>(p.order);
@@ -287,31 +321,43 @@ __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2) qgemm_sm_k
     lc_order_end<ORDERED>(p.order);
 }
 
-template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT, bool ORDERED>
-int launch_sm(lc_batch *b, bool serial, const SmParams &p, int tiles) {
-    auto kern = qgemm_sm_kernel<FMT, NT8, MTW, SINGLE, GEGLU, OutT, ORDERED>;
-    const size_t smem = (size_t)MTW * 16 * p.raw_rs + sizeof(float) * SM_NW * NT8 * 8 * (MTW * 16 + 4);
+template <int FMT, int NT8, int MTW, bool SINGLE, int COPY, bool GEGLU, typename OutT, bool ORDERED>
+int launch_sm(lc_batch *b, bool serial, const SmParams &p, const CUtensorMap &w_map, int tiles) {
+    auto kern = qgemm_sm_kernel<FMT, NT8, MTW, SINGLE, COPY, GEGLU, OutT, ORDERED>;
+    const size_t smem = 128 + raw_bytes(MTW * 16, p.raw_rs) + sizeof(float) * SM_NW * NT8 * 8 * (MTW * 16 + 4);
     static lc_smem_optin optin;
     LC_CUDA_TRY(lc_ensure_smem(kern, optin, b->ctx, smem));
-    LC_LAUNCH_CHECKED(lc_launch_as(serial, kern, dim3(tiles), dim3(SM_NT), smem, b, p));
+    if constexpr (COPY == COPY_BOX)
+        LC_LAUNCH_CHECKED(lc_launch_as(serial, kern, dim3(tiles), dim3(SM_NT), smem, b, p, w_map));
+    else
+        LC_LAUNCH_CHECKED(lc_launch_as(serial, kern, dim3(tiles), dim3(SM_NT), smem, b, p, NoMap()));
     b->dispatch_count++;
     return LC_OK;
 }
+// (rows of one step per warp are below 2 KB, and CTAs of 16 rows copy row by row)
+template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT, bool ORDERED>
+int launch_copy(lc_batch *b, bool serial, const SmParams &p, const CUtensorMap &w_map, int tiles, int copy) {
+    if constexpr (FMT == FMT_Q4_0)
+        if (copy == COPY_BOX) return launch_sm<FMT, NT8, MTW, SINGLE, COPY_BOX, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles);
+    if constexpr (!SINGLE)
+        if (copy == COPY_ROWS) return launch_sm<FMT, NT8, MTW, SINGLE, COPY_ROWS, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles);
+    return launch_sm<FMT, NT8, MTW, SINGLE, COPY_RANGE, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles);
+}
 template <int FMT, int NT8, bool GEGLU, typename OutT, bool ORDERED>
-int launch_rows(lc_batch *b, bool serial, const SmParams &p, int tiles, int rows) {
+int launch_rows(lc_batch *b, bool serial, const SmParams &p, const CUtensorMap &w_map, int tiles, int rows, int copy) {
     if (p.K <= SM_NW * SM_UNIT) {
-        if (rows == 64) return launch_sm<FMT, NT8, 4, true, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
-        if (rows == 32) return launch_sm<FMT, NT8, 2, true, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
-        return launch_sm<FMT, NT8, 1, true, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
+        if (rows == 64) return launch_copy<FMT, NT8, 4, true, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles, copy);
+        if (rows == 32) return launch_copy<FMT, NT8, 2, true, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles, copy);
+        return launch_sm<FMT, NT8, 1, true, COPY_ROWS, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles);
     }
-    if (rows == 32) return launch_sm<FMT, NT8, 2, false, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
-    return launch_sm<FMT, NT8, 1, false, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
+    if (rows == 32) return launch_copy<FMT, NT8, 2, false, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles, copy);
+    return launch_sm<FMT, NT8, 1, false, COPY_ROWS, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles);
 }
 template <int FMT, bool GEGLU, typename OutT>
-int launch_nt(lc_batch *b, bool serial, const SmParams &p, int tiles, int rows) {
+int launch_nt(lc_batch *b, bool serial, const SmParams &p, const CUtensorMap &w_map, int tiles, int rows, int copy) {
     if (p.order)
-        return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT, true>(b, serial, p, tiles, rows) : launch_rows<FMT, 2, GEGLU, OutT, true>(b, serial, p, tiles, rows);
-    return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT, false>(b, serial, p, tiles, rows) : launch_rows<FMT, 2, GEGLU, OutT, false>(b, serial, p, tiles, rows);
+        return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT, true>(b, serial, p, w_map, tiles, rows, copy) : launch_rows<FMT, 2, GEGLU, OutT, true>(b, serial, p, w_map, tiles, rows, copy);
+    return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT, false>(b, serial, p, w_map, tiles, rows, copy) : launch_rows<FMT, 2, GEGLU, OutT, false>(b, serial, p, w_map, tiles, rows, copy);
 }
 
 }  // namespace
@@ -334,7 +380,6 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     // a row's enclosing 16-byte range; an odd number of 32-byte pieces spreads the lanes' rows over the banks
     size_t rs = (rb + 15 + 15) / 16 * 16;
     rs += (32 + 64 - rs % 64) % 64;
-    p.raw_rs = (int)rs;
     uint64_t rows_all = 0;
     for (int g = 0; g < ng; g++) rows_all += ns[g];
     // Rows per CTA: the fewest CTAs that still give every SM one (a CTA reads all activations), but never so many rows that
@@ -348,6 +393,15 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     // Q4_0 with few steps per warp, 9 to 16 rows of activations and more than two waves of tiles: the register-direct kernel's
     // 64-row tiles read the activations half as often (11 x 1792 x 15996: 18.0 us here, 13.7 there, 16 x 2048 x 12000 15.0 and 12.9; at K = 3072 24 against 28).
     if (fmt == FMT_Q4_0 && !f32out && m > 8 && kk > SM_NW * SM_UNIT && kk <= 2560 && (rows_all + 31) / 32 > 2 * sms) return -1;
+    // (CTAs of 16 rows keep a copy per row: 1024 x 1024 Q4_0 at one row 1.62 us against 1.64 for a box, 1024 x 512 1.49 / 1.54 for a range.)
+    int copy = COPY_ROWS;
+    lc_encode_tiled_fn encode = nullptr;
+    if (rb < 2048 && rows >= 32) {
+        if (fmt != FMT_Q4_0 || rb % 32 != 0) copy = COPY_RANGE;
+        else if (ng == 1 && (encode = lc_encode_tiled()) != nullptr) copy = COPY_BOX;
+        if (copy != COPY_ROWS) rs = rb + (copy == COPY_BOX ? 16 : 0);
+    }
+    p.raw_rs = (int)rs;
     int tiles = 0;
     const int orows = geglu ? rows / 2 : rows;
     for (int g = 0; g < SM_GROUPS; g++) {
@@ -360,6 +414,17 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
         p.tile_end[g] = tiles;
     }
     if (tiles < 1) return -1;
+    CUtensorMap w_map = {};
+    if (copy == COPY_BOX) {
+        const cuuint64_t dims[2] = {rb / 8, ns[0]};
+        const cuuint64_t strides[1] = {rb};
+        const cuuint32_t box[2] = {(cuuint32_t)(rs / 8), (cuuint32_t)rows};
+        const cuuint32_t estr[2] = {1, 1};
+        const CUresult r = encode(&w_map, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<uint8_t *>(p.w[0]), dims, strides, box, estr,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return lc_fail(LC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+    }
     p.status = k->dev_status;
     p.wait_limit = k->test_wait_expiry ? 4096u : SM_WAIT_LIMIT;
     p.extra_arrivals = k->test_wait_expiry ? 1u : 0u;
@@ -377,9 +442,9 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     LcOrder order(b, input, (size_t)m * kk * 2, ng, weights, w_bytes, outputs, out_bytes, n_all * kk <= host_paced);
     p.order = order.flags;
     int st;
-    if (geglu) st = launch_nt<FMT_TQ2_0, true, __half>(b, order.serial, p, tiles, rows);
-    else if (fmt == FMT_Q4_0) st = f32out ? launch_nt<FMT_Q4_0, false, float>(b, order.serial, p, tiles, rows) : launch_nt<FMT_Q4_0, false, __half>(b, order.serial, p, tiles, rows);
-    else st = f32out ? launch_nt<FMT_TQ2_0, false, float>(b, order.serial, p, tiles, rows) : launch_nt<FMT_TQ2_0, false, __half>(b, order.serial, p, tiles, rows);
+    if (geglu) st = launch_nt<FMT_TQ2_0, true, __half>(b, order.serial, p, w_map, tiles, rows, copy);
+    else if (fmt == FMT_Q4_0) st = f32out ? launch_nt<FMT_Q4_0, false, float>(b, order.serial, p, w_map, tiles, rows, copy) : launch_nt<FMT_Q4_0, false, __half>(b, order.serial, p, w_map, tiles, rows, copy);
+    else st = f32out ? launch_nt<FMT_TQ2_0, false, float>(b, order.serial, p, w_map, tiles, rows, copy) : launch_nt<FMT_TQ2_0, false, __half>(b, order.serial, p, w_map, tiles, rows, copy);
     order.launched = st == LC_OK;
     return st;
 }

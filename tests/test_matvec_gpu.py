@@ -366,7 +366,8 @@ def test_matmul_nt_q4_0_wide_matrix(la, orc, ctx, kernels, m, k, n):
     rel_close(got, want32, TC_TOL_Q4, "wide q4_0 f16 out")
 
 
-@pytest.mark.parametrize("m,k,n", [(64, 1536, 6144), (33, 512, 200), (16, 256, 64), (64, 2048, 1000), (4, 512, 256), (70, 512, 256)])
+@pytest.mark.parametrize("m,k,n", [(64, 1536, 6144), (33, 512, 200), (16, 256, 64), (64, 2048, 1000), (4, 512, 256), (70, 512, 256), (3, 512, 3561),
+                                   (11, 2304, 1801)])
 def test_geglu_fused_equals_separate_launches(la, orc, ctx, kernels, m, k, n):
     """gelu_tanh(x Wg^T) * (x Wu^T): one launch for decode batches, the three separate dispatches otherwise; both
     must give what matmul, matmul, gelu_mul give (up to the f32 summation order of the K splits: gate and up are
@@ -424,6 +425,19 @@ def test_q4_0_streaming_columns(la, orc, ctx, kernels, m, k, n):
     assert b.dispatch_count() == 1
     b.commit_and_wait()
     rel_close(out.read(np.float32), orc.matmul_nt(orc.Q4_0, a, raw, m, k, n), 2e-4, "streaming q4_0")
+
+
+@pytest.mark.parametrize("fmt,m,k,n", [("tq2_0", 1, 256, 7105), ("tq2_0", 16, 768, 7137), ("tq2_0", 9, 2048, 3553), ("tq2_0", 3, 7936, 3555),
+                                       ("tq2_0", 12, 8192, 3553), ("q4_0", 1, 96, 7109), ("q4_0", 3, 512, 7111), ("q4_0", 16, 1536, 7103),
+                                       ("q4_0", 5, 2048, 3555), ("q4_0", 8, 3520, 3557), ("q4_0", 2, 3584, 3553), ("q4_0", 2, 4096, 3553)])
+def test_small_batch_rows_copied_together(la, orc, ctx, kernels, fmt, m, k, n):
+    """The small-batch kernel's CTAs of 32 and 64 rows: raw blocks as one range, as a box and row by row, a last tile that ends with the
+    matrix on and off a 16-byte boundary."""
+    raw = (la.synth.q4_0_weights if fmt == "q4_0" else la.synth.tq2_0_weights)(n, k, 19)
+    a = la.synth.normal_f16((m, k), 20)
+    got = run_matmul(la, ctx, kernels, f"matmul_nt_{fmt}_into", a, raw, m, k, n)
+    rel_close(got, orc.matmul_nt(orc.Q4_0 if fmt == "q4_0" else orc.TQ2_0, a, raw, m, k, n), TOL, f"small batch {fmt} m={m} k={k} n={n}")
+    device_status_ok(kernels)
 
 
 @pytest.mark.parametrize("m,k,n", [(1, 256, 19000), (8, 512, 20001), (2, 1536, 19100)])
