@@ -15,9 +15,8 @@
 //     and the MMA takes A from tensor memory and B, the activations, from shared memory.  All 512 columns are in use:
 //     four 64-column accumulators and two weight slots of 128 columns (256 k) each (127 registers x 416 threads
 //     keep this kernel at one CTA per SM, so no second CTA ever waits for tensor memory behind a cluster barrier);
-//   * before the dependency wait: TMEM allocation, barrier set-up, the raw quantized rows of the CTA's K range
-//     brought in by bulk copies (cp.async.bulk, one per row segment, completion counted on an mbarrier), and both
-//     weight slots dequantized -- none of it depends on the predecessor;
+//   * before the dependency wait: the raw quantized rows of the CTA's K range (whole rows as one bulk copy per matrix, parts of rows by
+//     cp.async), TMEM allocation, barrier set-up, and both weight slots dequantized -- none of it depends on the predecessor;
 //   * the pipeline runs in steps of 256 k (one TQ2_0 block per row), because every hand-over costs its thread a few
 //     hundred cycles whatever the amount of data behind it: a barrier test ~150, an MMA issue ~210, a commit ~90
 //     (measured), and the hand-overs of a step sit in series (slot released -> dequantize -> weights ready ->
@@ -83,7 +82,8 @@ struct TcdParams {
     int ngroups;
     int m, K, nb;        // nb = blocks per weight row
     int ks, bps;         // split-K: grid.z = cluster size = ks, bps = blocks per split
-    int raw_rs;          // bytes reserved per row of raw blocks (odd multiple of 16)
+    int raw_rs;          // bytes from row to row of raw blocks: an odd multiple of 16, or whole rows as they lie in the matrix (ks = 1)
+    int raw_bytes;       // reserved for them all
     int sa, sb;          // operand slots (one step each): weights in tensor memory (always SA) / activations in shared memory
     int geglu;           // 1: operand rows 0-63 are gate rows, 64-127 the same rows of the up matrix; out[0] = gelu(gate) * up
     int *status;
@@ -103,13 +103,12 @@ constexpr int NT = (NDQ + 1 + NISS) * 32;    // + activation loader warp + MMA i
 template <bool ORDERED>
 __global__ void __launch_bounds__(NT, 1)
 qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CUtensorMap x_map) {
-    constexpr int ROWS = TILE_ROWS;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // operand tiles start on 1024-byte boundaries
     const int SB = p.sb;
     uint8_t *b_s = smem;                                   // [SB][B_SLOT]; slot 0 is reused for the split-K exchange
-    uint8_t *raw = b_s + SB * B_SLOT;                      // [ROWS][raw_rs]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(raw + ROWS * p.raw_rs);
+    uint8_t *raw = b_s + SB * B_SLOT;                      // [TILE_ROWS][raw_rs]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(raw + p.raw_bytes);
     uint64_t *raw_full = bars;                             // 1
     uint64_t *a_full = bars + 1;                           // [MAX_STEPS] (SA used)
     uint64_t *b_full = a_full + MAX_STEPS;                 // [MAX_STEPS] (SB used)
@@ -140,6 +139,42 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
     auto wmat_of = [&](int r) -> const uint8_t * { return p.geglu ? p.w[r >> 6] : p.w[grp]; };
     auto wrow_of = [&](int r) -> int { return n0 + (p.geglu ? (r & 63) : r); };
 
+    // ---- raw rows, ahead of everything else: blocks [kbs, kbe) of each.  Whole rows (ks = 1) are one range per matrix and one bulk copy;
+    //      parts of rows come in by 16-byte cp.async, two threads a row, as the enclosing 16-byte range (rows are only 2-byte aligned).
+    //      (With a bulk copy per row after the barriers and tensor memory were ready, the step of 64 lanes at context 8192 took 1976 us, not 1913.) ----
+    const bool range = p.ks == 1;
+    if (range) {
+        if (tid == 0) {
+            mbar_init(smem_u32(raw_full), 1);
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+            const int parts = p.geglu ? 2 : 1;
+            const uint32_t want = (uint32_t)(max(0, min(rows_out, n_rows - n0)) * (int)rb);
+            const size_t a0 = (size_t)n0 * rb;   // (a multiple of 64 rows of an even number of bytes)
+            uint32_t bytes = (want + 15u) & ~15u;
+            if (a0 + bytes > w_bytes) {   // the last bytes of the matrix: nothing is read past its end
+                bytes -= 16;
+                for (int h = 0; h < parts; h++)
+#pragma unroll 1
+                    for (uint32_t i = bytes; i < want; i++) raw[h * rows_out * (int)rb + i] = p.w[p.geglu ? h : grp][a0 + i];
+            }
+            mbar_arrive_expect_tx(smem_u32(raw_full), bytes * (uint32_t)parts);
+            for (int h = 0; h < parts; h++)
+                if (bytes) bulk_g2s(smem_u32(raw) + (uint32_t)(h * rows_out * (int)rb), p.w[p.geglu ? h : grp] + a0, bytes, smem_u32(raw_full));
+        }
+    } else if (warp < NDQ) {
+        const int r = tid >> 1;
+        if (wrow_of(r) < n_rows && nblk > 0) {
+            const uint8_t *wm = wmat_of(r);
+            const size_t g0 = (size_t)wrow_of(r) * rb + (size_t)kbs * BB, end = g0 + (size_t)seg;
+            const uint32_t dst = smem_u32(raw) + (uint32_t)(r * p.raw_rs);
+            uint32_t off = (uint32_t)(tid & 1) * 16u;
+            for (size_t at = (g0 & ~(size_t)15) + off; at < end; at += 32, off += 32) {
+                const uint32_t n = w_bytes - at < 16 ? (uint32_t)(w_bytes - at) : 16u;   // nothing is read past the matrix
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst + off), "l"(wm + at), "r"(n) : "memory");
+            }
+        }
+    }
+
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
                      "r"((uint32_t)TMEM_COLS)
@@ -147,7 +182,6 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid == 0) {
-        mbar_init(smem_u32(raw_full), ROWS);
         for (int i = 0; i < MAX_STEPS; i++) mbar_init(smem_u32(&a_full[i]), NDQ + p.extra_arrivals);
         for (int i = 0; i < MAX_STEPS; i++) mbar_init(smem_u32(&b_full[i]), 1);
         for (int i = 0; i < NBAR; i++) mbar_init(smem_u32(&step_done[i]), NISS);
@@ -162,35 +196,20 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
 
     if (warp < NDQ) {
         // =========================== dequantizing warps ===========================
-        // ---- raw rows: thread r < ROWS brings in row r's blocks [kbs, kbe) as one bulk copy of the enclosing
-        //      16-byte range (rows are only 2-byte aligned) ----
-        if (tid < ROWS) {
-            const uint8_t *wm = wmat_of(tid);
-            const int row = wrow_of(tid);
-            const uint32_t bar = smem_u32(raw_full);
-            bool counted = false;
-            if (row < n_rows && nblk > 0) {
-                const size_t g0 = (size_t)row * rb + (size_t)kbs * BB, a0 = g0 & ~(size_t)15;
-                const uint32_t bytes = (uint32_t)(((g0 + seg - a0) + 15) & ~(size_t)15);
-                uint8_t *dst = raw + tid * p.raw_rs;
-                if (a0 + bytes <= w_bytes) {
-                    mbar_arrive_expect_tx(bar, bytes);
-                    bulk_g2s(smem_u32(dst), wm + a0, bytes, bar);
-                    counted = true;
-                } else {   // the last bytes of the matrix: plain loads, nothing is read past its end
-                    for (uint32_t i = 0; i < bytes; i++) dst[i] = (a0 + i < w_bytes) ? wm[a0 + i] : 0;
-                }
-            }
-            if (!counted) mbar_arrive(bar);
+        bool dead = false;
+        if (range) {
+            dead = !mbar_wait_warp(smem_u32(raw_full), 0u, p.wait_limit, abort_flag);
+        } else {
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+            asm volatile("bar.sync 1, %0;\n" ::"n"(NDQ * 32) : "memory");
         }
-        bool dead = !mbar_wait_warp(smem_u32(raw_full), 0u, p.wait_limit, abort_flag);
         // This thread's share of every step: operand row 32 (warp & 3) + lane and, of each 32-byte half h of the row's
         // block, the 16 code bytes 16 bq .. + 15 (bq = warp >> 2): 128 weights.
         const int r = 32 * (warp & 3) + lane, bq = warp >> 2;
         const int row = wrow_of(r);
         const bool rvalid = row < n_rows;
         const size_t g0 = (size_t)row * rb + (size_t)kbs * BB;
-        const uint8_t *rrow = raw + r * p.raw_rs + (int)(g0 & 15);
+        const uint8_t *rrow = raw + r * p.raw_rs + (range ? 0 : (int)(g0 & 15));
         // tensor-memory address of this warp's lane quarter, first column of the weight slots
         const uint32_t ta0 = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)A_BASE;
         for (int i = 0; i < total_steps && !dead; i++) {
@@ -201,8 +220,8 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
             const uint32_t p01 = (uint32_t)__half_as_ushort(__hneg(d));
             const uint32_t p23 = (uint32_t)__half_as_ushort(d) | ((uint32_t)__half_as_ushort(__hadd(d, d)) << 16);
             const uint32_t lut_lo = __byte_perm(p01, p23, 0x6420), lut_hi = __byte_perm(p01, p23, 0x7531);
-            // The first half block is converted before the wait for the slot (only the stores depend on the MMAs that
-            // read the slot SA steps ago); its stores then run beside the conversion of the second half.
+            // The step is converted before the wait for the slot: only the stores depend on the MMAs that read the slot SA steps ago.
+            uint32_t v[2][4][8];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 // 16 code bytes, 2-byte aligned: five aligned words, funnel-shifted into place
@@ -212,25 +231,28 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
                                         __funnelshift_r(w3, w4, sh)};
                 // element k = 128 h + 32 l + j of the block is bit pair l of code byte 32 h + j: for a given l this
                 // thread's bytes j = 16 bq .. + 15 are 16 consecutive k, i.e. the eight columns from (128 h + 32 l + 16 bq) / 2
-                uint32_t v[4][8];
 #pragma unroll
                 for (int l = 0; l < 4; l++) {
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        const uint32_t sel = ((cw[q] >> (2 * l)) & 0x03030303u) * 0x11u + 0x40404040u;
-                        v[l][2 * q] = __byte_perm(lut_lo, lut_hi, sel);
-                        v[l][2 * q + 1] = __byte_perm(lut_lo, lut_hi, sel >> 16);
+                        // (the upper two selectors by the multiply pipe too: shifts are the ALU's, which is the busy one)
+                        const uint32_t c = (cw[q] >> (2 * l)) & 0x03030303u;
+                        uint32_t sel_hi;
+                        asm("mad.hi.u32 %0, %1, 0x110000, 0x4040;\n" : "=r"(sel_hi) : "r"(c));
+                        v[h][l][2 * q] = __byte_perm(lut_lo, lut_hi, c * 0x11u + 0x40404040u);
+                        v[h][l][2 * q + 1] = __byte_perm(lut_lo, lut_hi, sel_hi);
                     }
                 }
-                if (h == 0 && i >= SA) {   // the MMAs that read this slot SA steps ago have completed
-                    const int u = i - SA;
-                    if (!mbar_wait_warp(smem_u32(&step_done[u % NBAR]), (uint32_t)((u / NBAR) & 1), p.wait_limit, abort_flag)) { dead = true; break; }
-                    tc_fence_after();
-                }
-#pragma unroll
-                for (int l = 0; l < 4; l++) tmem_st8(ta0 + (uint32_t)(s * A_COLS + 64 * h + 16 * l + 8 * bq), v[l]);
             }
-            if (dead) break;
+            if (i >= SA) {
+                const int u = i - SA;
+                if (!mbar_wait_warp(smem_u32(&step_done[u % NBAR]), (uint32_t)((u / NBAR) & 1), p.wait_limit, abort_flag)) { dead = true; break; }
+                tc_fence_after();
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int l = 0; l < 4; l++) tmem_st8(ta0 + (uint32_t)(s * A_COLS + 64 * h + 16 * l + 8 * bq), v[h][l]);
             asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
             tc_fence_before();
             __syncwarp();
@@ -504,13 +526,16 @@ int lc_qgemm_tcd_launch(lc_kernels *k, lc_batch *b, const lc_buf *input, int ng,
     p.bps = bps;
     p.raw_rs = ((bps * BB + 15 + 15) / 16) * 16;
     if ((p.raw_rs / 16) % 2 == 0) p.raw_rs += 16;
+    const int raw_bytes = rows * p.raw_rs;
+    if (ks == 1) p.raw_rs = p.nb * BB;
     p.status = k->dev_status;
     p.wait_limit = k->test_wait_expiry ? 4096u : WAIT_LIMIT;
     p.extra_arrivals = k->test_wait_expiry ? 1u : 0u;
     // Shared memory: the raw rows and up to three activation slots of one step each (the weight operand lives in
     // tensor memory); the first slot doubles as the staging of the split-K / GeGLU exchange (32 KB, exactly one slot).
     const int total = bps;
-    const size_t fixed = (size_t)rows * p.raw_rs + (1 + 2 * MAX_STEPS + NBAR) * 8 + 16 + 1024;   // + 1024: tile alignment slack
+    p.raw_bytes = raw_bytes;
+    const size_t fixed = (size_t)raw_bytes + (1 + 2 * MAX_STEPS + NBAR) * 8 + 16 + 1024;   // + 1024: tile alignment slack
     const size_t budget = k->ctx->smem_optin > 2048 ? k->ctx->smem_optin - 1024 : 0;
     static const int sb_cap = []() { const char *e = getenv("LOCAL_CUDA_TCD_SB"); const int v = e ? atoi(e) : 0; return v >= 1 && v <= MAX_STEPS ? v : 3; }();
     int sb = total < sb_cap ? total : sb_cap;

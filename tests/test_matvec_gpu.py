@@ -205,7 +205,8 @@ def device_status_ok(kernels):
 
 @pytest.mark.parametrize("m,k,n", [(70, 256, 96), (70, 512, 128), (16, 1536, 8192), (64, 1536, 8192), (64, 6144, 1536),
                                    (200, 512, 64), (9, 256, 1), (33, 2048, 1536), (17, 768, 130), (64, 1536, 2560),
-                                   (40, 1536, 12288), (64, 256, 31)])
+                                   (40, 1536, 12288), (64, 256, 31), (17, 512, 77), (64, 256, 129), (20, 1280, 131), (33, 2304, 1),
+                                   (50, 768, 255)])
 def test_matmul_nt_tq2_0_tensor_core(la, orc, ctx, tc_kernels, m, k, n):
     kernels = tc_kernels
     """kernels.rs:9551-9600 (m = 70 spans tiles) plus the benchmark shapes (config 2 at M = 16 and 64)."""
@@ -367,7 +368,7 @@ def test_matmul_nt_q4_0_wide_matrix(la, orc, ctx, kernels, m, k, n):
 
 
 @pytest.mark.parametrize("m,k,n", [(64, 1536, 6144), (33, 512, 200), (16, 256, 64), (64, 2048, 1000), (4, 512, 256), (70, 512, 256), (3, 512, 3561),
-                                   (11, 2304, 1801)])
+                                   (11, 2304, 1801), (40, 256, 201), (17, 1792, 67)])
 def test_geglu_fused_equals_separate_launches(la, orc, ctx, kernels, m, k, n):
     """gelu_tanh(x Wg^T) * (x Wu^T): one launch for decode batches, the three separate dispatches otherwise; both
     must give what matmul, matmul, gelu_mul give (up to the f32 summation order of the K splits: gate and up are
