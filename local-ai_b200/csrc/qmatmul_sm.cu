@@ -30,13 +30,10 @@ constexpr int SM_NW = 12, SM_NT = SM_NW * 32, SM_UNIT = 128;   // warps (each a 
 constexpr int SM_GROUPS = 3;
 constexpr uint32_t SM_WAIT_LIMIT = 1u << 22;
 // A bulk copy takes the copy engine some 70 cycles however short it is, and a CTA has up to 64 rows: rows below 2 KB come in together, as the
-// one range that they are, or, where rows an even number of 16-byte pieces long would start in the same banks, as a box of a tensor map
+// one range that they are, or, where rows a multiple of 64 bytes long would start in the same few banks, as a box of a tensor map
 // 16 bytes wider than the matrix.  (35 matrices in a graph: TQ2_0 8192 x 1536 at one row 109 -> 100 us, at 16 rows 154 -> 144; Q4_0 6144 x 1536 at
-// one row 115 -> 102, 4000 x 2048 at four 126 -> 116.)  Kernels of their own: decided at run time it cost CTAs of 16 rows 3 %.
+// one row 115 -> 102; enqueued one by one, 8192 x 1536 TQ2_0 at 16 rows 95.7 -> 90, 6000 x 2048 at eight 103 -> 92.)  Kernels of their own: decided at run time it cost CTAs of 16 rows 3 %.
 constexpr int COPY_ROWS = 0, COPY_RANGE = 1, COPY_BOX = 2;
-struct NoMap {};
-template <int COPY> struct SmMap { typedef NoMap type; };
-template <> struct SmMap<COPY_BOX> { typedef CUtensorMap type; };
 
 struct SmParams {
     const uint8_t *w[SM_GROUPS];
@@ -51,6 +48,12 @@ struct SmParams {
     uint32_t extra_arrivals;   // 0; 1 in the expiry self-test
     uint32_t order;            // LcOrder::flags
 };
+
+struct SmBoxParams : SmParams {
+    CUtensorMap w_map;
+};
+template <int COPY> struct SmArg { typedef SmParams type; };
+template <> struct SmArg<COPY_BOX> { typedef SmBoxParams type; };
 
 __device__ __forceinline__ void sm_store(__half *p, float v) { *p = __float2half_rn(v); }
 __device__ __forceinline__ void sm_store(float *p, float v) { *p = v; }
@@ -85,7 +88,7 @@ __host__ __device__ __forceinline__ int raw_bytes(int rows, int rs) { return (ro
 // step, so a tile's sums go to shared memory at once and four tiles fit the registers of two CTAs per SM.
 template <int FMT, int NT8, int MTW, bool SINGLE, int COPY, bool GEGLU, typename OutT, bool ORDERED>
 __global__ void __launch_bounds__(SM_NT, NT8 == 2 && !SINGLE ? 1 : 2)
-qgemm_sm_kernel(const __grid_constant__ SmParams p, const __grid_constant__ typename SmMap<COPY>::type w_map) {
+qgemm_sm_kernel(const __grid_constant__ typename SmArg<COPY>::type p) {
     constexpr int BB = FMT == FMT_Q4_0 ? 18 : 66;
     constexpr int ROWS = MTW * 16, OROWS = GEGLU ? ROWS / 2 : ROWS;
     constexpr int RS = ROWS + 4;                // padded column of partial sums
@@ -110,7 +113,7 @@ qgemm_sm_kernel(const __grid_constant__ SmParams p, const __grid_constant__ type
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         if constexpr (COPY == COPY_BOX) {
             mbar_arrive_expect_tx(bar, (uint32_t)(ROWS * p.raw_rs));
-            tma_load_2d(smem_u32(raw), &w_map, 0, n0, bar);
+            tma_load_2d(smem_u32(raw), &p.w_map, 0, n0, bar);
         } else if constexpr (COPY == COPY_RANGE) {   // (a tile starts on a multiple of 8 rows of an even number of bytes)
             const uint32_t want = (uint32_t)(min(OROWS, n_rows - n0) * (int)rb);
             const size_t a0 = (size_t)n0 * rb;
@@ -322,42 +325,39 @@ qgemm_sm_kernel(const __grid_constant__ SmParams p, const __grid_constant__ type
 }
 
 template <int FMT, int NT8, int MTW, bool SINGLE, int COPY, bool GEGLU, typename OutT, bool ORDERED>
-int launch_sm(lc_batch *b, bool serial, const SmParams &p, const CUtensorMap &w_map, int tiles) {
+int launch_sm(lc_batch *b, bool serial, const SmBoxParams &p, int tiles) {
     auto kern = qgemm_sm_kernel<FMT, NT8, MTW, SINGLE, COPY, GEGLU, OutT, ORDERED>;
     const size_t smem = 128 + raw_bytes(MTW * 16, p.raw_rs) + sizeof(float) * SM_NW * NT8 * 8 * (MTW * 16 + 4);
     static lc_smem_optin optin;
     LC_CUDA_TRY(lc_ensure_smem(kern, optin, b->ctx, smem));
-    if constexpr (COPY == COPY_BOX)
-        LC_LAUNCH_CHECKED(lc_launch_as(serial, kern, dim3(tiles), dim3(SM_NT), smem, b, p, w_map));
-    else
-        LC_LAUNCH_CHECKED(lc_launch_as(serial, kern, dim3(tiles), dim3(SM_NT), smem, b, p, NoMap()));
+    LC_LAUNCH_CHECKED(lc_launch_as(serial, kern, dim3(tiles), dim3(SM_NT), smem, b, static_cast<const typename SmArg<COPY>::type &>(p)));
     b->dispatch_count++;
     return LC_OK;
 }
-// (rows of one step per warp are below 2 KB, and CTAs of 16 rows copy row by row)
+// (rows of one step per warp are below 2 KB, TQ2_0's are one range then, and CTAs of 16 rows copy row by row)
 template <int FMT, int NT8, int MTW, bool SINGLE, bool GEGLU, typename OutT, bool ORDERED>
-int launch_copy(lc_batch *b, bool serial, const SmParams &p, const CUtensorMap &w_map, int tiles, int copy) {
+int launch_copy(lc_batch *b, bool serial, const SmBoxParams &p, int tiles, int copy) {
     if constexpr (FMT == FMT_Q4_0)
-        if (copy == COPY_BOX) return launch_sm<FMT, NT8, MTW, SINGLE, COPY_BOX, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles);
-    if constexpr (!SINGLE)
-        if (copy == COPY_ROWS) return launch_sm<FMT, NT8, MTW, SINGLE, COPY_ROWS, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles);
-    return launch_sm<FMT, NT8, MTW, SINGLE, COPY_RANGE, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles);
+        if (copy == COPY_BOX) return launch_sm<FMT, NT8, MTW, SINGLE, COPY_BOX, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
+    if constexpr (!SINGLE || FMT == FMT_Q4_0)
+        if (copy == COPY_ROWS) return launch_sm<FMT, NT8, MTW, SINGLE, COPY_ROWS, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
+    return launch_sm<FMT, NT8, MTW, SINGLE, COPY_RANGE, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
 }
 template <int FMT, int NT8, bool GEGLU, typename OutT, bool ORDERED>
-int launch_rows(lc_batch *b, bool serial, const SmParams &p, const CUtensorMap &w_map, int tiles, int rows, int copy) {
+int launch_rows(lc_batch *b, bool serial, const SmBoxParams &p, int tiles, int rows, int copy) {
     if (p.K <= SM_NW * SM_UNIT) {
-        if (rows == 64) return launch_copy<FMT, NT8, 4, true, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles, copy);
-        if (rows == 32) return launch_copy<FMT, NT8, 2, true, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles, copy);
-        return launch_sm<FMT, NT8, 1, true, COPY_ROWS, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles);
+        if (rows == 64) return launch_copy<FMT, NT8, 4, true, GEGLU, OutT, ORDERED>(b, serial, p, tiles, copy);
+        if (rows == 32) return launch_copy<FMT, NT8, 2, true, GEGLU, OutT, ORDERED>(b, serial, p, tiles, copy);
+        return launch_sm<FMT, NT8, 1, true, COPY_ROWS, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
     }
-    if (rows == 32) return launch_copy<FMT, NT8, 2, false, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles, copy);
-    return launch_sm<FMT, NT8, 1, false, COPY_ROWS, GEGLU, OutT, ORDERED>(b, serial, p, w_map, tiles);
+    if (rows == 32) return launch_copy<FMT, NT8, 2, false, GEGLU, OutT, ORDERED>(b, serial, p, tiles, copy);
+    return launch_sm<FMT, NT8, 1, false, COPY_ROWS, GEGLU, OutT, ORDERED>(b, serial, p, tiles);
 }
 template <int FMT, bool GEGLU, typename OutT>
-int launch_nt(lc_batch *b, bool serial, const SmParams &p, const CUtensorMap &w_map, int tiles, int rows, int copy) {
+int launch_nt(lc_batch *b, bool serial, const SmBoxParams &p, int tiles, int rows, int copy) {
     if (p.order)
-        return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT, true>(b, serial, p, w_map, tiles, rows, copy) : launch_rows<FMT, 2, GEGLU, OutT, true>(b, serial, p, w_map, tiles, rows, copy);
-    return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT, false>(b, serial, p, w_map, tiles, rows, copy) : launch_rows<FMT, 2, GEGLU, OutT, false>(b, serial, p, w_map, tiles, rows, copy);
+        return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT, true>(b, serial, p, tiles, rows, copy) : launch_rows<FMT, 2, GEGLU, OutT, true>(b, serial, p, tiles, rows, copy);
+    return p.m <= 8 ? launch_rows<FMT, 1, GEGLU, OutT, false>(b, serial, p, tiles, rows, copy) : launch_rows<FMT, 2, GEGLU, OutT, false>(b, serial, p, tiles, rows, copy);
 }
 
 }  // namespace
@@ -370,7 +370,7 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     if (m < 1 || m > 16 || ng < 1 || ng > SM_GROUPS || !lc_aligned(input->dptr, 16)) return -1;
     if (geglu && (ng != 2 || ns[0] != ns[1] || fmt != FMT_TQ2_0 || f32out)) return -1;
     if (fmt == FMT_Q4_0 && kk % 4 != 0) return -1;
-    SmParams p;
+    SmBoxParams p;
     p.x = (const __half *)input->dptr;
     p.m = (int)m;
     p.K = (int)kk;
@@ -393,12 +393,14 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     // Q4_0 with few steps per warp, 9 to 16 rows of activations and more than two waves of tiles: the register-direct kernel's
     // 64-row tiles read the activations half as often (11 x 1792 x 15996: 18.0 us here, 13.7 there, 16 x 2048 x 12000 15.0 and 12.9; at K = 3072 24 against 28).
     if (fmt == FMT_Q4_0 && !f32out && m > 8 && kk > SM_NW * SM_UNIT && kk <= 2560 && (rows_all + 31) / 32 > 2 * sms) return -1;
+    // A box costs the host 0.1 us a launch, which shows where launches side by side keep up with it (35 of 4000 x 2048 at three rows 93 us with a
+    // copy per row, 99 with boxes).
     // (CTAs of 16 rows keep a copy per row: 1024 x 1024 Q4_0 at one row 1.62 us against 1.64 for a box, 1024 x 512 1.49 / 1.54 for a range.)
     int copy = COPY_ROWS;
     lc_encode_tiled_fn encode = nullptr;
     if (rb < 2048 && rows >= 32) {
-        if (fmt != FMT_Q4_0 || rb % 32 != 0) copy = COPY_RANGE;
-        else if (ng == 1 && (encode = lc_encode_tiled()) != nullptr) copy = COPY_BOX;
+        if (fmt != FMT_Q4_0 || rb % 64 != 0) copy = COPY_RANGE;
+        else if (ng == 1 && rows_all * kk >= 1u << 24 && (encode = lc_encode_tiled()) != nullptr) copy = COPY_BOX;
         if (copy != COPY_ROWS) rs = rb + (copy == COPY_BOX ? 16 : 0);
     }
     p.raw_rs = (int)rs;
@@ -414,13 +416,12 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
         p.tile_end[g] = tiles;
     }
     if (tiles < 1) return -1;
-    CUtensorMap w_map = {};
     if (copy == COPY_BOX) {
         const cuuint64_t dims[2] = {rb / 8, ns[0]};
         const cuuint64_t strides[1] = {rb};
         const cuuint32_t box[2] = {(cuuint32_t)(rs / 8), (cuuint32_t)rows};
         const cuuint32_t estr[2] = {1, 1};
-        const CUresult r = encode(&w_map, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<uint8_t *>(p.w[0]), dims, strides, box, estr,
+        const CUresult r = encode(&p.w_map, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<uint8_t *>(p.w[0]), dims, strides, box, estr,
                                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return lc_fail(LC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
@@ -442,9 +443,9 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     LcOrder order(b, input, (size_t)m * kk * 2, ng, weights, w_bytes, outputs, out_bytes, n_all * kk <= host_paced);
     p.order = order.flags;
     int st;
-    if (geglu) st = launch_nt<FMT_TQ2_0, true, __half>(b, order.serial, p, w_map, tiles, rows, copy);
-    else if (fmt == FMT_Q4_0) st = f32out ? launch_nt<FMT_Q4_0, false, float>(b, order.serial, p, w_map, tiles, rows, copy) : launch_nt<FMT_Q4_0, false, __half>(b, order.serial, p, w_map, tiles, rows, copy);
-    else st = f32out ? launch_nt<FMT_TQ2_0, false, float>(b, order.serial, p, w_map, tiles, rows, copy) : launch_nt<FMT_TQ2_0, false, __half>(b, order.serial, p, w_map, tiles, rows, copy);
+    if (geglu) st = launch_nt<FMT_TQ2_0, true, __half>(b, order.serial, p, tiles, rows, copy);
+    else if (fmt == FMT_Q4_0) st = f32out ? launch_nt<FMT_Q4_0, false, float>(b, order.serial, p, tiles, rows, copy) : launch_nt<FMT_Q4_0, false, __half>(b, order.serial, p, tiles, rows, copy);
+    else st = f32out ? launch_nt<FMT_TQ2_0, false, float>(b, order.serial, p, tiles, rows, copy) : launch_nt<FMT_TQ2_0, false, __half>(b, order.serial, p, tiles, rows, copy);
     order.launched = st == LC_OK;
     return st;
 }

@@ -521,6 +521,9 @@ int lc_qgemv_mma_stream_group(int fmt, bool f32out, lc_kernels *k, lc_batch *b, 
                               const lc_buf *const *weights, lc_buf *const *outputs, uint32_t m, uint32_t kk, uint32_t n) {
     const int be = fmt == FMT_Q4_0 ? 32 : 256, bb = fmt == FMT_Q4_0 ? 18 : 66;
     if (count < 1 || count > MAX_MATRICES || m > 8 || kk % UNIT_K != 0 || kk % be != 0 || !lc_aligned(input->dptr, 16)) return -1;
+    // worth it only when every SM gets a few groups to stream
+    const int gpm = (int)((n + GROUP_ROWS - 1) / GROUP_ROWS);
+    if ((int64_t)gpm * count < 2 * k->ctx->sm_count) return -1;
     StreamParams p;
     for (int i = 0; i < MAX_MATRICES; i++) {
         const int j = i < count ? i : count - 1;
@@ -533,11 +536,9 @@ int lc_qgemv_mma_stream_group(int fmt, bool f32out, lc_kernels *k, lc_batch *b, 
     p.m = (int)m;
     p.K = (int)kk;
     p.nb = (int)(kk / be);
-    p.gpm = (int)((n + GROUP_ROWS - 1) / GROUP_ROWS);
+    p.gpm = gpm;
     p.status = k->dev_status;
     p.groups = p.gpm * count;
-    // worth it only when every SM gets a few groups to stream
-    if (p.groups < 2 * k->ctx->sm_count) return -1;
     if (fmt == FMT_Q4_0) return kk <= 16 * UNIT_K ? stream_q4_0(f32out, k, b, p) : -1;
     p.xs = (int)kk * 2 + 16;
     p.slot_bytes = (int)(((size_t)GROUP_ROWS * p.nb * bb + 15 + 15) / 16 * 16 + 16);

@@ -430,7 +430,7 @@ def test_q4_0_streaming_columns(la, orc, ctx, kernels, m, k, n):
 
 @pytest.mark.parametrize("fmt,m,k,n", [("tq2_0", 1, 256, 7105), ("tq2_0", 16, 768, 7137), ("tq2_0", 9, 2048, 3553), ("tq2_0", 3, 7936, 3555),
                                        ("tq2_0", 12, 8192, 3553), ("q4_0", 1, 96, 7109), ("q4_0", 3, 512, 7111), ("q4_0", 16, 1536, 7103),
-                                       ("q4_0", 5, 2048, 3555), ("q4_0", 8, 3520, 3557), ("q4_0", 2, 3584, 3553), ("q4_0", 2, 4096, 3553)])
+                                       ("q4_0", 5, 2048, 3555), ("q4_0", 5, 2048, 8195), ("q4_0", 11, 1024, 16385), ("q4_0", 8, 3520, 3557), ("q4_0", 2, 3584, 3553), ("q4_0", 2, 4096, 3553)])
 def test_small_batch_rows_copied_together(la, orc, ctx, kernels, fmt, m, k, n):
     """The small-batch kernel's CTAs of 32 and 64 rows: raw blocks as one range, as a box and row by row, a last tile that ends with the
     matrix on and off a 16-byte boundary."""
