@@ -183,9 +183,9 @@ class QuantMatvec:
 
     def kernel_name(self) -> str:
         if self.grouped:
-            return "qgemv_mma_stream_kernel (grouped)"
+            return f"qgemv_{self.fmt}_stream_kernel (grouped)"
         if self.m <= 8 and self.rows >= 18944:
-            return "qgemv_mma_stream_kernel"
+            return f"qgemv_{self.fmt}_stream_kernel"
         if self.m <= 16 and not (self.f32out and self.m > 8 and self.rows >= 18944):
             return "qgemm_sm_kernel"
         if self.f32out and 8 < self.m <= 64 and self.cols % 256 == 0 and self.rows >= 128 * 148:
