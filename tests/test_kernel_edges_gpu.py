@@ -214,6 +214,82 @@ def test_prefill_attention_keeps_large_value_norms_in_range(la, orc, ctx, kernel
     device_status_ok(kernels)
 
 
+# The same for the decode kernel, where the maximum may lag if P has two parts (all but tq2 at head_dim 256): one split per lane stored as it is,
+# splits merged in a cluster, splits and a merge launch, and work items.  A warp takes every eighth tile, so logits that step every 256 keys
+# (128 at head_dim 512) step along its tiles: by less than the lag, so that weights stay well above 1, past it, and down again.
+DECODE_FORMS = [   # head_dim, bits, form, lanes (0: a single one), rows of a lane, largest V norm
+    (128, 2, "one", 100, 1800, 1.0), (128, 3, "items", 80, 4200, 60000.0), (128, 4, "cluster", 60, 2000, 85.0), (128, 4, "merge", 60, 2000, 1000.0),
+    (256, 2, "items", 80, 4200, 60000.0), (256, 3, "cluster", 60, 2000, 60000.0), (256, 4, "items", 80, 4200, 121.0), (256, 4, "one", 100, 1800, 1000.0),
+    (256, 4, "merge", 0, 100000, 200.0), (512, 2, "merge", 60, 2000, 60000.0), (512, 3, "items", 50, 4200, 200.0), (512, 4, "cluster", 60, 2000, 60000.0)]
+
+
+@pytest.mark.parametrize("hd,bits,form,lanes,cap,vnorm", DECODE_FORMS)
+def test_decode_attention_keeps_large_value_norms_in_range(la, orc, ctx, kernels, hd, bits, form, lanes, cap, vnorm):
+    n_q, n = 8, max(lanes, 1)
+    levels, signs = la.tq_levels(hd, bits), la.tq_signs(hd, la.TQ_SEED)
+    cb = la.tq_code_bytes(hd, bits)
+    rng = np.random.default_rng(bits)
+    decode = lambda codes: levels[(np.unpackbits(codes.reshape(-1, cb), axis=1, bitorder="little").reshape(-1, hd, bits) * (1 << np.arange(bits))).sum(2)].astype(np.float64)
+    one = rng.integers(0, 256, cb, dtype=np.uint8)                      # every K row has one direction; its norms set the logits
+    k0 = decode(one)[0]
+    at = np.arange(cap)
+    step = np.array([0.5, 5.2, 0.8, 7.9, 1.4, 8.3, 6.0, 0.6])[at // (128 if hd == 512 else 256) % 8] + 6.0 * (at // 2048 % 2)
+    kn = np.tile((step + at % 7 / 20).astype(np.float16), n)
+    vn = np.tile(np.array([1.0, vnorm, 1.0, vnorm / 8, 1.0], np.float32)[at // 64 % 5].astype(np.float16), n)
+    kc, vc = np.tile(one, n * cap), rng.integers(0, 256, n * cap * cb, dtype=np.uint8)
+    positions = np.full(n, cap - 1, np.uint32)
+    if n > 1:
+        positions[1::2] = rng.integers(0, cap, positions[1::2].size)
+    rq = (np.linspace(0.75, 1.15, n * n_q)[rng.permutation(n * n_q)][:, None] * (k0 / (k0 @ k0))).astype(np.float32)   # logits 0.4 .. 16.9
+    q16 = orc.hadamard_rotate(rq.reshape(-1), signs, hd, n * n_q, False, True).astype(np.float16)
+    f = lambda a: la.CudaBuffer.from_slice(ctx, a)
+    bufs, pos, rows = (f(kc), f(kn), f(vc), f(vn), f(levels)), f(positions), n * n_q
+    shift = 8 if form == "merge" else 0   # (an output that 16-byte stores cannot reach keeps the first launch from merging)
+    outs = [la.CudaBuffer.from_slice(ctx, np.full(shift + rows * hd * e + 256, 0xA5, np.uint8)) for e in (4, 2)]
+    views = [la.CudaBuffer.wrap(ctx, o.device_ptr + shift, rows * hd * e) for o, e in zip(outs, (4, 2))]
+    launches = []
+    for fused in (False, True):
+        b = la.CommandBatch.new(ctx)
+        if lanes and fused:
+            kernels.tq_attention_batched_into(b, f(q16), *bufs, f(signs), views[1], pos, hd, cap, n_q, 1, 0, bits, n, 0, 1.0)
+        elif lanes:
+            kernels.flash_attention_tq_batched_into(b, f(rq), *bufs, views[0], pos, hd, cap, n_q, 1, 0, bits, n, 0, 1.0)
+        elif fused:
+            kernels.tq_attention_into(b, f(q16), *bufs, f(signs), views[1], hd, cap, cap - 1, n_q, 1, 0, bits, 0, 1.0)
+        else:
+            kernels.flash_attention_tq_into(b, f(rq), *bufs, views[0], hd, cap, cap - 1, n_q, 1, 0, bits, 0, 1.0)
+        launches.append(b.dispatch_count())
+        b.commit_and_wait()
+    assert launches == ([1, 1] if form in ("one", "cluster") else [2, 2])   # (of an aligned output, two are items and their merge)
+
+    def attend(x):   # in 64 bits
+        out = np.empty((n, n_q, hd))
+        for i, p in enumerate(positions):
+            rows_i = slice(i * cap, i * cap + int(p) + 1)
+            s = (x.astype(np.float64).reshape(n, n_q, hd)[i] @ k0)[:, None] * kn[rows_i].astype(np.float64)
+            w = np.exp(s - s.max(1, keepdims=True))
+            w /= w.sum(1, keepdims=True)
+            out[i] = (w * vn[rows_i].astype(np.float64)) @ decode(vc.reshape(-1, cb)[rows_i].copy())
+        return out.reshape(-1, hd)
+
+    # The weights sum to 1, and their errors count twice, in the sum and in its divisor.  tq2 at head_dim 256 rounds each P to f16: 2^-11 of it,
+    # and holds levels to 2^-18.  The others keep P, levels and query in two f16 parts, 2^-22 each, and a logit is a chain of head_dim / 16
+    # MMAs of up to 2^-23 of what is summed so far, half of the result in the mean: (head_dim / 16 + 4) 2^-24 of logits up to 17.  64 2^-24
+    # leaves room for f32 sums over a warp's tiles and for exponentials.  The inverse rotation keeps a row's 2-norm; its f16 result adds 2^-11.
+    most = np.abs(levels).max() * max(vnorm, 1.0)
+    tol = 2.0 * most * ((17.0 * (hd / 16 + 4) + 64.0) * 2.0 ** -24 + (2.0 ** -11 if bits == 2 and hd == 256 else 0.0))
+    raw = [o.as_slice(np.uint8) for o in outs]
+    assert all((r[:shift] == 0xA5).all() and (r[r.size - 256:] == 0xA5).all() for r in raw)
+    got, want = raw[0][shift:-256].view(np.float32).reshape(-1, hd), attend(rq)
+    assert np.isfinite(got).all() and np.abs(got - want).max() <= tol, np.abs(got - want).max() / tol
+    rotated = orc.hadamard_rotate(q16.astype(np.float32).reshape(-1), signs, hd, rows, True, False)
+    back = orc.hadamard_rotate(attend(rotated).astype(np.float32).reshape(-1), signs, hd, rows, False, True).reshape(-1, hd)
+    got = raw[1][shift:-256].view(np.float16).astype(np.float64).reshape(-1, hd)
+    off = np.linalg.norm(got - back, axis=1)
+    assert np.all(off <= tol * np.sqrt(hd) + 2.0 ** -11 * np.linalg.norm(back, axis=1)), off.max()
+    device_status_ok(kernels)
+
+
 # Q4_0 at 17 .. 64 rows goes to the kernel that is estimated to take less: shapes of both, their clusters and edges
 Q4_0_ROUTES = [(17, 1024, 8200), (24, 4096, 4600), (32, 1536, 4100), (20, 256, 19001), (29, 768, 20737), (33, 128, 75777), (64, 256, 75900),
                (45, 384, 19300), (32, 2048, 12300), (18, 160, 334)]
