@@ -481,3 +481,20 @@ def test_matvec_group_equals_single_launches(la, orc, ctx, kernels, fmt, rows, c
         if not streamed:
             assert np.array_equal(got.view(np.uint16), single.as_slice(np.uint16))
         rel_close(got, orc.matmul_nt(f, x, ws[i], 1, cols, rows).reshape(-1), 2e-3, f"group matvec {i}")
+
+
+@pytest.mark.parametrize("rows,cols,count", [(4101, 1024, 7), (2817, 896, 9), (4101, 1664, 7), (4109, 1920, 7), (4099, 2048, 7)])
+def test_streamed_q4_0_group_at_every_length_of_a_quarter(la, orc, ctx, kernels, rows, cols, count):
+    """Groups that the streaming kernel takes, with two and four units of 128 k to a warp's quarter (quarters that end early among them), rows of
+    a multiple of 512 k without the wider box, and last groups of 1 to 13 rows.  f32 sums against f64 (2e-4 of max(|want|, 1), as the single
+    launch) and an f16 result."""
+    ws = [la.synth.q4_0_weights(rows, cols, 80 + i) for i in range(count)]
+    x = la.synth.normal_f16((1, cols), 79)
+    outs = [Guarded(la, ctx, rows * 2) for _ in range(count)]
+    b = la.CommandBatch.new(ctx)
+    kernels.matvec_q4_0_group_into(b, [la.CudaBuffer.from_slice(ctx, w) for w in ws], count, la.CudaBuffer.from_slice(ctx, x), [o.view for o in outs], rows, cols)
+    assert b.dispatch_count() == 1
+    b.commit_and_wait()
+    for w, o in zip(ws, outs):
+        rel_close(o.read(np.float16), orc.matmul_nt(orc.Q4_0, x, w, 1, cols, rows).reshape(-1), 2e-4 + 2.0 ** -11, "streamed group")
+    device_status_ok(kernels)
