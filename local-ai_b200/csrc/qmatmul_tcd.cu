@@ -175,7 +175,7 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
         }
     }
 
-    if (warp == 0) {
+    if (warp == NDQ) {   // (whole, while the lanes of the raw rows' warps come from different code; that warp frees it, too)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
                      "r"((uint32_t)TMEM_COLS)
                      : "memory");
@@ -425,7 +425,7 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
     if (failed) tc_wait_expired(p.status, LC_DEV_STATUS_WAIT_EXPIRED_TCD, tid);
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) {
+    if (warp == NDQ) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS) : "memory");
     }
     lc_order_end<ORDERED>(p.order);
