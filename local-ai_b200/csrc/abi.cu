@@ -536,6 +536,7 @@ int lc_kernels_create(lc_ctx *ctx, lc_kernels **out) {
         if (v >= 0 && v <= 8) k->small_m = (uint32_t)v;
     }
     { const char *e = getenv("LOCAL_CUDA_TEST_WAIT_EXPIRY"); k->test_wait_expiry = e && strcmp(e, "1") == 0; }
+    { const char *e = getenv("LOCAL_CUDA_TEST_MAP_REFUSED"); k->test_map_refused = e && strcmp(e, "1") == 0; }
     const char *nm = getenv("LOCAL_CUDA_TQ_NORM");
     k->kv_norm_mode = (nm && strcmp(nm, "tree") == 0) ? 1 : 0;
     lc_cluster_capacity(ctx, k->cluster_cap);

@@ -91,6 +91,9 @@ struct lc_kernels {
     // prefill attention kernel use a short limit and wait for an arrival that never comes, so the expiry path (status word, early
     // exit, TMEM release) can be exercised on purpose.
     bool test_wait_expiry = false;
+    // LOCAL_CUDA_TEST_MAP_REFUSED=1 (read at creation): tensor maps over weights are as if the driver refused them, so that the copies
+    // that serve without one can be exercised.
+    bool test_map_refused = false;
 };
 
 // Values of the device-side status word (lc_kernels::dev_status).

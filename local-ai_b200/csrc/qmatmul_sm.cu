@@ -397,13 +397,10 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
     // copy per row, 99 with boxes).
     // (CTAs of 16 rows keep a copy per row: 1024 x 1024 Q4_0 at one row 1.62 us against 1.64 for a box, 1024 x 512 1.49 / 1.54 for a range.)
     int copy = COPY_ROWS;
-    lc_encode_tiled_fn encode = nullptr;
     if (rb < 2048 && rows >= 32) {
         if (fmt != FMT_Q4_0 || rb % 64 != 0) copy = COPY_RANGE;
-        else if (ng == 1 && rows_all * kk >= 1u << 24 && (encode = lc_encode_tiled()) != nullptr) copy = COPY_BOX;
-        if (copy != COPY_ROWS) rs = rb + (copy == COPY_BOX ? 16 : 0);
+        else if (ng == 1 && rows_all * kk >= 1u << 24) copy = COPY_BOX;
     }
-    p.raw_rs = (int)rs;
     int tiles = 0;
     const int orows = geglu ? rows / 2 : rows;
     for (int g = 0; g < SM_GROUPS; g++) {
@@ -416,16 +413,8 @@ int lc_qgemm_sm_launch(int fmt, bool f32out, lc_kernels *k, lc_batch *b, const l
         p.tile_end[g] = tiles;
     }
     if (tiles < 1) return -1;
-    if (copy == COPY_BOX) {
-        const cuuint64_t dims[2] = {rb / 8, ns[0]};
-        const cuuint64_t strides[1] = {rb};
-        const cuuint32_t box[2] = {(cuuint32_t)(rs / 8), (cuuint32_t)rows};
-        const cuuint32_t estr[2] = {1, 1};
-        const CUresult r = encode(&p.w_map, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<uint8_t *>(p.w[0]), dims, strides, box, estr,
-                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return lc_fail(LC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-    }
+    if (copy == COPY_BOX && !lc_wider_rows_map(&p.w_map, k->test_map_refused, p.w[0], rb, ns[0], (uint32_t)rows)) copy = COPY_ROWS;
+    p.raw_rs = (int)(copy == COPY_RANGE ? rb : copy == COPY_BOX ? rb + 16 : rs);
     p.status = k->dev_status;
     p.wait_limit = k->test_wait_expiry ? 4096u : SM_WAIT_LIMIT;
     p.extra_arrivals = k->test_wait_expiry ? 1u : 0u;

@@ -465,18 +465,7 @@ int stream_q4_0(bool f32out, lc_kernels *k, lc_batch *b, StreamParams &p) {
     const bool multi = p.groups > p.gpm;
     CUtensorMap w_map = {};
     p.pitch = (int)rb;
-    lc_encode_tiled_fn encode = lc_encode_tiled();
-    if (!multi && rb % 32 == 0 && encode) {
-        const cuuint64_t dims[2] = {rb / 8, (cuuint64_t)p.n};   // the box is wider: it ends each row with 16 bytes of zeros
-        const cuuint64_t strides[1] = {rb};
-        const cuuint32_t box[2] = {(rb + 16) / 8, GROUP_ROWS};
-        const cuuint32_t estr[2] = {1, 1};
-        const CUresult r = encode(&w_map, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<uint8_t *>(p.w[0]), dims, strides, box, estr,
-                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return lc_fail(LC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-        p.pitch = (int)rb + 16;
-    }
+    if (!multi && rb % 32 == 0 && lc_wider_rows_map(&w_map, k->test_map_refused, p.w[0], rb, (uint32_t)p.n, GROUP_ROWS)) p.pitch = (int)rb + 16;
     p.slot_bytes = (GROUP_ROWS * p.pitch + 16 + 127) / 128 * 128;
     const int nv = p.m <= 2 ? p.m : p.m <= 4 ? 4 : 8;
     auto bytes = [&](int slots) { return (size_t)128 + 4 * 256 * nv * sizeof(float) + (size_t)slots * p.slot_bytes; };

@@ -498,3 +498,19 @@ def test_streamed_q4_0_group_at_every_length_of_a_quarter(la, orc, ctx, kernels,
     for w, o in zip(ws, outs):
         rel_close(o.read(np.float16), orc.matmul_nt(orc.Q4_0, x, w, 1, cols, rows).reshape(-1), 2e-4 + 2.0 ** -11, "streamed group")
     device_status_ok(kernels)
+
+
+@pytest.mark.parametrize("m,k,n,f32", [(1, 512, 18945, True), (8, 2048, 18945, True), (2, 1536, 19001, False), (5, 2048, 8195, False), (16, 1024, 16391, False)])
+def test_a_refused_tensor_map_leaves_the_plain_copies(la, orc, ctx, monkeypatch, m, k, n, f32):
+    """Where the driver gives no map of the wider box, the streaming and the small-batch kernel bring their rows in without it: the same values
+    in the same order, so the same bits.  (LOCAL_CUDA_TEST_MAP_REFUSED=1 stands for the driver's refusal.)"""
+    raw, a = la.synth.q4_0_weights(n, k, 87), la.synth.normal_f16((m, k), 88)
+    entry, got = "matmul_nt_q4_0_f32out_into" if f32 else "matmul_nt_q4_0_into", []
+    for refused in ("0", "1"):
+        monkeypatch.setenv("LOCAL_CUDA_TEST_MAP_REFUSED", refused)
+        kk = la.Kernels.new(ctx)
+        got.append(run_matmul(la, ctx, kk, entry, a, raw, m, k, n, f32out=f32))
+        device_status_ok(kk)
+        kk.close()
+    rel_close(got[1], orc.matmul_nt(orc.Q4_0, a, raw, m, k, n), 2e-4 if f32 else TOL, "without the box")
+    assert np.array_equal(got[0], got[1])
