@@ -100,8 +100,8 @@ static int route(int fmt, bool f32out, const char *name, lc_kernels *k, lc_batch
     if (k->mma && m > 8) {
         if (m <= 64) {
             // Q4_0 from 17 rows: the large-batch kernel, or for a tall matrix at short K whichever kernel's estimate is less (large-batch
-            // against register-direct: 24 x 40000 x 512 16.2 us and 12.7; 24 x 24000 x 512 10.1 and 10.1; 48 x 40000 x 256 13.1 and 15.9;
-            // 48 x 71000 x 512 25.2 and 29.7; 64 x 262144 x 256 76 and 61).
+            // against register-direct: 24 x 40000 x 256 11.2 us and 9.0; 24 x 40000 x 512 14.2 and 13.6; 24 x 24000 x 512 9.3 and 10.8; 48 x 40000 x 256
+            // 11.9 and 16.5; 48 x 71000 x 512 21.1 and 30.4; 64 x 150000 x 256 35.3 and 32.3).
             // f32 outputs keep the other: its sums, 32 k at a time, are within 1e-7 of 64 bits, the tcgen05 accumulators' within 1e-6.  (An f16
             // output hides that: over 56 shapes 2.07e-4 off 64 bits from either, their ratio 1.00002 in the mean and 1.00025 at most.)
             const bool choose = k->decode_tc && fmt == 0 && m > SM_MAX_M && !f32out;

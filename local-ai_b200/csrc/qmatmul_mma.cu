@@ -592,7 +592,7 @@ static uint64_t narrow_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, ui
     const bool alone = 2 * (pl.smem + 1024) > 228 * 1024;   // one CTA fills an SM
     if (tiles > sms) {
         const uint64_t rounds = (tiles + sms - 1) / sms;
-        if (m <= 32) return rounds * (alone ? 2800 + 9 * K : 900 + 8 * K);
+        if (m <= 32) return alone ? rounds * (2800 + 9 * K) : 1500 + rounds * (600 + 8 * K);
         return rounds * (alone ? 3000 + 14 * K : 2600 + 9 * K);
     }
     return ~0ull - 1;   // fewer tiles than SMs: compared with nothing that could be slower

@@ -505,12 +505,15 @@ static TclPlan tcl_plan(int fmt, const lc_kernels *k, uint32_t m, uint32_t kk, i
 // What a launch over one Q4_0 matrix takes at 17 .. 64 rows, in ns, for the choice between this kernel and the register-direct one
 // (qmatmul_mma.cu) where there are more tiles than SMs; 0 with fewer, where this one is never the slower by more than 1 % (20 x 512 x 6144:
 // 5.45 us against 5.41; 24 x 16384 x 256 5.1 / 5.8; 24 x 4096 x 6144 15.4 / 17.4; eight of 24 x 1536 x 512 in one batch 25.8 / 37.7).
-// Fitted to n 24000 .. 262144, K 256 .. 1536: a wave costs its start and epilogue and about 720 a step.
+// A wave costs its start, 550 a unit of 128 k and 12 a batch column.  Fitted, with the other kernel's estimate, to both kernels' times over 1900 shapes
+// (n 19000 .. 262144, K 64 .. 1536, 17 .. 64 rows): the kernel that it picks takes 0.3 % longer than the faster one in the mean, more than 5 % at 2 % of
+// the shapes, 18 % at most (64 x 64 x 44000).  Among those that an older fit gave to the other kernel: 24 x 512 x 32000 13.0 us there, 10.2 here; 24 x 896 x
+// 44000 25.0 / 19.5; 24 x 768 x 262144 94.1 / 89.7.
 uint64_t lc_qgemm_tcl_estimate(const lc_kernels *k, uint32_t m, uint32_t kk, uint32_t n) {
     const uint64_t tiles = (n + ROWS - 1) / ROWS, sms = (uint64_t)k->ctx->sm_count;
     if (tiles <= sms) return 0;
     const TclPlan pl = tcl_plan(FMT_Q4_0, k, m, kk, (int)tiles);
-    return pl.waves * (3300 + 720 * (uint64_t)pl.ups);
+    return pl.waves * (2300 + 550 * (uint64_t)pl.ups + 12 * (uint64_t)pl.NB);
 }
 
 // Grouped launch: `ng` weight matrices [ns[g], kk] sharing the activations `input` [m, kk].  Returns LC_OK after a launch, a

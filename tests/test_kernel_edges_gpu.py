@@ -347,6 +347,38 @@ def test_q4_0_matmul_of_17_to_64_rows_is_not_the_slower_kernel(la, ctx, kernels,
     assert best[0] <= 1.1 * best[1], best
 
 
+@pytest.mark.parametrize("m,k,n", [(24, 512, 32000), (24, 896, 44000), (64, 192, 44000), (20, 768, 64000), (24, 384, 40000), (48, 256, 150000)])
+def test_q4_0_matmul_of_17_to_64_rows_is_the_faster_of_two_kernels(la, ctx, kernels, monkeypatch, m, k, n):
+    """The choice against either kernel alone (LOCAL_CUDA_DECODE_TC=0: register-direct, LOCAL_CUDA_DECODE_MMA=0: large-batch): at most 1.1 times the faster
+    one's time, at shapes where the other takes up to 1.33 times that."""
+    kerns = [kernels]
+    for off in ("LOCAL_CUDA_DECODE_TC", "LOCAL_CUDA_DECODE_MMA"):
+        monkeypatch.setenv(off, "0")
+        kerns.append(la.Kernels.new(ctx))
+        monkeypatch.delenv(off)
+    w, x, out = la.CudaBuffer.empty(ctx, n * k // 32 * 18), la.CudaBuffer.empty(ctx, m * k * 2), la.CudaBuffer.empty(ctx, m * n * 2)
+    w.zero(), x.zero()
+    graphs, best = [], [np.inf] * 3
+    for kern in kerns:
+        for begin in (la.CommandBatch.new, la.CommandBatch.capture):
+            b = begin(ctx)
+            for _ in range(20):
+                kern.matmul_nt_q4_0_into(b, x, w, out, m, k, n)
+            b.commit_and_wait() if begin == la.CommandBatch.new else graphs.append(b.end_capture())
+    for _ in range(8):
+        for i, g in enumerate(graphs):
+            ctx.synchronize()
+            t = time.perf_counter()
+            g.launch()
+            ctx.synchronize()
+            best[i] = min(best[i], time.perf_counter() - t)
+    for g in graphs:
+        g.destroy()
+    for kern in kerns[1:]:
+        kern.close()
+    assert best[0] <= 1.1 * min(best[1:]), best
+
+
 @pytest.mark.parametrize("bits,rows,start", [(2, 256, 768), (4, 150, 1900)])
 def test_prefill_attention_captured_without_an_eager_call_first(la, orc, ctx, bits, rows, start):
     """The prefill kernel's partials need scratch memory, which cannot grow while a graph is recorded: with none reserved the
