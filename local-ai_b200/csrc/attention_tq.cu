@@ -575,6 +575,26 @@ int launch_split_b(lc_batch *b, const TqAttnParams &p, dim3 grid, int g, unsigne
     }
 }
 
+// What the tensor-core kernels take, for the choice between their forms, in ns (keys: ps).  Fitted to graphs of calls on one B200, 8 heads on one kv head,
+// after the kernels' last change: decode kernel 1 .. 128 lanes x 256 .. 8192 keys at every split count, prefill kernel 8 .. 256 rows x 300 ..
+// 8192 keys at 1 .. 32 splits; both within 3 % in the mean.
+struct AttnTimes {
+    uint32_t start, wave, key;            // decode kernel: a launch, each further wave, a key of a CTA
+    uint32_t pf_start, pf_wave, pf_tile;  // prefill kernel: the same, a tile of keys
+};
+constexpr uint32_t ATTN_CLUSTER = 500;   // splits merged by the launch itself
+uint32_t attn_merge_ns(const lc_ctx *ctx, uint32_t rows, uint32_t splits, uint32_t hd) {   // splits merged by another launch
+    return cluster_merge_fits(ctx, rows, splits, hd) ? 2700 : 850 + 94 * splits;
+}
+AttnTimes attn_times(uint32_t hd, uint32_t bits) {
+    if (hd == 512) return {8800, 9200, bits == 2 ? 32400u : 35000u, 0, 0, 0};   // (the prefill kernel has no such heads)
+    if (hd == 256) {
+        if (bits == 2) return {7000, 7500, 7900, 14300, 9000, 1320};
+        return {7000, 7500, bits == 3 ? 16600u : 15300u, 13600, 7700, 1500};
+    }
+    return {5600, 5500, bits == 2 ? 8900u : bits == 3 ? 10800u : 9300u, 11200, 6300, 1490};
+}
+
 // Common host path.  `q_f16`/`out_f16` select the fused form.
 int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_or_q, bool fused,
                  const lc_buf *kc, const lc_buf *kn, const lc_buf *vc, const lc_buf *vn, const lc_buf *levels,
@@ -601,7 +621,7 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     if (fused) LC_REQUIRE(signs->bytes >= hd * 4u, "%s: signs buffer too small", name);
     // Rows a launch may touch: single form reads slots < min(kv_len, pos+1) (or < ring).
     size_t rows;
-    uint32_t len_max;
+    uint32_t len_max, seq_max = 0;   // the most keys a row attends; one cache: the keys in it
     if (positions) {
         LC_REQUIRE(positions->bytes >= (size_t)n_lanes * 4, "%s: positions buffer too small", name);
         LC_REQUIRE(ring <= lane_capacity, "%s: ring %u exceeds lane capacity %u", name, ring, lane_capacity);
@@ -610,6 +630,7 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     } else {
         const uint32_t last_pos = current_pos + (prefill ? n_rows - 1 : 0);   // the row that sees the most keys
         const uint32_t seq_len = kv_len < last_pos + 1 ? kv_len : last_pos + 1;
+        seq_max = seq_len;
         rows = ring ? (ring < seq_len ? ring : seq_len) : seq_len;
         const uint32_t ws = (window > 0 && last_pos + 1 > window) ? last_pos + 1 - window : 0;
         len_max = seq_len > ws ? seq_len - ws : 0;
@@ -650,23 +671,24 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     static const bool cluster_allowed = []() { const char *e = getenv("LOCAL_CUDA_ATTN_CLUSTER"); return !(e && e[0] == '0'); }();
     const bool clusters = use_mma && cluster_allowed && lc_aligned(out->dptr, 16) && (!fused || lc_aligned(signs->dptr, 16));
     uint64_t grid_cost = ~0ull;
-    const bool one_part = bits == 2 && hd == 256;   // levels and P in one f16 (attention_tq_mma.cu)
-    auto in_keys = [&](uint32_t tq2_keys) -> uint32_t { return tq2_keys * (one_part ? 8u : 5u) * 32u / hd; };
+    const AttnTimes t = attn_times(hd, bits);
+    auto keys_ns = [&](uint64_t keys) -> uint64_t { return keys * t.key / 1000u; };
     if (use_mma) {
-        // One CTA per SM (shared memory), so the launch runs in whole waves.  Pick the split count that minimises their
-        // time, in keys of tq2 at head_dim 256 (8.5 ns each; others take 8/5 of that per 256 dims): 700 for the launch, 1050 for
-        // every further wave, 640 for a merge launch.
+        // One CTA per SM (shared memory), so the launch runs in whole waves.  Pick the split count that minimises their time.
         // Short contexts split down to two 32-key tiles per CTA (two warps that have the table's banks to themselves finish a
         // tile sooner than eight), but into no more splits than one launch merges; long ones to half the warps.
         uint32_t max_s = len_max < 4096 ? len_max / 64u : len_max / 128u;
         if (len_max < 4096 && max_s > 8) max_s = 8;
         if (max_s < 1) max_s = 1;
         if (max_s > sms) max_s = sms;
+        // The lanes of a pool are as a rule shorter than its rows: splits save less there, and a merge costs the same (4 lanes of 16 heads over 7605 rows, full and
+        // ragged together: 8 splits in one launch 25.2 us, 18 and a merge 26.5).
+        auto merge_ns = [&](uint32_t s) -> uint32_t { return attn_merge_ns(b->ctx, (uint32_t)(qn / hd), s, hd) + (positions ? 2500u : 0u); };
         // Up to 8 splits are a cluster, and of those fewer fit at once (17 lanes x 512 keys: 8 splits 17.2 us, 6 splits 9.3).
         for (uint32_t s = 1; s <= max_s; s++) {
             const bool one_launch = s <= 8 && clusters;
             const uint64_t waves = one_launch ? (base + k->cluster_cap[s] - 1) / k->cluster_cap[s] : ((uint64_t)base * s + sms - 1) / sms;
-            const uint64_t cost = in_keys(700u) + waves * ((len_max + s - 1) / s) + (waves - 1) * in_keys(1050u) + (one_launch || s == 1 ? 0u : in_keys(640u));
+            const uint64_t cost = t.start + waves * keys_ns((len_max + s - 1) / s) + (waves - 1) * t.wave + (s == 1 ? 0u : one_launch ? ATTN_CLUSTER : merge_ns(s));
             if (cost < grid_cost) { grid_cost = cost; n_splits = s; }
         }
     }
@@ -677,22 +699,24 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     };
     // Queue form for pools of lanes that attend all of their keys.  Lanes differ in length, which the host cannot see, and
     // equal splits per lane leave most SMs waiting for the longest lane; so one persistent CTA per SM draws items of at
-    // most `chunk` keys.  An item after a CTA's first costs about 620 keys' worth more, and a merge launch follows.  The chunk minimises
-    // the sum of two estimates: every lane full, and lane lengths spread evenly up to the longest.  The splits above take
-    // their longest lane's time in both, in one launch, and stay unless the queue promises less: measured full / ragged,
-    // 32 lanes x 8192 tq2 keys 28.5 / 23.5 us against 36.8 / 22.1 for the queue, 64 lanes 46.6 / 44.3 against 57.4 / 33.3,
-    // 64 lanes of tq4 keys 74.5 / 72.3 against 85.7 / 48.3.
+    // most `chunk` keys; a merge launch follows.  The chunk minimises the sum of two estimates: every lane full, and lane lengths spread evenly up to
+    // the longest.  The splits above take their longest lane's time in both, in one launch, and stay unless the queue promises less: measured full / ragged,
+    // 32 lanes x 8192 tq2 keys 25.7 / 21.0 us against 34.7 / 21.8 for the queue, 64 lanes 40.1 / 38.3 against 50.7 / 29.4,
+    // 64 lanes of tq4 keys 70.9 / 68.4 against 80.4 / 44.0; over 76 pools the choice takes 0.7 % longer than the faster form
+    // and cut in the mean, 8 % at most.  (In a pool of few lanes the longest is often short, too, and the splits then gain as much: 17 lanes x 7600 tq4 keys at
+    // head_dim 128, two kv heads, 30.5 / 17.7 as splits, 35.9 / 20.7 as items; but 18 lanes x 7010 at head_dim 512 104.5 together, 95.9.)
     if (use_mma && positions && window == 0 && ring == 0 && n_lanes <= LC_ATTN_QUEUE_LANES && base * 16u >= sms && len_max > 2048) {
-        const uint32_t item = in_keys(620u), launch = in_keys(700u + 640u), lo_s = len_max > 32u * 2048u ? 32u : (len_max + 4095) / 4096;
-        uint64_t best_cost = ~0ull;
+        // an item after a CTA's first costs about three quarters of a launch's start more
+        const uint32_t lo_s = len_max > 32u * 2048u ? 32u : (len_max + 4095) / 4096, item = t.start * 3u / 4u, launches = t.start + 3500u + 6u * hd;
+        uint64_t best_cost = ~0ull / 128u;
         uint32_t best_chunk = 0;
         for (uint32_t s = lo_s; s <= 32; s++) {
             uint32_t per = ((len_max - 64u) / s + 255u) & ~255u;   // whole rounds of eight warps x 32 keys
             if (per < 256u) per = 256u;
-            const uint64_t rounds = ((uint64_t)base * s + sms - 1) / sms, full = rounds * per + (rounds - 1) * item;
-            const uint64_t mean = ((uint64_t)base * (len_max + item * (s + 1)) / 2) / sms;
-            const uint64_t cost = full + (mean > per ? mean : per) + 2u * launch;
-            if (cost < best_cost) { best_cost = cost; best_chunk = per + 64u; }   // (a few keys over do not make another item)
+            const uint64_t rounds = ((uint64_t)base * s + sms - 1) / sms, one = keys_ns(per), full = rounds * one + (rounds - 1) * item;
+            const uint64_t mean = base * (keys_ns(len_max) + (uint64_t)item * (s + 1)) / 2 / sms;
+            const uint64_t cost = full + (mean > one ? mean : one) + 2u * launches;
+            if (cost * 100u < best_cost * 99u) { best_cost = cost; best_chunk = per + 64u; }   // (a few keys over do not make another item; of near equals the fewer items)
         }
         const uint32_t most = best_chunk ? (len_max + best_chunk - 1) / best_chunk : 1u;
         if (best_cost < 2u * grid_cost && partials_fit(most, (size_t)n_kv * gchunks)) {
@@ -700,10 +724,11 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
             n_splits = most;
         }
     }
-    // Chunks of several rows: the prefill kernel shares each decoded key among 128 MMA rows, but takes 1900 keys' time (16 us)
-    // before and after its key tiles, of 240 (operands in one part; else 360) each.  Fewer than half a tile of rows, and chunks whose rows the decode
-    // kernel's CTAs finish sooner by the estimate above, stay there: 64 rows over 400 keys 9.7 us against 16.6, 256 over 330
-    // 20.0 against 19.5, 256 over 4096 87 against 38.
+    // Chunks of several rows: the prefill kernel shares each decoded key among 128 MMA rows, but takes longer before and after its key tiles and
+    // leaves a merge launch.  Fewer than half a tile of rows, and chunks whose rows the decode kernel's
+    // CTAs finish sooner, stay there (tq2): 64 rows over 400 keys 9.7 us against 15.9, 256 over 300 19.0 against 18.1, 256 over
+    // 4096 77 against 30; tq4 128 over 2000 39 against 26, at head_dim 128 64 over 8192 46 against 21.  Over 360 chunks the choice takes 0.7 % longer than
+    // the faster kernel at its best split in the mean, 19 % at most (16 tq3 rows over 8192 at head_dim 128: 22.0 against 18.5).
     uint32_t pf_heads = 1, pf_tiles = 0;
     if (prefill && use_mma && lc_tq_attn_prefill_supported(hd, bits)) {
         const uint32_t heads = group < 8 ? group : 8;
@@ -712,14 +737,27 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
         if (n_rows * 2 >= rows_per_tile) {
             pf_tiles = (n_rows + rows_per_tile - 1) / rows_per_tile;
             const uint32_t ctas = n_kv * gchunks * pf_tiles, tile = lc_tq_attn_prefill_tile_keys(hd, bits);
-            const uint32_t seen = len_max + (rows_per_tile < n_rows ? rows_per_tile : n_rows);   // keys of a tile of rows, at most
+            uint32_t seen = len_max + (rows_per_tile < n_rows ? rows_per_tile : n_rows);   // keys of a tile of rows, at most
+            if (seen > seq_max) seen = seq_max;
             const uint32_t key_tiles = (seen + tile - 1) / tile;
-            uint32_t splits = ctas < sms ? sms / ctas : 1;
-            if (splits > key_tiles) splits = key_tiles;
-            if (splits > MERGE_ROWS_MAX_SPLITS) splits = MERGE_ROWS_MAX_SPLITS;
-            const uint64_t waves = ((uint64_t)ctas * splits + sms - 1) / sms, steps = (key_tiles + splits - 1) / splits;
-            const uint64_t merge = (uint64_t)n_rows * n_q * splits * hd / 6400u;   // partials: 25 KB of them in a key's time
-            if (waves * (in_keys(1900u) + steps * in_keys(one_part ? 240u : 360u)) + in_keys((uint32_t)merge) < grid_cost && partials_fit(splits, 0))
+            uint32_t most = ctas < sms ? sms / ctas : 1;   // one wave
+            if (most > key_tiles) most = key_tiles;
+            if (most > MERGE_ROWS_MAX_SPLITS) most = MERGE_ROWS_MAX_SPLITS;
+            // The merge launch's blocks (MERGE_ROWS rows each) become resident ahead of their turn on the SMs that this launch leaves free, up to five on one, and
+            // read all their partials through those: some 90 bytes a ns and SM (64 rows of 8 heads over 4096 keys: 24 splits on 96 SMs 21.5 us, 32 on 128 26.0).
+            const uint32_t merge_blocks = (n_rows * n_q + MERGE_ROWS - 1) / MERGE_ROWS, split_bytes = hd * 4u;
+            const uint64_t waves = (ctas + sms - 1) / sms;
+            uint64_t best = ~0ull / 128u;
+            uint32_t splits = 1;
+            for (uint32_t sp = most; sp >= 1; sp--) {   // (of near equals the most splits: the first rows of a chunk see fewer keys)
+                const uint32_t free = (uint32_t)waves * sms - ctas * sp;
+                uint32_t crowd = 0;
+                if (free) crowd = merge_blocks > 5u * free ? 5u : (merge_blocks + free - 1) / free;
+                const uint64_t cost = t.pf_start + (waves - 1) * t.pf_wave + waves * ((key_tiles + sp - 1) / sp) * t.pf_tile +
+                                      (uint64_t)n_rows * n_q * sp * split_bytes * 11u / 100000u + crowd * MERGE_ROWS * 4u * sp * hd / 90u;
+                if (cost * 102u < best * 100u) { best = cost; splits = sp; }
+            }
+            if (best < grid_cost && partials_fit(splits, 0))
                 n_splits = splits;
             else
                 pf_tiles = 0;

@@ -379,6 +379,68 @@ def test_q4_0_matmul_of_17_to_64_rows_is_the_faster_of_two_kernels(la, ctx, kern
     assert best[0] <= 1.1 * min(best[1:]), best
 
 
+# Chunks that only the estimate of the kernels' times sends to the prefill kernel, and single lanes that it cuts into more splits than one launch merges
+@pytest.mark.parametrize("hd,n_q,n_kv,bits,rows,start,window", [
+    (128, 8, 1, 2, 64, 4000, 0), (256, 8, 1, 3, 24, 8100, 0), (256, 8, 1, 4, 100, 1900, 0), (128, 4, 1, 4, 40, 5000, 0), (128, 8, 2, 4, 130, 700, 300),
+    (256, 8, 1, 2, 1, 4200, 0), (128, 16, 1, 3, 1, 6677, 0), (512, 8, 1, 4, 1, 4100, 0)])
+def test_attention_of_two_launches(la, orc, ctx, kernels, hd, n_q, n_kv, bits, rows, start, window):
+    total = start + rows
+    c = Cache(la, orc, ctx, hd, n_kv, bits, total, seed=70 + total)
+    c.fill_single(total, 0)
+    kc, kn, vc, vn, lv, sg = c.device()
+    q = la.synth.normal_f16((rows, n_q, hd), 62)
+    rq = orc.hadamard_rotate(q.astype(np.float32), c.signs, hd, rows * n_q, True, False)
+    want = orc.flash_attention_tq_prefill(rq, c.kc, c.kn, c.vc, c.vn, c.levels, hd, total, start, rows, n_q, n_kv, window, bits, 0, 0.0625)
+    out, fused = Guarded(la, ctx, rows * n_q * hd * 4), Guarded(la, ctx, rows * n_q * hd * 2)
+    f = lambda x: la.CudaBuffer.from_slice(ctx, x)
+    b = la.CommandBatch.new(ctx)
+    if rows > 1:
+        kernels.flash_attention_tq_prefill_into(b, f(rq), kc, kn, vc, vn, lv, out.view, hd, total, start, rows, n_q, n_kv, window, bits, 0, 0.0625)
+        kernels.tq_attention_prefill_into(b, f(q), kc, kn, vc, vn, lv, sg, fused.view, hd, total, start, rows, n_q, n_kv, window, bits, 0, 0.0625)
+    else:
+        kernels.flash_attention_tq_into(b, f(rq), kc, kn, vc, vn, lv, out.view, hd, total, start, n_q, n_kv, window, bits, 0, 0.0625)
+        kernels.tq_attention_into(b, f(q), kc, kn, vc, vn, lv, sg, fused.view, hd, total, start, n_q, n_kv, window, bits, 0, 0.0625)
+    assert b.dispatch_count() == 4
+    b.commit_and_wait()
+    rel_close(out.read(np.float32), want, 1e-3, "two launches")
+    back = orc.hadamard_rotate(want, c.signs, hd, rows * n_q, False, True)
+    rel_close(fused.read(np.float16), back.astype(np.float16).astype(np.float32), 2e-3, "two launches, fused")
+    device_status_ok(kernels)
+
+
+@pytest.mark.parametrize("hd,bits,less,more", [(128, 2, (64, 8192), (128, 8192)), (256, 4, (128, 2000), (256, 2000)), (128, 4, (128, 2000), (256, 2000)),
+                                               (256, 3, (64, 4096), (128, 4096)), (128, 3, (1, 7000), (1, 16000)), (256, 4, (1, 6000), (1, 16000))])
+def test_attention_over_less_takes_no_longer(la, ctx, kernels, hd, bits, less, more):
+    """Fewer rows over the same keys, and fewer keys: at most 1.1 times as long, where a form chosen by a wrong estimate took up to 1.6 times."""
+    cb, (rows, total) = la.tq_code_bytes(hd, bits), more
+    zeros = lambda n: la.CudaBuffer.empty(ctx, n)
+    kc, kn, vc, vn = zeros(total * cb), zeros(total * 2), zeros(total * cb), zeros(total * 2)
+    lv, sg = la.CudaBuffer.from_slice(ctx, la.tq_levels(hd, bits)), la.CudaBuffer.from_slice(ctx, la.tq_signs(hd, la.TQ_SEED))
+    q, out = zeros(rows * 8 * hd * 2), zeros(rows * 8 * hd * 2)
+    graphs, best = [], [np.inf] * 2
+    for n, keys in (less, more):
+        def call(b):
+            if n > 1:
+                kernels.tq_attention_prefill_into(b, q, kc, kn, vc, vn, lv, sg, out, hd, keys, keys - n, n, 8, 1, 0, bits, 0, 0.0625)
+            else:
+                kernels.tq_attention_into(b, q, kc, kn, vc, vn, lv, sg, out, hd, keys, keys - 1, 8, 1, 0, bits, 0, 0.0625)
+        for begin in (la.CommandBatch.new, la.CommandBatch.capture):
+            b = begin(ctx)
+            for _ in range(20):
+                call(b)
+            b.commit_and_wait() if begin == la.CommandBatch.new else graphs.append(b.end_capture())
+    for _ in range(8):
+        for i, g in enumerate(graphs):
+            ctx.synchronize()
+            t = time.perf_counter()
+            g.launch()
+            ctx.synchronize()
+            best[i] = min(best[i], time.perf_counter() - t)
+    for g in graphs:
+        g.destroy()
+    assert best[0] <= 1.1 * best[1], best
+
+
 @pytest.mark.parametrize("bits,rows,start", [(2, 256, 768), (4, 150, 1900)])
 def test_prefill_attention_captured_without_an_eager_call_first(la, orc, ctx, bits, rows, start):
     """The prefill kernel's partials need scratch memory, which cannot grow while a graph is recorded: with none reserved the
