@@ -9,16 +9,17 @@
 //   * S^T[16 keys x 8 heads] = K[16 x HD] . RQ^T: the contraction index (dims) is free to permute, so thread (g, t) of a
 //     warp feeds the MMA with the HD / 4 dims held in its own quarter of the code bytes of keys g, g + 8;
 //   * O^T[HD dims x 8 heads] += V^T[HD x 16 keys] . P: the A operand wants (dim; two adjacent keys) per register, so
-//     thread (g, t) decodes its eighth of the code bytes of keys 2t, 2t + 1, 2t + 8, 2t + 9 and pairs the table entries of
-//     adjacent keys with byte permutes; P reaches the B operand through one movmatrix transpose per 8 keys.
+//     thread (g, t) takes its eighth of the code bytes of keys 2t, 2t + 1, 2t + 8, 2t + 9 and puts the codes of adjacent keys side by
+//     side before the lookup, whose two registers are then operand registers (attn_tile); at head_dim 512 the table entries of adjacent keys
+//     are paired by byte permutes.  P reaches the B operand through one movmatrix transpose per 8 keys.
 // A warp step is KT = 32 keys (16 at head_dim 512): two independent sets of accumulation chains, and the softmax, the
 // running-maximum shuffles and the refill arithmetic are paid once per 32 keys.  Codes stream through a per-warp
 // cp.async ring; consecutive lanes copy consecutive 16-byte pieces, so a tile of one kv-head is one contiguous read.
 //
-// What bounds it: instruction issue and fetch, not a pipe (ncu, tq2: 37 warp instructions per key against 55 with 16-key
-// steps and per-thread copies; ALU 38 %, tensor 27 %, shared memory 41 % busy; 12 or 16 warps with the query in shared memory
-// are no faster).  About 14 cycles per key and SM at tq2, 25 at tq4.  64 lanes x 8193 keys: 57 -> 47 us (tq2), 480 -> 79 us
-// (tq4, from the CUDA-core kernel); 64 ragged lanes up to 8192 keys at tq4: 259 -> 49 us.
+// What bounds it: instruction issue and fetch, not a pipe (ncu, tq2, 64 lanes x 8192 keys: 33 warp instructions per key, 0.46 issued per cycle and
+// scheduler; ALU 35 %, tensor 26 %, shared memory 47 % busy; 12 or 16 warps with the query in shared memory are no
+// faster).  At head_dim 256 a key takes an SM 15.5 cycles at tq2, 30 at tq4.  64 lanes x 8192 keys: 57 -> 47 -> 40 us (tq2), 480 (the CUDA-core kernel)
+// -> 85 -> 80 us (tq4); 64 ragged lanes up to 8192 keys at tq4: 259 -> 47 -> 44 us.
 //
 // Precision.  The query is split into an f16 and the f16 of the remainder (two MMAs), because logits reach |q||k| ~ head_dim
 // at softmax scale 1.  The table holds each level as an f16 and the f16 of its remainder, and so is P (three MMAs per contraction

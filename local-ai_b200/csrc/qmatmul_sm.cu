@@ -31,8 +31,9 @@ constexpr int SM_GROUPS = 3;
 constexpr uint32_t SM_WAIT_LIMIT = 1u << 22;
 // A bulk copy takes the copy engine some 70 cycles however short it is, and a CTA has up to 64 rows: rows below 2 KB come in together, as the
 // one range that they are, or, where rows a multiple of 64 bytes long would start in the same few banks, as a box of a tensor map
-// 16 bytes wider than the matrix.  (35 matrices in a graph: TQ2_0 8192 x 1536 at one row 109 -> 100 us, at 16 rows 154 -> 144; Q4_0 6144 x 1536 at
-// one row 115 -> 102; enqueued one by one, 8192 x 1536 TQ2_0 at 16 rows 95.7 -> 90, 6000 x 2048 at eight 103 -> 92.)  Kernels of their own: decided at run time it cost CTAs of 16 rows 3 %.
+// 16 bytes wider than the matrix.  (35 matrices in a graph, side by side, against a copy per row: TQ2_0 8192 x 1536 at one row 84.0 -> 65.6 us, at
+// 16 rows 101.0 -> 84.2; Q4_0 6144 x 1536 at one row 115 -> 102.  Enqueued call by call the host sets the pace, 2.6 to 3.1 us a call
+// from box to box, and 16 rows take 95 to 109 us either way.)  Kernels of their own: decided at run time it cost CTAs of 16 rows 3 %.
 constexpr int COPY_ROWS = 0, COPY_RANGE = 1, COPY_BOX = 2;
 
 struct SmParams {
