@@ -100,7 +100,10 @@ __device__ __forceinline__ uint2 pack4(float a, float b, float c, float d) {
 constexpr int NDQ = 8;                       // dequantizing warps (also the epilogue warps)
 constexpr int NT = (NDQ + 1 + NISS) * 32;    // + activation loader warp + MMA issuers
 
-template <bool ORDERED>
+// LANES: how many lanes bring in a row's part (ks > 1), 16 bytes each.  Two for the two or three blocks of a decode step's projections; eight, 128 bytes
+// at a time, for longer parts, which two lanes ask L2 for in 32-byte pieces (30 x 6912 x 5410, six blocks: 21.6 -> 20.6 us; with eight
+// for all the step of 64 lanes took 1919 us, not 1901, and with the choice at run time 1907 to 1910).
+template <bool ORDERED, int LANES>
 __global__ void __launch_bounds__(NT, 1)
 qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CUtensorMap x_map) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -140,7 +143,7 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
     auto wrow_of = [&](int r) -> int { return n0 + (p.geglu ? (r & 63) : r); };
 
     // ---- raw rows, ahead of everything else: blocks [kbs, kbe) of each.  Whole rows (ks = 1) are one range per matrix and one bulk copy;
-    //      parts of rows come in by 16-byte cp.async, two threads a row, as the enclosing 16-byte range (rows are only 2-byte aligned).
+    //      parts of rows come in by 16-byte cp.async, as the enclosing 16-byte range (rows are only 2-byte aligned).
     //      (With a bulk copy per row after the barriers and tensor memory were ready, the step of 64 lanes at context 8192 took 1976 us, not 1913.) ----
     const bool range = p.ks == 1;
     if (range) {
@@ -162,13 +165,15 @@ qgemm_tcd_kernel(const __grid_constant__ TcdParams p, const __grid_constant__ CU
                 if (bytes) bulk_g2s(smem_u32(raw) + (uint32_t)(h * rows_out * (int)rb), p.w[p.geglu ? h : grp] + a0, bytes, smem_u32(raw_full));
         }
     } else if (warp < NDQ) {
-        const int r = tid >> 1;
-        if (wrow_of(r) < n_rows && nblk > 0) {
+#pragma unroll
+        for (int r = tid / LANES; r < TILE_ROWS; r += NDQ * 32 / LANES) {
+            if (wrow_of(r) >= n_rows || nblk <= 0) continue;
             const uint8_t *wm = wmat_of(r);
             const size_t g0 = (size_t)wrow_of(r) * rb + (size_t)kbs * BB, end = g0 + (size_t)seg;
             const uint32_t dst = smem_u32(raw) + (uint32_t)(r * p.raw_rs);
-            uint32_t off = (uint32_t)(tid & 1) * 16u;
-            for (size_t at = (g0 & ~(size_t)15) + off; at < end; at += 32, off += 32) {
+            uint32_t off = (uint32_t)(tid % LANES) * 16u;
+#pragma unroll (LANES == 2 ? 4 : 1)
+            for (size_t at = (g0 & ~(size_t)15) + off; at < end; at += LANES * 16, off += LANES * 16) {
                 const uint32_t n = w_bytes - at < 16 ? (uint32_t)(w_bytes - at) : 16u;   // nothing is read past the matrix
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst + off), "l"(wm + at), "r"(n) : "memory");
             }
@@ -447,10 +452,10 @@ int make_x_map(CUtensorMap *map, const void *x, uint32_t m, uint32_t kk) {
     return LC_OK;
 }
 
-template <bool ORDERED>
+template <bool ORDERED, int LANES>
 int launch_tcd(lc_batch *b, bool serial, const TcdParams &p, const CUtensorMap &x_map, int tiles, size_t smem) {
     static lc_smem_optin optin;
-    LC_CUDA_TRY(lc_ensure_smem(qgemm_tcd_kernel<ORDERED>, optin, b->ctx, smem));
+    LC_CUDA_TRY(lc_ensure_smem(qgemm_tcd_kernel<ORDERED, LANES>, optin, b->ctx, smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles, 1, p.ks);
     cfg.blockDim = dim3(NT);
@@ -472,7 +477,7 @@ int launch_tcd(lc_batch *b, bool serial, const TcdParams &p, const CUtensorMap &
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    LC_LAUNCH_CHECKED(cudaLaunchKernelEx(&cfg, qgemm_tcd_kernel<ORDERED>, p, x_map));
+    LC_LAUNCH_CHECKED(cudaLaunchKernelEx(&cfg, qgemm_tcd_kernel<ORDERED, LANES>, p, x_map));
     b->dispatch_count++;
     return LC_OK;
 }
@@ -555,7 +560,8 @@ int lc_qgemm_tcd_launch(lc_kernels *k, lc_batch *b, const lc_buf *input, int ng,
     }
     LcOrder order(b, input, (size_t)m * kk * 2, ng, weights, w_bytes, outputs, out_bytes);
     p.order = order.flags;
-    st = p.order ? launch_tcd<true>(b, order.serial, p, x_map, tiles, smem) : launch_tcd<false>(b, order.serial, p, x_map, tiles, smem);
+    if (ks > 1 && bps > 3) st = p.order ? launch_tcd<true, 8>(b, order.serial, p, x_map, tiles, smem) : launch_tcd<false, 8>(b, order.serial, p, x_map, tiles, smem);
+    else st = p.order ? launch_tcd<true, 2>(b, order.serial, p, x_map, tiles, smem) : launch_tcd<false, 2>(b, order.serial, p, x_map, tiles, smem);
     order.launched = st == LC_OK;
     return st;
 }

@@ -514,3 +514,28 @@ def test_a_refused_tensor_map_leaves_the_plain_copies(la, orc, ctx, monkeypatch,
         kk.close()
     rel_close(got[1], orc.matmul_nt(orc.Q4_0, a, raw, m, k, n), 2e-4 if f32 else TOL, "without the box")
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("m,k,n", [(17, 4096, 4001), (64, 7936, 129), (30, 6912, 5410), (20, 2560, 13000)])
+@pytest.mark.parametrize("geglu", [False, True])
+def test_decode_matmul_over_long_parts_of_rows(la, orc, ctx, kernels, m, k, n, geglu):
+    """Splits of four to six blocks a row, whose raw bytes come in eight lanes a row: ragged last tiles (in a GeGLU tile the up rows follow
+    gate rows that do not exist), parts that start and end off a 16-byte boundary, the matrix's last bytes."""
+    raws = [la.synth.tq2_0_weights(n, k, 91 + i) for i in range(2)]
+    a = la.synth.normal_f16((m, k), 93)
+    if not geglu:
+        got = run_matmul(la, ctx, kernels, "matmul_nt_tq2_0_into", a, raws[0], m, k, n)
+        rel_close(got, orc.matmul_nt(orc.TQ2_0, a, raws[0], m, k, n), TC_TOL_TQ2, f"m={m} k={k} n={n}")
+        device_status_ok(kernels)
+        return
+    x, ws = la.CudaBuffer.from_slice(ctx, a), [la.CudaBuffer.from_slice(ctx, w) for w in raws]
+    t1, t2, out = la.CudaBuffer.empty(ctx, m * n * 2), la.CudaBuffer.empty(ctx, m * n * 2), Guarded(la, ctx, m * n * 2)
+    b = la.CommandBatch.new(ctx)
+    kernels.matmul_nt_tq2_0_geglu_into(b, x, ws[0], ws[1], t1, t2, out.view, m, k, n)
+    assert b.dispatch_count() == 1
+    b.commit_and_wait()
+    gate, up = (orc.matmul_nt(orc.TQ2_0, a, w, m, k, n).astype(np.float16).ravel() for w in raws)
+    # (gate and up each an f16 rounding off, which the product passes on, and its own result another: as above)
+    want = orc.gelu_mul(gate, up).astype(np.float32)
+    rel_close(out.read(np.float16), want, 4e-3, f"geglu m={m} k={k} n={n}")
+    device_status_ok(kernels)
