@@ -671,7 +671,11 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     static const bool cluster_allowed = []() { const char *e = getenv("LOCAL_CUDA_ATTN_CLUSTER"); return !(e && e[0] == '0'); }();
     const bool clusters = use_mma && cluster_allowed && lc_aligned(out->dptr, 16) && (!fused || lc_aligned(signs->dptr, 16));
     uint64_t grid_cost = ~0ull;
-    const AttnTimes t = attn_times(hd, bits);
+    // (Pools of tq2 rows at head_dim 256 are counted in keys of 8.5 ns, an older fit that chooses as well there: over 24 pools 0.5 % above the faster form in
+    // the mean, 0.6 with the times above.)
+    const bool counted = positions && bits == 2 && hd == 256;
+    const AttnTimes t = counted ? AttnTimes{700, 1050, 1000, 0, 0, 0} : attn_times(hd, bits);
+    const uint32_t cluster_cost = counted ? 0 : ATTN_CLUSTER;
     auto keys_ns = [&](uint64_t keys) -> uint64_t { return keys * t.key / 1000u; };
     if (use_mma) {
         // One CTA per SM (shared memory), so the launch runs in whole waves.  Pick the split count that minimises their time.
@@ -683,12 +687,12 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
         if (max_s > sms) max_s = sms;
         // The lanes of a pool are as a rule shorter than its rows: splits save less there, and a merge costs the same (4 lanes of 16 heads over 7605 rows, full and
         // ragged together: 8 splits in one launch 25.2 us, 18 and a merge 26.5).
-        auto merge_ns = [&](uint32_t s) -> uint32_t { return attn_merge_ns(b->ctx, (uint32_t)(qn / hd), s, hd) + (positions ? 2500u : 0u); };
+        auto merge_ns = [&](uint32_t s) -> uint32_t { return counted ? 640u : attn_merge_ns(b->ctx, (uint32_t)(qn / hd), s, hd) + (positions ? 2500u : 0u); };
         // Up to 8 splits are a cluster, and of those fewer fit at once (17 lanes x 512 keys: 8 splits 17.2 us, 6 splits 9.3).
         for (uint32_t s = 1; s <= max_s; s++) {
             const bool one_launch = s <= 8 && clusters;
             const uint64_t waves = one_launch ? (base + k->cluster_cap[s] - 1) / k->cluster_cap[s] : ((uint64_t)base * s + sms - 1) / sms;
-            const uint64_t cost = t.start + waves * keys_ns((len_max + s - 1) / s) + (waves - 1) * t.wave + (s == 1 ? 0u : one_launch ? ATTN_CLUSTER : merge_ns(s));
+            const uint64_t cost = t.start + waves * keys_ns((len_max + s - 1) / s) + (waves - 1) * t.wave + (s == 1 ? 0u : one_launch ? cluster_cost : merge_ns(s));
             if (cost < grid_cost) { grid_cost = cost; n_splits = s; }
         }
     }
@@ -707,7 +711,8 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
     // head_dim 128, two kv heads, 30.5 / 17.7 as splits, 35.9 / 20.7 as items; but 18 lanes x 7010 at head_dim 512 104.5 together, 95.9.)
     if (use_mma && positions && window == 0 && ring == 0 && n_lanes <= LC_ATTN_QUEUE_LANES && base * 16u >= sms && len_max > 2048) {
         // an item after a CTA's first costs about three quarters of a launch's start more
-        const uint32_t lo_s = len_max > 32u * 2048u ? 32u : (len_max + 4095) / 4096, item = t.start * 3u / 4u, launches = t.start + 3500u + 6u * hd;
+        const uint32_t lo_s = len_max > 32u * 2048u ? 32u : (len_max + 4095) / 4096, item = counted ? 620u : t.start * 3u / 4u,
+                       launches = counted ? 700u + 640u : t.start + 3500u + 6u * hd, enough = counted ? 100u : 99u;
         uint64_t best_cost = ~0ull / 128u;
         uint32_t best_chunk = 0;
         for (uint32_t s = lo_s; s <= 32; s++) {
@@ -716,7 +721,7 @@ int tq_attention(const char *name, lc_kernels *k, lc_batch *b, const lc_buf *rq_
             const uint64_t rounds = ((uint64_t)base * s + sms - 1) / sms, one = keys_ns(per), full = rounds * one + (rounds - 1) * item;
             const uint64_t mean = base * (keys_ns(len_max) + (uint64_t)item * (s + 1)) / 2 / sms;
             const uint64_t cost = full + (mean > one ? mean : one) + 2u * launches;
-            if (cost * 100u < best_cost * 99u) { best_cost = cost; best_chunk = per + 64u; }   // (a few keys over do not make another item; of near equals the fewer items)
+            if (cost * 100u < best_cost * enough) { best_cost = cost; best_chunk = per + 64u; }   // (a few keys over do not make another item; of near equals the fewer items)
         }
         const uint32_t most = best_chunk ? (len_max + best_chunk - 1) / best_chunk : 1u;
         if (best_cost < 2u * grid_cost && partials_fit(most, (size_t)n_kv * gchunks)) {
