@@ -471,10 +471,11 @@ int launch_tcl(lc_batch *b, bool serial, const TclParams &p, const CUtensorMap &
 
 }  // namespace
 
-// Batch rows per CTA and K splits of a launch of `tiles` 128-row tiles, the cheapest by an estimate in cycles fitted to all plans of 113
-// shapes (17 .. 512 rows, K 512 .. 8192, n 512 .. 16384, with and without an overlap of launches): the plan it picks takes 0.5 % longer
-// than the best one in the mean, 10 % at most.  352 x 1530 x 2048 TQ2_0 9.5 -> 7.9 us against a rule without a launch's true fixed part.
-// Clusters cannot use every SM, other launches can.
+// Batch rows per CTA and K splits of a launch of `tiles` 128-row tiles, the cheapest by an estimate in cycles.  Q4_0: fitted to all plans of 93
+// shapes (17 .. 512 rows, K 64 .. 8192, n 128 .. 16384), one call after the other and side by side, where plans of few CTAs win; a split costs by
+// its clusters and, in a launch of one wave, by how many CTAs they are.  The plan it picks takes 1.4 % longer than the best one in the mean, 13 % at most (3.5 and 31 % without
+// that term: 34 x 512 x 7872 6.9 us in 62 pairs, 5.4 in 62 CTAs; 291 x 512 x 1088 7.0 and 5.5).  TQ2_0 keeps the fit of its own 113 shapes, 2.0 % above the
+// best plan: other splits round differently, and in a decode step that flips KV codes.  Clusters cannot use every SM, other launches can.
 struct TclPlan {
     int m_tiles, NB, ks, ups, units;   // ks splits of ups units of two steps
     uint64_t waves;
@@ -487,8 +488,9 @@ static TclPlan tcl_plan(int fmt, const lc_kernels *k, uint32_t m, uint32_t kk, i
         const int nb = (((int)m + mt - 1) / mt + 15) / 16 * 16, real_mt = ((int)m + nb - 1) / nb;
         for (int ks = 1; ks <= MAX_KS && (ks == 1 || 2 * ks <= pl.units); ks++) {
             const uint64_t at_once = ks > 1 ? k->cluster_cap[ks] : (uint64_t)k->ctx->sm_count, waves = ((uint64_t)tiles * real_mt + at_once - 1) / at_once;
-            const uint64_t unit = 910u + (fmt == FMT_Q4_0 ? 4u : 7u) * (uint64_t)nb;
-            const uint64_t cost = waves * (6900u + (uint64_t)((pl.units + ks - 1) / ks) * unit + 9u * (uint64_t)nb + (ks > 1 ? 2000u + 100u * (uint64_t)ks : 0u));
+            const uint64_t unit = 910u + (fmt == FMT_Q4_0 ? 4u : 7u) * (uint64_t)nb, ctas = (uint64_t)tiles * real_mt;
+            const uint64_t split = ks == 1 ? 0u : fmt == FMT_Q4_0 && waves == 1 ? 800u + (400u + 25u * ctas) * (uint64_t)ks : 2000u + 100u * (uint64_t)ks;
+            const uint64_t cost = waves * (6900u + (uint64_t)((pl.units + ks - 1) / ks) * unit + 9u * (uint64_t)nb + split);
             if (cost < best) {
                 best = cost;
                 pl.m_tiles = real_mt;
